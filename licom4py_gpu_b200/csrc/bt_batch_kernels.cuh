@@ -54,7 +54,7 @@ __device__ __forceinline__ int member_of_warp(const int* off, int count, int ite
 // Stage pointers of member k at (substep, stage); the schedule of
 // barotr.py:41-87 as in the single-member round.
 template <typename T>
-__device__ StageIO<T> member_stage(const MemberDesc<T>& d, int rk, int step, int st) {
+__device__ StageIO<T> member_stage(const MemberDesc<T>& d, int n, int rk, int step, int st) {
   StageIO<T> io;
   const T* const* cur = step == 0 ? d.x0 : (const T* const*)d.x;
   const T* const* base = step == 0 ? d.b0 : (const T* const*)d.x;
@@ -71,6 +71,10 @@ __device__ StageIO<T> member_stage(const MemberDesc<T>& d, int rk, int step, int
   io.u_out = out[1];
   io.v_out = out[2];
   io.fx = d.fx;
+  const int sg = step * nst + st;  // the new-h bands alternate between consecutive stages
+  io.band_uv = d.band;
+  io.band_h = d.band + (3 + (sg & 1)) * band_plane(n);
+  io.band_hn = d.band + (4 - (sg & 1)) * band_plane(n);
   double dt;
   if (rk == 2) {
     dt = st == 0 ? d.dtb / 2.0 : d.dtb;
@@ -113,7 +117,7 @@ __device__ __forceinline__ void ctx_load(TileCtx<T>& ctx, const BatchArgs<T>& a,
       for (int w = threadIdx.x; w < (int)(sizeof(Geo<T>) / sizeof(int)); w += 32) gdst[w] = __ldg(gsrc + w);
       __syncwarp();
     }
-    if (threadIdx.x == 0) ctx.io = member_stage(ctx.d, a.rk, step, st);
+    if (threadIdx.x == 0) ctx.io = member_stage(ctx.d, ctx.g.n, a.rk, step, st);
   }
   __syncthreads();
   ctx.k = k;
@@ -234,16 +238,14 @@ __global__ void __launch_bounds__(kTileThreads, 2) k_batch_round(BatchArgs<T> a)
       ctx_load(ctx, a, k, step, st);
       const Geo<T>& g = ctx.g;
       const TileBox b = tile_box(make_tiling_dev(TI, TJ, g.n), g.n, tile - __ldg(a.off.tile + k));
-      EdgeCnt cnt;
-      int P;
       if (!uv) {
-        Gather<T, TI, TJ, false> gat;
-        tile_h_pro<T, TI, TJ>(g, ctx.io, b, sm, gat, cnt, P);
-        tile_h_main<T, TI, TJ>(g, ctx.io, b, sm, gat, cnt, P);
+        HPre<T, TI, TJ> pre;
+        tile_h_pro<T, TI, TJ>(g, ctx.io, b, sm, pre);
+        tile_h_main<T, TI, TJ>(g, ctx.io, b, sm, pre);
       } else {
-        Gather<T, TI, TJ, true> gat;
-        tile_uv_pro<T, TI, TJ>(g, ctx.io, b, sm, gat, cnt, P);
-        tile_uv_main<T, TI, TJ>(g, ctx.io, b, sm, gat, cnt, P);
+        UvPre<T, TI, TJ> pre;
+        tile_uv_pro<T, TI, TJ>(g, b, pre);
+        tile_uv_main<T, TI, TJ>(g, ctx.io, b, sm, pre);
       }
     }
     if (!grid_barrier(a.bar, gen, a.err, a.spin_limit)) {
@@ -266,7 +268,7 @@ namespace {
 template <typename T, int TI, int TJ, bool UV>
 size_t batch_tile_smem() {
   using S = TileShape<TI, TJ>;
-  return sizeof(T) * (UV ? S::kWordsUV : S::kWordsH) + sizeof(int) * kItemWords;
+  return sizeof(T) * (UV ? S::kWordsUV : S::kWordsH);
 }
 
 template <typename T, int TI, int TJ>

@@ -93,7 +93,8 @@ namespace {
 // interpolation weights (composition of communication.py:387-474 and
 // cube.py:40-127); route[f*4+side] packs the adjacency.
 template <typename T>
-int build_halo_host(int n, const T* coef, const int* li, const int* lj, int2* src, T* w, int* route) {
+int build_halo_host(int n, const T* coef, const int* li, const int* lj, int2* src, T* w, int* route,
+                    int* bsrc = nullptr) {
   const int m = n + 6, nh = halo_count(m);
   const size_t fe = (size_t)6 * m * m;
   for (int f = 0; f < 6; ++f)
@@ -147,6 +148,21 @@ int build_halo_host(int n, const T* coef, const int* li, const int* lj, int2* sr
         w[2 * k] = coef[2 * ob];
         w[2 * k + 1] = coef[2 * ob + 1];
       }
+  // the first sources of the band halo cells in band order (Geo::bsrc; locations checked above)
+  if (bsrc)
+    for (int f = 0; f < 6; ++f)
+      for (int dd = 0; dd < 4; ++dd) {
+        int nb, side, rev;
+        face_neighbor(f, dd, &nb, &side, &rev);
+        for (int c = 0; c < kHalo; ++c)
+          for (int k = 0; k < n; ++k) {
+            int ti, tj;
+            band_cell(dd, c, k, m, &ti, &tj);
+            const long o = cell(f, ti, tj, m);
+            const int pos = ((dd == kE || dd == kW) ? li[o] : lj[o]) - kHalo;
+            bsrc[((f * 4 + dd) * 3 + c) * n + k] = ((nb * 4 + side) * 3 + c) * n + (rev ? n - 1 - pos : pos);
+          }
+      }
   return BT_OK;
 }
 
@@ -172,21 +188,35 @@ int build_tables(bt_plan* p, const bt_grid_desc* d) {
       }
   std::vector<int2> src((size_t)6 * nh);
   std::vector<T> w((size_t)6 * nh * 2);
-  const int rc = build_halo_host<T>(p->n, coef.data(), li.data(), lj.data(), src.data(), w.data(), p->route);
+  std::vector<int> bsrc((size_t)72 * p->n);
+  const int rc =
+      build_halo_host<T>(p->n, coef.data(), li.data(), lj.data(), src.data(), w.data(), p->route, bsrc.data());
   if (rc != BT_OK) return rc;
   p->h_src = src;
-  BT_CUDA(cudaMalloc(&p->d_hsrc, src.size() * sizeof(int2)), "alloc halo table");
-  BT_CUDA(cudaMalloc(&p->d_hw, w.size() * sizeof(T)), "alloc halo weights");
-  BT_CUDA(cudaMemcpy(p->d_hsrc, src.data(), src.size() * sizeof(int2), cudaMemcpyHostToDevice), "upload table");
-  BT_CUDA(cudaMemcpy(p->d_hw, w.data(), w.size() * sizeof(T), cudaMemcpyHostToDevice), "upload weights");
+  // one block on the device: weights, sources, band sources (each part a multiple of 16 bytes: nh and n
+  // enter six- and 72-fold)
+  const size_t wb = w.size() * sizeof(T), sb = src.size() * sizeof(int2), bb = bsrc.size() * sizeof(int);
+  std::vector<unsigned char> blob(wb + sb + bb);
+  std::memcpy(blob.data(), w.data(), wb);
+  std::memcpy(blob.data() + wb, src.data(), sb);
+  std::memcpy(blob.data() + wb + sb, bsrc.data(), bb);
+  BT_CUDA(cudaMalloc(&p->d_hw, blob.size()), "alloc halo tables");
+  p->d_hsrc = (char*)p->d_hw + wb;
+  p->d_bsrc = (int*)((char*)p->d_hsrc + sb);
+  BT_CUDA(cudaMemcpy(p->d_hw, blob.data(), blob.size(), cudaMemcpyHostToDevice), "upload halo tables");
   return BT_OK;
 }
 
 template <typename T>
 StageIO<T> stage_io(const bt_plan* p, const T* h, const T* u, const T* v, const T* hp, const T* up, const T* vp,
-                    T* ho, T* uo, T* vo, double dt, double beta, int stored, int last) {
+                    T* ho, T* uo, T* vo, double dt, double beta, int stored, int last, int sg) {
   StageIO<T> io;
-  io.fx = (T*)p->face_x();
+  io.fx = (T*)p->terms();
+  T* const band = (T*)p->bands();
+  const size_t plane = (size_t)72 * p->n;
+  io.band_uv = band;  // the new-h bands alternate between consecutive stages
+  io.band_h = band + (3 + (sg & 1)) * plane;
+  io.band_hn = band + (4 - (sg & 1)) * plane;
   io.h = h;
   io.u = u;
   io.v = v;
@@ -233,20 +263,20 @@ cudaError_t enqueue_round(const bt_plan* p, const bt_state_in& in, const bt_stat
     if (rk == 2) {
       // barotr.py:50-56: dt/2 from the base, then dt from the same base
       e = run_stage<T>(p, g, stage_io<T>(p, cur[0], cur[1], cur[2], base[0], base[1], base[2], Y[0], Y[1], Y[2],
-                                         dtb / 2.0, 0.0, stored, 0), s);
+                                         dtb / 2.0, 0.0, stored, 0, 2 * step), s);
       if (e != cudaSuccess) return e;
       e = run_stage<T>(p, g, stage_io<T>(p, Y[0], Y[1], Y[2], base[0], base[1], base[2], X[0], X[1], X[2], dtb,
-                                         0.0, 0, 1), s);
+                                         0.0, 0, 1, 2 * step + 1), s);
     } else {
       // barotr.py:73-83: dt/3, dt/2, dt with beta_d = 1
       e = run_stage<T>(p, g, stage_io<T>(p, cur[0], cur[1], cur[2], base[0], base[1], base[2], Y[0], Y[1], Y[2],
-                                         dtb / 3.0, 1.0, stored, 0), s);
+                                         dtb / 3.0, 1.0, stored, 0, 3 * step), s);
       if (e != cudaSuccess) return e;
       e = run_stage<T>(p, g, stage_io<T>(p, Y[0], Y[1], Y[2], base[0], base[1], base[2], Z[0], Z[1], Z[2],
-                                         dtb / 2.0, 1.0, 0, 0), s);
+                                         dtb / 2.0, 1.0, 0, 0, 3 * step + 1), s);
       if (e != cudaSuccess) return e;
       e = run_stage<T>(p, g, stage_io<T>(p, Z[0], Z[1], Z[2], base[0], base[1], base[2], X[0], X[1], X[2], dtb,
-                                         1.0, 0, 1), s);
+                                         1.0, 0, 1, 3 * step + 2), s);
     }
     if (e != cudaSuccess) return e;
   }
@@ -269,7 +299,7 @@ cudaError_t enqueue_stage(const bt_plan* p, const bt_state_in& in, const bt_stat
   const Geo<T> g = p->geo<T>();
   T* X[3] = {(T*)out.h0, (T*)out.ub, (T*)out.vb};
   const StageIO<T> io = stage_io<T>(p, (const T*)in.h0, (const T*)in.ub, (const T*)in.vb, (const T*)in.h0p,
-                                    (const T*)in.ubp, (const T*)in.vbp, X[0], X[1], X[2], dt, beta, 1, last);
+                                    (const T*)in.ubp, (const T*)in.vbp, X[0], X[1], X[2], dt, beta, 1, last, 0);
   cudaError_t e = run_stage<T>(p, g, io, s);
   if (e != cudaSuccess) return e;
   if (out.diag[0]) {
@@ -347,7 +377,8 @@ RoundArgs<T> round_args(bt_plan* p, const bt_state_in& in, const bt_state_out& o
   a.x[0] = (T*)out.h0;
   a.x[1] = (T*)out.ub;
   a.x[2] = (T*)out.vb;
-  a.fx = (T*)p->face_x();
+  a.fx = (T*)p->terms();
+  a.band = (T*)p->bands();
   a.nbb = nbb;
   a.rk = rk;
   a.step0 = 0;
@@ -644,7 +675,6 @@ int bt_plan_destroy(bt_plan* p) {
   if (p->cap_stream) cudaStreamDestroy(p->cap_stream);
   if (p->scratch) cudaFree(p->scratch);
   if (p->d_flags) cudaFree(p->d_flags);
-  if (p->d_hsrc) cudaFree(p->d_hsrc);
   if (p->d_hw) cudaFree(p->d_hw);
   if (p->d_res) cudaFree(p->d_res);
   for (bt_plan::ConstBlocks& c : p->cblks)

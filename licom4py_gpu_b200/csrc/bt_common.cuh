@@ -71,11 +71,12 @@ struct Geo {
   const T* d_dx;
   const int2* hsrc; // (6, nh) source offsets (absolute within the member)
   const T* hw;      // (6, nh, 2) interpolation weights
+  const int* bsrc;  // (24, 3, n) first source of each band halo cell as a number in band order
+                    // (bt_stencil.cuh, band_no); the second is the next one along the edge
   // Tile constant blocks for tiles of cblk_ti x cblk_tj cells (TileShape::cW words
-  // per tile): the image of phase UV's shared-memory constant area
-  // (TileShape::uG .. uCEnd), then the depths of the tile's x and y faces; phase
-  // H of full interior tiles assembles its constants from its own block and its
-  // four neighbours'.  nullptr, or another tile shape: the arrays above are read.
+  // per tile: phase H's cell and face constants of the tile); phase H of full
+  // interior tiles assembles its constants from its own block and its four
+  // neighbours'.  nullptr, or another tile shape: the arrays above are read.
   const T* cblk;
   int cblk_ti, cblk_tj;
   int route[24];    // f*4 + side
@@ -93,9 +94,12 @@ struct StageIO {
   T* h_out;     // stage outputs (interior cells only)
   T* u_out;
   T* v_out;
-  T* fx;        // face cache, one block per tile (bt_stencil.cuh, TileShape::fW): for every x face
-                // and y face of the tile its averaged normal velocity, viscous correction and
-                // celerity flux, written by phase H, read by phase UV of the same tile
+  T* fx;        // momentum terms, one block per tile (bt_stencil.cuh, kTerms planes): written by phase
+                // H, read by phase UV of the same tile
+  T* band_uv;   // bands of the stage input's velocity, three planes: lon/lat components and the
+                // contravariant component normal to the band's side (read by phase H, rewritten by phase UV)
+  const T* band_h;  // bands of the stage input's h
+  T* band_hn;       // bands of the new h
   T dt;
   T beta;
   int stored_halo;  // 1: the inputs' halo cells hold valid values (first stage of a round)
@@ -137,7 +141,8 @@ struct RoundArgs {
   T* x[3];         // output / running state
   T* y[3];         // stage scratch
   T* z[3];         // second stage scratch (RK3)
-  T* fx;           // face cache blocks (phase H -> phase UV)
+  T* fx;           // momentum-term blocks (phase H -> phase UV)
+  T* band;         // bands (bt_stencil.cuh): velocity (3 planes), h (2 planes used in turn)
   int nbb, rk;      // substeps of this launch, RK order
   int step0;        // substep index of the launch's first substep within the round (0: reads x0/b0)
   double dtb;

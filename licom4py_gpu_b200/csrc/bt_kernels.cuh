@@ -21,13 +21,13 @@
 
 namespace bt {
 
-constexpr int kThreads = kTileThreads;
+constexpr int kThreads = 256;  // of the element-wise kernels
 
 
 // FP: the full-interior-tile path compiled in (multi-wave launches), else
 // every tile runs the edge path (one-wave launches: half the code to fetch).
 template <typename T, int TI, int TJ, bool FP>
-__global__ void __launch_bounds__(kThreads, PhaseBlocks<T, FP>::value) k_phase_h(Geo<T> g, StageIO<T> io, Tiling t) {
+__global__ void __launch_bounds__(kTileThreads, kPhaseBlocks) k_phase_h(Geo<T> g, StageIO<T> io, Tiling t) {
   extern __shared__ __align__(16) unsigned char smraw[];
   release_dependents();
   const TileBox b = tile_box(t, g.n, blockIdx.x);
@@ -35,7 +35,7 @@ __global__ void __launch_bounds__(kThreads, PhaseBlocks<T, FP>::value) k_phase_h
 }
 
 template <typename T, int TI, int TJ, bool FP>
-__global__ void __launch_bounds__(kThreads, PhaseBlocksUV<T>::value) k_phase_uv(Geo<T> g, StageIO<T> io, Tiling t) {
+__global__ void __launch_bounds__(kTileThreads, PhaseBlocksUV<T, TileShape<TI, TJ>::KP, FP>::value) k_phase_uv(Geo<T> g, StageIO<T> io, Tiling t) {
   extern __shared__ __align__(16) unsigned char smraw[];
   release_dependents();
   const TileBox b = tile_box(t, g.n, blockIdx.x);
@@ -49,7 +49,7 @@ __global__ void __launch_bounds__(kThreads, PhaseBlocksUV<T>::value) k_phase_uv(
 // overlap the barrier.  The loop runs per RK stage (phase H, barrier, phase
 // UV, barrier) so the two phases' gather states are never live together.
 template <typename T, int TI, int TJ>
-__global__ void __launch_bounds__(kThreads, 3) k_round(RoundArgs<T> a) {
+__global__ void __launch_bounds__(kTileThreads, 3) k_round(RoundArgs<T> a) {
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ StageIO<T> s_io[2];  // stage pointers, alternating between consecutive stages
   T* sm = reinterpret_cast<T*>(smraw);
@@ -58,24 +58,22 @@ __global__ void __launch_bounds__(kThreads, 3) k_round(RoundArgs<T> a) {
   const int nstage = a.nbb * nst;
   const int t0 = blockIdx.x;
   unsigned gen = 0;
-  EdgeCnt cnt;
-  int P = 0;
   if (threadIdx.x == 0) s_io[0] = round_stage(a, a.step0, 0);
   __syncthreads();
   // phase H of stage 0: the first tile's prologue
-  Gather<T, TI, TJ, false> gh;
-  if (t0 < ntiles) tile_h_pro<T, TI, TJ>(a.g, s_io[0], tile_box(a.t, a.g.n, t0), sm, gh, cnt, P);
+  HPre<T, TI, TJ> hpre;
+  if (t0 < ntiles) tile_h_pro<T, TI, TJ>(a.g, s_io[0], tile_box(a.t, a.g.n, t0), sm, hpre);
   for (int sg = 0; sg < nstage; ++sg) {
     const StageIO<T>& io = s_io[sg & 1];
     int k = 0;
     for (int tile = t0; tile < ntiles; tile += gridDim.x, ++k) {
       const TileBox b = tile_box(a.t, a.g.n, tile);
-      if (k > 0) tile_h_pro<T, TI, TJ>(a.g, io, b, sm, gh, cnt, P);
-      tile_h_main<T, TI, TJ>(a.g, io, b, sm, gh, cnt, P);
+      if (k > 0) tile_h_pro<T, TI, TJ>(a.g, io, b, sm, hpre);
+      tile_h_main<T, TI, TJ>(a.g, io, b, sm, hpre);
       __syncthreads();
     }
-    Gather<T, TI, TJ, true> gu;
-    if (t0 < ntiles) tile_uv_pro<T, TI, TJ>(a.g, io, tile_box(a.t, a.g.n, t0), sm, gu, cnt, P);
+    UvPre<T, TI, TJ> pre;
+    if (t0 < ntiles) tile_uv_pro<T, TI, TJ>(a.g, tile_box(a.t, a.g.n, t0), pre);
     if (!grid_barrier(a.bar, gen, a.err, a.spin_limit)) {
       cp_async_wait_all();  // no copy may be left in flight when the CTA leaves
       return;
@@ -83,14 +81,14 @@ __global__ void __launch_bounds__(kThreads, 3) k_round(RoundArgs<T> a) {
     k = 0;
     for (int tile = t0; tile < ntiles; tile += gridDim.x, ++k) {
       const TileBox b = tile_box(a.t, a.g.n, tile);
-      if (k > 0) tile_uv_pro<T, TI, TJ>(a.g, io, b, sm, gu, cnt, P);
-      tile_uv_main<T, TI, TJ>(a.g, io, b, sm, gu, cnt, P);
+      if (k > 0) tile_uv_pro<T, TI, TJ>(a.g, b, pre);
+      tile_uv_main<T, TI, TJ>(a.g, io, b, sm, pre);
       __syncthreads();
     }
     if (sg + 1 < nstage) {
       if (threadIdx.x == 0) s_io[(sg + 1) & 1] = round_stage(a, a.step0 + (sg + 1) / nst, (sg + 1) % nst);
       __syncthreads();
-      if (t0 < ntiles) tile_h_pro<T, TI, TJ>(a.g, s_io[(sg + 1) & 1], tile_box(a.t, a.g.n, t0), sm, gh, cnt, P);
+      if (t0 < ntiles) tile_h_pro<T, TI, TJ>(a.g, s_io[(sg + 1) & 1], tile_box(a.t, a.g.n, t0), sm, hpre);
     }
     if (!grid_barrier(a.bar, gen, a.err, a.spin_limit)) {
       cp_async_wait_all();
@@ -99,43 +97,31 @@ __global__ void __launch_bounds__(kThreads, 3) k_round(RoundArgs<T> a) {
   }
 }
 
-// Tile constant blocks: word w < uConstWords of tile t's block is what
-// tile_uv_consts stages at shared-memory word uG + w for that tile (gct, sina,
-// rda, rdx, rdy, a_f of its cells, c_dy of its x faces, d_dx of its y faces);
-// then dzph_x of its x faces and dzph_y of its y faces, indexed like phase H's
-// shared-memory planes.  Positions outside a partial tile and the padding are zero.
+// Tile constant blocks (TileShape::cW words per tile): rda, rdx, rdy, a_f of
+// the tile's cells, c_dy of its x faces, d_dx of its y faces, dzph_x of its x
+// faces and dzph_y of its y faces, the image of phase H's shared-memory
+// constant area.  Positions outside a partial tile and the padding are zero.
 template <typename T, int TI, int TJ>
 __global__ void __launch_bounds__(kThreads) k_const_blocks(Geo<T> g, Tiling t, T* out) {
   using S = TileShape<TI, TJ>;
   const long total = 6L * t.nti * t.ntj * S::cW;
   const int m = g.m;
   for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < total; k += (long)gridDim.x * blockDim.x) {
-    const int tile = (int)(k / S::cW), w = (int)(k - (long)tile * S::cW), o = S::uG + w;
+    const int tile = (int)(k / S::cW), w = (int)(k - (long)tile * S::cW);
     const TileBox b = tile_box_at(t, g.n, tile);
     T v = T(0);
-    if (w >= S::bDZX) {
-      if (w < S::bDZY) {
-        const int e = w - S::bDZX, a = e / TJ, q = e % TJ;
-        if (a <= b.ni && q < b.nj) v = g.dzph_x[cell(b.f, b.i0 + a, b.j0 + q, m)];
-      } else if (w < S::bDZY + S::FY) {
-        const int e = w - S::bDZY, r = e / (TJ + 1), qq = e % (TJ + 1);
-        if (r < b.ni && qq <= b.nj) v = g.dzph_y[cell(b.f, b.i0 + r, b.j0 + qq, m)];
-      }
-    } else if (o < S::uSN) {
-      const int e = (o - S::uG) / 4, comp = (o - S::uG) % 4, a = e / TJ, q = e % TJ;
-      if (a < b.ni && q < b.nj) v = g.gct[4 * cell(b.f, b.i0 + a, b.j0 + q, m) + comp];
-    } else if (o < S::uAF + S::C) {
-      const int arr = (o - S::uSN) / S::C, e = (o - S::uSN) % S::C, a = e / TJ, q = e % TJ;
+    if (w < S::bCDY) {
+      const int arr = w / S::C, e = w % S::C, a = e / TJ, q = e % TJ;
       if (a < b.ni && q < b.nj) {
         const long c = cell(b.f, b.i0 + a, b.j0 + q, m);
-        v = arr == 0 ? g.sina[c] : arr == 1 ? g.rda[c] : arr == 2 ? g.rdx[c] : arr == 3 ? g.rdy[c] : g.a_f[c];
+        v = arr == 0 ? g.rda[c] : arr == 1 ? g.rdx[c] : arr == 2 ? g.rdy[c] : g.a_f[c];
       }
-    } else if (o >= S::uCDY && o < S::uCDY + S::FX) {
-      const int e = o - S::uCDY, a = e / TJ, q = e % TJ;
-      if (a <= b.ni && q < b.nj) v = g.c_dy[cell(b.f, b.i0 + a, b.j0 + q, m)];
-    } else if (o >= S::uDDX && o < S::uDDX + S::FY) {
-      const int e = o - S::uDDX, r = e / (TJ + 1), qq = e % (TJ + 1);
-      if (r < b.ni && qq <= b.nj) v = g.d_dx[cell(b.f, b.i0 + r, b.j0 + qq, m)];
+    } else {
+      const bool xf = w < S::bDDX || (w >= S::bDZX && w < S::bDZY);
+      const T* src = w < S::bDDX ? g.c_dy : w < S::bDZX ? g.d_dx : w < S::bDZY ? g.dzph_x : g.dzph_y;
+      const int e = w - (w < S::bDDX ? S::bCDY : w < S::bDZX ? S::bDDX : w < S::bDZY ? S::bDZX : S::bDZY);
+      const int W = xf ? TJ : TJ + 1, a = e / W, q = e % W;
+      if (xf ? (a <= b.ni && q < b.nj) : (a < b.ni && q <= b.nj)) v = src[cell(b.f, b.i0 + a, b.j0 + q, m)];
     }
     out[k] = v;
   }
@@ -167,10 +153,16 @@ bool tile_cfg_supported(TileCfg c) {
 }
 
 namespace {
-template <int TI, int TJ>
-size_t face_cache_elems_tile(int n) {
+template <typename T, int TI, int TJ>
+size_t terms_elems_tile(int n) {
   const size_t nti = (n + TI - 1) / TI, ntj = (n + TJ - 1) / TJ;
-  return 6 * nti * ntj * (size_t)TileShape<TI, TJ>::fW;
+  return 6 * nti * ntj * (size_t)(kTerms<T> * TI * TJ);
+}
+template <typename T>
+size_t terms_elems_all(int n) {
+  const size_t s[6] = {terms_elems_tile<T, 7, 32>(n),  terms_elems_tile<T, 8, 32>(n), terms_elems_tile<T, 15, 32>(n),
+                       terms_elems_tile<T, 16, 32>(n), terms_elems_tile<T, 8, 16>(n), terms_elems_tile<T, 16, 16>(n)};
+  return *std::max_element(s, s + 6);
 }
 }  // namespace
 
@@ -192,12 +184,7 @@ size_t const_block_elems(TileCfg c, int n) {
   return 0;
 }
 
-size_t face_cache_elems(int n) {
-  const size_t s[6] = {face_cache_elems_tile<7, 32>(n), face_cache_elems_tile<8, 32>(n),
-                       face_cache_elems_tile<15, 32>(n), face_cache_elems_tile<16, 32>(n),
-                       face_cache_elems_tile<8, 16>(n), face_cache_elems_tile<16, 16>(n)};
-  return *std::max_element(s, s + 6);
-}
+size_t terms_elems(int n, size_t esize) { return esize == 8 ? terms_elems_all<double>(n) : terms_elems_all<float>(n); }
 
 Tiling make_tiling(TileCfg c, int n) {
   Tiling t;
@@ -214,7 +201,7 @@ namespace {
 template <typename T, int TI, int TJ, bool UV>
 size_t tile_smem() {
   using S = TileShape<TI, TJ>;
-  return sizeof(T) * (UV ? S::kWordsUV : S::kWordsH) + sizeof(int) * kItemWords;
+  return sizeof(T) * (UV ? S::kWordsUV : S::kWordsH);
 }
 
 // The persistent kernel runs both phases in one allocation: the larger of the two.
@@ -240,7 +227,7 @@ cudaError_t record_wave_slots() {
   if (dev < 0 || dev >= kMaxDevices) return cudaSuccess;  // the launch then keeps the full-tile path
   if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
   auto kern = UV ? k_phase_uv<T, TI, TJ, false> : k_phase_h<T, TI, TJ, false>;
-  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, tile_smem<T, TI, TJ, UV>())) !=
+  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kTileThreads, tile_smem<T, TI, TJ, UV>())) !=
       cudaSuccess)
     return e;
   wave_slots<T, TI, TJ, UV>()[dev].store(sms * per_sm, std::memory_order_relaxed);
@@ -275,7 +262,7 @@ cudaError_t launch_round_tile(RoundArgs<T> a, int max_ctas, cudaStream_t s, int*
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_round<T, TI, TJ>, kThreads, smem)) !=
+  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_round<T, TI, TJ>, kTileThreads, smem)) !=
       cudaSuccess)
     return e;
   a.t = make_tiling({TI, TJ}, a.g.n);
@@ -284,7 +271,7 @@ cudaError_t launch_round_tile(RoundArgs<T> a, int max_ctas, cudaStream_t s, int*
   if (grid < 1) return cudaErrorInvalidConfiguration;
   if (grid_out) *grid_out = grid;
   void* args[] = {&a};
-  return cudaLaunchCooperativeKernel((const void*)k_round<T, TI, TJ>, dim3(grid), dim3(kThreads), args, smem, s);
+  return cudaLaunchCooperativeKernel((const void*)k_round<T, TI, TJ>, dim3(grid), dim3(kTileThreads), args, smem, s);
 }
 
 // Whether a phase launch at n cells per face edge runs the full-tile kernel:
@@ -311,7 +298,7 @@ cudaError_t launch_tile(const Geo<T>& g, const StageIO<T>& io, cudaStream_t s, i
   // previous kernel's tail; it waits (griddepcontrol.wait) before reading state
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(6 * t.tiles_per_face());
-  cfg.blockDim = dim3(kThreads);
+  cfg.blockDim = dim3(kTileThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cudaLaunchAttribute attr[1];

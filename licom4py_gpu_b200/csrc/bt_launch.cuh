@@ -22,9 +22,12 @@ bool tile_cfg_supported(TileCfg c);
 size_t const_block_elems(TileCfg c, int n);
 template <typename T>
 cudaError_t launch_const_blocks(const Geo<T>& g, TileCfg c, T* out, cudaStream_t s);
-// Elements of the face cache blocks of one member at n cells per face edge,
-// enough for every supported tile shape (the plan's tile can change later).
-size_t face_cache_elems(int n);
+// Elements of the momentum-term blocks of one member at n cells per face edge
+// in a type of esize bytes, enough for every supported tile shape (the plan's
+// tile can change later).
+size_t terms_elems(int n, size_t esize);
+// Elements of the bands of one member (velocity: 3 planes, h: 2).
+inline size_t band_elems(int n) { return 5 * (size_t)72 * n; }
 Tiling make_tiling(TileCfg c, int n);
 
 // Set kernel attributes (dynamic shared memory opt-in) for the current device.

@@ -5,14 +5,14 @@
 // the device memory pool), a Fortran or C model driver that reserves all of its
 // GPU memory up front, or a service that must not change its memory footprint
 // once it is serving.  bt_round does allocate (its plan owns stage scratch,
-// face caches and the halo gather tables), so this file offers one entry point
+// momentum terms and the halo gather tables), so this file offers one entry point
 // that keeps all of that scratch in a fixed array of device memory that the
 // library declares statically.
 //
 // The array (kScratchBytes, 6 MiB) belongs to every GPU that loads the library
 // and stays allocated until the process exits.  It holds, in this order: a
-// status word, the halo gather tables, the stage fields (3, or 6 for RK3) and
-// the face cache blocks of the 8 x 16 tiles.  The largest sizes that fit: float64 N <= 112 (RK2) /
+// status word, the halo gather tables, the stage fields (3, or 6 for RK3),
+// the momentum-term blocks of the 8 x 16 tiles and the bands.  The sizes it serves: float64 N <= 112 (RK2) /
 // 96 (RK3), float32 N <= 160 (RK2) / 136 (RK3); larger sizes are rejected with
 // BT_EINVAL.
 //
@@ -134,7 +134,7 @@ __device__ __forceinline__ long band_source(const RouteTable& rt, int f, int ti,
 // out of bounds (k_check_tables has rejected tables that would need it).
 template <typename T>
 __global__ void k_build_halo(int n, const T* coef, const int* li, const int* lj, RouteTable rt, int2* src,
-                             T* w) {
+                             T* w, int* bsrc) {
   const int m = n + 6, nh = halo_count(m);
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= 6 * nh) return;
@@ -171,6 +171,13 @@ __global__ void k_build_halo(int n, const T* coef, const int* li, const int* lj,
   src[k] = make_int2((int)s0, (int)s1);
   w[2 * k] = coef[2 * ob];
   w[2 * k + 1] = coef[2 * ob + 1];
+  if (bi != i) return;  // corner
+  // the first source in band order (Geo::bsrc)
+  const int d = along_i ? (j < kHalo ? kW : kE) : (i < kHalo ? kS : kN);
+  const int c = d == kW ? j : d == kE ? j - (m - kHalo) : d == kS ? i : i - (m - kHalo);
+  const int pos = loc - kHalo, r = rt.r[f * 4 + d];
+  bsrc[band_no(f, d, c, (along_i ? i : j) - kHalo, n)] =
+      band_no(route_nb(r), route_side(r), c, route_rev(r) ? n - 1 - pos : pos, n);
 }
 
 // The checks of bt_plan_create on the device, one thread per cell of the
@@ -235,7 +242,7 @@ int check_tables_once(unsigned char* base, const bt_grid_desc& d, cudaStream_t s
 
 template <typename T>
 StageIO<T> io_of(const T* h, const T* u, const T* v, const T* hp, const T* up, const T* vp, T* ho, T* uo, T* vo,
-                 T* fx, double dt, double beta, int stored, int last) {
+                 T* fx, T* band, int n, double dt, double beta, int stored, int last, int sg) {
   StageIO<T> io;
   io.h = h;
   io.u = u;
@@ -247,6 +254,9 @@ StageIO<T> io_of(const T* h, const T* u, const T* v, const T* hp, const T* up, c
   io.u_out = uo;
   io.v_out = vo;
   io.fx = fx;
+  io.band_uv = band;  // the new-h bands alternate between consecutive stages
+  io.band_h = band + (3 + (sg & 1)) * band_plane(n);
+  io.band_hn = band + (4 - (sg & 1)) * band_plane(n);
   io.dt = (T)dt;
   io.beta = (T)beta;
   io.stored_halo = stored;
@@ -254,33 +264,43 @@ StageIO<T> io_of(const T* h, const T* u, const T* v, const T* hp, const T* up, c
   return io;
 }
 
+// Largest N served per type and RK order (include/licom_bt.h).
+template <typename T>
+constexpr int max_n(int rk) {
+  return sizeof(T) == 8 ? (rk == 2 ? 112 : 96) : (rk == 2 ? 160 : 136);
+}
+
 template <typename T>
 int run_noalloc(unsigned char* base, const bt_grid_desc& d, const bt_state_in& in, const bt_state_out& out, int nbb,
                 double dtb, int rk, cudaStream_t s) {
   const int n = d.n, m = n + 6, nh = halo_count(m);
-  // face cache blocks of the 8 x 16 tiles this entry point runs
+  // momentum-term blocks of the 8 x 16 tiles this entry point runs
   const size_t fe = (size_t)6 * m * m,
-               face = (size_t)6 * ((n + 7) / 8) * ((n + 15) / 16) * TileShape<8, 16>::fW;
+               terms = (size_t)6 * ((n + 7) / 8) * ((n + 15) / 16) * (kTerms<T> * TileShape<8, 16>::C);
   const size_t o_src = kStatusBytes;
   const size_t o_w = o_src + align256((size_t)6 * nh * sizeof(int2));
   const size_t o_f = o_w + align256((size_t)6 * nh * 2 * sizeof(T));
   const int nfields = rk == 2 ? 3 : 6;
   const size_t o_fx = o_f + align256((size_t)nfields * fe * sizeof(T));
-  const size_t need = o_fx + align256(face * sizeof(T));
-  if (need > kScratchBytes)
-    return set_error(BT_EINVAL, "bt_round_noalloc: N = " + std::to_string(n) + " needs " + std::to_string(need) +
-                                    " bytes of scratch, more than the library's fixed " +
-                                    std::to_string(kScratchBytes) + "; use bt_plan_create/bt_round");
+  const size_t o_band = o_fx + align256(terms * sizeof(T));
+  const size_t o_bsrc = o_band + align256(band_elems(n) * sizeof(T));
+  const size_t need = o_bsrc + align256((size_t)72 * n * sizeof(int));
+  if (n > max_n<T>(rk) || need > kScratchBytes)
+    return set_error(BT_EINVAL, "bt_round_noalloc: N = " + std::to_string(n) + " is more than the library's fixed " +
+                                    std::to_string(kScratchBytes) + " bytes of scratch serve (N <= " +
+                                    std::to_string(max_n<T>(rk)) + "); use bt_plan_create/bt_round");
   const int rc = check_tables_once<T>(base, d, s);
   if (rc != BT_OK) return rc;
   int2* hsrc = (int2*)(base + o_src);
   T* hw = (T*)(base + o_w);
   T* F = (T*)(base + o_f);
   T* fx = (T*)(base + o_fx);
+  T* band = (T*)(base + o_band);
+  int* bsrc = (int*)(base + o_bsrc);
   const RouteTable rt = make_routes();
   const int cells = 6 * nh, th = 256;
   k_build_halo<T><<<(cells + th - 1) / th, th, 0, s>>>(n, (const T*)d.k2e_coef, d.loc_i_local, d.loc_j_local, rt,
-                                                       hsrc, hw);
+                                                       hsrc, hw, bsrc);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return set_error(BT_ECUDA, std::string("bt_round_noalloc: ") + cudaGetErrorString(e));
 
@@ -302,7 +322,8 @@ int run_noalloc(unsigned char* base, const bt_grid_desc& d, const bt_state_in& i
   g.d_dx = (const T*)d.d_dx;
   g.hsrc = hsrc;
   g.hw = hw;
-  g.cblk = nullptr;  // no prepared constant blocks: phase UV reads the constant arrays
+  g.bsrc = bsrc;
+  g.cblk = nullptr;  // no prepared constant blocks: the phases read the constant arrays
   g.cblk_ti = g.cblk_tj = 0;
   for (int k = 0; k < 24; ++k) g.route[k] = rt.r[k];
 
@@ -321,17 +342,20 @@ int run_noalloc(unsigned char* base, const bt_grid_desc& d, const bt_state_in& i
     const T* const* bs = step == 0 ? B0 : (const T* const*)X;
     const int stored = step == 0 ? 1 : 0;
     if (rk == 2) {
-      e = stage(io_of<T>(cur[0], cur[1], cur[2], bs[0], bs[1], bs[2], Y[0], Y[1], Y[2], fx, dtb / 2.0, 0.0,
-                         stored, 0));
+      e = stage(io_of<T>(cur[0], cur[1], cur[2], bs[0], bs[1], bs[2], Y[0], Y[1], Y[2], fx, band, n, dtb / 2.0, 0.0,
+                         stored, 0, 2 * step));
       if (e == cudaSuccess)
-        e = stage(io_of<T>(Y[0], Y[1], Y[2], bs[0], bs[1], bs[2], X[0], X[1], X[2], fx, dtb, 0.0, 0, 1));
+        e = stage(io_of<T>(Y[0], Y[1], Y[2], bs[0], bs[1], bs[2], X[0], X[1], X[2], fx, band, n, dtb, 0.0, 0, 1,
+                         2 * step + 1));
     } else {
-      e = stage(io_of<T>(cur[0], cur[1], cur[2], bs[0], bs[1], bs[2], Y[0], Y[1], Y[2], fx, dtb / 3.0, 1.0,
-                         stored, 0));
+      e = stage(io_of<T>(cur[0], cur[1], cur[2], bs[0], bs[1], bs[2], Y[0], Y[1], Y[2], fx, band, n, dtb / 3.0, 1.0,
+                         stored, 0, 3 * step));
       if (e == cudaSuccess)
-        e = stage(io_of<T>(Y[0], Y[1], Y[2], bs[0], bs[1], bs[2], Z[0], Z[1], Z[2], fx, dtb / 2.0, 1.0, 0, 0));
+        e = stage(io_of<T>(Y[0], Y[1], Y[2], bs[0], bs[1], bs[2], Z[0], Z[1], Z[2], fx, band, n, dtb / 2.0, 1.0, 0,
+                         0, 3 * step + 1));
       if (e == cudaSuccess)
-        e = stage(io_of<T>(Z[0], Z[1], Z[2], bs[0], bs[1], bs[2], X[0], X[1], X[2], fx, dtb, 1.0, 0, 1));
+        e = stage(io_of<T>(Z[0], Z[1], Z[2], bs[0], bs[1], bs[2], X[0], X[1], X[2], fx, band, n, dtb, 1.0, 0, 1,
+                         3 * step + 2));
     }
   }
   if (e == cudaSuccess && out.diag[0]) {

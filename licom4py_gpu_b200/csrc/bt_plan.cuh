@@ -36,9 +36,10 @@ struct bt_plan {
   int mode = BT_MODE_STREAM;
   const void* c[17] = {};
   int route[24] = {};
+  void* d_hw = nullptr;    // T[6*nh*2]; the halo tables are one allocation, d_hsrc and d_bsrc point into it
   void* d_hsrc = nullptr;  // int2[6*nh]
-  void* d_hw = nullptr;    // T[6*nh*2]
-  void* scratch = nullptr; // Y (3 fields) + Y2 (3 fields) + edge lines
+  int* d_bsrc = nullptr;   // int[72*n]
+  void* scratch = nullptr; // Y (3 fields) + Z (3 fields) + edge lines + bands + momentum terms
   size_t field_elems = 0;
   cudaStream_t cap_stream = nullptr;
   cudaEvent_t ev_in = nullptr, ev_out = nullptr;
@@ -98,13 +99,14 @@ struct bt_plan {
   }
 
   size_t esize() const { return dtype == BT_F64 ? 8 : 4; }
-  // scratch layout: 6 stage fields, edge lines (24 n), then on a 256-byte boundary (16-byte copies)
-  // the face cache blocks, sized for every tile shape
-  size_t face_offset() const { return ((6 * field_elems + 24 * (size_t)n) * esize() + 255) & ~(size_t)255; }
-  size_t scratch_bytes() const { return face_offset() + face_cache_elems(n) * esize(); }
+  // scratch layout: 6 stage fields, edge lines (24 n), bands, then on a 256-byte boundary the
+  // momentum-term blocks, sized for every tile shape
+  size_t terms_offset() const { return ((6 * field_elems + 24 * (size_t)n + band_elems(n)) * esize() + 255) & ~(size_t)255; }
+  size_t scratch_bytes() const { return terms_offset() + terms_elems(n, esize()) * esize(); }
   void* scratch_field(int k) const { return (char*)scratch + (size_t)k * field_elems * esize(); }
   void* edge_lines() const { return scratch_field(6); }
-  void* face_x() const { return (char*)scratch + face_offset(); }
+  void* bands() const { return (char*)edge_lines() + 24 * (size_t)n * esize(); }
+  void* terms() const { return (char*)scratch + terms_offset(); }
 
   // geometry for kernels of tile shape t (its constant blocks if built)
   template <typename T>
@@ -141,6 +143,7 @@ struct bt_plan {
     g.d_dx = (const T*)c[16];
     g.hsrc = (const int2*)d_hsrc;
     g.hw = (const T*)d_hw;
+    g.bsrc = d_bsrc;
     g.cblk = nullptr;
     g.cblk_ti = g.cblk_tj = 0;
     std::memcpy(g.route, route, sizeof(route));

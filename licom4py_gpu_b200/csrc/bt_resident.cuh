@@ -6,12 +6,10 @@
 // round in one cooperative launch with ONE CTA PER TILE, and each CTA keeps
 // everything that does not change during the round on chip:
 //
-//   * the tile's constants of both phases (metric, depths, spacings) are
-//     staged into shared memory once, at launch;
-//   * phase H leaves the face cache (edge-averaged normal velocity, its
-//     viscous correction and the celerity flux of every face of the tile) and
-//     the raw velocities of the stencil region in phase UV's shared-memory
-//     layout, so phase UV reads only the new h of its region from memory.
+//   * the tile's cell and face constants (depths, spacings) are staged into
+//     shared memory once, at launch;
+//   * phase H leaves the momentum terms of the tile's cells in shared memory,
+//     so phase UV reads only the new h of its region and the base velocities.
 //
 // Tiles synchronise with their neighbours only: after each phase a CTA
 // publishes the number of phases it has completed (release store of its own
@@ -43,15 +41,15 @@ struct ResBlocks {
   static constexpr int value = (sizeof(T) == 8 && TI * TJ > 128) ? 2 : 3;
 };
 
-// Shared-memory layout of a resident CTA (words of T): phase H layout, phase
-// H face fluxes, phase UV layout, then the gather item scratch (ints).
+// Shared-memory layout of a resident CTA (words of T): phase H layout,
+// momentum terms, phase UV layout.
 template <typename T, int TI, int TJ>
 struct ResLayout {
   using S = TileShape<TI, TJ>;
-  static constexpr int kPQ = up4(S::kWordsH);
-  static constexpr int kUV = up4(kPQ + S::FX + S::FY);
+  static constexpr int kTermsAt = up4(S::kWordsH);
+  static constexpr int kUV = up4(kTermsAt + kTerms<T> * S::C);
   static constexpr int kWords = up4(kUV + S::kWordsUV);
-  static constexpr size_t kBytes = sizeof(T) * kWords + sizeof(int) * kItemWords;
+  static constexpr size_t kBytes = sizeof(T) * kWords;
 };
 
 // Publish that this CTA has completed ``phases`` phases: every thread's global
@@ -109,24 +107,17 @@ template <typename T, int TI, int TJ, bool FULL>
 __device__ __forceinline__ bool res_stage(const RoundArgs<T>& a, const ResSync& rsy, const StageIO<T>& io,
                                           const TileBox& b, T* sm, const ResSm<T>& rs, int tile, int done) {
   {
-    Gather<T, TI, TJ, false, true> gat;
-    EdgeCnt cnt;
-    int P;
-    tile_desc<T, TI, TJ, FULL, false, true>(a.g, io, b, gat, cnt, P, rs.items);
+    HPre<T, TI, TJ> pre;
+    tile_h_points<T, TI, TJ, FULL>(a.g, io, b, sm, pre);
     if (done > 0 && !res_wait(rsy, tile, done, a.err, a.spin_limit)) return false;
-    tile_h_main_t<T, TI, TJ, FULL, true>(a.g, io, b, sm, gat, cnt, P, rs);
+    tile_h_main_t<T, TI, TJ, FULL, true>(a.g, io, b, sm, pre, rs);
     res_publish(rsy.flags + tile * kResFlagStride, done + 1);
   }
   {
-    Gather<T, TI, TJ, true, true> gat;
-    EdgeCnt cnt;
-    int P;
-    tile_desc<T, TI, TJ, FULL, true, true>(a.g, io, b, gat, cnt, P, rs.items);
-    if (!res_wait(rsy, tile, done + 1, a.err, a.spin_limit)) {
-      cp_async_wait_all();
-      return false;
-    }
-    tile_uv_main_t<T, TI, TJ, FULL, true>(a.g, io, b, rs.uv, gat, cnt, P, rs);  // phase UV's own layout
+    UvPre<T, TI, TJ> pre;
+    tile_uv_pro_t<T, TI, TJ, FULL>(a.g, b, pre);
+    if (!res_wait(rsy, tile, done + 1, a.err, a.spin_limit)) return false;
+    tile_uv_main_t<T, TI, TJ, FULL, true>(a.g, io, b, sm + ResLayout<T, TI, TJ>::kUV, pre, rs);
     res_publish(rsy.flags + tile * kResFlagStride, done + 2);
   }
   return true;
@@ -135,27 +126,16 @@ __device__ __forceinline__ bool res_stage(const RoundArgs<T>& a, const ResSync& 
 // One CTA per tile (face-major order); the grid is exactly the tile count.
 template <typename T, int TI, int TJ>
 __global__ void __launch_bounds__(kTileThreads, ResBlocks<T, TI, TJ>::value) k_resident(RoundArgs<T> a, ResSync rsy) {
-  using RL = ResLayout<T, TI, TJ>;
-  using S = TileShape<TI, TJ>;
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ StageIO<T> s_io;
   T* const sm = reinterpret_cast<T*>(smraw);
   ResSm<T> rs;
-  rs.uv = sm + RL::kUV;
-  rs.pq = sm + RL::kPQ;
-  rs.hs = sm + S::hH;
-  rs.items = reinterpret_cast<int*>(sm + RL::kWords);
+  rs.terms = sm + ResLayout<T, TI, TJ>::kTermsAt;
   const int tile = blockIdx.x;
   const TileBox b = tile_box_at(a.t, a.g.n, tile);
   const bool full = tile_full(b, a.g.m, TI, TJ);
-  // the constants of both phases, once per round (awaited by the first phase's barrier)
-  if (full) {
-    tile_h_consts<T, TI, TJ, true>(a.g, b, sm);
-    tile_uv_consts<T, TI, TJ, true>(a.g, b, rs.uv);
-  } else {
-    tile_h_consts<T, TI, TJ, false>(a.g, b, sm);
-    tile_uv_consts<T, TI, TJ, false>(a.g, b, rs.uv);
-  }
+  // the constants, once per round (awaited by the first phase's barrier)
+  tile_h_consts<T, TI, TJ>(a.g, b, sm);
   const int nst = a.rk == 2 ? 2 : 3;
   const int nstage = a.nbb * nst;
   for (int sg = 0; sg < nstage; ++sg) {

@@ -3,18 +3,35 @@
 // One RK stage (src/licom/momentum/barotr_pure.py:100-168) is split at its two
 // global dependencies into two tile phases:
 //
-//   phase H  (tile_h):  celerity, A->C remap, C-grid edge average, D-grid
-//            upwind, velocity viscosity, mass flux (+ flux edge average on
-//            the last stage), divergence, new h = h_base - div*dt.
-//   phase UV (tile_uv): the same C/D-grid face quantities recomputed from the
-//            stage input, vorticity/kinetic-energy advection, celerity
-//            viscosity, pressure gradient of the new h, momentum update.
+//   phase H  (tile_h):  everything that depends on the stage input alone:
+//            celerity, A->C remap, C-grid edge average, D-grid upwind,
+//            velocity viscosity, mass flux (+ flux edge average on the last
+//            stage), divergence, new h = h_base - div*dt, and the momentum
+//            terms other than the pressure gradient (vorticity / kinetic
+//            energy advection, Coriolis, celerity viscosity) of each cell.
+//   phase UV (tile_uv): what needs the new h: its pressure gradient, and the
+//            momentum update from that and phase H's terms.
+//
+// Everything local to the stage input runs in phase H, so that phase UV reads 11
+// words per cell in float64 (7 in float32) instead of the 26 it took when it
+// recomputed the advection from the faces' cache, and gathers only h at the
+// face edges.  Both are bound by latency at one-wave sizes (loads, two to four
+// barriers, one float64 face chain) and by issue and memory latency at
+// C384.  Measured before and after this split with the band gathers, 16-byte
+// constant copies and 288 threads (us per substep): float64 C96 8 x 16 15.2 /
+// 14.0, C192 8 x 32 39.5 / 36.1, C384 16 x 16 149 / 137, 16 x 32 184 / 155;
+// float32 C96 8 x 16 11.9 / 10.8, C192 16 x 32 24.3 / 22.1, C384 16 x 32 70.0 / 65.9.
 //
 // The ext_scalar / ext_vector halo fills of the reference (cube.py:130-153)
-// become gathers done by whoever reads a halo cell (fetch_s / fetch_v), and
-// the boundary_communication edge averages (communication.py:504-570) are
-// computed in place by recomputing the neighbouring face's edge value from
-// that face's data (nb_normal_raw / nb_mass_flux).
+// are computed by whoever reads a halo cell.  Both of a halo cell's sources
+// lie on one of the three interior lines next to the shared edge, side by
+// side; each phase therefore also writes what the halo remap reads -- the new
+// h, or the lon/lat velocity -- of those lines into band buffers ordered along
+// the edge, so that the reads of neighbouring halo cells are runs of
+// consecutive words whatever the two faces' orientation.  The
+// boundary_communication edge averages (communication.py:504-570) are computed
+// in place by recomputing the neighbouring face's edge value from that face's
+// data.
 //
 // Every arithmetic expression keeps the reference's operand order; with
 // -fmad=false the float64 instantiation rounds exactly like the NumPy run of
@@ -149,35 +166,6 @@ __device__ T nb_normal_raw(const Geo<T>& g, const T* U, const T* V, int stored, 
   return T(0.5) * (rplus(p, 1) + rminus(p + 1, 1));
 }
 
-// The neighbour's mass flux at the shared edge on the last stage, given the
-// (already averaged, hence common) edge velocity ``bc`` (barotr_pure.py:29-49
-// evaluated on the neighbour, then communication.py:504-570 on the fluxes).
-template <typename T>
-__device__ T nb_mass_flux(const Geo<T>& g, const T* H, int stored, int f, int side, int k, T bc) {
-  const int r = g.route[f * 4 + side];
-  const int nb = route_nb(r), ns = route_side(r);
-  const int kk = route_rev(r) ? g.n - 1 - k : k;
-  const int y = (ns == kE || ns == kW);
-  T p[6];
-  int fi = 0, fj = 0;
-#pragma unroll
-  for (int q = 0; q < 6; ++q) {
-    int i, j;
-    edge_point(ns, kk, q, g.m, i, j);
-    if (q == 3) {
-      fi = i;
-      fj = j;
-    }
-    p[q] = fetch_s(H, g, nb, i, j, stored);
-  }
-  const long o = cell(nb, fi, fj, g.m);
-  const T dz = y ? g.dzph_y[o] : g.dzph_x[o];
-  const T he = rplus(p, 1), hw = rminus(p + 1, 1);
-  const T c = celerity(mid6(p, 1), dz);
-  const T vis = bc + (T(4.9) / c) * (he - hw);
-  return dz * vis + (vis > T(0.0) ? he : hw) * vis;
-}
-
 // Side of a face whose C-grid edge lies at x-face index i (or y-face index j).
 __device__ __forceinline__ int xface_side(int i, int m) {
   return i == kHalo ? kS : (i == m - kHalo ? kN : -1);
@@ -189,37 +177,38 @@ __device__ __forceinline__ int yface_side(int j, int m) {
 // ---------------------------------------------------------------------------
 // Tile phases
 // ---------------------------------------------------------------------------
-// A CTA of kTileThreads threads computes one TI x TJ tile of one face.  Thread
-// t works on column q = t % TJ of the tile and on the rows sl, sl + NS, ...
-// (sl = t / TJ, NS = kTileThreads / TJ row slots), so a warp always covers
-// consecutive columns of one row: every global access is a run of
-// consecutive cells and every shared-memory stencil read is conflict-free.
+// A CTA of kTileThreads threads computes one TI x TJ tile of one face, as lists
+// of independent items spread over the CTA: the points of the tile's stencil
+// region, its faces, its cells.  The lists are row-major, so every global
+// access of a warp is a run of consecutive cells and the shared-memory reads
+// are conflict-free or nearly so.
 //
 // The stencil region of a tile is a cross: the tile's columns extended by 3
 // rows on each side (the "vertical bar", read along i by the x faces) and
 // the tile's rows extended by 3 columns on each side (the "horizontal bar",
-// read along j by the y faces).  Each thread loads the state of its own
-// interior region points straight into registers and stores the quantities
-// the stencils read (h and the contravariant velocity normal to the faces
-// that read the point); halo points of the region are gathered by the
-// Gather items from the neighbouring face.  Constants are staged with
-// cp.async in a prologue that does not depend on the state.
-constexpr int kTileThreads = 256;
+// read along j by the y faces).  A region point is loaded, or gathered from
+// the neighbouring face's bands where it lies in the halo, by one thread, which
+// stores what the stencils read: h, the contravariant velocity normal to the
+// faces that read the point, and the raw velocity tangential to them.  Cell
+// and face constants are staged with cp.async in a prologue that does not
+// depend on the state.
+//
+// 288 threads: with 8 x 16 tiles (the one-wave sizes) the 272 region points,
+// the 280 faces and the gather items each fit one pass, so a CTA runs one face
+// chain, not two; 8 x 32 and 16 x 16 tiles need two (552 and 544 faces; three
+// with 256 threads), 16 x 32 four (1072).
+constexpr int kTileThreads = 288;
 
-// Resident CTAs per SM the phase H kernels are compiled for (register cap
-// 65536 / (256 * blocks)): float64 tiles need more registers per thread.  The
-// float32 build with the full-tile path runs 4 (multi-wave launches: C384 7 %
-// faster than at 3); the edge-path-only build, which runs the one-wave launches,
-// 3 (C96 8 x 16 13.15 -> 11.93 us per substep, C48 12.43 -> 11.51).
-template <typename T, bool FP = true>
-struct PhaseBlocks {
-  static constexpr int value = sizeof(T) == 8 ? 3 : (FP ? 4 : 3);
-};
-// Phase UV runs 3 CTAs per SM in both precisions: at 4 its shared-memory
-// traffic throttles (MIO) and the best tile shape per size measured faster at 3.
-template <typename T>
+// Resident CTAs per SM the phase kernels are compiled for (registers 65536 /
+// (288 * blocks), rounded down to a multiple of 8): 3 in phase H.
+constexpr int kPhaseBlocks = 3;
+template <typename T, int KP, bool FP>
 struct PhaseBlocksUV {
-  static constexpr int value = 3;
+  // float64 tiles of two region points per thread in multi-wave launches: 4 (C384 16 x 16 136.7 us per
+  // substep against 144.3 at 3, 8 x 32 151.5 against 156.4); in one-wave launches (C96 8 x 32 21.2 at 4
+  // against 19.5) and with one point (C48 8 x 16 14.4 against 12.9) or three (C384 16 x 32 156.5
+  // against 154.0): 3
+  static constexpr int value = sizeof(T) == 8 && KP == 2 && FP ? 4 : 3;
 };
 
 constexpr int up4(int x) { return (x + 3) & ~3; }  // shared-memory offsets in words, 16-byte aligned
@@ -227,113 +216,109 @@ constexpr int up4(int x) { return (x + 3) & ~3; }  // shared-memory offsets in w
 template <int TI, int TJ>
 struct TileShape {
   static_assert(TJ == 16 || TJ == 32, "tile columns must be 16 or 32");
-  static_assert(TI <= 32, "the east y-face column is one lane per tile row");
-  static constexpr int RI = TI + 6, RJ = TJ + 6;
-  static constexpr int NS = kTileThreads / TJ;      // row slots
+  static constexpr int RI = TI + 6, RJ = TJ + 6;    // stencil region
   static constexpr int VB = RI * TJ;                // vertical-bar points (r * TJ + q)
-  static constexpr int SB = 6 * TI;                 // side points: 3 W + 3 E columns per tile row
-  static constexpr int NP = VB + SB;                // staged region points
+  static constexpr int NP = VB + 6 * TI;            // region points: vertical bar, then 3 W + 3 E columns per tile row
   static constexpr int FX = (TI + 1) * TJ;          // x faces (a * TJ + q)
   static constexpr int FY = TI * (TJ + 1);          // y faces (r * (TJ + 1) + q)
   static constexpr int C = TI * TJ;                 // cells (a * TJ + q)
   static constexpr int EW = TI > TJ ? TI : TJ;
-  // face cache block of a tile (words): the three x-face planes [3][FX], then the three y-face planes
-  // [3][FY], each part padded to 16 bytes (four words)
-  static constexpr int fXB = (3 * FX + 3) & ~3, fYB = (3 * FY + 3) & ~3, fW = fXB + fYB;
   static constexpr int NE = 4 * EW;                 // edge slots: 4 kinds x max(TI, TJ) positions
-  static constexpr int KV = (RI + NS - 1) / NS;     // row iterations over the vertical bar
-  static constexpr int KX = (TI + 1 + NS - 1) / NS; // over x-face rows
-  static constexpr int KC = (TI + NS - 1) / NS;     // over tile rows
-  // phase H (words): s_h [RI][RJ], s_uc [VB], s_vc [TI][RJ], s_g [NP][4], s_sn [NP],
-  // s_dzx/s_cdy [FX], s_dzy/s_ddx [FY], s_rda [C], neighbour lines; s_P [FX] and
-  // s_Q [FY] alias s_g (dead once the region is staged)
-  static constexpr int hH = 0, hUC = up4(hH + RI * RJ), hVC = up4(hUC + VB), hG = up4(hVC + TI * RJ),
-                       hSN = up4(hG + 4 * NP), hDZX = up4(hSN + NP), hCDY = up4(hDZX + FX),
-                       hDZY = up4(hCDY + FX), hDDX = up4(hDZY + FY), hRDA = up4(hDDX + FY),
-                       hNP = up4(hRDA + C), hNH = hNP + 6 * NE, hNDZ = hNH + 6 * NE, kWordsH = up4(hNDZ + NE);
-  static constexpr int hP = hG, hQ = hG + FX;
-  static_assert(FX + FY <= 4 * NP, "face fluxes must fit in the metric block they alias");
-  // phase UV (words): s_v [VB], s_u [TI][RJ], s_hn [RI][RJ], s_hb [RI][RJ] (stage h of
-  // the fb blend, RK3); the constants, contiguous [uG, uCEnd): cells g [C][4], sina, rda,
-  // rdx, rdy, a_f, x faces c_dy, y faces d_dx; then x faces cache [3][FX], kinetic energy,
-  // v_t * c_dy; y faces cache [3][FY], kinetic energy, u_t * d_dx
-  static constexpr int uV = 0, uU = up4(uV + VB), uHN = up4(uU + TI * RJ), uHB = up4(uHN + RI * RJ),
-                       uG = up4(uHB + RI * RJ),
-                       uSN = up4(uG + 4 * C), uRDA = uSN + C, uRDX = uRDA + C, uRDY = uRDX + C, uAF = uRDY + C,
-                       uCDY = up4(uAF + C), uDDX = up4(uCDY + FX), uCEnd = up4(uDDX + FY),
-                       uXC = uCEnd, uKU = up4(uXC + 3 * FX), uVX = up4(uKU + FX),
-                       uYC = up4(uVX + FX), uKV = up4(uYC + 3 * FY), uUY = up4(uKV + FY),
-                       kWordsUV = up4(uUY + FY);
-  static constexpr int uConstWords = uCEnd - uG;  // phase UV's constants of one tile
-  // tile constant block (words): phase UV's constant area image, then dzph_x of the x faces [FX]
-  // and dzph_y of the y faces [FY] (padded); plane offsets within the block
-  static constexpr int bSN = uSN - uG, bRDA = uRDA - uG, bCDY = uCDY - uG, bDDX = uDDX - uG,
-                       bDZX = uConstWords, bDZY = bDZX + FX, cW = bDZY + ((FY + 3) & ~3);
+  static constexpr int KP = (NP + kTileThreads - 1) / kTileThreads;  // region points per thread
+  static constexpr int KC = (C + kTileThreads - 1) / kTileThreads;   // cells per thread
+  // with one region point per thread its constants (metric, halo weights) are held in registers
+  // across the wait for the previous phase; with more they are staged in shared memory
+  static constexpr bool kHeld = KP == 1;
+  // tile constant block (words): cells rda, rdx, rdy, a_f [C] each; x faces c_dy, y faces d_dx, x
+  // faces dzph_x, y faces dzph_y
+  static constexpr int FXP = up4(FX), FYP = up4(FY);
+  static constexpr int bCDY = 4 * C, bDDX = bCDY + FXP, bDZX = bDDX + FYP, bDZY = bDZX + FXP, cW = bDZY + FYP;
+  // phase H (words): s_h [RI][RJ], contravariant s_uc [VB] / s_vc [TI][RJ], raw s_v [VB] /
+  // s_u [TI][RJ] (tangential reconstructions), face results x [4][FXP] and y [4][FYP] (sharing
+  // memory with the staged region metric s_g [NP][4], s_sn [NP], dead by then), the constant
+  // block, neighbour lines
+  static constexpr int kFaceWords = 4 * (FXP + FYP), kMetricWords = kHeld ? 0 : 5 * NP;
+  static constexpr int hH = 0, hUC = up4(hH + RI * RJ), hVC = up4(hUC + VB), hV = up4(hVC + TI * RJ),
+                       hU = up4(hV + VB), hFX = up4(hU + TI * RJ), hFY = hFX + 4 * FXP,
+                       hC = up4(hFX + (kFaceWords > kMetricWords ? kFaceWords : kMetricWords)), hNP = up4(hC + cW),
+                       hNH = hNP + 6 * NE, hNDZ = hNH + 6 * NE, kWordsH = up4(hNDZ + NE);
+  // phase UV (words): s_hn [RI][RJ], the (blended) new h of the region
+  static constexpr int kWordsUV = up4(RI * RJ);
 };
+
+// Momentum terms of a cell handed from phase H to phase UV, one block of
+// kTerms planes [TI][TJ] per tile.  float64 keeps the three terms of each
+// component apart, because the reference adds them to the pressure gradient one
+// by one (barotr_pure.py:149-150); float32 sums them.
+template <typename T>
+constexpr int kTerms = sizeof(T) == 8 ? 6 : 2;
 
 struct TileBox {
   int f, i0, j0, ni, nj;
+  int idx;  // number of the tile in face-major, row-major order
 };
 
-// Work order of the tiles: the tiles on the ring of each face's tile grid
-// (those touching a face edge: halo gathers and edge averages make them the
-// slowest) come first, the interior tiles after them, so that the long tiles
-// start in the first wave instead of finishing a launch alone (largest work
-// first).  Item b < 6 R (R = ring tiles of one face) is ring tile b % R of face
-// b / R; the rest are the interior tiles face by face.  Returns the tile's
-// face-major, row-major index.
-__device__ __forceinline__ int edge_first_tile(const Tiling& t, int b) {
-  const int nti = t.nti, ntj = t.ntj;
-  if (nti < 3 || ntj < 3) return b;  // every tile touches a face edge
-  const int R = 2 * ntj + 2 * (nti - 2);
-  int f, ti, tj;
-  if (b < 6 * R) {
-    f = b / R;
-    int r = b - f * R;
-    if (r < ntj) {
-      ti = 0;
-      tj = r;
-    } else if ((r -= ntj) < ntj) {
-      ti = nti - 1;
-      tj = r;
-    } else if ((r -= ntj) < nti - 2) {
-      ti = 1 + r;
-      tj = 0;
-    } else {
-      ti = 1 + r - (nti - 2);
-      tj = ntj - 1;
-    }
-  } else {
-    const int I = (nti - 2) * (ntj - 2), k = b - 6 * R;
-    f = k / I;
-    const int rr = k - f * I;
-    ti = 1 + rr / (ntj - 2);
-    tj = 1 + rr % (ntj - 2);
-  }
-  return (f * nti + ti) * ntj + tj;
+// a / b for 0 <= a < 2^24, b >= 1, without the integer division's long
+// sequence (the quotient by reciprocal is off by one at most).
+__device__ __forceinline__ int div24(int a, int b) {
+  int q = __float2int_rz(__int2float_rn(a) * __frcp_rn(__int2float_rn(b)));
+  const int r = a - q * b;
+  if (r < 0) --q;
+  if (r >= b) ++q;
+  return q;
 }
 
-// Tile number ``tile`` in face-major, row-major order.
-__device__ __forceinline__ TileBox tile_box_at(const Tiling& t, int n, int tile) {
+__device__ __forceinline__ TileBox tile_box_rc(const Tiling& t, int n, int f, int ti, int tj) {
   TileBox b;
-  const int per_face = t.nti * t.ntj;
-  b.f = tile / per_face;
-  const int r = tile - b.f * per_face;
-  const int ti = r / t.ntj, tj = r - ti * t.ntj;
+  b.f = f;
   b.i0 = kHalo + ti * t.ti;
   b.j0 = kHalo + tj * t.tj;
   b.ni = min(t.ti, n - ti * t.ti);
   b.nj = min(t.tj, n - tj * t.tj);
+  b.idx = (f * t.nti + ti) * t.ntj + tj;
   return b;
 }
 
+// Tile number ``tile`` in face-major, row-major order.
+__device__ __forceinline__ TileBox tile_box_at(const Tiling& t, int n, int tile) {
+  const int f = div24(tile, t.nti * t.ntj), r = tile - f * (t.nti * t.ntj), ti = div24(r, t.ntj);
+  return tile_box_rc(t, n, f, ti, r - ti * t.ntj);
+}
+
 // The tile that work item ``item`` (a CTA of a phase launch, or a step of a
-// persistent CTA's tile loop) computes, in edge_first_tile order.  The
-// batched phase kernels keep the face-major order instead (tile_box_at): with
-// many members in one launch the last wave is short anyway, and neighbouring
-// tiles running together share their halo rows in L2 (2.7 % faster there).
+// persistent CTA's tile loop) computes.  The tiles on the ring of each face's
+// tile grid (those touching a face edge: halo gathers and edge averages make
+// them the slowest) come first, the interior tiles after them, so that the
+// long tiles start in the first wave instead of finishing a launch alone
+// (largest work first); the faces take turns.  The batched phase kernels keep
+// the face-major order instead (tile_box_at): with many members in one launch
+// the last wave is short anyway, and neighbouring tiles running together share
+// their halo rows in L2 (2.7 % faster there).
 __device__ __forceinline__ TileBox tile_box(const Tiling& t, int n, int item) {
-  return tile_box_at(t, n, edge_first_tile(t, item));
+  const int nti = t.nti, ntj = t.ntj, f = item % 6;
+  int r = item / 6, ti, tj;
+  if (nti < 3 || ntj < 3) {  // every tile touches a face edge
+    ti = div24(r, ntj);
+    tj = r - ti * ntj;
+  } else if (r < ntj) {
+    ti = 0;
+    tj = r;
+  } else if ((r -= ntj) < ntj) {
+    ti = nti - 1;
+    tj = r;
+  } else if ((r -= ntj) < nti - 2) {
+    ti = 1 + r;
+    tj = 0;
+  } else if ((r -= nti - 2) < nti - 2) {
+    ti = 1 + r;
+    tj = ntj - 1;
+  } else {
+    r -= nti - 2;
+    const int k = div24(r, ntj - 2);
+    ti = 1 + k;
+    tj = 1 + r - k * (ntj - 2);
+  }
+  return tile_box_rc(t, n, f, ti, tj);
 }
 
 // A full interior tile: TI x TJ cells whose whole stencil region (3 cells
@@ -347,27 +332,6 @@ __device__ __forceinline__ bool tile_full(const TileBox& b, int m, int ti, int t
 
 // 32-bit offset of cell (i, j) of face f (fields of up to 2^31 elements).
 __device__ __forceinline__ int cell32(int f, int i, int j, int m) { return (f * m + i) * m + j; }
-
-// Row handled by this thread in the tile's east y-face column (faces at column
-// TJ of full-width tiles): lane r of the last warp.  With TI = 8k - 1 rows the
-// x-face rows (TI + 1) fill every warp evenly and the last warp has one tile
-// row fewer, so the extra column evens out the face work across the warps.
-__device__ __forceinline__ int east_row() { return (int)threadIdx.x - (kTileThreads - 32); }
-
-// Offset of a tile's face cache block (TileShape::fW words per tile, tiles in
-// face-major, row-major order).  Each tile writes every face it computes into
-// its own block (the faces it shares with the next tile are computed by both,
-// identically), so phase UV of a tile reads only its own block: one
-// contiguous range, loaded with 16-byte copies.
-template <int TI, int TJ>
-__device__ __forceinline__ int tile_index(const TileBox& b, int n) {
-  const int nti = (n + TI - 1) / TI, ntj = (n + TJ - 1) / TJ;
-  return (b.f * nti + (b.i0 - kHalo) / TI) * ntj + (b.j0 - kHalo) / TJ;
-}
-template <int TI, int TJ>
-__device__ __forceinline__ long face_block_off(const TileBox& b, int n) {
-  return (long)tile_index<TI, TJ>(b, n) * TileShape<TI, TJ>::fW;
-}
 
 // ---- asynchronous global -> shared copies ---------------------------------
 template <int BYTES>
@@ -425,22 +389,6 @@ __device__ __forceinline__ void ld_pair(const double* p, double& a, double& b) {
   b = v.y;
 }
 
-// ---- halo gathers in two steps (descriptor, then sources) ------------------
-template <typename T>
-struct Pull {
-  int2 s;
-  T w0, w1;
-};
-template <typename T>
-__device__ __forceinline__ Pull<T> pull_desc(const Geo<T>& g, int f, int i, int j) {
-  const int k = f * g.nh + halo_id(i, j, g.m);
-  Pull<T> p;
-  p.s = g.hsrc[k];
-  p.w0 = g.hw[2 * k];
-  p.w1 = g.hw[2 * k + 1];
-  return p;
-}
-
 // ---- the tile's face-edge positions ----------------------------------------
 // Item q of a tile's edge list: kind 0/1 = x faces of side S/N (position along
 // the tile's columns), kind 2/3 = y faces of side W/E (along the tile's rows).
@@ -483,272 +431,86 @@ __device__ __forceinline__ EdgeItem edge_item(const TileBox& b, const EdgeCnt& c
   return e;
 }
 
-// Work items of a tile that touches face edges, spread over the whole CTA:
-//   item t < 3P:  halo point at depth t % 3 outside edge position t / 3 of the
-//                 tile: its h and normal contravariant velocity (phase H), or
-//                 its raw tangential-reading velocity and new h (phase UV) --
-//                 read directly when the stored halo is valid, else gathered
-//                 from the neighbouring face;
-//   item t >= 3P: point q = (t - 3P) % 6 of the neighbour's 6-point line normal
-//                 to the shared edge at position (t - 3P) / 6: its contravariant
-//                 normal velocity (and h for the mass-flux average).
-// P is the number of edge positions of the tile.  Descriptor loads of all
-// items go out in a first sweep, source loads in a second, so a CTA waits for
-// two L2 round trips instead of one chain per point.
-struct ItemCell {
-  int f, i, j;      // cell whose value the item needs
-  int o;            // its offset within the member, cell32(f, i, j, m)
-  int kind;         // edge kind 0..3 (S, N, W, E)
-  int r, c;         // region row / column (region items)
-  int slot;         // line item: edge slot * 6 + q
-  int line, y, q;   // line item: 1, normal axis (1 = y), point index
-};
+// ---- halo values from the bands ---------------------------------------------
+// Band order: cell k along side s of face f, line c (0..2, increasing i or j)
+// has number ((f * 4 + s) * 3 + c) * n + k, for the halo cells outside the side
+// and for the interior cells inside it alike.
+__device__ __forceinline__ int band_no(int f, int s, int c, int k, int n) { return ((f * 4 + s) * 3 + c) * n + k; }
 
-// Shared-memory words (ints) past a phase's layout where each thread keeps
-// its first gather item, decoded in the prologue: the offset o at [t] and the
-// other fields the item needs at [kTileThreads + t], packed as
-// r | c << 6 | slot << 12 | line << 22 | kind << 23 | y << 25 | (q == 3) << 26.
-// Only the writing thread reads them back (after the grid dependency), so the
-// decode's cold code stays off the critical path without holding registers.
-constexpr int kItemWords = 2 * kTileThreads;
-__device__ __forceinline__ int pack_item(const ItemCell& c) {
-  return c.r | (c.c << 6) | (c.slot << 12) | (c.line << 22) | (c.kind << 23) | (c.y << 25) | ((c.q == 3) << 26);
-}
-__device__ __forceinline__ ItemCell unpack_item(int o, int pk) {
-  ItemCell c;
-  c.f = c.i = c.j = 0;  // not needed past the descriptor sweep
-  c.o = o;
-  c.r = pk & 63;
-  c.c = (pk >> 6) & 63;
-  c.slot = (pk >> 12) & 1023;
-  c.line = (pk >> 22) & 1;
-  c.kind = (pk >> 23) & 3;
-  c.y = (pk >> 25) & 1;
-  c.q = ((pk >> 26) & 1) ? 3 : 0;
-  return c;
-}
-
-__device__ __forceinline__ ItemCell decode_item(const TileBox& b, const EdgeCnt& cnt, int P, int t, int m, int n,
-                                                int EW) {
-  ItemCell c;
-  if (t < 3 * P) {
-    const EdgeItem e = edge_item(b, cnt, t / 3);
-    const int d = t % 3;
-    int r, cc;
-    switch (e.kind) {
-      case 0: r = d; cc = e.pos + kHalo; break;                  // S: region rows 0..2
-      case 1: r = b.ni + kHalo + d; cc = e.pos + kHalo; break;   // N: rows ni+3..ni+5
-      case 2: r = e.pos + kHalo; cc = d; break;                  // W: region cols 0..2
-      default: r = e.pos + kHalo; cc = b.nj + kHalo + d; break;  // E: cols nj+3..nj+5
+// A point of a face by its coordinates: interior, or line c, position k of the
+// halo band outside ``side`` (the corner blocks are never asked for).
+struct PointKind {
+  int side, c, k;  // side -1: interior
+  __device__ __forceinline__ PointKind(int i, int j, int m) {
+    side = -1;
+    c = k = 0;
+    if (i < kHalo) {
+      side = kS;
+      c = i;
+      k = j - kHalo;
+    } else if (i >= m - kHalo) {
+      side = kN;
+      c = i - (m - kHalo);
+      k = j - kHalo;
+    } else if (j < kHalo) {
+      side = kW;
+      c = j;
+      k = i - kHalo;
+    } else if (j >= m - kHalo) {
+      side = kE;
+      c = j - (m - kHalo);
+      k = i - kHalo;
     }
-    c.f = b.f;
-    c.i = b.i0 - kHalo + r;
-    c.j = b.j0 - kHalo + cc;
-    c.o = cell32(c.f, c.i, c.j, m);
-    c.kind = e.kind;
-    c.r = r;
-    c.c = cc;
-    c.slot = 0;
-    c.line = 0;
-    c.y = 0;
-    c.q = 0;
-  } else {
-    const int t2 = t - 3 * P;
-    const EdgeItem e = edge_item(b, cnt, t2 / 6);
-    const int q = t2 % 6;
-    const int r = (cnt.routes >> (8 * e.kind)) & 0xff;
-    const int ns = route_side(r);
-    const int kk = route_rev(r) ? n - 1 - e.k : e.k;
-    c.f = route_nb(r);
-    edge_point(ns, kk, q, m, c.i, c.j);
-    c.o = cell32(c.f, c.i, c.j, m);
-    c.kind = e.kind;
-    c.r = 0;
-    c.c = 0;
-    c.slot = (e.kind * EW + e.pos) * 6 + q;
-    c.line = 1;
-    c.y = (ns == kE || ns == kW);
-    c.q = q;
   }
-  return c;
-}
-
-// Shared-memory destinations of the gather items of one phase.
-template <typename T>
-struct GatherSink {
-  T* h;    // H: region h [RI][RJ]        UV: blended new h [RI][RJ]
-  T* vb;   // H: s_uc [VB]                UV: raw v [VB]
-  T* hb;   // H: s_vc [TI][RJ]            UV: raw u [TI][RJ]
-  T* np;   // H: neighbour lines (contravariant normal velocity, h, depth)
-  T* nh;
-  T* ndz;
-  // tile-resident round only (RES): phase H also leaves the raw velocities of
-  // the region halo in phase UV's arrays, and phase UV blends with the stage
-  // h phase H staged
-  T* rv = nullptr;        // H: phase UV's raw v [VB]
-  T* ru = nullptr;        // H: phase UV's raw u [TI][RJ]
-  const T* hs = nullptr;  // UV: phase H's region h [RI][RJ]
 };
 
-// Shared-memory pointers of the tile-resident round kernel: phase H and phase
-// UV keep separate layouts, so constants and the face cache stay in place
-// for the whole round.
+// The two band cells and weights a halo cell is interpolated from (cube.py:40-127).
+template <typename T>
+struct HaloRef {
+  int b0, d;  // the second source is number b0 + d (added at use: the first is still in flight here)
+  T w0, w1;
+  __device__ __forceinline__ void load(const Geo<T>& g, int f, int side, int c, int k) {
+    b0 = g.bsrc[band_no(f, side, c, k, g.n)];
+    d = route_rev(g.route[f * 4 + side]) ? -1 : 1;  // the next along our edge
+    const int id = side == kS   ? c * g.m + kHalo + k
+                   : side == kN ? (3 + c) * g.m + kHalo + k
+                                : 6 * g.m + (side == kE ? 3 * g.n : 0) + 3 * k + c;
+    ld_pair(g.hw + 2 * (f * g.nh + id), w0, w1);
+  }
+  __device__ __forceinline__ T lerp(const T* band) const { return w0 * band[b0] + w1 * band[b0 + d]; }
+};
+
+// Halo velocity (ext_vector, cube.py:137-153) from the bands' lon/lat velocity
+// and the target's l2c.
+template <typename T>
+__device__ __forceinline__ void halo_uv(const StageIO<T>& io, const HaloRef<T>& r, int plane, const T* l2, T& u, T& v) {
+  const T ull = r.lerp(io.band_uv), vll = r.lerp(io.band_uv + plane);
+  u = l2[0] * ull + l2[1] * vll;
+  v = l2[2] * ull + l2[3] * vll;
+}
+
+// Words of one band plane.
+__host__ __device__ __forceinline__ int band_plane(int n) { return 72 * n; }
+
+// Whether a cell lies on one of the three lines next to a side of its face.
+__device__ __forceinline__ bool in_bands(int i, int j, int n) {
+  return min(i, j) < 2 * kHalo || max(i, j) >= n;
+}
+
+// Run fn(side, band number) for every side whose three interior lines hold cell (i, j) of face f.
+template <typename F>
+__device__ __forceinline__ void for_bands(int f, int i, int j, int n, F fn) {
+  const int a = i - kHalo, b = j - kHalo;
+  if (a < kHalo) fn((int)kS, band_no(f, kS, a, b, n));
+  if (a >= n - kHalo) fn((int)kN, band_no(f, kN, a - (n - kHalo), b, n));
+  if (b < kHalo) fn((int)kW, band_no(f, kW, b, a, n));
+  if (b >= n - kHalo) fn((int)kE, band_no(f, kE, b - (n - kHalo), a, n));
+}
+
+// Shared-memory pointers of the tile-resident round kernel.
 template <typename T>
 struct ResSm {
-  T* uv;      // phase UV layout (constants, face cache, raw velocities of the stage)
-  T* pq;      // phase H face fluxes [FX + FY] (alias the metric block otherwise)
-  T* hs;      // phase H region h [RI][RJ]: the stage h of the fb blend in phase UV
-  int* items; // gather item scratch (kItemWords)
-};
-
-template <typename T, int TI, int TJ, bool UV, bool RES = false>
-struct Gather {
-  using S = TileShape<TI, TJ>;
-  // phase H gathers the region halo and the neighbour edge lines (9 items per
-  // edge position); phase UV only the region halo (3 per position)
-  static constexpr int kPerPos = UV ? 3 : 9;
-  Pull<T> pd;  // descriptor of the thread's first item
-  bool pl;
-
-  __device__ __forceinline__ static bool needs_pull(const StageIO<T>& io, const ItemCell& c, int m) {
-    return !is_interior(c.i, c.j, m) && (!io.stored_halo || (UV && !c.line));
-  }
-
-  // sweep 1: the descriptor of the thread's first item (constants, may
-  // precede the grid dependency)
-  __device__ __forceinline__ void descriptors(const Geo<T>& g, const StageIO<T>& io, const TileBox& b,
-                                              const EdgeCnt& cnt, int P, int* s_items) {
-    pl = false;
-    pd.s = make_int2(0, 0);
-    pd.w0 = pd.w1 = T(0.0);
-    if ((int)threadIdx.x < kPerPos * P) {
-      const ItemCell c = decode_item(b, cnt, P, threadIdx.x, g.m, g.n, S::EW);
-      s_items[threadIdx.x] = c.o;
-      s_items[kTileThreads + threadIdx.x] = pack_item(c);
-      if (needs_pull(io, c, g.m)) {
-        pd = pull_desc(g, c.f, c.i, c.j);
-        pl = true;
-      }
-    }
-  }
-
-  // One item.  Every lane issues the same loads whatever its item's kind --
-  // the two sources of an interpolated halo value, or the cell itself twice
-  // for a direct read -- so a warp mixing kinds waits for one memory round
-  // trip, not one per kind; the results are selected afterwards (a direct
-  // read stays exact), and all loads precede the item's shared-memory stores.
-  __device__ __forceinline__ void one(const Geo<T>& g, const StageIO<T>& io, const ItemCell& c, const Pull<T>& p,
-                                      bool pull, const GatherSink<T>& k) {
-    if constexpr (UV && RES) {
-      // resident phase UV: the raw velocities and the stage h of the halo
-      // point were staged by phase H; only the new h is interpolated here
-      T hn = p.w0 * ((const T*)io.h_out)[p.s.x] + p.w1 * ((const T*)io.h_out)[p.s.y];
-      const int e = c.r * S::RJ + c.c;
-      if (io.beta != T(0.0)) hn = (T(1.0) - io.beta) * hn + io.beta * k.hs[e];  // fb_scheme
-      k.h[e] = hn;
-      return;
-    }
-    const int o = c.o;
-    const bool vpull = UV ? !io.stored_halo : pull;  // velocity interpolated (else read directly)
-    const int sa = vpull ? p.s.x : o, sb = vpull ? p.s.y : o;
-    const T ua = io.u[sa], va = io.v[sa], ub = io.u[sb], vb = io.v[sb];
-    T c0[4], c1[4], l2[4];
-    ld_quad(g.c2l + 4 * (long)sa, c0);
-    ld_quad(g.c2l + 4 * (long)sb, c1);
-    ld_quad(g.l2c + 4 * (long)o, l2);
-    if (!UV) {
-      const bool want_h = !c.line || io.last;  // region h, or the neighbour h of the mass-flux average
-      T ha = T(0.0), hb = T(0.0), dz = T(0.0);
-      if (want_h) {
-        ha = io.h[sa];
-        hb = io.h[sb];
-      }
-      const bool yaxis = c.line ? c.y : c.kind >= 2;  // contravariant component normal to the faces read
-      T g0, g1;
-      ld_pair(g.gct + 4 * (long)o + (yaxis ? 2 : 0), g0, g1);
-      const T sn = g.sina[o];
-      if (c.line && want_h && c.q == 3) dz = (c.y ? g.dzph_y : g.dzph_x)[o];
-      T u = ua, v = va, h = ha;
-      if (vpull) {  // ext_vector / ext_scalar, cube.py:130-153
-        const T ull0 = c0[0] * ua + c0[1] * va, vll0 = c0[2] * ua + c0[3] * va;
-        const T ull1 = c1[0] * ub + c1[1] * vb, vll1 = c1[2] * ub + c1[3] * vb;
-        const T ull = p.w0 * ull0 + p.w1 * ull1;
-        const T vll = p.w0 * vll0 + p.w1 * vll1;
-        u = l2[0] * ull + l2[1] * vll;
-        v = l2[2] * ull + l2[3] * vll;
-        h = p.w0 * ha + p.w1 * hb;
-      }
-      const T ct = (g0 * u + g1 * v) * sn;  // remap.py:34-39
-      if (!c.line) {
-        k.h[c.r * S::RJ + c.c] = h;
-        if (c.kind < 2)  // S/N halo rows belong to the vertical bar
-          k.vb[c.r * TJ + (c.c - kHalo)] = ct;
-        else
-          k.hb[(c.r - kHalo) * S::RJ + c.c] = ct;
-        if constexpr (RES) {  // phase UV's raw (tangential-reading) velocity at the same point
-          if (c.kind < 2)
-            k.rv[c.r * TJ + (c.c - kHalo)] = v;
-          else
-            k.ru[(c.r - kHalo) * S::RJ + c.c] = u;
-        }
-      } else {
-        k.np[c.slot] = ct;
-        if (want_h) {
-          k.nh[c.slot] = h;
-          if (c.q == 3) k.ndz[c.slot / 6] = dz;
-        }
-      }
-    } else {  // region items only; the new h never has a stored halo
-      const bool blend = io.beta != T(0.0);
-      const T n0 = ((const T*)io.h_out)[p.s.x], n1 = ((const T*)io.h_out)[p.s.y];
-      T ba = T(0.0), bb = T(0.0);
-      if (blend) {
-        ba = io.h[sa];
-        bb = io.h[sb];
-      }
-      T u = ua, v = va, h = ba;
-      if (vpull) {
-        const T ull0 = c0[0] * ua + c0[1] * va, vll0 = c0[2] * ua + c0[3] * va;
-        const T ull1 = c1[0] * ub + c1[1] * vb, vll1 = c1[2] * ub + c1[3] * vb;
-        const T ull = p.w0 * ull0 + p.w1 * ull1;
-        const T vll = p.w0 * vll0 + p.w1 * vll1;
-        u = l2[0] * ull + l2[1] * vll;
-        v = l2[2] * ull + l2[3] * vll;
-        h = p.w0 * ba + p.w1 * bb;
-      }
-      T hn = p.w0 * n0 + p.w1 * n1;
-      if (blend) hn = (T(1.0) - io.beta) * hn + io.beta * h;  // fb_scheme, barotr_pure.py:52-54
-      k.h[c.r * S::RJ + c.c] = hn;
-      if (c.kind < 2)
-        k.vb[c.r * TJ + (c.c - kHalo)] = v;
-      else
-        k.hb[(c.r - kHalo) * S::RJ + c.c] = u;
-    }
-  }
-
-  // sweep 2: sources (state, after the grid dependency) and the items'
-  // values.  One rolled loop, so the item code exists once in the kernel (the
-  // edge path is cold code: at small sizes each CTA runs it once and waits on
-  // instruction fetch); items past the first of a thread (tiles with more than
-  // kTileThreads items) load their descriptor here.
-  __device__ __forceinline__ void sources(const Geo<T>& g, const StageIO<T>& io, const TileBox& b,
-                                          const EdgeCnt& cnt, int P, const GatherSink<T>& k, const int* s_items) {
-    const int nitems = kPerPos * P;
-#pragma unroll 1
-    for (int t = threadIdx.x; t < nitems; t += kTileThreads) {
-      bool pull = pl;
-      Pull<T> p = pd;
-      ItemCell c;
-      if (t < kTileThreads) {
-        c = unpack_item(s_items[t], s_items[kTileThreads + t]);
-      } else {
-        c = decode_item(b, cnt, P, t, g.m, g.n, S::EW);
-        pull = needs_pull(io, c, g.m);
-        if (pull) p = pull_desc(g, c.f, c.i, c.j);
-      }
-      one(g, io, c, p, pull, k);
-    }
-  }
+  T* terms;  // momentum terms [kTerms][TI][TJ]
 };
 
 // Normal velocity of the neighbour's line (6 contravariant values) before averaging.
@@ -790,237 +552,164 @@ __device__ __forceinline__ void celerity_coef(T hface, T dz, T& c, T& coef) {
   }
 }
 
-// Region points a thread stages itself: interior points, and halo points that
-// no gather item covers -- the halo rows (columns) that the region of a tile
-// next to a tile thinner than 3 cells reaches without the tile touching that
-// face edge; those are fetched point by point.
-struct EdgeCover {
-  bool s, n, w, e;  // the tile touches face edge S / N / W / E (its halo points there are gather items)
-  __device__ __forceinline__ EdgeCover(const TileBox& b, int m)
-      : s(b.i0 == kHalo), n(b.i0 + b.ni == m - kHalo), w(b.j0 == kHalo), e(b.j0 + b.nj == m - kHalo) {}
-  __device__ __forceinline__ bool row_staged(int i, int m) const {
-    return !((i < kHalo && s) || (i >= m - kHalo && n));
-  }
-  __device__ __forceinline__ bool col_staged(int j, int m) const {
-    return !((j < kHalo && w) || (j >= m - kHalo && e));
-  }
-};
-
 // ---- phase H ----------------------------------------------------------------
 template <typename T, int TI, int TJ>
 struct LayoutH {
   using S = TileShape<TI, TJ>;
-  T *s_h, *s_uc, *s_vc, *s_g, *s_sn, *s_dzx, *s_cdy, *s_dzy, *s_ddx, *s_rda, *s_P, *s_Q, *s_np, *s_nh, *s_ndz;
+  T *s_h, *s_uc, *s_vc, *s_v, *s_u, *s_g, *s_sn, *s_fx, *s_fy, *s_cell, *s_cdy, *s_ddx, *s_dzx, *s_dzy, *s_np, *s_nh,
+      *s_ndz;
   __device__ __forceinline__ explicit LayoutH(T* sm) {
     s_h = sm + S::hH;
     s_uc = sm + S::hUC;
     s_vc = sm + S::hVC;
-    s_g = sm + S::hG;
-    s_sn = sm + S::hSN;
-    s_dzx = sm + S::hDZX;
-    s_cdy = sm + S::hCDY;
-    s_dzy = sm + S::hDZY;
-    s_ddx = sm + S::hDDX;
-    s_rda = sm + S::hRDA;
-    s_P = sm + S::hP;
-    s_Q = sm + S::hQ;
+    s_v = sm + S::hV;
+    s_u = sm + S::hU;
+    s_g = sm + S::hFX;
+    s_sn = s_g + 4 * S::NP;
+    s_fx = sm + S::hFX;
+    s_fy = sm + S::hFY;
+    s_cell = sm + S::hC;
+    s_cdy = s_cell + S::bCDY;
+    s_ddx = s_cell + S::bDDX;
+    s_dzx = s_cell + S::bDZX;
+    s_dzy = s_cell + S::bDZY;
     s_np = sm + S::hNP;
     s_nh = sm + S::hNH;
     s_ndz = sm + S::hNDZ;
   }
 };
 
-template <typename T, int TI, int TJ>
-struct LayoutUV {
-  using S = TileShape<TI, TJ>;
-  T *s_v, *s_u, *s_hn, *s_hb, *s_g, *s_sn, *s_rda, *s_rdx, *s_rdy, *s_af, *s_xc, *s_cdy, *s_ku, *s_vx, *s_yc,
-      *s_ddx, *s_kv, *s_uy;
-  __device__ __forceinline__ explicit LayoutUV(T* sm) {
-    s_v = sm + S::uV;
-    s_u = sm + S::uU;
-    s_hn = sm + S::uHN;
-    s_hb = sm + S::uHB;
-    s_g = sm + S::uG;
-    s_sn = sm + S::uSN;
-    s_rda = sm + S::uRDA;
-    s_rdx = sm + S::uRDX;
-    s_rdy = sm + S::uRDY;
-    s_af = sm + S::uAF;
-    s_xc = sm + S::uXC;
-    s_cdy = sm + S::uCDY;
-    s_ku = sm + S::uKU;
-    s_vx = sm + S::uVX;
-    s_yc = sm + S::uYC;
-    s_ddx = sm + S::uDDX;
-    s_kv = sm + S::uKV;
-    s_uy = sm + S::uUY;
+// Region point number p of a tile: region row r and column c, and whether the
+// tile has it (partial tiles).
+template <int TI, int TJ, bool FULL>
+struct RegionPoint {
+  int r, c;
+  bool on, vbar, hbar;  // on the vertical bar (tile columns) / horizontal bar (tile rows)
+  __device__ __forceinline__ RegionPoint(const TileBox& b, int p) {
+    using S = TileShape<TI, TJ>;
+    const int ni = FULL ? TI : b.ni, nj = FULL ? TJ : b.nj;
+    if (p < S::VB) {
+      r = p / TJ;
+      c = p % TJ + kHalo;
+      vbar = true;
+      hbar = r >= kHalo && r < ni + kHalo;
+      on = r < ni + 6 && c < nj + kHalo;
+    } else {
+      const int s = p - S::VB, a = s / 6, d = s - 6 * a;
+      r = a + kHalo;
+      c = d < 3 ? d : nj + d;
+      vbar = false;
+      hbar = true;
+      on = a < ni;
+    }
   }
 };
 
-// 16-byte copies of ``words`` words (a multiple of 16 bytes) from global src to shared dst.
-template <typename T, int WORDS>
-__device__ __forceinline__ void cp_async_run(T* dst, const T* src) {
-  constexpr int V = 16 / sizeof(T);
-  static_assert(WORDS % V == 0, "runs of whole 16-byte chunks");
-#pragma unroll
-  for (int w = threadIdx.x * V; w < WORDS; w += kTileThreads * V) cp_async<16>(dst + w, src + w);
-}
+// Depth d (0..2) of the neighbour's lines normal to the shared edge: a line has
+// six points at edge position e of the tile, three inside the neighbouring face
+// nb (line d inside its side ns) and three in its halo (line d outside), at
+// position kk along that side; slots of the two points in the tile's line
+// arrays, and which of them is the first point past the edge face (the depth
+// is read there).
+struct LinePoint {
+  int nb, ns, kk, d, slot_in, slot_out;
+  bool low, y;  // low: the halo points come first; y: the lines run along axis -1
+  __device__ __forceinline__ LinePoint(const TileBox& b, const EdgeCnt& cnt, int P, int t, int n, int EW) {
+    d = div24(t, P);
+    const EdgeItem e = edge_item(b, cnt, t - d * P);
+    const int r = (cnt.routes >> (8 * e.kind)) & 0xff;
+    nb = route_nb(r);
+    ns = route_side(r);
+    kk = route_rev(r) ? n - 1 - e.k : e.k;
+    low = ns == kS || ns == kW;
+    y = ns == kE || ns == kW;
+    const int base = (e.kind * EW + e.pos) * 6;
+    slot_in = base + (low ? 3 + d : d);
+    slot_out = base + (low ? d : 3 + d);
+  }
+  __device__ __forceinline__ int offset(bool out, int m) const {  // cell offset of the halo / inside point
+    int i, j;
+    edge_point(ns, kk, out == low ? d : 3 + d, m, i, j);
+    return cell32(nb, i, j, m);
+  }
+};
 
-// Phase H constants of a full interior tile from the tile constant blocks: the
-// region metric (vertical bar: 3 rows of the tile above, the tile's own rows, 3
-// rows of the tile below; side points: 3 columns of the tiles left and right --
-// all four exist on the same face for a full tile and hold at least 3 rows /
-// columns) and the tile's own face and cell constants, in 16-byte copies.
-template <typename T, int TI, int TJ>
-__device__ __forceinline__ void tile_h_consts_blocks(const Geo<T>& g, const TileBox& b, T* sm) {
-  using S = TileShape<TI, TJ>;
-  const LayoutH<T, TI, TJ> L(sm);
-  const int ntj = (g.n + TJ - 1) / TJ;
-  const T* own = g.cblk + (long)tile_index<TI, TJ>(b, g.n) * S::cW;
-  const T* above = own - (long)ntj * S::cW;
-  const T* below = own + (long)ntj * S::cW;
-  const T* left = own - S::cW;
-  const T* right = own + S::cW;
-  cp_async_run<T, 4 * 3 * TJ>(L.s_g, above + 4 * (TI - 3) * TJ);
-  cp_async_run<T, 4 * TI * TJ>(L.s_g + 4 * 3 * TJ, own);
-  cp_async_run<T, 4 * 3 * TJ>(L.s_g + 4 * (TI + 3) * TJ, below);
-  cp_async_run<T, 3 * TJ>(L.s_sn, above + S::bSN + (TI - 3) * TJ);
-  cp_async_run<T, TI * TJ>(L.s_sn + 3 * TJ, own + S::bSN);
-  cp_async_run<T, 3 * TJ>(L.s_sn + (TI + 3) * TJ, below + S::bSN);
-  if (threadIdx.x < 6 * TI) {  // side point (r, c): columns TJ-3.. of the left tile, 0..2 of the right one
-    const int t = threadIdx.x, r = t / 6, c = t - 6 * r;
-    const T* nb = c < 3 ? left : right;
-    const int e = c < 3 ? r * TJ + TJ - 3 + c : r * TJ + c - 3;  // the cell within the neighbour's block
-    cp_async_mat(L.s_g + 4 * (S::VB + t), nb + 4 * e);            // metric plane first, 4 words per cell
-    cp_async_t(L.s_sn + S::VB + t, nb + S::bSN + e);
-  }
-  cp_async_run<T, S::C>(L.s_rda, own + S::bRDA);
-  cp_async_run<T, S::FX>(L.s_cdy, own + S::bCDY);
-  cp_async_run<T, S::FX>(L.s_dzx, own + S::bDZX);
-  cp_async_run<T, (S::FY + 3) & ~3>(L.s_ddx, own + S::bDDX);
-  cp_async_run<T, (S::FY + 3) & ~3>(L.s_dzy, own + S::bDZY);
-}
-
-// Phase H constants of the tile (cp.async, not yet awaited).
-template <typename T, int TI, int TJ, bool FULL>
-__device__ __forceinline__ void tile_h_consts(const Geo<T>& g, const TileBox& b, T* sm) {
-  using S = TileShape<TI, TJ>;
-  if (FULL && g.cblk != nullptr && g.cblk_ti == TI && g.cblk_tj == TJ) {
-    tile_h_consts_blocks<T, TI, TJ>(g, b, sm);
-    return;
-  }
-  const LayoutH<T, TI, TJ> L(sm);
-  const int m = g.m, q = threadIdx.x % TJ, sl = threadIdx.x / TJ;
-  const int ni = FULL ? TI : b.ni, nj = FULL ? TJ : b.nj;
-  // region metric (halo points of edge tiles are also read by the gather items, from global memory)
-  if (q < nj) {
-    const int o0 = cell32(b.f, b.i0 - kHalo, b.j0 + q, m);
-#pragma unroll
-    for (int k = 0; k < S::KV; ++k) {
-      const int r = sl + k * S::NS;
-      if (r < ni + 6) {
-        const int o = o0 + r * m, p = r * TJ + q;
-        cp_async_mat(L.s_g + 4 * p, g.gct + 4 * (long)o);
-        cp_async_t(L.s_sn + p, g.sina + o);
-      }
-    }
-  }
-  if (threadIdx.x < 6 * ni) {
-    const int t = threadIdx.x, r = t / 6, c = t - 6 * r, cc = c < 3 ? c : nj + c;
-    const int o = cell32(b.f, b.i0 + r, b.j0 - kHalo + cc, m), p = S::VB + t;
-    cp_async_mat(L.s_g + 4 * p, g.gct + 4 * (long)o);
-    cp_async_t(L.s_sn + p, g.sina + o);
-  }
-  // face and cell constants
-  if (q < nj) {
-    const int o0 = cell32(b.f, b.i0, b.j0 + q, m);
-#pragma unroll
-    for (int k = 0; k < S::KX; ++k) {
-      const int a = sl + k * S::NS;
-      if (a <= ni) {
-        cp_async_t(L.s_dzx + a * TJ + q, g.dzph_x + o0 + a * m);
-        cp_async_t(L.s_cdy + a * TJ + q, g.c_dy + o0 + a * m);
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < S::KC; ++k) {
-      const int a = sl + k * S::NS;
-      if (a < ni) cp_async_t(L.s_rda + a * TJ + q, g.rda + o0 + a * m);
-    }
-  }
-  if (q <= nj) {
-    const int o0 = cell32(b.f, b.i0, b.j0 + q, m);
-#pragma unroll
-    for (int k = 0; k < S::KC; ++k) {
-      const int r = sl + k * S::NS;
-      if (r < ni) {
-        cp_async_t(L.s_dzy + r * (TJ + 1) + q, g.dzph_y + o0 + r * m);
-        cp_async_t(L.s_ddx + r * (TJ + 1) + q, g.d_dx + o0 + r * m);
-      }
-    }
-  }
-  if (nj == TJ && east_row() >= 0 && east_row() < ni) {  // the last y-face column of full-width tiles
-    const int r = east_row(), o = cell32(b.f, b.i0 + r, b.j0 + TJ, m);
-    cp_async_t(L.s_dzy + r * (TJ + 1) + TJ, g.dzph_y + o);
-    cp_async_t(L.s_ddx + r * (TJ + 1) + TJ, g.d_dx + o);
-  }
-}
-
-// Halo-gather descriptors of a tile phase (edge tiles; P = 0 for full tiles).
-template <typename T, int TI, int TJ, bool FULL, bool UV, bool RES>
-__device__ __forceinline__ void tile_desc(const Geo<T>& g, const StageIO<T>& io, const TileBox& b,
-                                          Gather<T, TI, TJ, UV, RES>& gat, EdgeCnt& cnt, int& P, int* items) {
-  if (FULL) {
-    P = 0;
-  } else {
-    P = edge_count(b, g.m, g.route, cnt);
-    if (P > 0) gat.descriptors(g, io, b, cnt, P, items);
-  }
-}
-
-// Phase H prologue: constants of the tile (cp.async, not yet awaited) and the
-// halo-gather descriptors.  Independent of the state, so it may run before the
-// previous phase has finished (programmatic launch, or before a grid barrier).
-template <typename T, int TI, int TJ, bool FULL>
-__device__ __forceinline__ void tile_h_pro_t(const Geo<T>& g, const StageIO<T>& io, const TileBox& b, T* sm,
-                                             Gather<T, TI, TJ, false>& gat, EdgeCnt& cnt, int& P) {
-  using S = TileShape<TI, TJ>;
-  tile_h_consts<T, TI, TJ, FULL>(g, b, sm);
-  tile_desc<T, TI, TJ, FULL, false, false>(g, io, b, gat, cnt, P, reinterpret_cast<int*>(sm + S::kWordsH));
-}
-
-// The neighbour's side of every edge face of a tile, from its gathered 6-point
-// lines (slot = edge kind x EW + position): its raw C-grid normal velocity
-// (line_raw) replaces the line's first velocity value and, on the last stage,
-// its reconstructed face h values and celerity viscosity coefficient replace
-// the line's first three h values.  Run between the staging barriers, one edge
-// position per thread counted from the CTA's last thread (the threads with the
-// fewest region points), so that the face pass of an edge face carries one
-// square root and division chain instead of two.  float64 only: measured on a
-// B200 it shortens the float64 round (C96 16.60 -> 16.15 us per substep, C384
-// 160.3 -> 157.9) and lengthens the float32 one (C384 69.1 -> 70.7, C768
-// 293.5 -> 313.4), whose face chains are short and whose extra staging pass
-// costs more than it saves.
+// Constants of one halo value: its two sources and l2c, and for a line's halo
+// point the metric row along the line.
 template <typename T>
-__host__ __device__ constexpr bool edge_lines_staged() { return sizeof(T) == 8; }
+struct HaloWork {
+  HaloRef<T> ref;
+  T l2[4], g0, g1, sn;
+  __device__ __forceinline__ void line_constants(const Geo<T>& g, const LinePoint& p) {
+    const int o = p.offset(true, g.m);
+    ld_quad(g.l2c + 4 * (long)o, l2);
+    ld_pair(g.gct + 4 * (long)o + (p.y ? 2 : 0), g0, g1);
+    sn = g.sina[o];
+  }
+};
 
+// The lines' inside points (and depths) of an edge tile, line point t: the
+// contravariant velocity along the line and, on the last stage, h come from the
+// neighbour's bands as they are (cp.async).
+template <typename T, int TI, int TJ>
+__device__ __forceinline__ void line_inside(const Geo<T>& g, const StageIO<T>& io, const LinePoint& p,
+                                            const LayoutH<T, TI, TJ>& L) {
+  const int e = band_no(p.nb, p.ns, p.d, p.kk, g.n);
+  cp_async_t(L.s_np + p.slot_in, (const T*)io.band_uv + 2 * band_plane(g.n) + e);
+  if (io.last) cp_async_t(L.s_nh + p.slot_in, io.band_h + e);
+}
+template <typename T, int TI, int TJ>
+__device__ __forceinline__ void line_depth(const Geo<T>& g, const LinePoint& p, const LayoutH<T, TI, TJ>& L) {
+  if (p.d == 0) {  // point 3 of the line: the first past the edge face
+    const int slot = (p.slot_in < p.slot_out ? p.slot_in : p.slot_out) / 6;
+    cp_async_t(L.s_ndz + slot, (p.y ? g.dzph_y : g.dzph_x) + p.offset(!p.low, g.m));
+  }
+}
+// The lines' halo points: line point t, its value gathered like a halo point's.
+template <typename T, int TI, int TJ>
+__device__ __forceinline__ void line_outside(const StageIO<T>& io, int slot, const HaloWork<T>& w, int plane,
+                                             const LayoutH<T, TI, TJ>& L) {
+  T u, v;
+  halo_uv(io, w.ref, plane, w.l2, u, v);
+  L.s_np[slot] = (w.g0 * u + w.g1 * v) * w.sn;  // remap.py:34-39
+  if (io.last) L.s_nh[slot] = w.ref.lerp(io.band_h);
+}
+// Both points of a line read directly (first stage of a round: the halo cells are stored).
+template <typename T, int TI, int TJ>
+__device__ __forceinline__ void line_stored(const Geo<T>& g, const StageIO<T>& io, const LinePoint& p,
+                                            const LayoutH<T, TI, TJ>& L) {
+#pragma unroll 1
+  for (int k = 0; k < 2; ++k) {
+    const int o = p.offset(k != 0, g.m), slot = k ? p.slot_out : p.slot_in;
+    L.s_np[slot] = contra(g, (long)o, io.u[o], io.v[o], p.y);
+    if (io.last) L.s_nh[slot] = io.h[o];
+  }
+}
+
+// On the last stage the mass flux of an edge face is averaged with the
+// neighbour's: from the gathered 6-point lines (slot = edge kind x EW +
+// position) the neighbour's reconstructed face h values and celerity viscosity
+// coefficient replace the line's first three h values, and its raw C-grid
+// normal velocity (line_raw) the first velocity value.  Run between two
+// barriers, one edge position per thread, so that the face pass of an edge
+// face carries one square root and division chain instead of two; on the other
+// stages the face pass forms line_raw itself and the extra barrier is saved.
 template <typename T, int EW>
-__device__ __forceinline__ void edge_lines(const StageIO<T>& io, const TileBox& b, const EdgeCnt& cnt, int P, T* s_np,
-                                           T* s_nh, const T* s_ndz) {
-  for (int k = kTileThreads - 1 - (int)threadIdx.x; k < P; k += kTileThreads) {
+__device__ __forceinline__ void edge_lines(const TileBox& b, const EdgeCnt& cnt, int P, T* s_np, T* s_nh,
+                                           const T* s_ndz) {
+#pragma unroll 1
+  for (int k = threadIdx.x; k < P; k += kTileThreads) {
     const EdgeItem e = edge_item(b, cnt, k);
     const int slot = e.kind * EW + e.pos;
     T* np = s_np + 6 * slot;
+    T* nh = s_nh + 6 * slot;
     const T lr = line_raw(np);
-    if (io.last) {
-      T* nh = s_nh + 6 * slot;
-      const T nhe = rplus(nh, 1), nhw = rminus(nh + 1, 1);
-      T nc, ncoef;
-      celerity_coef(mid6(nh, 1), s_ndz[slot], nc, ncoef);
-      nh[0] = nhe;
-      nh[1] = nhw;
-      nh[2] = ncoef;
-    }
+    const T nhe = rplus(nh, 1), nhw = rminus(nh + 1, 1);
+    T nc, ncoef;
+    celerity_coef(mid6(nh, 1), s_ndz[slot], nc, ncoef);
+    nh[0] = nhe;
+    nh[1] = nhw;
+    nh[2] = ncoef;
     np[0] = lr;
   }
 }
@@ -1028,24 +717,28 @@ __device__ __forceinline__ void edge_lines(const StageIO<T>& io, const TileBox& 
 // Phase H of one x face or y face: C-grid normal velocity (remap.py:41-55)
 // and its edge average (communication.py:504-570), upwind mass flux with the
 // celerity-based velocity viscosity (barotr_pure.py:21-49) and its edge
-// average on the last stage, and the face cache of phase UV.
-// ph / pu: the 6 h / contravariant values along the face normal (strides sh / su).
+// average on the last stage, upwind tangential component (remap.py:73-95),
+// kinetic energy (barotr_pure.py:91-92) and celerity-viscosity flux
+// (barotr_pure.py:68-69).  ph / pu / pt: the 6 h / contravariant / raw
+// tangential values along the face normal (strides sh / su / su); len: c_dy or
+// d_dx of the face; side, slot: the face edge it lies on (-1: none) and its
+// staged line.  Writes four planes ``plane`` words apart: mass flux x len,
+// kinetic energy, tangential velocity x len, celerity-viscosity flux.
 template <typename T>
-__device__ __forceinline__ T face_h(const StageIO<T>& io, const T* ph, int sh, const T* pu, int su, int side,
-                                    int slot, T dz, const T* s_np, const T* s_nh, const T* s_ndz, T* fc,
-                                    int pstride) {
-  T hh[6], uu[6];
+__device__ __forceinline__ void face_h(const StageIO<T>& io, const T* ph, int sh, const T* pu, const T* pt, int su,
+                                       int side, int slot, T dz, T len, const T* s_np, const T* s_nh, const T* s_ndz,
+                                       T* fo, int plane) {
+  T hh[6], uu[6], tt[6];
 #pragma unroll
   for (int k = 0; k < 6; ++k) {
     hh[k] = ph[k * sh];
     uu[k] = pu[k * su];
+    tt[k] = pt[k * su];
   }
   const T ue = rplus(uu, 1), uw = rminus(uu + 1, 1);
   T bc = T(0.5) * (ue + uw);
-  if (side >= 0) {  // the neighbour's raw normal velocity
-    const T nraw = edge_lines_staged<T>() ? s_np[6 * slot] : line_raw(s_np + 6 * slot);
-    bc = (bc + nraw) / T(2.0);
-  }
+  if (side >= 0)  // with the neighbour's raw normal velocity
+    bc = (bc + (io.last ? s_np[6 * slot] : line_raw(s_np + 6 * slot))) / T(2.0);
   const T he = rplus(hh, 1), hw = rminus(hh + 1, 1);
   T cc, coef;
   celerity_coef(mid6(hh, 1), dz, cc, coef);
@@ -1054,461 +747,500 @@ __device__ __forceinline__ T face_h(const StageIO<T>& io, const T* ph, int sh, c
   if (io.last && side >= 0) {  // the neighbour's flux at the same edge face (barotr_pure.py:29-49)
     const T* nh = s_nh + 6 * slot;
     const T ndz = s_ndz[slot];
-    T nhe, nhw, ncoef;
-    if constexpr (edge_lines_staged<T>()) {  // its face values and viscosity coefficient, staged
-      nhe = nh[0];
-      nhw = nh[1];
-      ncoef = nh[2];
-    } else {
-      nhe = rplus(nh, 1);
-      nhw = rminus(nh + 1, 1);
-      T nc;
-      celerity_coef(mid6(nh, 1), ndz, nc, ncoef);
-    }
-    const T nvis = bc + ncoef * (nhe - nhw);
-    fl = (fl + (ndz * nvis + (nvis > T(0.0) ? nhe : nhw) * nvis)) / T(2.0);
+    const T nvis = bc + nh[2] * (nh[0] - nh[1]);
+    fl = (fl + (ndz * nvis + (nvis > T(0.0) ? nh[0] : nh[1]) * nvis)) / T(2.0);
   }
-  // face cache for phase UV: three planes pstride apart
-  fc[0] = bc;
-  fc[pstride] = vis;
-  fc[2 * pstride] = T(0.5) * cc * (ue - uw);  // celerity viscosity flux, barotr_pure.py:68-69
-  return fl;
+  const T vt = bc > T(0.0) ? rplus(tt, 1) : rminus(tt + 1, 1);
+  fo[0] = fl * len;
+  fo[plane] = T(0.5) * (vis * vis + vt * vt);
+  fo[2 * plane] = vt * len;
+  fo[3 * plane] = T(0.5) * cc * (ue - uw);
 }
 
-// Phase H of one tile: writes the new h on the tile's interior cells.
-// RES (tile-resident round): the constants are already in shared memory, the
-// face fluxes get their own area, and the face cache and the raw velocities
-// of the region go to phase UV's layout (rs.uv) instead of global memory.
+// The tile's cell and face constants (cp.async, not yet awaited): its prepared
+// block with 16-byte copies when the plan has one for this tile shape, else
+// element by element from the constant arrays.
+template <typename T, int TI, int TJ>
+__device__ __forceinline__ void tile_h_consts(const Geo<T>& g, const TileBox& b, T* sm) {
+  using S = TileShape<TI, TJ>;
+  if (g.cblk != nullptr && g.cblk_ti == TI && g.cblk_tj == TJ) {
+    constexpr int V = 16 / sizeof(T);
+    const T* blk = g.cblk + (long)b.idx * S::cW;
+#pragma unroll
+    for (int w = 0; w < S::cW; w += kTileThreads * V) {
+      const int e = w + (int)threadIdx.x * V;
+      if (w + kTileThreads * V <= S::cW || e < S::cW) cp_async<16>(sm + S::hC + e, blk + e);
+    }
+    return;
+  }
+  const LayoutH<T, TI, TJ> L(sm);
+  const int m = g.m, o0 = cell32(b.f, b.i0, b.j0, m);
+#pragma unroll 1
+  for (int e = threadIdx.x; e < S::FX; e += kTileThreads) {
+    const int a = e / TJ, q = e % TJ, o = o0 + a * m + q;
+    if (a > b.ni || q >= b.nj) continue;
+    cp_async_t(L.s_dzx + e, g.dzph_x + o);
+    cp_async_t(L.s_cdy + e, g.c_dy + o);
+    if (a == b.ni) continue;
+    cp_async_t(L.s_cell + e, g.rda + o);
+    cp_async_t(L.s_cell + S::C + e, g.rdx + o);
+    cp_async_t(L.s_cell + 2 * S::C + e, g.rdy + o);
+    cp_async_t(L.s_cell + 3 * S::C + e, g.a_f + o);
+  }
+#pragma unroll 1
+  for (int e = threadIdx.x; e < S::FY; e += kTileThreads) {
+    const int r = e / (TJ + 1), q = e - r * (TJ + 1), o = o0 + r * m + q;
+    if (r >= b.ni || q > b.nj) continue;
+    cp_async_t(L.s_dzy + e, g.dzph_y + o);
+    cp_async_t(L.s_ddx + e, g.d_dx + o);
+  }
+}
+
+// State-independent data of a tile held in registers from the prologue to the
+// main part.  With one region point per thread (TileShape::kHeld) its metric,
+// and one halo value's constants: those of the thread's region point if that
+// lies in the halo, else -- float32 -- those of the line point it gathers.
+// float64 has the registers for that line point's sources only (C96, 8 x 16:
+// 13.97 us per substep; 14.54 with all its constants held and 11 registers
+// spilled; float32 10.66 with all held against 11.56).  With more points per
+// thread only the points' halo sources are held.
+template <typename T, int TI, int TJ>
+struct HPre {
+  using S = TileShape<TI, TJ>;
+  HaloRef<T> ref[S::kHeld ? 1 : S::KP];
+  static constexpr bool kLineHeld = sizeof(T) == 4;
+  HaloWork<T> halo;
+  HaloRef<T> lref;
+  T g[4], sn;
+  int slot;  // the line halo point whose constants (kLineHeld) or sources are held, -1: none
+  EdgeCnt cnt;
+  int P;  // edge positions of the tile (0 for tiles that touch no face edge)
+};
+
+// Line points of a tile (3 per edge position) go to the threads from
+// line_thread0 on, whose region points lie on the tile's own rows: interior
+// points, except in tiles thinner than TI next to an N edge.
+template <int TI, int TJ>
+__device__ __forceinline__ int line_first() {
+  constexpr int line_thread0 = kHalo * TJ;
+  const int t = (int)threadIdx.x - line_thread0;
+  return t >= 0 ? t : t + kTileThreads;
+}
+
+// Metric, halo sources and line constants of the tile.
+template <typename T, int TI, int TJ, bool FULL>
+__device__ __forceinline__ void tile_h_points(const Geo<T>& g, const StageIO<T>& io, const TileBox& b, T* sm,
+                                              HPre<T, TI, TJ>& pre) {
+  using S = TileShape<TI, TJ>;
+  const int m = g.m;
+  const LayoutH<T, TI, TJ> L(sm);
+  pre.P = FULL ? 0 : edge_count(b, m, g.route, pre.cnt);
+  pre.slot = -1;
+  bool halo = false;
+#pragma unroll
+  for (int k = 0; k < S::KP; ++k) {
+    const int p = k * kTileThreads + (int)threadIdx.x;
+    if (p >= S::NP) continue;
+    const RegionPoint<TI, TJ, FULL> pt(b, p);
+    if (!pt.on) continue;
+    const int i = b.i0 - kHalo + pt.r, j = b.j0 - kHalo + pt.c, o = cell32(b.f, i, j, m);
+    if (!FULL && !io.stored_halo) {
+      const PointKind pk(i, j, m);
+      if (pk.side >= 0) {
+        halo = true;
+        if (S::kHeld) {
+          pre.halo.ref.load(g, b.f, pk.side, pk.c, pk.k);
+          ld_quad(g.l2c + 4 * (long)o, pre.halo.l2);
+        } else {
+          pre.ref[k].load(g, b.f, pk.side, pk.c, pk.k);
+        }
+      }
+    }
+    if constexpr (S::kHeld) {
+      ld_quad(g.gct + 4 * (long)o, pre.g);
+      pre.sn = g.sina[o];
+    } else {
+      cp_async_mat(L.s_g + 4 * p, g.gct + 4 * (long)o);
+      cp_async_t(L.s_sn + p, g.sina + o);
+    }
+  }
+  if (!FULL && pre.P > 0) {
+#pragma unroll 1
+    for (int t = line_first<TI, TJ>(); t < 3 * pre.P; t += kTileThreads) {
+      const LinePoint lp(b, pre.cnt, pre.P, t, g.n, S::EW);
+      if (io.last) line_depth<T, TI, TJ>(g, lp, L);
+      if (S::kHeld && !io.stored_halo && t < kTileThreads) {
+        if (!HPre<T, TI, TJ>::kLineHeld) {
+          pre.slot = lp.slot_out;
+          pre.lref.load(g, lp.nb, lp.ns, lp.d, lp.kk);
+        } else if (!halo) {
+          pre.slot = lp.slot_out;
+          pre.halo.ref.load(g, lp.nb, lp.ns, lp.d, lp.kk);
+          pre.halo.line_constants(g, lp);
+        }
+      }
+    }
+  }
+}
+
+// Phase H prologue: constants of the tile, metric, halo sources.  Independent
+// of the state, so it may run before the previous phase has finished
+// (programmatic launch, or before a grid barrier).
+template <typename T, int TI, int TJ, bool FULL>
+__device__ __forceinline__ void tile_h_pro_t(const Geo<T>& g, const StageIO<T>& io, const TileBox& b, T* sm,
+                                             HPre<T, TI, TJ>& pre) {
+  tile_h_consts<T, TI, TJ>(g, b, sm);
+  tile_h_points<T, TI, TJ, FULL>(g, io, b, sm, pre);
+}
+
+// Phase H of one tile: writes the new h and the momentum terms of the tile's
+// interior cells, and the new h of its cells in the face's bands.  RES
+// (tile-resident round): the terms stay on chip.
 template <typename T, int TI, int TJ, bool FULL, bool RES = false>
 __device__ __forceinline__ void tile_h_main_t(const Geo<T>& g, const StageIO<T>& io, const TileBox& b, T* sm,
-                                              Gather<T, TI, TJ, false, RES>& gat, const EdgeCnt& cnt, int P,
-                                              const ResSm<T>& rs = ResSm<T>{}) {
+                                              const HPre<T, TI, TJ>& pre, const ResSm<T>& rs = ResSm<T>{}) {
   using S = TileShape<TI, TJ>;
   constexpr int RJ = S::RJ;
-  static_assert(6 * TI <= kTileThreads, "one side point per thread");
-  const int m = g.m, n = g.n, f = b.f, q = threadIdx.x % TJ, sl = threadIdx.x / TJ;
+  const int m = g.m, n = g.n, f = b.f;
   const int ni = FULL ? TI : b.ni, nj = FULL ? TJ : b.nj;
-  LayoutH<T, TI, TJ> L(sm);
-  const LayoutUV<T, TI, TJ> U(RES ? rs.uv : sm);  // RES only
-  if constexpr (RES) {
-    L.s_P = rs.pq;
-    L.s_Q = rs.pq + S::FX;
-  }
-  int* const items = RES ? rs.items : reinterpret_cast<int*>(sm + S::kWordsH);
-  // state of the thread's interior region points and base h of its cells, into registers
-  T hv[S::KV], uv[S::KV], vv[S::KV], hpc[S::KC];
-  T hs = T(0.0), us = T(0.0), vs = T(0.0);
-  const EdgeCover ec(b, m);
-  const int ov = cell32(f, b.i0 - kHalo, b.j0 + q, m);
+  const LayoutH<T, TI, TJ> L(sm);
+  const int o0 = cell32(f, b.i0, b.j0, m);
+
+  // region: state of the thread's points (halo points from the bands) and base h of its cells
+  T hv[S::KP], uv[S::KP], vv[S::KP], hpc[S::KC];
 #pragma unroll
-  for (int k = 0; k < S::KV; ++k) {
-    const int r = sl + k * S::NS, i = b.i0 - kHalo + r;
-    if (q < nj && r < ni + 6 && (FULL || (i >= kHalo && i < m - kHalo))) {  // halo rows: see below
-      const int o = ov + r * m;
-      hv[k] = io.h[o];
-      uv[k] = io.u[o];
-      vv[k] = io.v[o];
+  for (int k = 0; k < S::KP; ++k) {
+    const int p = k * kTileThreads + (int)threadIdx.x;
+    if (p >= S::NP) continue;
+    const RegionPoint<TI, TJ, FULL> pt(b, p);
+    if (!pt.on) continue;
+    const int o = o0 + (pt.r - kHalo) * m + pt.c - kHalo;
+    if (!FULL && !io.stored_halo) {
+      const int i = b.i0 - kHalo + pt.r, j = b.j0 - kHalo + pt.c;
+      const PointKind pk(i, j, m);
+      if (pk.side >= 0) {
+        T l2[4];
+        if (!S::kHeld) ld_quad(g.l2c + 4 * (long)o, l2);
+        const HaloRef<T>& ref = S::kHeld ? pre.halo.ref : pre.ref[k];
+        halo_uv(io, ref, band_plane(n), S::kHeld ? pre.halo.l2 : l2, uv[k], vv[k]);
+        hv[k] = ref.lerp(io.band_h);
+        continue;
+      }
     }
-  }
-  const int t6 = threadIdx.x;
-  const int sr = t6 / 6, sc = t6 - 6 * sr, scc = sc < 3 ? sc : nj + sc, sj = b.j0 - kHalo + scc;
-  const bool side_pt = t6 < 6 * ni && (FULL || ec.col_staged(sj, m));
-  if (side_pt) {
-    if (FULL || (sj >= kHalo && sj < m - kHalo)) {
-      const int o = cell32(f, b.i0 + sr, sj, m);
-      hs = io.h[o];
-      us = io.u[o];
-      vs = io.v[o];
-    } else {
-      hs = fetch_s(io.h, g, f, b.i0 + sr, sj, io.stored_halo);
-      fetch_v(io.u, io.v, g, f, b.i0 + sr, sj, io.stored_halo, us, vs);
-    }
+    hv[k] = io.h[o];
+    uv[k] = io.u[o];
+    vv[k] = io.v[o];
   }
 #pragma unroll
   for (int k = 0; k < S::KC; ++k) {
-    const int a = sl + k * S::NS;
-    if (q < nj && a < ni) hpc[k] = io.hp[ov + (a + kHalo) * m];
+    const int c = k * kTileThreads + (int)threadIdx.x, a = c / TJ, q = c % TJ;
+    if (a < ni && q < nj) hpc[k] = io.hp[o0 + a * m + q];
   }
-  if (!FULL && P > 0) {
-    GatherSink<T> sink{L.s_h, L.s_uc, L.s_vc, L.s_np, L.s_nh, L.s_ndz};
-    if constexpr (RES) {
-      sink.rv = U.s_v;
-      sink.ru = U.s_u;
-    }
-    gat.sources(g, io, b, cnt, P, sink, items);
-  }
-  cp_async_wait_all();
-  __syncthreads();
-
-  // h and contravariant velocities of the region (remap.py:34-39)
-#pragma unroll
-  for (int k = 0; k < S::KV; ++k) {
-    const int r = sl + k * S::NS, i = b.i0 - kHalo + r;
-    if (q < nj && r < ni + 6 && (FULL || (i >= kHalo && i < m - kHalo))) {
-      const int p = r * TJ + q;
-      const T* G = L.s_g + 4 * p;
-      const T sn = L.s_sn[p], u = uv[k], v = vv[k];
-      const bool row = r >= kHalo && r < ni + kHalo;
-      L.s_h[r * RJ + q + kHalo] = hv[k];
-      L.s_uc[p] = (G[0] * u + G[1] * v) * sn;
-      if (row) L.s_vc[(r - kHalo) * RJ + q + kHalo] = (G[2] * u + G[3] * v) * sn;
-      if constexpr (RES) {  // phase UV's raw velocities (tangential reconstructions)
-        U.s_v[p] = v;
-        if (row) U.s_u[(r - kHalo) * RJ + q + kHalo] = u;
-      }
-    }
-  }
-  if (!FULL) {
-    // halo rows of the region that no gather item covers (EdgeCover), fetched
-    // point by point; a rolled loop keeps this rarely run code small
+  if (!FULL && pre.P > 0) {
 #pragma unroll 1
-    for (int k = 0; k < S::KV; ++k) {
-      const int r = sl + k * S::NS, i = b.i0 - kHalo + r;
-      if (q < nj && r < ni + 6 && ec.row_staged(i, m) && !(i >= kHalo && i < m - kHalo)) {
-        T u, v;
-        const T h = fetch_s(io.h, g, f, i, b.j0 + q, io.stored_halo);
-        fetch_v(io.u, io.v, g, f, i, b.j0 + q, io.stored_halo, u, v);
-        const int p = r * TJ + q;
-        const T* G = L.s_g + 4 * p;
-        const T sn = L.s_sn[p];
-        L.s_h[r * RJ + q + kHalo] = h;
-        L.s_uc[p] = (G[0] * u + G[1] * v) * sn;
-        if constexpr (RES) U.s_v[p] = v;
+    for (int t = line_first<TI, TJ>(); t < 3 * pre.P; t += kTileThreads) {
+      const LinePoint lp(b, pre.cnt, pre.P, t, n, S::EW);
+      if (io.stored_halo) {
+        line_stored<T, TI, TJ>(g, io, lp, L);
+      } else {
+        line_inside<T, TI, TJ>(g, io, lp, L);
+        const bool held = S::kHeld && lp.slot_out == pre.slot;
+        if (!(HPre<T, TI, TJ>::kLineHeld && held)) {
+          HaloWork<T> w;
+          if (held)
+            w.ref = pre.lref;
+          else
+            w.ref.load(g, lp.nb, lp.ns, lp.d, lp.kk);
+          w.line_constants(g, lp);
+          line_outside<T, TI, TJ>(io, lp.slot_out, w, band_plane(n), L);
+        }
       }
     }
+    if (S::kHeld && HPre<T, TI, TJ>::kLineHeld && pre.slot >= 0)
+      line_outside<T, TI, TJ>(io, pre.slot, pre.halo, band_plane(n), L);
   }
-  if (side_pt) {
-    const T* G = L.s_g + 4 * (S::VB + t6);
-    const T sn = L.s_sn[S::VB + t6];
-    L.s_h[(sr + kHalo) * RJ + scc] = hs;
-    L.s_vc[sr * RJ + scc] = (G[2] * us + G[3] * vs) * sn;
-    if constexpr (RES) U.s_u[sr * RJ + scc] = us;
+  if (!S::kHeld) {
+    cp_async_wait_all();
+    __syncthreads();
   }
-  if (edge_lines_staged<T>() && !FULL && P > 0) edge_lines<T, S::EW>(io, b, cnt, P, L.s_np, L.s_nh, L.s_ndz);
-  __syncthreads();
+  // h, raw and contravariant velocities (remap.py:34-39)
+#pragma unroll
+  for (int k = 0; k < S::KP; ++k) {
+    const int p = k * kTileThreads + (int)threadIdx.x;
+    if (p >= S::NP) continue;
+    const RegionPoint<TI, TJ, FULL> pt(b, p);
+    if (!pt.on) continue;
+    const T* G = S::kHeld ? pre.g : L.s_g + 4 * p;
+    const T sn = S::kHeld ? pre.sn : L.s_sn[p];
+    const T u = uv[k], v = vv[k];
+    L.s_h[pt.r * RJ + pt.c] = hv[k];
+    if (pt.vbar) {
+      L.s_uc[pt.r * TJ + pt.c - kHalo] = (G[0] * u + G[1] * v) * sn;
+      L.s_v[pt.r * TJ + pt.c - kHalo] = v;
+    }
+    if (pt.hbar) {
+      L.s_vc[(pt.r - kHalo) * RJ + pt.c] = (G[2] * u + G[3] * v) * sn;
+      L.s_u[(pt.r - kHalo) * RJ + pt.c] = u;
+    }
+  }
+  if (S::kHeld) {
+    cp_async_wait_all();
+    __syncthreads();
+  }
+  const bool lines = !FULL && pre.P > 0 && io.last;
+  if (lines) edge_lines<T, S::EW>(b, pre.cnt, pre.P, L.s_np, L.s_nh, L.s_ndz);
+  if (!S::kHeld || lines) __syncthreads();
 
-  // faces; their fluxes (times c_dy / d_dx) alias the metric block, no longer read.  The face
-  // cache of every face goes to the tile's block (phase UV's shared-memory layout when resident)
-  T* const fblk = RES ? nullptr : io.fx + face_block_off<TI, TJ>(b, n);
-  if (q < nj) {
-#pragma unroll
-    for (int k = 0; k < S::KX; ++k) {
-      const int a = sl + k * S::NS;
-      if (a <= ni) {
-        const int side =
-            FULL ? -1 : ((a == 0 && b.i0 == kHalo) ? kS : ((a == ni && b.i0 + ni == m - kHalo) ? kN : -1));
-        const int e = a * TJ + q;
-        T* fc = RES ? U.s_xc + e : fblk + e;
-        const T fl = face_h<T>(io, L.s_h + a * RJ + q + kHalo, RJ, L.s_uc + a * TJ + q, TJ, side,
-                               (side == kS ? 0 : 1) * S::EW + q, L.s_dzx[e], L.s_np, L.s_nh, L.s_ndz, fc, S::FX);
-        L.s_P[e] = fl * L.s_cdy[e];
-      }
-    }
-  }
-  // y faces: (r, qq) with qq = q, plus qq = TJ for full-width tiles (lanes of the last warp)
-#pragma unroll
-  for (int k = 0; k <= S::KC; ++k) {
-    int r, qq;
-    if (k < S::KC) {
-      r = sl + k * S::NS;
-      qq = q;
-      if (r >= ni || q > nj) continue;
-    } else {
-      r = east_row();
-      qq = TJ;
-      if (nj != TJ || r < 0 || r >= ni) continue;
-    }
+  // faces: x faces, then y faces.  When all of them fit one pass they run
+  // one copy of the face code with run-time strides (a warp may hold both kinds,
+  // and the code is fetched once); else each kind starts at a warp boundary.
+  auto x_face = [&](int e) {
+    const int a = e / TJ, q = e % TJ;
+    if (!FULL && (a > ni || q >= nj)) return;
     const int side =
-        FULL ? -1 : ((qq == 0 && b.j0 == kHalo) ? kW : ((qq == nj && b.j0 + nj == m - kHalo) ? kE : -1));
-    const int e = r * (TJ + 1) + qq;
-    T* fc = RES ? U.s_yc + e : fblk + S::fXB + e;
-    const T fl = face_h<T>(io, L.s_h + (r + kHalo) * RJ + qq, 1, L.s_vc + r * RJ + qq, 1, side,
-                           (side == kW ? 2 : 3) * S::EW + r, L.s_dzy[e], L.s_np, L.s_nh, L.s_ndz, fc, S::FY);
-    L.s_Q[e] = fl * L.s_ddx[e];
+        FULL ? -1 : ((a == 0 && b.i0 == kHalo) ? kS : ((a == ni && b.i0 + ni == m - kHalo) ? kN : -1));
+    face_h<T>(io, L.s_h + a * RJ + q + kHalo, RJ, L.s_uc + e, L.s_v + e, TJ, side, (side == kS ? 0 : S::EW) + q,
+              L.s_dzx[e], L.s_cdy[e], L.s_np, L.s_nh, L.s_ndz, L.s_fx + e, S::FXP);
+  };
+  auto y_face = [&](int e) {
+    const int r = e / (TJ + 1), q = e - r * (TJ + 1);
+    if (!FULL && (r >= ni || q > nj)) return;
+    const int side =
+        FULL ? -1 : ((q == 0 && b.j0 == kHalo) ? kW : ((q == nj && b.j0 + nj == m - kHalo) ? kE : -1));
+    face_h<T>(io, L.s_h + (r + kHalo) * RJ + q, 1, L.s_vc + r * RJ + q, L.s_u + r * RJ + q, 1, side,
+              (side == kW ? 2 : 3) * S::EW + r, L.s_dzy[e], L.s_ddx[e], L.s_np, L.s_nh, L.s_ndz, L.s_fy + e, S::FYP);
+  };
+  if constexpr (S::FX + S::FY <= kTileThreads) {
+    const int t = threadIdx.x;
+    if (t < S::FX + S::FY) {
+      const bool y = t >= S::FX;
+      const int e = y ? t - S::FX : t;
+      const int a = y ? e / (TJ + 1) : e / TJ, q = y ? e - a * (TJ + 1) : e % TJ;
+      const bool on = y ? (a < ni && q <= nj) : (a <= ni && q < nj);
+      if (FULL || on) {
+        int side = -1;
+        if (!FULL) {
+          const int z = y ? q : a, w = y ? nj : ni, i0 = y ? b.j0 : b.i0;
+          if (z == 0 && i0 == kHalo) side = y ? kW : kS;
+          if (z == w && i0 + w == m - kHalo) side = y ? kE : kN;
+        }
+        const int slot = y ? (side == kW ? 2 : 3) * S::EW + a : (side == kS ? 0 : S::EW) + q;
+        const int at = y ? a * RJ + q : e;
+        face_h<T>(io, L.s_h + (y ? (a + kHalo) * RJ + q : a * RJ + q + kHalo), y ? 1 : RJ,
+                  (y ? L.s_vc : L.s_uc) + at, (y ? L.s_u : L.s_v) + at, y ? 1 : TJ, side, slot,
+                  (y ? L.s_dzy : L.s_dzx)[e], (y ? L.s_ddx : L.s_cdy)[e], L.s_np, L.s_nh, L.s_ndz,
+                  (y ? L.s_fy : L.s_fx) + e, y ? S::FYP : S::FXP);
+      }
+    }
+  } else {
+    constexpr int XS = (S::FX + 31) & ~31;  // y faces start here
+#pragma unroll
+    for (int z = 0; z < XS + S::FY; z += kTileThreads) {
+      const int t = z + (int)threadIdx.x;
+      if (z < S::FX && t < S::FX)
+        x_face(t);
+      else if (z + kTileThreads > XS && t >= XS && t < XS + S::FY)
+        y_face(t - XS);
+    }
   }
   __syncthreads();
 
-  // cells: divergence (agrid.py:43-53) and the h update (barotr_pure.py:119-120)
-  if (q < nj) {
+  // cells: divergence (agrid.py:43-53) and the h update (barotr_pure.py:119-120), vorticity
+  // (agrid.py:31-41), advection (barotr_pure.py:78-97), Coriolis, celerity viscosity
+  // (barotr_pure.py:63-75)
+  T* const tb = RES ? rs.terms : io.fx + (long)b.idx * (kTerms<T> * S::C);
 #pragma unroll
-    for (int k = 0; k < S::KC; ++k) {
-      const int a = sl + k * S::NS;
-      if (a < ni) {
-        const int x0 = a * TJ + q, y0 = a * (TJ + 1) + q;
-        const T div = L.s_rda[x0] * (L.s_P[x0 + TJ] - L.s_P[x0] + L.s_Q[y0 + 1] - L.s_Q[y0]);
-        io.h_out[ov + (a + kHalo) * m] = hpc[k] - div * io.dt;
+  for (int k = 0; k < S::KC; ++k) {
+    const int e = k * kTileThreads + (int)threadIdx.x, a = e / TJ, q = e % TJ;
+    if (a < ni && q < nj) {
+      const T* X = L.s_fx + e;
+      const T* Y = L.s_fy + a * (TJ + 1) + q;
+      const T* c = L.s_cell + e;
+      const T rda = c[0], rdx = c[S::C], rdy = c[2 * S::C], af = c[3 * S::C];
+      const T div = rda * (X[TJ] - X[0] + Y[1] - Y[0]);
+      const T hn = hpc[k] - div * io.dt;
+      io.h_out[o0 + a * m + q] = hn;
+      if (!FULL) for_bands(f, b.i0 + a, b.j0 + q, n, [&](int, int z) { io.band_hn[z] = hn; });
+      const T uct = L.s_uc[(a + kHalo) * TJ + q], vct = L.s_vc[a * RJ + q + kHalo];
+      const T* kx = X + S::FXP;
+      const T* ky = Y + S::FYP;
+      const T* tx = X + 2 * S::FXP;
+      const T* ty = Y + 2 * S::FYP;
+      const T* vx = X + 3 * S::FXP;
+      const T* vy = Y + 3 * S::FYP;
+      const T vort = rda * (ty[0] + tx[TJ] - ty[1] - tx[0]);
+      const T advx = vort * vct - (kx[TJ] - kx[0]) * rdx;
+      const T advy = -vort * uct - (ky[1] - ky[0]) * rdy;
+      const T visx = -(rdx * (vx[TJ] - vx[0]));
+      const T visy = -(rdy * (vy[1] - vy[0]));
+      T* const t = tb + e;
+      if constexpr (kTerms<T> == 6) {
+        t[0] = advx;
+        t[S::C] = af * vct;
+        t[2 * S::C] = visx;
+        t[3 * S::C] = advy;
+        t[4 * S::C] = af * uct;
+        t[5 * S::C] = visy;
+      } else {
+        t[0] = advx + af * vct + visx;
+        t[S::C] = advy - af * uct + visy;
       }
     }
   }
 }
 
 // ---- phase UV -----------------------------------------------------------------
-// Phase UV cell and face constants of the tile (cp.async, not yet awaited):
-// the tile's prepared block with 16-byte copies when the plan has one for this
-// tile shape, else element by element from the constant arrays.
+// State-independent data of phase UV held in registers from the prologue: the
+// thread's cell constants (with the metric of cells in the bands) and, with one
+// region point per thread, its halo sources.
+template <typename T, int TI, int TJ>
+struct UvPre {
+  using S = TileShape<TI, TJ>;
+  T rdx[S::KC], rdy[S::KC];
+  HaloRef<T> ref[S::KP];
+  static constexpr bool kBandHeld = S::KC == 1;
+  T c2[4], g[4], sn;  // of a cell in the bands (kBandHeld; else loaded at use)
+};
+
 template <typename T, int TI, int TJ, bool FULL>
-__device__ __forceinline__ void tile_uv_consts(const Geo<T>& g, const TileBox& b, T* sm) {
+__device__ __forceinline__ void tile_uv_pro_t(const Geo<T>& g, const TileBox& b, UvPre<T, TI, TJ>& pre) {
   using S = TileShape<TI, TJ>;
-  if (g.cblk != nullptr && g.cblk_ti == TI && g.cblk_tj == TJ) {
-    constexpr int V = 16 / sizeof(T);
-    const T* blk = g.cblk + (long)tile_index<TI, TJ>(b, g.n) * S::cW;
-#pragma unroll
-    for (int w = threadIdx.x * V; w < S::uConstWords; w += kTileThreads * V) cp_async<16>(sm + S::uG + w, blk + w);
-    return;
-  }
-  const LayoutUV<T, TI, TJ> L(sm);
-  const int m = g.m, q = threadIdx.x % TJ, sl = threadIdx.x / TJ;
+  const int m = g.m, o0 = cell32(b.f, b.i0, b.j0, m);
   const int ni = FULL ? TI : b.ni, nj = FULL ? TJ : b.nj;
-  const int o0 = cell32(b.f, b.i0, b.j0 + q, m);
-  if (q < nj) {
 #pragma unroll
-    for (int k = 0; k < S::KC; ++k) {
-      const int a = sl + k * S::NS;
-      if (a < ni) {
-        const int o = o0 + a * m, e = a * TJ + q;
-        cp_async_mat(L.s_g + 4 * e, g.gct + 4 * (long)o);
-        cp_async_t(L.s_sn + e, g.sina + o);
-        cp_async_t(L.s_rda + e, g.rda + o);
-        cp_async_t(L.s_rdx + e, g.rdx + o);
-        cp_async_t(L.s_rdy + e, g.rdy + o);
-        cp_async_t(L.s_af + e, g.a_f + o);
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < S::KX; ++k) {
-      const int a = sl + k * S::NS;
-      if (a <= ni) cp_async_t(L.s_cdy + a * TJ + q, g.c_dy + o0 + a * m);
-    }
-  }
-  if (q <= nj) {
-#pragma unroll
-    for (int k = 0; k < S::KC; ++k) {
-      const int r = sl + k * S::NS;
-      if (r < ni) cp_async_t(L.s_ddx + r * (TJ + 1) + q, g.d_dx + o0 + r * m);
-    }
-  }
-  if (nj == TJ && east_row() >= 0 && east_row() < ni) {
-    const int r = east_row();
-    cp_async_t(L.s_ddx + r * (TJ + 1) + TJ, g.d_dx + cell32(b.f, b.i0 + r, b.j0 + TJ, m));
-  }
-}
-
-// Phase UV prologue: cell and face constants (cp.async) and the halo-gather descriptors.
-template <typename T, int TI, int TJ, bool FULL>
-__device__ __forceinline__ void tile_uv_pro_t(const Geo<T>& g, const StageIO<T>& io, const TileBox& b, T* sm,
-                                              Gather<T, TI, TJ, true>& gat, EdgeCnt& cnt, int& P) {
-  using S = TileShape<TI, TJ>;
-  tile_uv_consts<T, TI, TJ, FULL>(g, b, sm);
-  tile_desc<T, TI, TJ, FULL, true, false>(g, io, b, gat, cnt, P, reinterpret_cast<int*>(sm + S::kWordsUV));
-}
-
-// RES (tile-resident round): the constants, the face cache and the raw
-// velocities of the region are already in shared memory (left there by phase
-// H of the same stage), and the stage h of the fb blend is phase H's region h
-// (rs.hs); only the new h of the region is read from global memory.
-template <typename T, int TI, int TJ, bool FULL, bool RES = false>
-__device__ __forceinline__ void tile_uv_main_t(const Geo<T>& g, const StageIO<T>& io, const TileBox& b, T* sm,
-                                               Gather<T, TI, TJ, true, RES>& gat, const EdgeCnt& cnt, int P,
-                                               const ResSm<T>& rs = ResSm<T>{}) {
-  using S = TileShape<TI, TJ>;
-  constexpr int RJ = S::RJ;
-  static_assert(6 * TI <= kTileThreads, "one side point per thread");
-  const int m = g.m, n = g.n, f = b.f, q = threadIdx.x % TJ, sl = threadIdx.x / TJ;
-  const int ni = FULL ? TI : b.ni, nj = FULL ? TJ : b.nj;
-  const LayoutUV<T, TI, TJ> L(sm);
-  const bool blend = io.beta != T(0.0);  // fb_scheme needs the stage h only when beta_d != 0
-  const T* hn_src = (const T*)io.h_out;
-  const T* const hb = RES ? rs.hs : L.s_hb;  // stage h of the blend, region layout [RI][RJ]
-  const int* const items = RES ? rs.items : reinterpret_cast<const int*>(sm + S::kWordsUV);
-
-  // the tile's face cache block of this stage (written by phase H) -> shared memory, 16 bytes a copy
-  if (!RES) {
-    constexpr int V = 16 / sizeof(T);
-    const T* blk = io.fx + face_block_off<TI, TJ>(b, n);
-#pragma unroll
-    for (int w = threadIdx.x * V; w < S::fXB; w += kTileThreads * V) cp_async<16>(L.s_xc + w, blk + w);
-#pragma unroll
-    for (int w = threadIdx.x * V; w < S::fYB; w += kTileThreads * V) cp_async<16>(L.s_yc + w, blk + S::fXB + w);
-  }
-
-  // state of the region: interior points by cp.async straight into shared
-  // memory (new h, raw v on the vertical bar, raw u on the tile rows and side
-  // points, the stage h of the fb blend when beta != 0); halo points that no
-  // gather item covers are fetched point by point and stored blended
-  T upc[S::KC], vpc[S::KC];
-  const EdgeCover ec(b, m);
-  const int ov = cell32(f, b.i0 - kHalo, b.j0 + q, m);
-#pragma unroll
-  for (int k = 0; k < S::KV; ++k) {
-    const int r = sl + k * S::NS, i = b.i0 - kHalo + r;
-    if (q < nj && r < ni + 6 && (FULL || (i >= kHalo && i < m - kHalo))) {  // halo rows: see below
-      const bool row = r >= kHalo && r < ni + kHalo;
-      const int e = r * RJ + q + kHalo;
-      const int o = ov + r * m;
-      cp_async_t(L.s_hn + e, hn_src + o);
-      if (!RES) {
-        if (blend) cp_async_t(L.s_hb + e, io.h + o);
-        cp_async_t(L.s_v + r * TJ + q, io.v + o);
-        if (row) cp_async_t(L.s_u + (r - kHalo) * RJ + q + kHalo, io.u + o);
+  for (int k = 0; k < S::KC; ++k) {
+    const int c = k * kTileThreads + (int)threadIdx.x, a = c / TJ, q = c % TJ;
+    if (a < ni && q < nj) {
+      pre.rdx[k] = g.rdx[o0 + a * m + q];
+      pre.rdy[k] = g.rdy[o0 + a * m + q];
+      if (!FULL && UvPre<T, TI, TJ>::kBandHeld && in_bands(b.i0 + a, b.j0 + q, g.n)) {
+        const long o = o0 + a * m + q;
+        ld_quad(g.c2l + 4 * o, pre.c2);
+        ld_quad(g.gct + 4 * o, pre.g);
+        pre.sn = g.sina[o];
       }
     }
   }
   if (!FULL) {
-    // halo rows of the region that no gather item covers (EdgeCover), fetched
-    // point by point and stored blended (the new h never has a stored halo)
-#pragma unroll 1
-    for (int k = 0; k < S::KV; ++k) {
-      const int r = sl + k * S::NS, i = b.i0 - kHalo + r;
-      if (q < nj && r < ni + 6 && ec.row_staged(i, m) && !(i >= kHalo && i < m - kHalo)) {
-        const int e = r * RJ + q + kHalo;
-        T hn = fetch_s(hn_src, g, f, i, b.j0 + q, 0);
-        if (RES) {  // raw velocities and the stage h staged by phase H
-          if (blend) hn = (T(1.0) - io.beta) * hn + io.beta * hb[e];
-          L.s_hn[e] = hn;
-          continue;
-        }
-        T u, v;
-        fetch_v(io.u, io.v, g, f, i, b.j0 + q, io.stored_halo, u, v);
-        if (blend) hn = (T(1.0) - io.beta) * hn + io.beta * fetch_s(io.h, g, f, i, b.j0 + q, io.stored_halo);
-        L.s_hn[e] = hn;
-        L.s_v[r * TJ + q] = v;
-        if (r >= kHalo && r < ni + kHalo) L.s_u[(r - kHalo) * RJ + q + kHalo] = u;
-      }
+#pragma unroll
+    for (int k = 0; k < S::KP; ++k) {
+      const int p = k * kTileThreads + (int)threadIdx.x;
+      if (p >= S::NP) continue;
+      const RegionPoint<TI, TJ, FULL> pt(b, p);
+      if (!pt.on) continue;
+      const PointKind pk(b.i0 - kHalo + pt.r, b.j0 - kHalo + pt.c, m);
+      if (pk.side >= 0) pre.ref[k].load(g, b.f, pk.side, pk.c, pk.k);
     }
   }
-  const int t6 = threadIdx.x;
-  const int sr = t6 / 6, sc = t6 - 6 * sr, scc = sc < 3 ? sc : nj + sc, sj = b.j0 - kHalo + scc;
-  const bool side_pt = t6 < 6 * ni && (FULL || ec.col_staged(sj, m));
-  const bool side_in = FULL || (sj >= kHalo && sj < m - kHalo);
-  if (side_pt) {
-    const int e = (sr + kHalo) * RJ + scc;
-    if (side_in) {
-      const int o = cell32(f, b.i0 + sr, sj, m);
-      cp_async_t(L.s_hn + e, hn_src + o);
-      if (!RES) {
-        if (blend) cp_async_t(L.s_hb + e, io.h + o);
-        cp_async_t(L.s_u + sr * RJ + scc, io.u + o);
+}
+
+// Phase UV of one tile: pressure gradient of the new h (agrid.py:55-69,
+// barotr_pure.py:57-60) and the momentum update (barotr_pure.py:149-150) with
+// phase H's terms; the lon/lat and normal contravariant velocity of the tile's
+// cells in the face's bands.  RES (tile-resident round): the terms are in
+// shared memory.
+template <typename T, int TI, int TJ, bool FULL, bool RES = false>
+__device__ __forceinline__ void tile_uv_main_t(const Geo<T>& g, const StageIO<T>& io, const TileBox& b, T* sm,
+                                               const UvPre<T, TI, TJ>& pre, const ResSm<T>& rs = ResSm<T>{}) {
+  using S = TileShape<TI, TJ>;
+  constexpr int RJ = S::RJ;
+  const int m = g.m, n = g.n, f = b.f;
+  const int ni = FULL ? TI : b.ni, nj = FULL ? TJ : b.nj;
+  const bool blend = io.beta != T(0.0);  // fb_scheme needs the stage h only when beta_d != 0
+  const T* hn_src = (const T*)io.h_out;
+  const T* hn_band = (const T*)io.band_hn;
+  const int o0 = cell32(f, b.i0, b.j0, m);
+
+  // new h of the region, blended with the stage h (fb_scheme, barotr_pure.py:52-54)
+  T hn[S::KP], hs[S::KP];
+#pragma unroll
+  for (int k = 0; k < S::KP; ++k) {
+    const int p = k * kTileThreads + (int)threadIdx.x;
+    if (p >= S::NP) continue;
+    const RegionPoint<TI, TJ, FULL> pt(b, p);
+    if (!pt.on) continue;
+    const int o = o0 + (pt.r - kHalo) * m + pt.c - kHalo;
+    if (!FULL) {
+      const PointKind pk(b.i0 - kHalo + pt.r, b.j0 - kHalo + pt.c, m);
+      if (pk.side >= 0) {  // the new h never has a stored halo
+        hn[k] = pre.ref[k].lerp(hn_band);
+        if (blend) hs[k] = io.stored_halo ? io.h[o] : pre.ref[k].lerp(io.band_h);
+        continue;
       }
-    } else if (RES) {
-      T hn = fetch_s(hn_src, g, f, b.i0 + sr, sj, 0);
-      if (blend) hn = (T(1.0) - io.beta) * hn + io.beta * hb[e];
-      L.s_hn[e] = hn;
-    } else {
-      T hn = fetch_s(hn_src, g, f, b.i0 + sr, sj, 0), u, v;
-      fetch_v(io.u, io.v, g, f, b.i0 + sr, sj, io.stored_halo, u, v);
-      if (blend) hn = (T(1.0) - io.beta) * hn + io.beta * fetch_s(io.h, g, f, b.i0 + sr, sj, io.stored_halo);
-      L.s_hn[e] = hn;
-      L.s_u[sr * RJ + scc] = u;
     }
+    hn[k] = hn_src[o];
+    if (blend) hs[k] = io.h[o];
   }
+  // base velocities and terms of the thread's cells
+  T upc[S::KC], vpc[S::KC], tm[S::KC][kTerms<T>];
+  const T* const tb = RES ? rs.terms : io.fx + (long)b.idx * (kTerms<T> * S::C);
 #pragma unroll
   for (int k = 0; k < S::KC; ++k) {
-    const int a = sl + k * S::NS;
-    if (q < nj && a < ni) {
-      upc[k] = io.up[ov + (a + kHalo) * m];
-      vpc[k] = io.vp[ov + (a + kHalo) * m];
-    }
-  }
-  if (!FULL && P > 0) {
-    GatherSink<T> sink{L.s_hn, L.s_v, L.s_u, nullptr, nullptr, nullptr};
-    sink.hs = hb;
-    gat.sources(g, io, b, cnt, P, sink, items);
-  }
-  cp_async_wait_all();
-  __syncthreads();
-  if (blend) {  // fb_scheme, barotr_pure.py:52-54, on the points staged by cp.async
+    const int c = k * kTileThreads + (int)threadIdx.x, a = c / TJ, q = c % TJ;
+    if (a < ni && q < nj) {
+      upc[k] = io.up[o0 + a * m + q];
+      vpc[k] = io.vp[o0 + a * m + q];
 #pragma unroll
-    for (int k = 0; k < S::KV; ++k) {
-      const int r = sl + k * S::NS, i = b.i0 - kHalo + r;
-      if (q < nj && r < ni + 6 && (FULL || (i >= kHalo && i < m - kHalo))) {
-        const int e = r * RJ + q + kHalo;
-        L.s_hn[e] = (T(1.0) - io.beta) * L.s_hn[e] + io.beta * hb[e];
-      }
-    }
-    if (side_pt && side_in) {
-      const int e = (sr + kHalo) * RJ + scc;
-      L.s_hn[e] = (T(1.0) - io.beta) * L.s_hn[e] + io.beta * hb[e];
-    }
-    __syncthreads();
-  }
-
-  // faces: upwind tangential component (remap.py:73-95) and kinetic energy (barotr_pure.py:91-92)
-  if (q < nj) {
-#pragma unroll
-    for (int k = 0; k < S::KX; ++k) {
-      const int a = sl + k * S::NS;
-      if (a <= ni) {
-        const int e = a * TJ + q;
-        const T* pt = L.s_v + a * TJ + q;
-        T p6[6];
-#pragma unroll
-        for (int z = 0; z < 6; ++z) p6[z] = pt[z * TJ];
-        const T bc = L.s_xc[e], vis = L.s_xc[S::FX + e];
-        const T vt = bc > T(0.0) ? rplus(p6, 1) : rminus(p6 + 1, 1);
-        L.s_ku[e] = T(0.5) * (vis * vis + vt * vt);
-        L.s_vx[e] = vt * L.s_cdy[e];
-      }
+      for (int z = 0; z < kTerms<T>; ++z) tm[k][z] = tb[z * S::C + c];
     }
   }
 #pragma unroll
-  for (int k = 0; k <= S::KC; ++k) {
-    int r, qq;
-    if (k < S::KC) {
-      r = sl + k * S::NS;
-      qq = q;
-      if (r >= ni || q > nj) continue;
-    } else {
-      r = east_row();
-      qq = TJ;
-      if (nj != TJ || r < 0 || r >= ni) continue;
-    }
-    const int e = r * (TJ + 1) + qq;
-    const T* pt = L.s_u + r * RJ + qq;
-    T p6[6];
-#pragma unroll
-    for (int z = 0; z < 6; ++z) p6[z] = pt[z];
-    const T bc = L.s_yc[e], vis = L.s_yc[S::FY + e];
-    const T ut = bc > T(0.0) ? rplus(p6, 1) : rminus(p6 + 1, 1);
-    L.s_kv[e] = T(0.5) * (vis * vis + ut * ut);
-    L.s_uy[e] = ut * L.s_ddx[e];
+  for (int k = 0; k < S::KP; ++k) {
+    const int p = k * kTileThreads + (int)threadIdx.x;
+    if (p >= S::NP) continue;
+    const RegionPoint<TI, TJ, FULL> pt(b, p);
+    if (!pt.on) continue;
+    sm[pt.r * RJ + pt.c] = blend ? (T(1.0) - io.beta) * hn[k] + io.beta * hs[k] : hn[k];
   }
   __syncthreads();
-
-  if (q < nj) {
 #pragma unroll
-    for (int k = 0; k < S::KC; ++k) {
-      const int a = sl + k * S::NS;
-      if (a >= ni) continue;
-      const int e = a * TJ + q;
-      const int xf0 = e, xf1 = e + TJ;
-      const int yf0 = a * (TJ + 1) + q, yf1 = yf0 + 1;
-      const T* G = L.s_g + 4 * e;
-      const T u = L.s_u[a * RJ + q + kHalo], v = L.s_v[(a + kHalo) * TJ + q], sn = L.s_sn[e];
-      const T uct = (G[0] * u + G[1] * v) * sn, vct = (G[2] * u + G[3] * v) * sn;  // remap.py:34-39
-      const T rdx = L.s_rdx[e], rdy = L.s_rdy[e];
-      // vorticity (agrid.py:31-41) and advection (barotr_pure.py:78-97)
-      const T vort = L.s_rda[e] * (L.s_uy[yf0] + L.s_vx[xf1] - L.s_uy[yf1] - L.s_vx[xf0]);
-      const T advx = vort * vct - (L.s_ku[xf1] - L.s_ku[xf0]) * rdx;
-      const T advy = -vort * uct - (L.s_kv[yf1] - L.s_kv[yf0]) * rdy;
-      // celerity viscosity (barotr_pure.py:63-75) from the cached face fluxes
-      const T visx = -(rdx * (L.s_xc[2 * S::FX + xf1] - L.s_xc[2 * S::FX + xf0]));
-      const T visy = -(rdy * (L.s_yc[2 * S::FY + yf1] - L.s_yc[2 * S::FY + yf0]));
-      // pressure gradient of the new h (agrid.py:55-69, barotr_pure.py:57-60)
-      const T* pbx = L.s_hn + (a * RJ + (q + kHalo));
-      const T* pby = L.s_hn + ((a + kHalo) * RJ + q);
+  for (int k = 0; k < S::KC; ++k) {
+    const int c = k * kTileThreads + (int)threadIdx.x, a = c / TJ, q = c % TJ;
+    if (a < ni && q < nj) {
       T hx[7], hy[7];
 #pragma unroll
       for (int z = 0; z < 7; ++z) {
-        hx[z] = pbx[z * RJ];
-        hy[z] = pby[z];
+        hx[z] = sm[(a + z) * RJ + q + kHalo];
+        hy[z] = sm[(a + kHalo) * RJ + q + z];
       }
-      const T pgu = T(-9.80) * (rdx * (mid6(hx + 1, 1) - mid6(hx, 1)));
-      const T pgv = T(-9.80) * (rdy * (mid6(hy + 1, 1) - mid6(hy, 1)));
-      const T af = L.s_af[e];
-      // momentum update (barotr_pure.py:149-150)
-      const int o = ov + (a + kHalo) * m;
-      io.u_out[o] = upc[k] + (pgu + advx + af * vct + visx) * io.dt;
-      io.v_out[o] = vpc[k] + (pgv + advy - af * uct + visy) * io.dt;
+      const T pgu = T(-9.80) * (pre.rdx[k] * (mid6(hx + 1, 1) - mid6(hx, 1)));
+      const T pgv = T(-9.80) * (pre.rdy[k] * (mid6(hy + 1, 1) - mid6(hy, 1)));
+      const int o = o0 + a * m + q;
+      T u, v;
+      if constexpr (kTerms<T> == 6) {
+        u = upc[k] + (pgu + tm[k][0] + tm[k][1] + tm[k][2]) * io.dt;
+        v = vpc[k] + (pgv + tm[k][3] - tm[k][4] + tm[k][5]) * io.dt;
+      } else {
+        u = upc[k] + (pgu + tm[k][0]) * io.dt;
+        v = vpc[k] + (pgv + tm[k][1]) * io.dt;
+      }
+      io.u_out[o] = u;
+      io.v_out[o] = v;
+      if (!FULL && in_bands(b.i0 + a, b.j0 + q, n)) {
+        // the bands: lon/lat velocity (cube.py:137-145) and normal contravariant component (remap.py:34-39)
+        T c2[4], G[4], sn;
+        if constexpr (UvPre<T, TI, TJ>::kBandHeld) {
+#pragma unroll
+          for (int z = 0; z < 4; ++z) {
+            c2[z] = pre.c2[z];
+            G[z] = pre.g[z];
+          }
+          sn = pre.sn;
+        } else {
+          ld_quad(g.c2l + 4 * (long)o, c2);
+          ld_quad(g.gct + 4 * (long)o, G);
+          sn = g.sina[o];
+        }
+        const T ull = c2[0] * u + c2[1] * v, vll = c2[2] * u + c2[3] * v;
+        const T uct = (G[0] * u + G[1] * v) * sn, vct = (G[2] * u + G[3] * v) * sn;
+        T* const bu = io.band_uv;
+        const int plane = band_plane(n);
+        for_bands(f, b.i0 + a, b.j0 + q, n, [&](int side, int z) {
+          bu[z] = ull;
+          bu[plane + z] = vll;
+          bu[2 * plane + z] = side == kE || side == kW ? vct : uct;
+        });
+      }
     }
   }
 }
@@ -1523,55 +1255,50 @@ __device__ __forceinline__ void tile_uv_main_t(const Geo<T>& g, const StageIO<T>
 // the same tile box.
 template <typename T, int TI, int TJ, bool FP = true>
 __device__ __forceinline__ void tile_h_pro(const Geo<T>& g, const StageIO<T>& io, const TileBox& b, T* sm,
-                                           Gather<T, TI, TJ, false>& gat, EdgeCnt& cnt, int& P) {
+                                           HPre<T, TI, TJ>& pre) {
   if (FP && tile_full(b, g.m, TI, TJ))
-    tile_h_pro_t<T, TI, TJ, true>(g, io, b, sm, gat, cnt, P);
+    tile_h_pro_t<T, TI, TJ, true>(g, io, b, sm, pre);
   else
-    tile_h_pro_t<T, TI, TJ, false>(g, io, b, sm, gat, cnt, P);
+    tile_h_pro_t<T, TI, TJ, false>(g, io, b, sm, pre);
 }
 template <typename T, int TI, int TJ, bool FP = true>
 __device__ __forceinline__ void tile_h_main(const Geo<T>& g, const StageIO<T>& io, const TileBox& b, T* sm,
-                                            Gather<T, TI, TJ, false>& gat, const EdgeCnt& cnt, int P) {
+                                            const HPre<T, TI, TJ>& pre) {
   if (FP && tile_full(b, g.m, TI, TJ))
-    tile_h_main_t<T, TI, TJ, true>(g, io, b, sm, gat, cnt, P);
+    tile_h_main_t<T, TI, TJ, true>(g, io, b, sm, pre);
   else
-    tile_h_main_t<T, TI, TJ, false>(g, io, b, sm, gat, cnt, P);
+    tile_h_main_t<T, TI, TJ, false>(g, io, b, sm, pre);
 }
 template <typename T, int TI, int TJ, bool FP = true>
-__device__ __forceinline__ void tile_uv_pro(const Geo<T>& g, const StageIO<T>& io, const TileBox& b, T* sm,
-                                            Gather<T, TI, TJ, true>& gat, EdgeCnt& cnt, int& P) {
+__device__ __forceinline__ void tile_uv_pro(const Geo<T>& g, const TileBox& b, UvPre<T, TI, TJ>& pre) {
   if (FP && tile_full(b, g.m, TI, TJ))
-    tile_uv_pro_t<T, TI, TJ, true>(g, io, b, sm, gat, cnt, P);
+    tile_uv_pro_t<T, TI, TJ, true>(g, b, pre);
   else
-    tile_uv_pro_t<T, TI, TJ, false>(g, io, b, sm, gat, cnt, P);
+    tile_uv_pro_t<T, TI, TJ, false>(g, b, pre);
 }
 template <typename T, int TI, int TJ, bool FP = true>
 __device__ __forceinline__ void tile_uv_main(const Geo<T>& g, const StageIO<T>& io, const TileBox& b, T* sm,
-                                             Gather<T, TI, TJ, true>& gat, const EdgeCnt& cnt, int P) {
+                                             const UvPre<T, TI, TJ>& pre) {
   if (FP && tile_full(b, g.m, TI, TJ))
-    tile_uv_main_t<T, TI, TJ, true>(g, io, b, sm, gat, cnt, P);
+    tile_uv_main_t<T, TI, TJ, true>(g, io, b, sm, pre);
   else
-    tile_uv_main_t<T, TI, TJ, false>(g, io, b, sm, gat, cnt, P);
+    tile_uv_main_t<T, TI, TJ, false>(g, io, b, sm, pre);
 }
 
 // One tile phase with the prologue issued first (the stream/graph kernels).
 template <typename T, int TI, int TJ, bool FP = true>
 __device__ __forceinline__ void tile_h(const Geo<T>& g, const StageIO<T>& io, const TileBox& b, T* sm) {
-  Gather<T, TI, TJ, false> gat;
-  EdgeCnt cnt;
-  int P;
-  tile_h_pro<T, TI, TJ, FP>(g, io, b, sm, gat, cnt, P);
+  HPre<T, TI, TJ> pre;
+  tile_h_pro<T, TI, TJ, FP>(g, io, b, sm, pre);
   wait_prior_grid();
-  tile_h_main<T, TI, TJ, FP>(g, io, b, sm, gat, cnt, P);
+  tile_h_main<T, TI, TJ, FP>(g, io, b, sm, pre);
 }
 template <typename T, int TI, int TJ, bool FP = true>
 __device__ __forceinline__ void tile_uv(const Geo<T>& g, const StageIO<T>& io, const TileBox& b, T* sm) {
-  Gather<T, TI, TJ, true> gat;
-  EdgeCnt cnt;
-  int P;
-  tile_uv_pro<T, TI, TJ, FP>(g, io, b, sm, gat, cnt, P);
+  UvPre<T, TI, TJ> pre;
+  tile_uv_pro<T, TI, TJ, FP>(g, b, pre);
   wait_prior_grid();
-  tile_uv_main<T, TI, TJ, FP>(g, io, b, sm, gat, cnt, P);
+  tile_uv_main<T, TI, TJ, FP>(g, io, b, sm, pre);
 }
 
 
@@ -1636,6 +1363,10 @@ __device__ __forceinline__ StageIO<T> round_stage(const RoundArgs<T>& a, int ste
   io.u_out = last ? a.x[1] : (st == 0 ? a.y[1] : a.z[1]);
   io.v_out = last ? a.x[2] : (st == 0 ? a.y[2] : a.z[2]);
   io.fx = a.fx;
+  const int sg = step * nst + st;  // the new-h bands alternate between consecutive stages
+  io.band_uv = a.band;
+  io.band_h = a.band + (3 + (sg & 1)) * band_plane(a.g.n);
+  io.band_hn = a.band + (4 - (sg & 1)) * band_plane(a.g.n);
   double dt;
   if (a.rk == 2) {
     dt = st == 0 ? a.dtb / 2.0 : a.dtb;      // barotr.py:50-56
