@@ -37,7 +37,7 @@ CUDA_SOURCES = [("bt_kernels_f64.cu", ["-fmad=false"]), ("bt_kernels_f32.cu", ["
                 ("bt_batch_f32.cu", ["-fmad=true"]), ("bt_batch_capi.cu", ["-fmad=false"]),
                 ("bt_resident_f64.cu", ["-fmad=false"]), ("bt_resident_f32.cu", ["-fmad=true"])]
 CUDA_HEADERS = ["bt_common.cuh", "bt_stencil.cuh", "bt_launch.cuh", "bt_kernels.cuh", "bt_plan.cuh",
-                "bt_batch.cuh", "bt_batch_kernels.cuh", "bt_resident.cuh"]
+                "bt_batch.cuh", "bt_batch_kernels.cuh", "bt_resident.cuh", "bt_fused.cuh"]
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 

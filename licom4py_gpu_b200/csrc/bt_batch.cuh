@@ -25,7 +25,7 @@ struct MemberDesc {
   T* x[3];         // output state (written by the last stage of each substep)
   T* y[3];         // stage scratch
   T* z[3];         // second stage scratch (RK3)
-  T* fx;           // momentum-term blocks
+  T* fx;           // momentum terms
   T* band;         // bands (5 planes)
   T* diag[10];     // STATE_KEYS[6:16] outputs, all null when not wanted
   double dtb;

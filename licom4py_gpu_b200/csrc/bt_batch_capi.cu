@@ -29,7 +29,7 @@ constexpr int kMaxGeo = 16;
 size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 // Member scratch layout: stage fields Y (3) [+ Z (3) for RK3], then the
-// momentum-term blocks and the bands, every part 256-byte aligned.
+// momentum terms and the bands, every part 256-byte aligned.
 struct ScratchLayout {
   size_t field, terms, bands, total;
   int nfields;

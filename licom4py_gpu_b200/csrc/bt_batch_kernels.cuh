@@ -17,6 +17,7 @@ __device__ __forceinline__ Tiling make_tiling_dev(int ti, int tj, int n) {
   t.tj = tj;
   t.nti = (n + ti - 1) / ti;
   t.ntj = (n + tj - 1) / tj;
+  t.bi = t.ri = t.bj = t.rj = t.late = 0;
   return t;
 }
 

@@ -94,7 +94,7 @@ namespace {
 // cube.py:40-127); route[f*4+side] packs the adjacency.
 template <typename T>
 int build_halo_host(int n, const T* coef, const int* li, const int* lj, int2* src, T* w, int* route,
-                    int* bsrc = nullptr) {
+                    int* bsrc = nullptr, bool* near_sources = nullptr) {
   const int m = n + 6, nh = halo_count(m);
   const size_t fe = (size_t)6 * m * m;
   for (int f = 0; f < 6; ++f)
@@ -161,9 +161,28 @@ int build_halo_host(int n, const T* coef, const int* li, const int* lj, int2* sr
             const long o = cell(f, ti, tj, m);
             const int pos = ((dd == kE || dd == kW) ? li[o] : lj[o]) - kHalo;
             bsrc[((f * 4 + dd) * 3 + c) * n + k] = ((nb * 4 + side) * 3 + c) * n + (rev ? n - 1 - pos : pos);
+            // the fused stage kernel's patches (EdgePatch::lo / hi) hold both sources of a halo cell d + 1
+            // outside the edge if they lie at most d + 1 positions towards the edge's middle
+            const int d = dd == kS || dd == kW ? 2 - c : c;
+            const bool first = 2 * k < n;
+            if (near_sources && !(first ? pos >= k && pos <= k + d : pos >= k - 1 - d && pos <= k - 1))
+              *near_sources = false;
           }
       }
   return BT_OK;
+}
+
+// Sizes the fused stage kernel takes: at least two tiles along each axis of a face (a tile touches at most one
+// of two opposite edges), none thinner than 6 cells (the 6 cells around a tile that touches no edge are inside
+// the face) -- and those where it is the faster form.  It saves a launch and a load round trip per stage but
+// forms the velocity of 2.1 x the tile's cells, so it wins while latency bounds the stage: float64 up to two
+// tiles per SM (us per substep, fused / phases: C48 8.9 / 13.1, C64 12.0 / 14.1, C72 14.3 / 14.4; C96, three
+// tiles per SM, 14.4 / 14.1), in RK3, whose blend doubles the h reads, up to one and a half (C64 20.7 / 21.5; C70
+// 23.8 / 22.4), float32 up to six (C48 5.9 / 10.2, C96 8.4 / 10.8, C144 18.4 / 23.0; C128 RK3 25.3 / 27.1).
+bool fused_size(int n, int dtype, int rk, int sms) {
+  const Tiling t = make_even_tiling(kFusedTile, n);
+  const int most = dtype == BT_F32 ? 6 * sms : rk == 2 ? 2 * sms : sms + sms / 2;
+  return t.nti >= 2 && t.ntj >= 2 && t.bi >= 6 && t.bj >= 6 && 6 * t.tiles_per_face() <= most;
 }
 
 template <typename T>
@@ -189,10 +208,15 @@ int build_tables(bt_plan* p, const bt_grid_desc* d) {
   std::vector<int2> src((size_t)6 * nh);
   std::vector<T> w((size_t)6 * nh * 2);
   std::vector<int> bsrc((size_t)72 * p->n);
+  bool near = true;
   const int rc =
-      build_halo_host<T>(p->n, coef.data(), li.data(), lj.data(), src.data(), w.data(), p->route, bsrc.data());
+      build_halo_host<T>(p->n, coef.data(), li.data(), lj.data(), src.data(), w.data(), p->route, bsrc.data(), &near);
   if (rc != BT_OK) return rc;
   p->h_src = src;
+  int sms = 0;
+  BT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device), "device attributes");
+  p->fused = near && fused_size(p->n, p->dtype, 2, sms);
+  p->fused_rk3 = p->fused && fused_size(p->n, p->dtype, 3, sms);
   // one block on the device: weights, sources, band sources (each part a multiple of 16 bytes: nh and n
   // enter six- and 72-fold)
   const size_t wb = w.size() * sizeof(T), sb = src.size() * sizeof(int2), bb = bsrc.size() * sizeof(int);
@@ -245,10 +269,141 @@ cudaError_t run_stage(const bt_plan* p, const Geo<T>& g, const StageIO<T>& io, c
   return e;
 }
 
+// Whether stream and graph rounds of plan p run the fused stage kernel: its tile shape is the plan's, nothing
+// asks for the phase kernels by themselves (their timing, one of their builds), and the plan has the buffers.
+bool fused_round(const bt_plan* p, int rk) {
+  return p->fused && (rk == 2 || p->fused_rk3) && p->tile.ti == kFusedTile.ti && p->tile.tj == kFusedTile.tj && !p->timing && p->full_tiles < 0 &&
+         (p->mode == BT_MODE_STREAM || p->mode == BT_MODE_GRAPH);
+}
+
+// The fused stage kernel's tables and constant blocks, built ahead of the plan's first fused round (like the
+// tile constant blocks: the stream is synchronised, so rounds on any stream may use them afterwards).
+template <typename T>
+int ensure_stage_tables_t(bt_plan* p, cudaStream_t s) {
+  if (p->stage_ready) return BT_OK;
+  cudaError_t e = launch_stage_tables<T>(p->geo_arrays<T>(), p->stage_tables(), s);
+  if (e == cudaSuccess) e = launch_const_blocks<T>(p->geo_arrays<T>(), kFusedTile, true, (T*)p->even_blocks(), s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  if (e != cudaSuccess) return cuda_fail(e, "fused stage tables");
+  p->stage_ready = true;
+  return BT_OK;
+}
+int ensure_stage_tables(bt_plan* p, cudaStream_t s) {
+  return p->dtype == BT_F64 ? ensure_stage_tables_t<double>(p, s) : ensure_stage_tables_t<float>(p, s);
+}
+
+// The diagnostics of the last stage (input h, u, v) and the halo fill of the result.
+template <typename T>
+cudaError_t enqueue_end(const Geo<T>& g, const bt_state_out& out, T* h, T* u, T* v, cudaStream_t s) {
+  if (out.diag[0]) {
+    cudaError_t e = launch_fill_halo<T>(g, h, u, v, s);
+    if (e != cudaSuccess) return e;
+    DiagOut<T> d;
+    T** dp = (T**)&d;
+    for (int k = 0; k < 10; ++k) dp[k] = (T*)out.diag[k];
+    e = launch_diag<T>(g, h, u, v, d, s);
+    if (e != cudaSuccess) return e;
+  }
+  return launch_fill_halo<T>(g, (T*)out.h0, (T*)out.ub, (T*)out.vb, s);
+}
+
+// The launch sequence of one round with the fused stage kernel (bt_fused.cuh):
+// phase H of the first stage, a fused kernel per further stage, phase UV of the
+// last.  h rotates like the stage outputs (scratch 0, scratch 3 in RK3, the
+// output); the velocity of a substep's start alternates between scratch 1, 2
+// and 4, 5.
+template <typename T>
+cudaError_t enqueue_round_fused(const bt_plan* p, const bt_state_in& in, const bt_state_out& out, int nbb, double dtb,
+                                int rk, cudaStream_t s) {
+  const Geo<T> g = p->geo<T>(), ge = p->geo_fused<T>();
+  T* const Yh = (T*)p->scratch_field(0);
+  T* const Zh = (T*)p->scratch_field(3);
+  T* const Xh = (T*)out.h0;
+  T* const ku[2] = {(T*)p->scratch_field(1), (T*)p->scratch_field(4)};
+  T* const kv[2] = {(T*)p->scratch_field(2), (T*)p->scratch_field(5)};
+  T* const fx[2] = {(T*)p->terms(0), (T*)p->terms(1)};
+  T* const band = (T*)p->bands();
+  const size_t plane = (size_t)72 * p->n;
+  const int S = nbb * rk;
+  auto h_of = [&](int st) { return st % rk == 0 ? Xh : st % rk == 1 ? Yh : Zh; };  // input h of stage st >= 1
+  auto h_in = [&](int st) { return st == 0 ? (const T*)in.h0 : (const T*)h_of(st); };
+  auto bands = [&](int st) { return band + (3 + st % 3) * plane; };
+  auto dt_of = [&](int st) {
+    const int k = st % rk;
+    return rk == 2 ? (k == 0 ? dtb / 2.0 : dtb) : (k == 0 ? dtb / 3.0 : k == 1 ? dtb / 2.0 : dtb);
+  };
+  auto base_u = [&](int st) { return st < rk ? (const T*)in.ubp : (const T*)ku[(st / rk) & 1]; };
+  auto base_v = [&](int st) { return st < rk ? (const T*)in.vbp : (const T*)kv[(st / rk) & 1]; };
+  const double beta = rk == 2 ? 0.0 : 1.0;
+  auto stage = [&](int st) {
+    StageIO<T> io = {};
+    io.h = h_in(st);
+    io.hp = st < rk ? (const T*)in.h0p : Xh;
+    io.h_out = h_of(st + 1);
+    io.fx = fx[st & 1];
+    io.band_uv = band;
+    io.band_h = bands(st);
+    io.band_hn = bands(st + 1);
+    io.dt = (T)dt_of(st);
+    io.beta = (T)beta;
+    io.stored_halo = st == 0 ? 1 : 0;
+    io.last = st % rk == rk - 1 ? 1 : 0;
+    return io;
+  };
+  StageIO<T> first = stage(0);
+  first.u = (const T*)in.ub;
+  first.v = (const T*)in.vb;
+  cudaError_t e = launch_phase_h<T>(g, first, p->tile, s);
+  int st0 = 1;
+  if (rk == 3 && e == cudaSuccess) {  // stage 0's phase UV and stage 1's phase H apart
+    first.up = base_u(0);
+    first.vp = base_v(0);
+    first.u_out = ku[0];
+    first.v_out = kv[0];
+    e = launch_phase_uv<T>(g, first, p->tile, s);
+    StageIO<T> second = stage(1);
+    second.u = ku[0];
+    second.v = kv[0];
+    if (e == cudaSuccess) e = launch_phase_h<T>(g, second, p->tile, s);
+    st0 = 2;
+  }
+  for (int st = st0; st < S && e == cudaSuccess; ++st) {
+    FusedIO<T> f;
+    f.io = stage(st);
+    f.h_prev = h_in(st - 1);
+    f.band_hprev = bands(st - 1);
+    f.terms_prev = fx[(st - 1) & 1];
+    f.u_base = base_u(st - 1);
+    f.v_base = base_v(st - 1);
+    f.dt_prev = (T)dt_of(st - 1);
+    f.beta_prev = (T)beta;
+    // kept: the velocity of a substep's start, and the last stage's input for the diagnostics (in the buffer
+    // that is not the last substep's base)
+    const int k = st / rk;
+    f.u_keep = f.v_keep = nullptr;
+    if (st % rk == 0 || (st == S - 1 && out.diag[0])) {
+      const int w = st % rk == 0 ? k & 1 : (k + 1) & 1;
+      f.u_keep = ku[w];
+      f.v_keep = kv[w];
+    }
+    e = launch_stage<T>(ge, f, p->stage_tables(), s);
+  }
+  if (e != cudaSuccess) return e;
+  StageIO<T> last = stage(S - 1);
+  last.up = base_u(S - 1);
+  last.vp = base_v(S - 1);
+  last.u_out = (T*)out.ub;
+  last.v_out = (T*)out.vb;
+  if ((e = launch_phase_uv<T>(g, last, p->tile, s)) != cudaSuccess) return e;
+  const int w = (nbb - 1 + 1) & 1;
+  return enqueue_end<T>(g, out, h_of(S - 1), ku[w], kv[w], s);
+}
+
 // The launch sequence of one round (stream order).
 template <typename T>
 cudaError_t enqueue_round(const bt_plan* p, const bt_state_in& in, const bt_state_out& out, int nbb,
                           double dtb, int rk, cudaStream_t s) {
+  if (fused_round(p, rk)) return enqueue_round_fused<T>(p, in, out, nbb, dtb, rk, s);
   const Geo<T> g = p->geo<T>();
   T* Y[3] = {(T*)p->scratch_field(0), (T*)p->scratch_field(1), (T*)p->scratch_field(2)};
   T* Z[3] = {(T*)p->scratch_field(3), (T*)p->scratch_field(4), (T*)p->scratch_field(5)};
@@ -280,17 +435,8 @@ cudaError_t enqueue_round(const bt_plan* p, const bt_state_in& in, const bt_stat
     }
     if (e != cudaSuccess) return e;
   }
-  if (out.diag[0]) {
-    T* const* L = rk == 2 ? Y : Z;  // input of the last stage
-    e = launch_fill_halo<T>(g, L[0], L[1], L[2], s);
-    if (e != cudaSuccess) return e;
-    DiagOut<T> d;
-    T** dp = (T**)&d;
-    for (int k = 0; k < 10; ++k) dp[k] = (T*)out.diag[k];
-    e = launch_diag<T>(g, L[0], L[1], L[2], d, s);
-    if (e != cudaSuccess) return e;
-  }
-  return launch_fill_halo<T>(g, X[0], X[1], X[2], s);
+  T* const* L = rk == 2 ? Y : Z;  // input of the last stage
+  return enqueue_end<T>(g, out, L[0], L[1], L[2], s);
 }
 
 template <typename T>
@@ -334,7 +480,7 @@ int ensure_const_blocks(bt_plan* p, TileCfg t, cudaStream_t s) {
     slot->ptr = nullptr;
     return BT_OK;
   }
-  cudaError_t e = launch_const_blocks<T>(p->geo_arrays<T>(), t, (T*)slot->ptr, s);
+  cudaError_t e = launch_const_blocks<T>(p->geo_arrays<T>(), t, false, (T*)slot->ptr, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) {
     cudaFree(slot->ptr);
@@ -720,7 +866,8 @@ int bt_round(bt_plan* p, const bt_state_in* in, const bt_state_out* out, int nbb
       if (!out->diag[k]) return fail(BT_EINVAL, "bt_round: diag outputs must be all set or diag[0] NULL");
   cudaStream_t s = (cudaStream_t)stream;
   {
-    const int rc = ensure_const_blocks_any(p, p->tile, s);
+    int rc = ensure_const_blocks_any(p, p->tile, s);
+    if (rc == BT_OK && fused_round(p, rk)) rc = ensure_stage_tables(p, s);
     if (rc != BT_OK) return rc;
   }
   if (p->mode == BT_MODE_RESIDENT)

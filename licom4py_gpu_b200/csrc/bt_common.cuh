@@ -94,8 +94,7 @@ struct StageIO {
   T* h_out;     // stage outputs (interior cells only)
   T* u_out;
   T* v_out;
-  T* fx;        // momentum terms, one block per tile (bt_stencil.cuh, kTerms planes): written by phase
-                // H, read by phase UV of the same tile
+  T* fx;        // momentum terms (bt_stencil.cuh, kTerms planes): written by phase H, read by phase UV
   T* band_uv;   // bands of the stage input's velocity, three planes: lon/lat components and the
                 // contravariant component normal to the band's side (read by phase H, rewritten by phase UV)
   const T* band_h;  // bands of the stage input's h
@@ -117,6 +116,10 @@ struct RoundArgs;
 struct Tiling {
   int ti, tj;        // tile extent (rows, cols)
   int nti, ntj;      // tiles per face along i and j
+  // even split (fused stage kernel): the first ri of the nti tile rows have bi + 1 cells, the others bi, and
+  // alike along j, so that no tile is thinner than half its shape; bi = 0: full tiles and one remainder
+  int bi, ri, bj, rj;
+  int late;          // phase kernels: 1 = release the dependent kernel after the wait for the previous one
   __host__ __device__ int tiles_per_face() const { return nti * ntj; }
 };
 
@@ -141,7 +144,7 @@ struct RoundArgs {
   T* x[3];         // output / running state
   T* y[3];         // stage scratch
   T* z[3];         // second stage scratch (RK3)
-  T* fx;           // momentum-term blocks (phase H -> phase UV)
+  T* fx;           // momentum terms (phase H -> phase UV)
   T* band;         // bands (bt_stencil.cuh): velocity (3 planes), h (2 planes used in turn)
   int nbb, rk;      // substeps of this launch, RK order
   int step0;        // substep index of the launch's first substep within the round (0: reads x0/b0)

@@ -17,11 +17,13 @@
 #include <algorithm>
 #include <atomic>
 
+#include "bt_fused.cuh"
 #include "bt_launch.cuh"
 
 namespace bt {
 
 constexpr int kThreads = 256;  // of the element-wise kernels
+constexpr int kSms = 148;
 
 
 // FP: the full-interior-tile path compiled in (multi-wave launches), else
@@ -29,17 +31,17 @@ constexpr int kThreads = 256;  // of the element-wise kernels
 template <typename T, int TI, int TJ, bool FP>
 __global__ void __launch_bounds__(kTileThreads, kPhaseBlocks) k_phase_h(Geo<T> g, StageIO<T> io, Tiling t) {
   extern __shared__ __align__(16) unsigned char smraw[];
-  release_dependents();
+  if (!t.late) release_dependents();
   const TileBox b = tile_box(t, g.n, blockIdx.x);
-  tile_h<T, TI, TJ, FP>(g, io, b, reinterpret_cast<T*>(smraw));
+  tile_h<T, TI, TJ, FP>(g, io, b, reinterpret_cast<T*>(smraw), t.late);
 }
 
 template <typename T, int TI, int TJ, bool FP>
 __global__ void __launch_bounds__(kTileThreads, PhaseBlocksUV<T, TileShape<TI, TJ>::KP, FP>::value) k_phase_uv(Geo<T> g, StageIO<T> io, Tiling t) {
   extern __shared__ __align__(16) unsigned char smraw[];
-  release_dependents();
+  if (!t.late) release_dependents();
   const TileBox b = tile_box(t, g.n, blockIdx.x);
-  tile_uv<T, TI, TJ, FP>(g, io, b, reinterpret_cast<T*>(smraw));
+  tile_uv<T, TI, TJ, FP>(g, io, b, reinterpret_cast<T*>(smraw), t.late);
 }
 
 // One whole round of one member in a single cooperative launch: every CTA
@@ -152,19 +154,14 @@ bool tile_cfg_supported(TileCfg c) {
          (c.tj == 16 && (c.ti == 8 || c.ti == 16));
 }
 
-namespace {
-template <typename T, int TI, int TJ>
-size_t terms_elems_tile(int n) {
-  const size_t nti = (n + TI - 1) / TI, ntj = (n + TJ - 1) / TJ;
-  return 6 * nti * ntj * (size_t)(kTerms<T> * TI * TJ);
+size_t terms_elems(int n, size_t esize) {
+  size_t most = terms_plane_elems(n, esize);
+  for (TileCfg c : {TileCfg{7, 32}, TileCfg{8, 32}, TileCfg{15, 32}, TileCfg{16, 32}, TileCfg{16, 16}}) {
+    const size_t tiles = (size_t)6 * ((n + c.ti - 1) / c.ti) * ((n + c.tj - 1) / c.tj);
+    most = std::max(most, tiles * c.ti * c.tj * (esize == 8 ? 6 : 2));
+  }
+  return most;
 }
-template <typename T>
-size_t terms_elems_all(int n) {
-  const size_t s[6] = {terms_elems_tile<T, 7, 32>(n),  terms_elems_tile<T, 8, 32>(n), terms_elems_tile<T, 15, 32>(n),
-                       terms_elems_tile<T, 16, 32>(n), terms_elems_tile<T, 8, 16>(n), terms_elems_tile<T, 16, 16>(n)};
-  return *std::max_element(s, s + 6);
-}
-}  // namespace
 
 namespace {
 template <int TI, int TJ>
@@ -184,15 +181,27 @@ size_t const_block_elems(TileCfg c, int n) {
   return 0;
 }
 
-size_t terms_elems(int n, size_t esize) { return esize == 8 ? terms_elems_all<double>(n) : terms_elems_all<float>(n); }
-
 Tiling make_tiling(TileCfg c, int n) {
   Tiling t;
   t.ti = c.ti;
   t.tj = c.tj;
   t.nti = (n + c.ti - 1) / c.ti;
   t.ntj = (n + c.tj - 1) / c.tj;
+  t.bi = t.ri = t.bj = t.rj = t.late = 0;
   return t;
+}
+
+Tiling make_even_tiling(TileCfg c, int n) {
+  Tiling t = make_tiling(c, n);
+  t.bi = n / t.nti;
+  t.ri = n % t.nti;
+  t.bj = n / t.ntj;
+  t.rj = n % t.ntj;
+  return t;
+}
+
+size_t stage_table_bytes(int n, size_t esize) {
+  return (size_t)6 * make_even_tiling(kFusedTile, n).tiles_per_face() * kTileThreads * (3 * sizeof(int4) + 2 * esize);
 }
 #endif
 
@@ -250,6 +259,11 @@ cudaError_t prime_tile() {
   e = cudaFuncSetAttribute(k_round<T, TI, TJ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)round_smem<T, TI, TJ>());
   if (e != cudaSuccess) return e;
+  if constexpr (TI == 8 && TJ == 16) {
+    e = cudaFuncSetAttribute(k_stage<T, TI, TJ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)(sizeof(T) * FusedShape<TI, TJ>::kWords));
+    if (e != cudaSuccess) return e;
+  }
   if ((e = record_wave_slots<T, TI, TJ, false>()) != cudaSuccess) return e;
   return record_wave_slots<T, TI, TJ, true>();
 }
@@ -290,7 +304,11 @@ bool full_path(int n, int full_tiles) {
 template <typename T, int TI, int TJ, bool UV>
 cudaError_t launch_tile(const Geo<T>& g, const StageIO<T>& io, cudaStream_t s, int full_tiles) {
   const size_t smem = tile_smem<T, TI, TJ, UV>();
-  const Tiling t = make_tiling({TI, TJ}, g.n);
+  Tiling t = make_tiling({TI, TJ}, g.n);
+  // up to one tile per SM the next kernel starts only when this one runs: its CTAs, and those of the kernels
+  // after it, would otherwise share SMs with this kernel's while other SMs idle (C48 8 x 16 float64 12.9 -> 12.0
+  // us per substep); with more, the early start is the faster (C384 16 x 16 float64 137 against 165)
+  t.late = 6 * t.tiles_per_face() <= kSms ? 1 : 0;
   const bool fp = full_path<T, TI, TJ, UV>(g.n, full_tiles);
   auto kern = UV ? (fp ? k_phase_uv<T, TI, TJ, true> : k_phase_uv<T, TI, TJ, false>)
                  : (fp ? k_phase_h<T, TI, TJ, true> : k_phase_h<T, TI, TJ, false>);
@@ -369,9 +387,37 @@ cudaError_t launch_phase_uv(const Geo<T>& g, const StageIO<T>& io, TileCfg cfg, 
   return dispatch<T, true>(g, io, cfg, s, full_tiles);
 }
 
+template <typename T>
+cudaError_t launch_stage_tables(const Geo<T>& g, void* out, cudaStream_t s) {
+  const Tiling t = make_even_tiling(kFusedTile, g.n);
+  const int tiles = 6 * t.tiles_per_face();
+  int4* const rec = (int4*)out;
+  k_stage_tables<T, 8, 16><<<tiles, kTileThreads, 0, s>>>(g, t, rec, (T*)(rec + (size_t)tiles * 3 * kTileThreads));
+  return cudaGetLastError();
+}
+
+template <typename T>
+cudaError_t launch_stage(const Geo<T>& g, const FusedIO<T>& p, const void* tables, cudaStream_t s) {
+  using F = FusedShape<8, 16>;
+  const Tiling t = make_even_tiling(kFusedTile, g.n);
+  const int4* const rec = (const int4*)tables;
+  const T* const weights = (const T*)(rec + (size_t)6 * t.tiles_per_face() * 3 * kTileThreads);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(6 * t.tiles_per_face());
+  cfg.blockDim = dim3(kTileThreads);
+  cfg.dynamicSmemBytes = sizeof(T) * (p.beta_prev != T(0) ? F::kWords : F::kHP);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k_stage<T, 8, 16>, g, p, t, rec, weights);
+}
+
 template <typename T, int TI, int TJ>
-cudaError_t launch_const_blocks_tile(const Geo<T>& g, T* out, cudaStream_t s) {
-  const Tiling t = make_tiling({TI, TJ}, g.n);
+cudaError_t launch_const_blocks_tile(const Geo<T>& g, bool even, T* out, cudaStream_t s) {
+  const Tiling t = even ? make_even_tiling({TI, TJ}, g.n) : make_tiling({TI, TJ}, g.n);
   const long total = 6L * t.nti * t.ntj * TileShape<TI, TJ>::cW;
   const int grid = (int)std::min<long>((total + kThreads - 1) / kThreads, 148L * 16);
   k_const_blocks<T, TI, TJ><<<grid, kThreads, 0, s>>>(g, t, out);
@@ -379,13 +425,13 @@ cudaError_t launch_const_blocks_tile(const Geo<T>& g, T* out, cudaStream_t s) {
 }
 
 template <typename T>
-cudaError_t launch_const_blocks(const Geo<T>& g, TileCfg c, T* out, cudaStream_t s) {
-  if (c.ti == 7 && c.tj == 32) return launch_const_blocks_tile<T, 7, 32>(g, out, s);
-  if (c.ti == 8 && c.tj == 32) return launch_const_blocks_tile<T, 8, 32>(g, out, s);
-  if (c.ti == 15 && c.tj == 32) return launch_const_blocks_tile<T, 15, 32>(g, out, s);
-  if (c.ti == 16 && c.tj == 32) return launch_const_blocks_tile<T, 16, 32>(g, out, s);
-  if (c.ti == 8 && c.tj == 16) return launch_const_blocks_tile<T, 8, 16>(g, out, s);
-  if (c.ti == 16 && c.tj == 16) return launch_const_blocks_tile<T, 16, 16>(g, out, s);
+cudaError_t launch_const_blocks(const Geo<T>& g, TileCfg c, bool even, T* out, cudaStream_t s) {
+  if (c.ti == 7 && c.tj == 32) return launch_const_blocks_tile<T, 7, 32>(g, even, out, s);
+  if (c.ti == 8 && c.tj == 32) return launch_const_blocks_tile<T, 8, 32>(g, even, out, s);
+  if (c.ti == 15 && c.tj == 32) return launch_const_blocks_tile<T, 15, 32>(g, even, out, s);
+  if (c.ti == 16 && c.tj == 32) return launch_const_blocks_tile<T, 16, 32>(g, even, out, s);
+  if (c.ti == 8 && c.tj == 16) return launch_const_blocks_tile<T, 8, 16>(g, even, out, s);
+  if (c.ti == 16 && c.tj == 16) return launch_const_blocks_tile<T, 16, 16>(g, even, out, s);
   return cudaErrorInvalidValue;
 }
 
@@ -410,7 +456,9 @@ cudaError_t launch_diag(const Geo<T>& g, const T* h, const T* u, const T* v, con
   template cudaError_t launch_phase_h<T>(const Geo<T>&, const StageIO<T>&, TileCfg, cudaStream_t, int);  \
   template cudaError_t launch_phase_uv<T>(const Geo<T>&, const StageIO<T>&, TileCfg, cudaStream_t, int); \
   template cudaError_t launch_fill_halo<T>(const Geo<T>&, T*, T*, T*, cudaStream_t);                \
-  template cudaError_t launch_const_blocks<T>(const Geo<T>&, TileCfg, T*, cudaStream_t);               \
+  template cudaError_t launch_const_blocks<T>(const Geo<T>&, TileCfg, bool, T*, cudaStream_t);         \
+  template cudaError_t launch_stage_tables<T>(const Geo<T>&, void*, cudaStream_t);                     \
+  template cudaError_t launch_stage<T>(const Geo<T>&, const FusedIO<T>&, const void*, cudaStream_t);   \
   template cudaError_t launch_round<T>(const RoundArgs<T>&, TileCfg, int, cudaStream_t, int*);      \
   template cudaError_t launch_diag<T>(const Geo<T>&, const T*, const T*, const T*, const DiagOut<T>&, \
                                       cudaStream_t);

@@ -17,18 +17,20 @@ struct TileCfg {
 
 // Tile shapes compiled into the library (rows x columns of interior cells).
 bool tile_cfg_supported(TileCfg c);
-// Tile constant blocks (Geo::cblk) for tile shape c: elements needed, and a
-// stream-ordered build from the constant arrays of g.
+// Tile constant blocks (Geo::cblk) for tile shape c (even: the even split):
+// elements needed, and a stream-ordered build from the constant arrays of g.
 size_t const_block_elems(TileCfg c, int n);
 template <typename T>
-cudaError_t launch_const_blocks(const Geo<T>& g, TileCfg c, T* out, cudaStream_t s);
-// Elements of the momentum-term blocks of one member at n cells per face edge
-// in a type of esize bytes, enough for every supported tile shape (the plan's
-// tile can change later).
+cudaError_t launch_const_blocks(const Geo<T>& g, TileCfg c, bool even, T* out, cudaStream_t s);
+// Elements of the momentum terms of one member at n cells per face edge in a
+// type of esize bytes: enough for every supported tile shape (the plan's tile
+// can change later), and for the planes of the 8 x 16 tiles alone.
 size_t terms_elems(int n, size_t esize);
-// Elements of the bands of one member (velocity: 3 planes, h: 2).
-inline size_t band_elems(int n) { return 5 * (size_t)72 * n; }
+inline size_t terms_plane_elems(int n, size_t esize) { return (esize == 8 ? 6 : 2) * (size_t)6 * n * n; }
+// Elements of the bands of one member (velocity: 3 planes, h: 2, or 3 with the fused stage kernel).
+inline size_t band_elems(int n, bool fused = false) { return (fused ? 6 : 5) * (size_t)72 * n; }
 Tiling make_tiling(TileCfg c, int n);
+Tiling make_even_tiling(TileCfg c, int n);
 
 // Set kernel attributes (dynamic shared memory opt-in) for the current device.
 template <typename T>
@@ -45,6 +47,16 @@ template <typename T>
 int phase_full_paths(TileCfg cfg, int n, int full_tiles);
 template <typename T>
 cudaError_t launch_phase_uv(const Geo<T>& g, const StageIO<T>& io, TileCfg cfg, cudaStream_t s, int full_tiles = -1);
+// The fused stage kernel (bt_fused.cuh), its tile shape, and the tables of decoded work it reads (built once
+// per plan, stream ordered).
+constexpr TileCfg kFusedTile{8, 16};
+template <typename T>
+struct FusedIO;
+size_t stage_table_bytes(int n, size_t esize);
+template <typename T>
+cudaError_t launch_stage_tables(const Geo<T>& g, void* out, cudaStream_t s);
+template <typename T>
+cudaError_t launch_stage(const Geo<T>& g, const FusedIO<T>& p, const void* tables, cudaStream_t s);
 // Persistent cooperative launch of a whole round (phases of all substeps);
 // max_ctas > 0 caps the grid.  The grid size used is returned in *grid_out.
 template <typename T>

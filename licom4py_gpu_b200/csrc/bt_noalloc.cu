@@ -12,7 +12,7 @@
 // The array (kScratchBytes, 6 MiB) belongs to every GPU that loads the library
 // and stays allocated until the process exits.  It holds, in this order: a
 // status word, the halo gather tables, the stage fields (3, or 6 for RK3),
-// the momentum-term blocks of the 8 x 16 tiles and the bands.  The sizes it serves: float64 N <= 112 (RK2) /
+// the momentum terms and the bands.  The sizes it serves: float64 N <= 112 (RK2) /
 // 96 (RK3), float32 N <= 160 (RK2) / 136 (RK3); larger sizes are rejected with
 // BT_EINVAL.
 //
@@ -274,9 +274,7 @@ template <typename T>
 int run_noalloc(unsigned char* base, const bt_grid_desc& d, const bt_state_in& in, const bt_state_out& out, int nbb,
                 double dtb, int rk, cudaStream_t s) {
   const int n = d.n, m = n + 6, nh = halo_count(m);
-  // momentum-term blocks of the 8 x 16 tiles this entry point runs
-  const size_t fe = (size_t)6 * m * m,
-               terms = (size_t)6 * ((n + 7) / 8) * ((n + 15) / 16) * (kTerms<T> * TileShape<8, 16>::C);
+  const size_t fe = (size_t)6 * m * m, terms = terms_plane_elems(n, sizeof(T));  // it runs the 8 x 16 tiles
   const size_t o_src = kStatusBytes;
   const size_t o_w = o_src + align256((size_t)6 * nh * sizeof(int2));
   const size_t o_f = o_w + align256((size_t)6 * nh * 2 * sizeof(T));

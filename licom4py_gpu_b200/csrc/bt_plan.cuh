@@ -12,6 +12,7 @@
 #include <cstring>
 #include <vector>
 
+#include "bt_fused.cuh"
 #include "bt_launch.cuh"
 #include "licom_bt.h"
 
@@ -70,6 +71,9 @@ struct bt_plan {
   int max_ctas = 0;
   long long spin_limit = 1ll << 24;
   int full_tiles = -1;  // BT_OPT_FULL_TILES
+  bool fused = false;   // the scratch and the halo tables allow the fused stage kernel
+  bool stage_ready = false;  // its tables and constant blocks are built (first use)
+  bool fused_rk3 = false;  // whether RK3 rounds use it too
   int last_grid = 0;
   // optional kernel timing: event pairs on the launch stream around the round
   // kernel (persistent mode) or each phase kernel (stream mode), with their kind
@@ -100,13 +104,24 @@ struct bt_plan {
 
   size_t esize() const { return dtype == BT_F64 ? 8 : 4; }
   // scratch layout: 6 stage fields, edge lines (24 n), bands, then on a 256-byte boundary the
-  // momentum-term blocks, sized for every tile shape
-  size_t terms_offset() const { return ((6 * field_elems + 24 * (size_t)n + band_elems(n)) * esize() + 255) & ~(size_t)255; }
-  size_t scratch_bytes() const { return terms_offset() + terms_elems(n, esize()) * esize(); }
+  // momentum terms
+  size_t terms_offset() const {
+    return ((6 * field_elems + 24 * (size_t)n + band_elems(n, fused)) * esize() + 255) & ~(size_t)255;
+  }
+  // with the fused stage kernel: a second set of terms, its tables, the constant blocks of its even split
+  size_t stage_offset() const {
+    return (terms_offset() + (fused ? 2 : 1) * terms_elems(n, esize()) * esize() + 255) & ~(size_t)255;
+  }
+  size_t even_offset() const { return (stage_offset() + stage_table_bytes(n, esize()) + 255) & ~(size_t)255; }
+  size_t scratch_bytes() const {
+    return fused ? even_offset() + const_block_elems(kFusedTile, n) * esize() : stage_offset();
+  }
+  void* stage_tables() const { return (char*)scratch + stage_offset(); }
+  void* even_blocks() const { return (char*)scratch + even_offset(); }
   void* scratch_field(int k) const { return (char*)scratch + (size_t)k * field_elems * esize(); }
   void* edge_lines() const { return scratch_field(6); }
   void* bands() const { return (char*)edge_lines() + 24 * (size_t)n * esize(); }
-  void* terms() const { return (char*)scratch + terms_offset(); }
+  void* terms(int k = 0) const { return (char*)scratch + terms_offset() + (size_t)k * terms_elems(n, esize()) * esize(); }
 
   // geometry for kernels of tile shape t (its constant blocks if built)
   template <typename T>
@@ -121,6 +136,15 @@ struct bt_plan {
   template <typename T>
   Geo<T> geo() const {
     return geo_tile<T>(tile);
+  }
+  // geometry for the fused stage kernel
+  template <typename T>
+  Geo<T> geo_fused() const {
+    Geo<T> g = geo_arrays<T>();
+    g.cblk = (const T*)even_blocks();
+    g.cblk_ti = kFusedTile.ti;
+    g.cblk_tj = kFusedTile.tj;
+    return g;
   }
   // geometry without constant blocks (the arrays only)
   template <typename T>

@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(kTileThreads, ResBlocks<T, TI, TJ>::value) k_r
   const TileBox b = tile_box_at(a.t, a.g.n, tile);
   const bool full = tile_full(b, a.g.m, TI, TJ);
   // the constants, once per round (awaited by the first phase's barrier)
-  tile_h_consts<T, TI, TJ>(a.g, b, sm);
+  tile_consts<T, TI, TJ>(a.g, b, LayoutH<T, TI, TJ>(sm));
   const int nst = a.rk == 2 ? 2 : 3;
   const int nstage = a.nbb * nst;
   for (int sg = 0; sg < nstage; ++sg) {

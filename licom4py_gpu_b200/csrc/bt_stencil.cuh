@@ -246,10 +246,14 @@ struct TileShape {
   static constexpr int kWordsUV = up4(RI * RJ);
 };
 
-// Momentum terms of a cell handed from phase H to phase UV, one block of
-// kTerms planes [TI][TJ] per tile.  float64 keeps the three terms of each
-// component apart, because the reference adds them to the pressure gradient one
-// by one (barotr_pure.py:149-150); float32 sums them.
+// Momentum terms of a cell handed from phase H to phase UV, kTerms planes.
+// float64 keeps the three terms of each component apart, because the reference
+// adds them to the pressure gradient one by one (barotr_pure.py:149-150); float32
+// sums them.  The 8 x 16 tiles, whose terms the fused stage kernel reads beyond
+// its own tile, keep planes over the interior cells of the faces, (6, N, N) each;
+// the other shapes a block of planes [TI][TJ] per tile, at offsets known when the
+// kernel is compiled (C384 float64 16 x 16 139.5 -> 137 us per substep, 16 x 32 163
+// -> 155).
 template <typename T>
 constexpr int kTerms = sizeof(T) == 8 ? 6 : 2;
 
@@ -271,10 +275,17 @@ __device__ __forceinline__ int div24(int a, int b) {
 __device__ __forceinline__ TileBox tile_box_rc(const Tiling& t, int n, int f, int ti, int tj) {
   TileBox b;
   b.f = f;
-  b.i0 = kHalo + ti * t.ti;
-  b.j0 = kHalo + tj * t.tj;
-  b.ni = min(t.ti, n - ti * t.ti);
-  b.nj = min(t.tj, n - tj * t.tj);
+  if (t.bi > 0) {  // even split
+    b.i0 = kHalo + ti * t.bi + min(ti, t.ri);
+    b.j0 = kHalo + tj * t.bj + min(tj, t.rj);
+    b.ni = t.bi + (ti < t.ri ? 1 : 0);
+    b.nj = t.bj + (tj < t.rj ? 1 : 0);
+  } else {
+    b.i0 = kHalo + ti * t.ti;
+    b.j0 = kHalo + tj * t.tj;
+    b.ni = min(t.ti, n - ti * t.ti);
+    b.nj = min(t.tj, n - tj * t.tj);
+  }
   b.idx = (f * t.nti + ti) * t.ntj + tj;
   return b;
 }
@@ -333,6 +344,22 @@ __device__ __forceinline__ bool tile_full(const TileBox& b, int m, int ti, int t
 // 32-bit offset of cell (i, j) of face f (fields of up to 2^31 elements).
 __device__ __forceinline__ int cell32(int f, int i, int j, int m) { return (f * m + i) * m + j; }
 
+// Where a tile's momentum terms are.
+template <typename T, int TI, int TJ, bool PLANAR>
+struct TermsAt {
+  T* p;
+  int n;
+  __device__ __forceinline__ TermsAt(T* fx, const TileBox& b, int n_)
+      : p(PLANAR ? fx + (b.f * n_ + b.i0 - kHalo) * n_ + b.j0 - kHalo : fx + (long)b.idx * (kTerms<T> * TI * TJ)),
+        n(n_) {}
+  __device__ __forceinline__ explicit TermsAt(T* block) : p(block), n(0) {}  // a tile's block in shared memory
+  __device__ __forceinline__ T& at(int z, int a, int q) const {
+    return PLANAR ? p[z * (6 * n * n) + a * n + q] : p[z * (TI * TJ) + a * TJ + q];
+  }
+};
+template <int TI, int TJ>
+constexpr bool kPlanarTerms = TI == 8 && TJ == 16;
+
 // ---- asynchronous global -> shared copies ---------------------------------
 template <int BYTES>
 __device__ __forceinline__ void cp_async(void* dst, const void* src) {
@@ -359,6 +386,13 @@ __device__ __forceinline__ void cp_async_mat(T* dst, const T* src) {  // 4 conse
   } else {
     cp_async<16>(dst, src);
   }
+}
+
+// N (2 or 4) consecutive values from an address aligned to two values.
+template <int N, typename T>
+__device__ __forceinline__ void cp_async_pairs(T* dst, const T* src) {
+#pragma unroll
+  for (int k = 0; k < N; k += 2) cp_async<2 * sizeof(T)>(dst + k, src + k);
 }
 
 // One 2x2 matrix (four consecutive values) or one row of it with vector
@@ -472,10 +506,13 @@ struct HaloRef {
   __device__ __forceinline__ void load(const Geo<T>& g, int f, int side, int c, int k) {
     b0 = g.bsrc[band_no(f, side, c, k, g.n)];
     d = route_rev(g.route[f * 4 + side]) ? -1 : 1;  // the next along our edge
-    const int id = side == kS   ? c * g.m + kHalo + k
-                   : side == kN ? (3 + c) * g.m + kHalo + k
-                                : 6 * g.m + (side == kE ? 3 * g.n : 0) + 3 * k + c;
-    ld_pair(g.hw + 2 * (f * g.nh + id), w0, w1);
+    ld_pair(g.hw + 2 * (f * g.nh + halo_word(g, side, c, k)), w0, w1);
+  }
+  // halo_id of a band cell
+  __device__ __forceinline__ static int halo_word(const Geo<T>& g, int side, int c, int k) {
+    return side == kS   ? c * g.m + kHalo + k
+           : side == kN ? (3 + c) * g.m + kHalo + k
+                        : 6 * g.m + (side == kE ? 3 * g.n : 0) + 3 * k + c;
   }
   __device__ __forceinline__ T lerp(const T* band) const { return w0 * band[b0] + w1 * band[b0 + d]; }
 };
@@ -556,6 +593,7 @@ __device__ __forceinline__ void celerity_coef(T hface, T dz, T& c, T& coef) {
 template <typename T, int TI, int TJ>
 struct LayoutH {
   using S = TileShape<TI, TJ>;
+  static constexpr int kSlotS = 0, kSlotN = S::EW, kSlotW = 2 * S::EW, kSlotE = 3 * S::EW;  // neighbour lines
   T *s_h, *s_uc, *s_vc, *s_v, *s_u, *s_g, *s_sn, *s_fx, *s_fy, *s_cell, *s_cdy, *s_ddx, *s_dzx, *s_dzy, *s_np, *s_nh,
       *s_ndz;
   __device__ __forceinline__ explicit LayoutH(T* sm) {
@@ -760,8 +798,8 @@ __device__ __forceinline__ void face_h(const StageIO<T>& io, const T* ph, int sh
 // The tile's cell and face constants (cp.async, not yet awaited): its prepared
 // block with 16-byte copies when the plan has one for this tile shape, else
 // element by element from the constant arrays.
-template <typename T, int TI, int TJ>
-__device__ __forceinline__ void tile_h_consts(const Geo<T>& g, const TileBox& b, T* sm) {
+template <typename T, int TI, int TJ, typename LAY>
+__device__ __forceinline__ void tile_consts(const Geo<T>& g, const TileBox& b, const LAY& L) {
   using S = TileShape<TI, TJ>;
   if (g.cblk != nullptr && g.cblk_ti == TI && g.cblk_tj == TJ) {
     constexpr int V = 16 / sizeof(T);
@@ -769,11 +807,10 @@ __device__ __forceinline__ void tile_h_consts(const Geo<T>& g, const TileBox& b,
 #pragma unroll
     for (int w = 0; w < S::cW; w += kTileThreads * V) {
       const int e = w + (int)threadIdx.x * V;
-      if (w + kTileThreads * V <= S::cW || e < S::cW) cp_async<16>(sm + S::hC + e, blk + e);
+      if (w + kTileThreads * V <= S::cW || e < S::cW) cp_async<16>(L.s_cell + e, blk + e);
     }
     return;
   }
-  const LayoutH<T, TI, TJ> L(sm);
   const int m = g.m, o0 = cell32(b.f, b.i0, b.j0, m);
 #pragma unroll 1
   for (int e = threadIdx.x; e < S::FX; e += kTileThreads) {
@@ -889,8 +926,118 @@ __device__ __forceinline__ void tile_h_points(const Geo<T>& g, const StageIO<T>&
 template <typename T, int TI, int TJ, bool FULL>
 __device__ __forceinline__ void tile_h_pro_t(const Geo<T>& g, const StageIO<T>& io, const TileBox& b, T* sm,
                                              HPre<T, TI, TJ>& pre) {
-  tile_h_consts<T, TI, TJ>(g, b, sm);
+  tile_consts<T, TI, TJ>(g, b, LayoutH<T, TI, TJ>(sm));
   tile_h_points<T, TI, TJ, FULL>(g, io, b, sm, pre);
+}
+
+// The faces of a tile whose region is staged: x faces, then y faces.  When all
+// of them fit one pass they run one copy of the face code with run-time strides
+// (a warp may hold both kinds, and the code is fetched once); else each kind
+// starts at a warp boundary.  hx0 / hy0: the first of the six h values of x face
+// (0, 0) / y face (0, 0), rows HP apart; L: the tile's arrays (LayoutH or alike).
+template <typename T, int TI, int TJ, bool FULL, int HP, typename LAY>
+__device__ __forceinline__ void tile_faces(const StageIO<T>& io, const TileBox& b, int m, int ni, int nj, const T* hx0,
+                                           const T* hy0, const LAY& L) {
+  using S = TileShape<TI, TJ>;
+  constexpr int RJ = S::RJ;
+  auto x_face = [&](int e) {
+    const int a = e / TJ, q = e % TJ;
+    if (!FULL && (a > ni || q >= nj)) return;
+    const int side =
+        FULL ? -1 : ((a == 0 && b.i0 == kHalo) ? kS : ((a == ni && b.i0 + ni == m - kHalo) ? kN : -1));
+    face_h<T>(io, hx0 + a * HP + q, HP, L.s_uc + e, L.s_v + e, TJ, side, (side == kS ? LAY::kSlotS : LAY::kSlotN) + q,
+              L.s_dzx[e], L.s_cdy[e], L.s_np, L.s_nh, L.s_ndz, L.s_fx + e, S::FXP);
+  };
+  auto y_face = [&](int e) {
+    const int r = e / (TJ + 1), q = e - r * (TJ + 1);
+    if (!FULL && (r >= ni || q > nj)) return;
+    const int side =
+        FULL ? -1 : ((q == 0 && b.j0 == kHalo) ? kW : ((q == nj && b.j0 + nj == m - kHalo) ? kE : -1));
+    face_h<T>(io, hy0 + r * HP + q, 1, L.s_vc + r * RJ + q, L.s_u + r * RJ + q, 1, side,
+              (side == kW ? LAY::kSlotW : LAY::kSlotE) + r, L.s_dzy[e], L.s_ddx[e], L.s_np, L.s_nh, L.s_ndz, L.s_fy + e, S::FYP);
+  };
+  if constexpr (S::FX + S::FY <= kTileThreads) {
+    const int t = threadIdx.x;
+    if (t < S::FX + S::FY) {
+      const bool y = t >= S::FX;
+      const int e = y ? t - S::FX : t;
+      const int a = y ? e / (TJ + 1) : e / TJ, q = y ? e - a * (TJ + 1) : e % TJ;
+      const bool on = y ? (a < ni && q <= nj) : (a <= ni && q < nj);
+      if (FULL || on) {
+        int side = -1;
+        if (!FULL) {
+          const int z = y ? q : a, w = y ? nj : ni, i0 = y ? b.j0 : b.i0;
+          if (z == 0 && i0 == kHalo) side = y ? kW : kS;
+          if (z == w && i0 + w == m - kHalo) side = y ? kE : kN;
+        }
+        const int slot = y ? (side == kW ? LAY::kSlotW : LAY::kSlotE) + a : (side == kS ? LAY::kSlotS : LAY::kSlotN) + q;
+        const int at = y ? a * RJ + q : e;
+        face_h<T>(io, (y ? hy0 : hx0) + a * HP + q, y ? 1 : HP,
+                  (y ? L.s_vc : L.s_uc) + at, (y ? L.s_u : L.s_v) + at, y ? 1 : TJ, side, slot,
+                  (y ? L.s_dzy : L.s_dzx)[e], (y ? L.s_ddx : L.s_cdy)[e], L.s_np, L.s_nh, L.s_ndz,
+                  (y ? L.s_fy : L.s_fx) + e, y ? S::FYP : S::FXP);
+      }
+    }
+  } else {
+    constexpr int XS = (S::FX + 31) & ~31;  // y faces start here
+#pragma unroll
+    for (int z = 0; z < XS + S::FY; z += kTileThreads) {
+      const int t = z + (int)threadIdx.x;
+      if (z < S::FX && t < S::FX)
+        x_face(t);
+      else if (z + kTileThreads > XS && t >= XS && t < XS + S::FY)
+        y_face(t - XS);
+    }
+  }
+}
+
+// The cells of a tile whose faces are computed: divergence (agrid.py:43-53) and
+// the h update (barotr_pure.py:119-120), vorticity (agrid.py:31-41), advection
+// (barotr_pure.py:78-97), Coriolis, celerity viscosity (barotr_pure.py:63-75).
+// hpc: the base h of the thread's cells.
+template <typename T, int TI, int TJ, bool FULL, typename LAY, typename TERMS>
+__device__ __forceinline__ void tile_cells(const StageIO<T>& io, const TileBox& b, int n, int m, int ni, int nj,
+                                           const T* hpc, const TERMS& ta, const LAY& L) {
+  using S = TileShape<TI, TJ>;
+  constexpr int RJ = S::RJ;
+  const int f = b.f, o0 = cell32(f, b.i0, b.j0, m);
+#pragma unroll
+  for (int k = 0; k < S::KC; ++k) {
+    const int e = k * kTileThreads + (int)threadIdx.x, a = e / TJ, q = e % TJ;
+    if (a < ni && q < nj) {
+      const T* X = L.s_fx + e;
+      const T* Y = L.s_fy + a * (TJ + 1) + q;
+      const T* c = L.s_cell + e;
+      const T rda = c[0], rdx = c[S::C], rdy = c[2 * S::C], af = c[3 * S::C];
+      const T div = rda * (X[TJ] - X[0] + Y[1] - Y[0]);
+      const T hn = hpc[k] - div * io.dt;
+      io.h_out[o0 + a * m + q] = hn;
+      if (!FULL) for_bands(f, b.i0 + a, b.j0 + q, n, [&](int, int z) { io.band_hn[z] = hn; });
+      const T uct = L.s_uc[(a + kHalo) * TJ + q], vct = L.s_vc[a * RJ + q + kHalo];
+      const T* kx = X + S::FXP;
+      const T* ky = Y + S::FYP;
+      const T* tx = X + 2 * S::FXP;
+      const T* ty = Y + 2 * S::FYP;
+      const T* vx = X + 3 * S::FXP;
+      const T* vy = Y + 3 * S::FYP;
+      const T vort = rda * (ty[0] + tx[TJ] - ty[1] - tx[0]);
+      const T advx = vort * vct - (kx[TJ] - kx[0]) * rdx;
+      const T advy = -vort * uct - (ky[1] - ky[0]) * rdy;
+      const T visx = -(rdx * (vx[TJ] - vx[0]));
+      const T visy = -(rdy * (vy[1] - vy[0]));
+      if constexpr (kTerms<T> == 6) {
+        ta.at(0, a, q) = advx;
+        ta.at(1, a, q) = af * vct;
+        ta.at(2, a, q) = visx;
+        ta.at(3, a, q) = advy;
+        ta.at(4, a, q) = af * uct;
+        ta.at(5, a, q) = visy;
+      } else {
+        ta.at(0, a, q) = advx + af * vct + visx;
+        ta.at(1, a, q) = advy - af * uct + visy;
+      }
+    }
+  }
 }
 
 // Phase H of one tile: writes the new h and the momentum terms of the tile's
@@ -991,102 +1138,12 @@ __device__ __forceinline__ void tile_h_main_t(const Geo<T>& g, const StageIO<T>&
   if (lines) edge_lines<T, S::EW>(b, pre.cnt, pre.P, L.s_np, L.s_nh, L.s_ndz);
   if (!S::kHeld || lines) __syncthreads();
 
-  // faces: x faces, then y faces.  When all of them fit one pass they run
-  // one copy of the face code with run-time strides (a warp may hold both kinds,
-  // and the code is fetched once); else each kind starts at a warp boundary.
-  auto x_face = [&](int e) {
-    const int a = e / TJ, q = e % TJ;
-    if (!FULL && (a > ni || q >= nj)) return;
-    const int side =
-        FULL ? -1 : ((a == 0 && b.i0 == kHalo) ? kS : ((a == ni && b.i0 + ni == m - kHalo) ? kN : -1));
-    face_h<T>(io, L.s_h + a * RJ + q + kHalo, RJ, L.s_uc + e, L.s_v + e, TJ, side, (side == kS ? 0 : S::EW) + q,
-              L.s_dzx[e], L.s_cdy[e], L.s_np, L.s_nh, L.s_ndz, L.s_fx + e, S::FXP);
-  };
-  auto y_face = [&](int e) {
-    const int r = e / (TJ + 1), q = e - r * (TJ + 1);
-    if (!FULL && (r >= ni || q > nj)) return;
-    const int side =
-        FULL ? -1 : ((q == 0 && b.j0 == kHalo) ? kW : ((q == nj && b.j0 + nj == m - kHalo) ? kE : -1));
-    face_h<T>(io, L.s_h + (r + kHalo) * RJ + q, 1, L.s_vc + r * RJ + q, L.s_u + r * RJ + q, 1, side,
-              (side == kW ? 2 : 3) * S::EW + r, L.s_dzy[e], L.s_ddx[e], L.s_np, L.s_nh, L.s_ndz, L.s_fy + e, S::FYP);
-  };
-  if constexpr (S::FX + S::FY <= kTileThreads) {
-    const int t = threadIdx.x;
-    if (t < S::FX + S::FY) {
-      const bool y = t >= S::FX;
-      const int e = y ? t - S::FX : t;
-      const int a = y ? e / (TJ + 1) : e / TJ, q = y ? e - a * (TJ + 1) : e % TJ;
-      const bool on = y ? (a < ni && q <= nj) : (a <= ni && q < nj);
-      if (FULL || on) {
-        int side = -1;
-        if (!FULL) {
-          const int z = y ? q : a, w = y ? nj : ni, i0 = y ? b.j0 : b.i0;
-          if (z == 0 && i0 == kHalo) side = y ? kW : kS;
-          if (z == w && i0 + w == m - kHalo) side = y ? kE : kN;
-        }
-        const int slot = y ? (side == kW ? 2 : 3) * S::EW + a : (side == kS ? 0 : S::EW) + q;
-        const int at = y ? a * RJ + q : e;
-        face_h<T>(io, L.s_h + (y ? (a + kHalo) * RJ + q : a * RJ + q + kHalo), y ? 1 : RJ,
-                  (y ? L.s_vc : L.s_uc) + at, (y ? L.s_u : L.s_v) + at, y ? 1 : TJ, side, slot,
-                  (y ? L.s_dzy : L.s_dzx)[e], (y ? L.s_ddx : L.s_cdy)[e], L.s_np, L.s_nh, L.s_ndz,
-                  (y ? L.s_fy : L.s_fx) + e, y ? S::FYP : S::FXP);
-      }
-    }
-  } else {
-    constexpr int XS = (S::FX + 31) & ~31;  // y faces start here
-#pragma unroll
-    for (int z = 0; z < XS + S::FY; z += kTileThreads) {
-      const int t = z + (int)threadIdx.x;
-      if (z < S::FX && t < S::FX)
-        x_face(t);
-      else if (z + kTileThreads > XS && t >= XS && t < XS + S::FY)
-        y_face(t - XS);
-    }
-  }
+  tile_faces<T, TI, TJ, FULL, RJ>(io, b, m, ni, nj, L.s_h + kHalo, L.s_h + kHalo * RJ, L);
   __syncthreads();
-
-  // cells: divergence (agrid.py:43-53) and the h update (barotr_pure.py:119-120), vorticity
-  // (agrid.py:31-41), advection (barotr_pure.py:78-97), Coriolis, celerity viscosity
-  // (barotr_pure.py:63-75)
-  T* const tb = RES ? rs.terms : io.fx + (long)b.idx * (kTerms<T> * S::C);
-#pragma unroll
-  for (int k = 0; k < S::KC; ++k) {
-    const int e = k * kTileThreads + (int)threadIdx.x, a = e / TJ, q = e % TJ;
-    if (a < ni && q < nj) {
-      const T* X = L.s_fx + e;
-      const T* Y = L.s_fy + a * (TJ + 1) + q;
-      const T* c = L.s_cell + e;
-      const T rda = c[0], rdx = c[S::C], rdy = c[2 * S::C], af = c[3 * S::C];
-      const T div = rda * (X[TJ] - X[0] + Y[1] - Y[0]);
-      const T hn = hpc[k] - div * io.dt;
-      io.h_out[o0 + a * m + q] = hn;
-      if (!FULL) for_bands(f, b.i0 + a, b.j0 + q, n, [&](int, int z) { io.band_hn[z] = hn; });
-      const T uct = L.s_uc[(a + kHalo) * TJ + q], vct = L.s_vc[a * RJ + q + kHalo];
-      const T* kx = X + S::FXP;
-      const T* ky = Y + S::FYP;
-      const T* tx = X + 2 * S::FXP;
-      const T* ty = Y + 2 * S::FYP;
-      const T* vx = X + 3 * S::FXP;
-      const T* vy = Y + 3 * S::FYP;
-      const T vort = rda * (ty[0] + tx[TJ] - ty[1] - tx[0]);
-      const T advx = vort * vct - (kx[TJ] - kx[0]) * rdx;
-      const T advy = -vort * uct - (ky[1] - ky[0]) * rdy;
-      const T visx = -(rdx * (vx[TJ] - vx[0]));
-      const T visy = -(rdy * (vy[1] - vy[0]));
-      T* const t = tb + e;
-      if constexpr (kTerms<T> == 6) {
-        t[0] = advx;
-        t[S::C] = af * vct;
-        t[2 * S::C] = visx;
-        t[3 * S::C] = advy;
-        t[4 * S::C] = af * uct;
-        t[5 * S::C] = visy;
-      } else {
-        t[0] = advx + af * vct + visx;
-        t[S::C] = advy - af * uct + visy;
-      }
-    }
-  }
+  if constexpr (RES)
+    tile_cells<T, TI, TJ, FULL>(io, b, n, m, ni, nj, hpc, TermsAt<T, TI, TJ, false>(rs.terms), L);
+  else
+    tile_cells<T, TI, TJ, FULL>(io, b, n, m, ni, nj, hpc, TermsAt<T, TI, TJ, kPlanarTerms<TI, TJ>>(io.fx, b, n), L);
 }
 
 // ---- phase UV -----------------------------------------------------------------
@@ -1173,7 +1230,12 @@ __device__ __forceinline__ void tile_uv_main_t(const Geo<T>& g, const StageIO<T>
   }
   // base velocities and terms of the thread's cells
   T upc[S::KC], vpc[S::KC], tm[S::KC][kTerms<T>];
-  const T* const tb = RES ? rs.terms : io.fx + (long)b.idx * (kTerms<T> * S::C);
+  const auto ta = [&] {
+    if constexpr (RES)
+      return TermsAt<T, TI, TJ, false>(rs.terms);
+    else
+      return TermsAt<T, TI, TJ, kPlanarTerms<TI, TJ>>(io.fx, b, n);
+  }();
 #pragma unroll
   for (int k = 0; k < S::KC; ++k) {
     const int c = k * kTileThreads + (int)threadIdx.x, a = c / TJ, q = c % TJ;
@@ -1181,7 +1243,7 @@ __device__ __forceinline__ void tile_uv_main_t(const Geo<T>& g, const StageIO<T>
       upc[k] = io.up[o0 + a * m + q];
       vpc[k] = io.vp[o0 + a * m + q];
 #pragma unroll
-      for (int z = 0; z < kTerms<T>; ++z) tm[k][z] = tb[z * S::C + c];
+      for (int z = 0; z < kTerms<T>; ++z) tm[k][z] = ta.at(z, a, q);
     }
   }
 #pragma unroll
@@ -1287,17 +1349,21 @@ __device__ __forceinline__ void tile_uv_main(const Geo<T>& g, const StageIO<T>& 
 
 // One tile phase with the prologue issued first (the stream/graph kernels).
 template <typename T, int TI, int TJ, bool FP = true>
-__device__ __forceinline__ void tile_h(const Geo<T>& g, const StageIO<T>& io, const TileBox& b, T* sm) {
+__device__ __forceinline__ void tile_h(const Geo<T>& g, const StageIO<T>& io, const TileBox& b, T* sm,
+                                       int late = 0) {
   HPre<T, TI, TJ> pre;
   tile_h_pro<T, TI, TJ, FP>(g, io, b, sm, pre);
   wait_prior_grid();
+  if (late) release_dependents();
   tile_h_main<T, TI, TJ, FP>(g, io, b, sm, pre);
 }
 template <typename T, int TI, int TJ, bool FP = true>
-__device__ __forceinline__ void tile_uv(const Geo<T>& g, const StageIO<T>& io, const TileBox& b, T* sm) {
+__device__ __forceinline__ void tile_uv(const Geo<T>& g, const StageIO<T>& io, const TileBox& b, T* sm,
+                                       int late = 0) {
   UvPre<T, TI, TJ> pre;
   tile_uv_pro<T, TI, TJ, FP>(g, b, pre);
   wait_prior_grid();
+  if (late) release_dependents();
   tile_uv_main<T, TI, TJ, FP>(g, io, b, sm, pre);
 }
 
