@@ -47,10 +47,19 @@ def _store(key: str, cfg: dict) -> None:
         pass
 
 
-def heuristic(n: int) -> dict:
+def heuristic(n: int, dtype: Optional[torch.dtype] = None) -> dict:
     """Static choice from B200 measurements: CUDA graphs everywhere (at C48-C96
     the graph with programmatic launch beat the tile-resident and persistent
-    rounds), small tiles for small grids."""
+    rounds), small tiles for small grids.  With ``dtype`` the tile is the fastest
+    one of that type (us per substep): float64 8 x 16 up to C112 (18.8 against 20.7),
+    16 x 16 beyond (C117 20.0 against 23.1; C384 137 against 151 with 8 x 32, 155 with
+    16 x 32); float32 8 x 16 up to C112 (C112 13.8 against 15.4), 8 x 32 up to
+    C160 (C144 16.9 against 20.3), 16 x 32 beyond (C176 22.3 against 24.4)."""
+    if dtype == torch.float64:
+        return {"mode": "graph", "tile": [8, 16] if n <= 112 else [16, 16], "source": "heuristic"}
+    if dtype == torch.float32:
+        tile = [8, 16] if n <= 112 else [8, 32] if n <= 164 else [16, 32]
+        return {"mode": "graph", "tile": tile, "source": "heuristic"}
     if n <= 96:
         return {"mode": "graph", "tile": [8, 16], "source": "heuristic"}
     if n <= 192:
@@ -113,7 +122,7 @@ def choose_config(n: int, dtype: torch.dtype = torch.float64, consts: Optional[S
         if cfg is not None:
             return cfg
     if consts is None:
-        return heuristic(n)
+        return heuristic(n, dtype)
     return tune(n, dtype, consts, dev)
 
 

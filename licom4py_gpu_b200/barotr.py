@@ -24,6 +24,7 @@ from typing import Dict, Sequence, Tuple
 import numpy as np
 import torch
 
+from .autotune import heuristic
 from .plan import BtPlan, DIAG_NAMES, to_device
 
 N_STATE = 23
@@ -48,7 +49,8 @@ def get_plan(consts: Sequence, dtype=torch.float64, device=None) -> BtPlan:
     if plan is None:
         if len(_PLANS) >= _PLAN_CACHE_MAX:
             _PLANS.pop(next(iter(_PLANS))).close()
-        plan = BtPlan(consts, dtype=dtype, device=dev)
+        n = consts[2].shape[-1] - 6  # the drop-in calls pick the tile shape; every shape gives the same result
+        plan = BtPlan(consts, dtype=dtype, device=dev, tile=tuple(heuristic(n, dtype)["tile"]))
         plan._const_refs = tuple(consts[:N_CONSTS])  # keep the key's objects alive
         _PLANS[key] = plan
     return plan
