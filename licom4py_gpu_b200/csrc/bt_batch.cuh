@@ -36,6 +36,7 @@ struct MemberDesc {
 // Prefix offsets of the member list (count + 1 entries each).
 struct BatchOffsets {
   const int* tile;  // tiles of members [0, k)
+  const int* geo;   // index of member k's geometry (not an offset)
   const int* fill;  // halo items of the output fill (6 nh per member)
   const int* lfill; // halo items of the last-stage-input fill (members with diagnostics)
   const int* diag;  // diagnostic cells (6 M^2 per member with diagnostics)

@@ -83,7 +83,8 @@ int batch_round(bt_batch* b, const bt_member* mem, int count, int rk, cudaStream
   MemberDesc<T>* hm = reinterpret_cast<MemberDesc<T>*>(h + b->geo_bytes);
   int* hoff = reinterpret_cast<int*>(h + b->geo_bytes + b->desc_bytes);
   const int stride = b->max_members + 1;
-  int *o_tile = hoff, *o_fill = hoff + stride, *o_lfill = hoff + 2 * stride, *o_diag = hoff + 3 * stride;
+  int *o_tile = hoff, *o_fill = hoff + stride, *o_lfill = hoff + 2 * stride, *o_diag = hoff + 3 * stride,
+      *o_geo = hoff + 4 * stride;
 
   std::vector<const bt_plan*> plans;
   o_tile[0] = o_fill[0] = o_lfill[0] = o_diag[0] = 0;
@@ -122,6 +123,7 @@ int batch_round(bt_batch* b, const bt_member* mem, int count, int rk, cudaStream
     for (int k = 0; k < 10; ++k) md.diag[k] = dg ? (T*)u.out.diag[k] : nullptr;
     md.dtb = u.dtb;
     md.geo = gi;
+    o_geo[q] = gi;
     md.nbb = u.nbb;
     const Tiling t = make_tiling(b->tile, p->n);
     o_tile[q + 1] = o_tile[q] + 6 * t.tiles_per_face();
@@ -141,6 +143,7 @@ int batch_round(bt_batch* b, const bt_member* mem, int count, int rk, cudaStream
   a.off.fill = doff + stride;
   a.off.lfill = doff + 2 * stride;
   a.off.diag = doff + 3 * stride;
+  a.off.geo = doff + 4 * stride;
   a.count = count;
   a.rk = rk;
   a.max_nbb = mem[order[0]].nbb;
@@ -220,7 +223,7 @@ int bt_batch_create(int dtype, int max_members, bt_batch** out) {
   const size_t msz = dtype == BT_F64 ? sizeof(MemberDesc<double>) : sizeof(MemberDesc<float>);
   b->geo_bytes = align256(kMaxGeo * gsz);
   b->desc_bytes = align256((size_t)max_members * msz);
-  b->off_bytes = align256(4 * sizeof(int) * ((size_t)max_members + 1));
+  b->off_bytes = align256(5 * sizeof(int) * ((size_t)max_members + 1));
   b->slot_bytes = b->geo_bytes + b->desc_bytes + b->off_bytes;
   cudaError_t e = dtype == BT_F64 ? prime_batch<double>() : prime_batch<float>();
   if (e != cudaSuccess) {

@@ -36,19 +36,27 @@ __device__ __forceinline__ int member_of(const int* off, int count, int item) {
 
 // The same search by one warp: each round the 32 lanes test 32 evenly spaced
 // offsets of the remaining range at once, so a list of up to 32 members takes
-// one load round trip and up to 1024 two.  Every lane returns the result.
-__device__ __forceinline__ int member_of_warp(const int* off, int count, int item) {
+// one load round trip and up to 1024 two.  Every lane returns the result, the
+// member's offset and its geometry's index (loaded with the offsets).
+__device__ __forceinline__ int member_of_warp(const int* off, const int* geo, int count, int item, int& first,
+                                              int& gi) {
   const int lane = threadIdx.x & 31;
   int lo = 0, hi = count;  // answer in [lo, hi)
-  while (hi - lo > 1) {
+  do {
     const int step = (hi - lo + 31) >> 5;
     const int idx = lo + lane * step;
-    const bool le = idx < hi && __ldg(off + idx) <= item;
-    const unsigned m = __ballot_sync(0xffffffffu, le);  // lane 0 always set: off[lo] <= item
+    int o = 0, q = 0;
+    if (idx < hi) {
+      o = __ldg(off + idx);
+      q = __ldg(geo + idx);
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, idx < hi && o <= item);  // lane 0 always set: off[lo] <= item
     const int last = 31 - __clz(m);
+    first = __shfl_sync(0xffffffffu, o, last);
+    gi = __shfl_sync(0xffffffffu, q, last);
     lo += last * step;
     hi = min(hi, lo + step);
-  }
+  } while (hi - lo > 1);
   return lo;
 }
 
@@ -130,32 +138,58 @@ __device__ __forceinline__ int active_members(const BatchArgs<T>& a, int act, in
   return act;
 }
 
-// Resident CTAs per SM of the batched phase kernels: their member geometry and
-// stage pointers live in shared memory, so the pointers occupy registers; 3
-// CTAs (85 registers) measured faster than 4 (spills) or 2 (occupancy).
-constexpr int kBatchPhaseBlocks = 3;
+// Resident CTAs per SM of the batched phase kernels, whose member geometry and
+// stage pointers live in shared memory, so that the pointers occupy registers.
+// float32 launches of more than one wave: 4 (phase H 56 registers with 52 bytes
+// spilled, phase UV none; a mixed ensemble of 8 C48, 6 C96 and 2 C192 members
+// 4070 -> 3946 us against 3 CTAs of phase H; 5 of phase UV spill and give
+// nothing); else 3.
+template <typename T, bool FP>
+constexpr int kBatchPhaseBlocks = sizeof(T) == 4 && FP ? 4 : 3;
 
 // Tile phase of every active member (one launch per phase): blockIdx.x is the
 // tile in the member-major tile list.  FP: the full-interior-tile path
 // compiled in (launches of more than one wave), else the smaller edge-path-only
 // code (launches whose CTAs all fit at once).
 template <typename T, int TI, int TJ, bool UV, bool FP>
-__global__ void __launch_bounds__(kTileThreads, kBatchPhaseBlocks) k_batch_phase(BatchArgs<T> a, int step, int st, int act) {
+__global__ void __launch_bounds__(kTileThreads, (kBatchPhaseBlocks<T, FP>)) k_batch_phase(BatchArgs<T> a, int step, int st, int act) {
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ TileCtx<T> ctx;
   release_dependents();
+  // Warp 0 finds the member and copies its record and geometry at once: two load round trips ahead of the
+  // tile's own loads
   const int tile = blockIdx.x;
-  __shared__ int s_k;
+  __shared__ int s_first;
   if (threadIdx.x < 32) {
-    const int k = member_of_warp(a.off.tile, act, tile);
-    if (threadIdx.x == 0) s_k = k;
+    int first, gi;
+    const int k = member_of_warp(a.off.tile, a.off.geo, act, tile, first, gi);
+    const int* src = reinterpret_cast<const int*>(a.mem + k);
+    const int* gsrc = reinterpret_cast<const int*>(a.geos + gi);
+    int* dst = reinterpret_cast<int*>(&ctx.d);
+    int* gdst = reinterpret_cast<int*>(&ctx.g);
+    constexpr int nd = sizeof(MemberDesc<T>) / sizeof(int), ng = sizeof(Geo<T>) / sizeof(int);
+    int w[(nd + 31) / 32 + (ng + 31) / 32];
+#pragma unroll
+    for (int q = 0; q < (nd + 31) / 32; ++q)
+      if (q * 32 + (int)threadIdx.x < nd) w[q] = __ldg(src + q * 32 + threadIdx.x);
+#pragma unroll
+    for (int q = 0; q < (ng + 31) / 32; ++q)
+      if (q * 32 + (int)threadIdx.x < ng) w[(nd + 31) / 32 + q] = __ldg(gsrc + q * 32 + threadIdx.x);
+#pragma unroll
+    for (int q = 0; q < (nd + 31) / 32; ++q)
+      if (q * 32 + (int)threadIdx.x < nd) dst[q * 32 + threadIdx.x] = w[q];
+#pragma unroll
+    for (int q = 0; q < (ng + 31) / 32; ++q)
+      if (q * 32 + (int)threadIdx.x < ng) gdst[q * 32 + threadIdx.x] = w[(nd + 31) / 32 + q];
+    __syncwarp();
+    if (threadIdx.x == 0) {
+      ctx.io = member_stage(ctx.d, ctx.g.n, a.rk, step, st);
+      s_first = first;
+    }
   }
-  ctx.k = -1;
   __syncthreads();
-  const int k = s_k;
-  ctx_load(ctx, a, k, step, st);
   const Geo<T>& g = ctx.g;
-  const TileBox b = tile_box_at(make_tiling_dev(TI, TJ, g.n), g.n, tile - __ldg(a.off.tile + k));
+  const TileBox b = tile_box_at(make_tiling_dev(TI, TJ, g.n), g.n, tile - s_first);
   T* sm = reinterpret_cast<T*>(smraw);
   if (!UV)
     tile_h<T, TI, TJ, FP>(g, ctx.io, b, sm);

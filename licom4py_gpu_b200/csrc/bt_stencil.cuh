@@ -200,15 +200,25 @@ __device__ __forceinline__ int yface_side(int j, int m) {
 constexpr int kTileThreads = 288;
 
 // Resident CTAs per SM the phase kernels are compiled for (registers 65536 /
-// (288 * blocks), rounded down to a multiple of 8): 3 in phase H.
-constexpr int kPhaseBlocks = 3;
+// (288 * blocks), rounded down to a multiple of 8).  A tile spends more than half
+// of its time waiting (loads, barriers, the face chain), so what counts in
+// multi-wave launches (FP) is how many tiles share the SM.  Phase H: float32 has
+// the registers for 4 (56; C384 16 x 32 66.6 -> 62.4 us per substep; 5 with 52
+// bytes spilled 61.2 against 59.4, with phase UV at 5), float64 for 3 (72; C384
+// 16 x 16 141.3, with 4 and 60 bytes spilled 153.1).  One-wave launches keep 3:
+// no more tiles are there to share.
+template <typename T, bool FP>
+struct PhaseBlocksH {
+  static constexpr int value = sizeof(T) == 4 && FP ? 4 : 3;
+};
 template <typename T, int KP, bool FP>
 struct PhaseBlocksUV {
   // float64 tiles of two region points per thread in multi-wave launches: 4 (C384 16 x 16 136.7 us per
   // substep against 144.3 at 3, 8 x 32 151.5 against 156.4); in one-wave launches (C96 8 x 32 21.2 at 4
   // against 19.5) and with one point (C48 8 x 16 14.4 against 12.9) or three (C384 16 x 32 156.5
-  // against 154.0): 3
-  static constexpr int value = sizeof(T) == 8 && KP == 2 && FP ? 4 : 3;
+  // against 154.0): 3.  float32 multi-wave: 5 (40 registers; C384 16 x 32 62.4 -> 59.4; 6 with 8 bytes
+  // spilled 59.7).
+  static constexpr int value = sizeof(T) == 4 ? (FP ? 5 : 3) : KP == 2 && FP ? 4 : 3;
 };
 
 constexpr int up4(int x) { return (x + 3) & ~3; }  // shared-memory offsets in words, 16-byte aligned
