@@ -427,12 +427,18 @@ __global__ void __launch_bounds__(kTileThreads, 3)
 
   // ---- ahead of the previous kernel: the thread's work and constants -------------
   const int4* const r = rec + (long)b.idx * 3 * kTileThreads + tid;
-  const int4 re = __ldg(r), rj = __ldg(r + 2 * kTileThreads), rh = __ldg(r + kTileThreads);
-  T w0, w1;
-  ld_pair(weights + ((long)b.idx * kTileThreads + tid) * 2, w0, w1);
-  tile_consts<T, TI, TJ>(g, b, L);
+  const int4 re = __ldg(r);
   EdgeCnt cnt;
   const int P = edge_count(b, m, g.route, cnt);
+  // only tiles at a face edge have halo points, patches and lines: the others need a quarter of the record
+  int4 rj = make_int4(0, 0, 0, -1), rh = make_int4(0, 0, 0, -1);
+  T w0 = T(0.0), w1 = T(0.0);
+  if (P > 0) {
+    rj = __ldg(r + 2 * kTileThreads);
+    rh = __ldg(r + kTileThreads);
+    ld_pair(weights + ((long)b.idx * kTileThreads + tid) * 2, w0, w1);
+  }
+  tile_consts<T, TI, TJ>(g, b, L);
   const int ev = re.z & 3, eo = re.x;
   T* const s_ec = sm + F::kEC;
   if (ev) {

@@ -213,6 +213,25 @@ size_t tile_smem() {
   return sizeof(T) * (UV ? S::kWordsUV : S::kWordsH);
 }
 
+// Shared memory a one-wave float64 launch of up to two tiles per SM asks for at
+// least, so that no SM takes more tiles than an even spread gives it: the CTAs
+// start as those of the kernel before leave, and without the limit the SMs that
+// are done first take three while others get one.  us per substep without / with
+// it: fused kernel C24 8.05 / 7.71, C48 8.87 / 8.24, C64 12.1 / 9.6, C72 14.2 /
+// 10.0; phase kernels C64 14.2 / 13.6, C72 14.5 / 13.1.  The request stays just
+// above the limit, which leaves the rest to L1 (C72 11.7 with all of it).  With
+// three tiles per SM the registers set the limit already and the larger request
+// only costs (C96 14.2 / 14.6, C128 16 x 16 20.9 / 21.8); phase launches of up to
+// one tile per SM are late (launch_tile) and lose with it (C48 12.1 / 12.9);
+// float32 tiles are short enough for the start of the next kernel's tiles beside
+// them to be worth more (C64 6.99 / 7.11).
+template <typename T>
+size_t spread_smem(int tiles) {
+  constexpr size_t per_sm = 228 * 1024, per_cta = 1024;  // sm_100: shared memory of an SM, reserved by each CTA
+  if (sizeof(T) == 4 || tiles > 2 * kSms) return 0;
+  return per_sm / (tiles > kSms ? 3 : 2) - per_cta + 256;
+}
+
 // The persistent kernel runs both phases in one allocation: the larger of the two.
 template <typename T, int TI, int TJ>
 size_t round_smem() {
@@ -248,20 +267,21 @@ cudaError_t record_wave_slots() {
 template <typename T, int TI, int TJ>
 cudaError_t prime_tile() {
   cudaError_t e;
+  const size_t spread = spread_smem<T>(1);  // the most it asks for
   for (auto k : {k_phase_h<T, TI, TJ, true>, k_phase_h<T, TI, TJ, false>})
     if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)tile_smem<T, TI, TJ, false>())) != cudaSuccess)
+                                  (int)std::max(tile_smem<T, TI, TJ, false>(), spread))) != cudaSuccess)
       return e;
   for (auto k : {k_phase_uv<T, TI, TJ, true>, k_phase_uv<T, TI, TJ, false>})
     if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)tile_smem<T, TI, TJ, true>())) != cudaSuccess)
+                                  (int)std::max(tile_smem<T, TI, TJ, true>(), spread))) != cudaSuccess)
       return e;
   e = cudaFuncSetAttribute(k_round<T, TI, TJ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)round_smem<T, TI, TJ>());
   if (e != cudaSuccess) return e;
   if constexpr (TI == 8 && TJ == 16) {
     e = cudaFuncSetAttribute(k_stage<T, TI, TJ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)(sizeof(T) * FusedShape<TI, TJ>::kWords));
+                             (int)std::max(sizeof(T) * FusedShape<TI, TJ>::kWords, spread));
     if (e != cudaSuccess) return e;
   }
   if ((e = record_wave_slots<T, TI, TJ, false>()) != cudaSuccess) return e;
@@ -317,7 +337,7 @@ cudaError_t launch_tile(const Geo<T>& g, const StageIO<T>& io, cudaStream_t s, i
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(6 * t.tiles_per_face());
   cfg.blockDim = dim3(kTileThreads);
-  cfg.dynamicSmemBytes = smem;
+  cfg.dynamicSmemBytes = fp || t.late ? smem : std::max(smem, spread_smem<T>(6 * t.tiles_per_face()));
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -405,7 +425,8 @@ cudaError_t launch_stage(const Geo<T>& g, const FusedIO<T>& p, const void* table
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(6 * t.tiles_per_face());
   cfg.blockDim = dim3(kTileThreads);
-  cfg.dynamicSmemBytes = sizeof(T) * (p.beta_prev != T(0) ? F::kWords : F::kHP);
+  cfg.dynamicSmemBytes = std::max(sizeof(T) * (p.beta_prev != T(0) ? F::kWords : F::kHP),
+                                  spread_smem<T>(6 * t.tiles_per_face()));
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;

@@ -25,7 +25,7 @@ def inputs(g, seed, dtype):
             for a in (s["h0"], b["h0"], s["ub"], s["vb"], b["ub"], b["vb"])]
 
 
-@pytest.mark.parametrize("n", [17, 18, 25, 33, 41, 48, 58, 72])
+@pytest.mark.parametrize("n", [17, 18, 25, 33, 41, 48, 58, 72, 80])
 @pytest.mark.parametrize("rk", [2, 3])
 def test_fused_round_bitwise_equals_phases_f64(n, rk, grids):
     g = grids(n)
