@@ -175,14 +175,15 @@ int build_halo_host(int n, const T* coef, const int* li, const int* lj, int2* sr
 // Sizes the fused stage kernel takes: at least two tiles along each axis of a face (a tile touches at most one
 // of two opposite edges), none thinner than 6 cells (the 6 cells around a tile that touches no edge are inside
 // the face) -- and those where it is the faster form.  It saves a launch and a load round trip per stage but
-// forms the velocity of 2.1 x the tile's cells, so it wins while latency bounds the stage: float64 up to 2.25
-// tiles per SM (us per substep, fused / phases: C48 8.2 / 12.1, C72 10.0 / 13.1, C76 14.1 / 14.5, C80 13.5 / 14.6;
-// C88 14.6 / 14.5 and C96 14.25 / 14.2 with three), in RK3, whose blend doubles the h reads, up to two (C72 16.7 /
-// 20.4; C80 23.4 / 22.4), float32 up to six (C48 5.9 / 10.2, C96 8.4 / 10.8, C144 18.4 / 23.0; C128 RK3 25.3 /
+// forms the velocity of 1.9-2.1 x the tile's cells, so it wins while latency bounds the stage: float64 up to two
+// tiles per SM (us per substep, fused / phases: C48 8.2 / 12.1, C72 10.0 / 13.1, C80 12.0 / 14.5, C96 13.2 / 14.15),
+// in RK3, whose blend doubles the h reads, up to 1.75 of the 12 x 16 tiles (C72 16.7 / 20.4, C80 20.2 / 22.4; C90
+// 22.0 / 21.9, C96 22.0 / 21.7), float32 up to six (C48 5.9 / 10.2, C96 8.2 / 10.8, C144 18.4 / 23.0; C128 RK3 25.3 /
 // 27.1).
 bool fused_size(int n, int dtype, int rk, int sms) {
-  const Tiling t = make_even_tiling(kFusedTile, n);
-  const int most = dtype == BT_F32 ? 6 * sms : rk == 2 ? 2 * sms + sms / 4 : 2 * sms;
+  const TileCfg c = fused_tile(n);
+  const Tiling t = make_even_tiling(c, n);
+  const int most = dtype == BT_F32 ? 6 * sms : rk == 3 && c.ti != kFusedTile.ti ? sms + 3 * sms / 4 : 2 * sms;
   return t.nti >= 2 && t.ntj >= 2 && t.bi >= 6 && t.bj >= 6 && 6 * t.tiles_per_face() <= most;
 }
 
@@ -283,7 +284,7 @@ template <typename T>
 int ensure_stage_tables_t(bt_plan* p, cudaStream_t s) {
   if (p->stage_ready) return BT_OK;
   cudaError_t e = launch_stage_tables<T>(p->geo_arrays<T>(), p->stage_tables(), s);
-  if (e == cudaSuccess) e = launch_const_blocks<T>(p->geo_arrays<T>(), kFusedTile, true, (T*)p->even_blocks(), s);
+  if (e == cudaSuccess) e = launch_const_blocks<T>(p->geo_arrays<T>(), fused_tile(p->n), true, (T*)p->even_blocks(), s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return cuda_fail(e, "fused stage tables");
   p->stage_ready = true;

@@ -60,6 +60,7 @@ struct FusedIO {
 template <int TI, int TJ>
 struct FusedShape {
   using S = TileShape<TI, TJ>;
+  static constexpr int kT = S::kT;
   static constexpr int PW = TJ + 12, HR = TI + 12;  // own h: rows i0 - 6 .., columns j0 - 6 ..
   static constexpr int XA = TJ + 12, XB = TI + 12;  // h patch behind an S/N and a W/E edge: 9 lines each
   static constexpr int OA = TJ + 6, OB = TI + 6;    // evaluated lines, 3 each
@@ -67,15 +68,15 @@ struct FusedShape {
   static constexpr int kJobs = 6 * (TI + TJ), kJobWords = 10;
   // halo points of h and patch points beside the evaluated ones: one per thread
   static constexpr int kHaloA = 3 * S::RJ, kPatchA = 3 * (TJ + 3), kHaloB = 3 * S::RI, kPatchB = 3 * (TI + 3);
-  static_assert(kHaloA + kPatchA + kHaloB + kPatchB + 36 <= kTileThreads, "one halo point per thread");
+  static_assert(kHaloA + kPatchA + kHaloB + kPatchB + 36 <= kT, "one halo point per thread");
   // evaluations of an interior, S/N-edge, W/E-edge and corner tile: one per thread
-  static_assert(S::NP <= kTileThreads && (TI + 3) * TJ + 6 * TI + 3 * TJ + 6 <= kTileThreads &&
-                    S::VB + 6 * TI + 6 <= kTileThreads && (TI + 3) * TJ + 3 * TI + 3 * TJ + 3 * TI + 12 <= kTileThreads,
+  static_assert(S::NP <= kT && (TI + 3) * TJ + 6 * TI + 3 * TJ + 6 <= kT &&
+                    S::VB + 6 * TI + 6 <= kT && (TI + 3) * TJ + 3 * TI + 3 * TJ + 3 * TI + 12 <= kT,
                 "one evaluation per thread");
-  static_assert(kJobs <= kTileThreads && S::C <= kTileThreads, "one pass");
+  static_assert(kJobs <= kT && S::C <= kT, "one pass");
   static constexpr int NE = 2 * S::EW;  // line slots: patch A, patch B
   // evaluation constants per thread: pairs gct, c2l (4), then rdx, rdy, sina
-  static constexpr int kEvalWords = 11 * kTileThreads;
+  static constexpr int kEvalWords = 11 * kT;
   static constexpr int kFaces = 4 * (S::FXP + S::FYP);
   // shared memory (words): h_s, contravariant and raw velocities, evaluation constants (the face
   // results share their memory: evaluated by then), interpolation constants, constant block, lines,
@@ -148,7 +149,7 @@ struct EdgePatch {
 // Line number (0..2, increasing i or j) of the halo cells d + 1 outside side s.
 __device__ __forceinline__ int outer_line(int s, int d) { return s == kS || s == kW ? 2 - d : d; }
 
-// A thread's decoded work (three int4 per thread, planes of kTileThreads):
+// A thread's decoded work (three int4 per thread, planes of S::kT):
 //   0: evaluation: cell offset, position in a terms plane, pack_eval, destination
 //      (region point: row | column << 8; patch: lon/lat word | (line slot + 1) << 9 | y << 20)
 //   1: halo point of h: cell offset, or band number for an interpolated one; its
@@ -170,7 +171,7 @@ struct StageRec {
 
 // Builds the tables of the fused kernel: one CTA per tile.
 template <typename T, int TI, int TJ>
-__global__ void __launch_bounds__(kTileThreads) k_stage_tables(Geo<T> g, Tiling t, int4* rec, T* weights) {
+__global__ void __launch_bounds__(TileShape<TI, TJ>::kT) k_stage_tables(Geo<T> g, Tiling t, int4* rec, T* weights) {
   using S = TileShape<TI, TJ>;
   using F = FusedShape<TI, TJ>;
   constexpr int RJ = S::RJ, PW = F::PW;
@@ -395,11 +396,11 @@ __global__ void __launch_bounds__(kTileThreads) k_stage_tables(Geo<T> g, Tiling 
     jpack = StageRec::pack_job(jb == 2 ? 3 : jside < 2 ? 1 : 2, src, jstep, jdst, jy);
   }
 
-  int4* const r = rec + (long)b.idx * 3 * kTileThreads + tid;
+  int4* const r = rec + (long)b.idx * 3 * S::kT + tid;
   r[0] = make_int4(ev ? eo : 0, et, pack1, pack2);
-  r[kTileThreads] = make_int4(hlerp ? hb : ho, hdst < 0 ? 0 : hdst | ((hlerp ? (hd < 0 ? 3 : 2) : 1) << 12), po, pdst);
-  r[2 * kTileThreads] = make_int4(jpack, jo, jw, jz < 0 ? -1 : jz | (jslot << 24));
-  T* const w = weights + ((long)b.idx * kTileThreads + tid) * 2;
+  r[S::kT] = make_int4(hlerp ? hb : ho, hdst < 0 ? 0 : hdst | ((hlerp ? (hd < 0 ? 3 : 2) : 1) << 12), po, pdst);
+  r[2 * S::kT] = make_int4(jpack, jo, jw, jz < 0 ? -1 : jz | (jslot << 24));
+  T* const w = weights + ((long)b.idx * S::kT + tid) * 2;
   w[0] = w0;
   w[1] = w1;
 }
@@ -411,7 +412,7 @@ __global__ void __launch_bounds__(kTileThreads) k_stage_tables(Geo<T> g, Tiling 
 // substep, two phase kernels per stage / fused: C48 float64 13.1 / 8.9, float32
 // 10.2 / 5.9; C96 float32 10.8 / 8.4; C90 RK3 float32 18.0 / 14.6.
 template <typename T, int TI, int TJ>
-__global__ void __launch_bounds__(kTileThreads, 3)
+__global__ void __launch_bounds__(TileShape<TI, TJ>::kT, TI == 8 ? 3 : 2)
     k_stage(Geo<T> g, FusedIO<T> p, Tiling t, const int4* rec, const T* weights) {
   using S = TileShape<TI, TJ>;
   using F = FusedShape<TI, TJ>;
@@ -426,7 +427,7 @@ __global__ void __launch_bounds__(kTileThreads, 3)
   const bool blend = p.beta_prev != T(0.0);
 
   // ---- ahead of the previous kernel: the thread's work and constants -------------
-  const int4* const r = rec + (long)b.idx * 3 * kTileThreads + tid;
+  const int4* const r = rec + (long)b.idx * 3 * S::kT + tid;
   const int4 re = __ldg(r);
   EdgeCnt cnt;
   const int P = edge_count(b, m, g.route, cnt);
@@ -434,23 +435,23 @@ __global__ void __launch_bounds__(kTileThreads, 3)
   int4 rj = make_int4(0, 0, 0, -1), rh = make_int4(0, 0, 0, -1);
   T w0 = T(0.0), w1 = T(0.0);
   if (P > 0) {
-    rj = __ldg(r + 2 * kTileThreads);
-    rh = __ldg(r + kTileThreads);
-    ld_pair(weights + ((long)b.idx * kTileThreads + tid) * 2, w0, w1);
+    rj = __ldg(r + 2 * S::kT);
+    rh = __ldg(r + S::kT);
+    ld_pair(weights + ((long)b.idx * S::kT + tid) * 2, w0, w1);
   }
   tile_consts<T, TI, TJ>(g, b, L);
   const int ev = re.z & 3, eo = re.x;
   T* const s_ec = sm + F::kEC;
   if (ev) {
     cp_async_pairs<2>(s_ec + 2 * tid, g.gct + 4 * (long)eo);
-    cp_async_pairs<2>(s_ec + 2 * (tid + kTileThreads), g.gct + 4 * (long)eo + 2);
+    cp_async_pairs<2>(s_ec + 2 * (tid + S::kT), g.gct + 4 * (long)eo + 2);
     if (P > 0) {
-      cp_async_pairs<2>(s_ec + 2 * (tid + 2 * kTileThreads), g.c2l + 4 * (long)eo);
-      cp_async_pairs<2>(s_ec + 2 * (tid + 3 * kTileThreads), g.c2l + 4 * (long)eo + 2);
+      cp_async_pairs<2>(s_ec + 2 * (tid + 2 * S::kT), g.c2l + 4 * (long)eo);
+      cp_async_pairs<2>(s_ec + 2 * (tid + 3 * S::kT), g.c2l + 4 * (long)eo + 2);
     }
-    cp_async_t(s_ec + 8 * kTileThreads + tid, g.rdx + eo);
-    cp_async_t(s_ec + 9 * kTileThreads + tid, g.rdy + eo);
-    cp_async_t(s_ec + 10 * kTileThreads + tid, g.sina + eo);
+    cp_async_t(s_ec + 8 * S::kT + tid, g.rdx + eo);
+    cp_async_t(s_ec + 9 * S::kT + tid, g.rdy + eo);
+    cp_async_t(s_ec + 10 * S::kT + tid, g.sina + eo);
   }
   const int jb = rj.x & 3;
   if (jb) {
@@ -472,7 +473,7 @@ __global__ void __launch_bounds__(kTileThreads, 3)
 
   // ---- 1. h, and what the evaluations read -------------------------------------
 #pragma unroll
-  for (int k = 0; k < F::HR * PW; k += kTileThreads) {
+  for (int k = 0; k < F::HR * PW; k += S::kT) {
     const int q = k + tid, row = q / PW, col = q - row * PW, i = b.i0 - 6 + row, j = b.j0 - 6 + col;
     if (q < F::HR * PW && row < ni + 12 && col < nj + 12 && is_interior(i, j, m)) {
       const int o = cell32(f, i, j, m);
@@ -496,8 +497,8 @@ __global__ void __launch_bounds__(kTileThreads, 3)
   const int hk = rh.y >> 12;
   if (hk) {
     const int at = rh.y & 0xfff, e2 = rh.x + (hk == 2 ? 1 : -1);
-    sm[F::kH + at] = hk == 1 ? io.h[rh.x] : w0 * io.band_h[rh.x] + w1 * io.band_h[e2];
-    if (blend) sm[F::kHP + at] = hk == 1 ? p.h_prev[rh.x] : w0 * p.band_hprev[rh.x] + w1 * p.band_hprev[e2];
+    sm[F::kH + at] = hk == 1 ? io.h[rh.x] : lin2(w0, io.band_h[rh.x], w1, io.band_h[e2]);
+    if (blend) sm[F::kHP + at] = hk == 1 ? p.h_prev[rh.x] : lin2(w0, p.band_hprev[rh.x], w1, p.band_hprev[e2]);
   }
   cp_async_wait_all();
   __syncthreads();
@@ -516,12 +517,12 @@ __global__ void __launch_bounds__(kTileThreads, 3)
       const T* const B = sm + F::kHP + at;
 #pragma unroll
       for (int z = 0; z < 7; ++z) {
-        hx[z] = (T(1.0) - p.beta_prev) * hx[z] + p.beta_prev * B[(z - 3) * si];
-        hy[z] = (T(1.0) - p.beta_prev) * hy[z] + p.beta_prev * B[(z - 3) * sj];
+        hx[z] = lin2(T(1.0) - p.beta_prev, hx[z], p.beta_prev, B[(z - 3) * si]);
+        hy[z] = lin2(T(1.0) - p.beta_prev, hy[z], p.beta_prev, B[(z - 3) * sj]);
       }
     }
     // agrid.py:55-69, barotr_pure.py:57-60, 149-150
-    const T rdx = s_ec[8 * kTileThreads + tid], rdy = s_ec[9 * kTileThreads + tid];
+    const T rdx = s_ec[8 * S::kT + tid], rdy = s_ec[9 * S::kT + tid];
     const T pgu = T(-9.80) * (rdx * (mid6(hx + 1, 1) - mid6(hx, 1)));
     const T pgv = T(-9.80) * (rdy * (mid6(hy + 1, 1) - mid6(hy, 1)));
     T u, v;
@@ -534,16 +535,16 @@ __global__ void __launch_bounds__(kTileThreads, 3)
     }
     T G[4];
     ld_pair(s_ec + 2 * tid, G[0], G[1]);
-    ld_pair(s_ec + 2 * (tid + kTileThreads), G[2], G[3]);
-    const T sn = s_ec[10 * kTileThreads + tid];
-    const T uct = (G[0] * u + G[1] * v) * sn, vct = (G[2] * u + G[3] * v) * sn;  // remap.py:34-39
+    ld_pair(s_ec + 2 * (tid + S::kT), G[2], G[3]);
+    const T sn = s_ec[10 * S::kT + tid];
+    const T uct = lin2(G[0], u, G[1], v) * sn, vct = lin2(G[2], u, G[3], v) * sn;  // remap.py:34-39
     T ull = T(0.0), vll = T(0.0);
     if (P > 0) {  // cube.py:137-145
       T c2[4];
-      ld_pair(s_ec + 2 * (tid + 2 * kTileThreads), c2[0], c2[1]);
-      ld_pair(s_ec + 2 * (tid + 3 * kTileThreads), c2[2], c2[3]);
-      ull = c2[0] * u + c2[1] * v;
-      vll = c2[2] * u + c2[3] * v;
+      ld_pair(s_ec + 2 * (tid + 2 * S::kT), c2[0], c2[1]);
+      ld_pair(s_ec + 2 * (tid + 3 * S::kT), c2[2], c2[3]);
+      ull = lin2(c2[0], u, c2[1], v);
+      vll = lin2(c2[2], u, c2[3], v);
     }
     constexpr int WA = 3 * F::OA, WP = 3 * (F::OA + F::OB);  // words of patch A, of both
     if (ev == 1) {
@@ -589,9 +590,9 @@ __global__ void __launch_bounds__(kTileThreads, 3)
       const T* const s = sm + F::kJ + tid * F::kJobWords;
       const T* const src = sm + F::kPU + ((rj.x >> 2) & 0xfff);
       const int step = (rj.x >> 14) & 1 ? -1 : 1, at = (rj.x >> 15) & 0x7fff;
-      const T ull = s[6] * src[0] + s[7] * src[step], vll = s[6] * src[WP] + s[7] * src[WP + step];
-      const T u = s[0] * ull + s[1] * vll, v = s[2] * ull + s[3] * vll;  // cube.py:137-153
-      const T ct = (s[4] * u + s[5] * v) * s[8];
+      const T ull = lin2(s[6], src[0], s[7], src[step]), vll = lin2(s[6], src[WP], s[7], src[WP + step]);
+      const T u = lin2(s[0], ull, s[1], vll), v = lin2(s[2], ull, s[3], vll);  // cube.py:137-153
+      const T ct = lin2(s[4], u, s[5], v) * s[8];
       if (jb == 3) {
         L.s_np[at] = ct;
       } else if (jb == 1) {

@@ -177,6 +177,7 @@ size_t const_block_elems(TileCfg c, int n) {
   if (c.ti == 15 && c.tj == 32) return const_block_elems_tile<15, 32>(n);
   if (c.ti == 16 && c.tj == 32) return const_block_elems_tile<16, 32>(n);
   if (c.ti == 8 && c.tj == 16) return const_block_elems_tile<8, 16>(n);
+  if (c.ti == 12 && c.tj == 16) return const_block_elems_tile<12, 16>(n);
   if (c.ti == 16 && c.tj == 16) return const_block_elems_tile<16, 16>(n);
   return 0;
 }
@@ -200,8 +201,20 @@ Tiling make_even_tiling(TileCfg c, int n) {
   return t;
 }
 
+// Tile shape of the fused stage kernel: 8 x 16, and 12 x 16 (416 threads, two CTAs
+// per SM) where that makes three tiles per SM two: it evaluates 1.9 velocities per
+// cell against 2.1, and two tiles of 13 warps spread evenly.  us per substep, 8 x
+// 16 / 12 x 16: float64 C80 13.5 / 12.0, C96 14.25 /
+// 13.2; float32 C80 8.00 / 7.93, C96 8.31 / 8.17, C90 RK3 14.6 / 14.3.
+TileCfg fused_tile(int n) {
+  const auto tiles = [n](TileCfg c) { return 6 * make_even_tiling(c, n).tiles_per_face(); };
+  const TileCfg wide{12, 16};
+  return tiles(kFusedTile) > 2 * kSms && tiles(wide) <= 2 * kSms ? wide : kFusedTile;
+}
+
 size_t stage_table_bytes(int n, size_t esize) {
-  return (size_t)6 * make_even_tiling(kFusedTile, n).tiles_per_face() * kTileThreads * (3 * sizeof(int4) + 2 * esize);
+  const TileCfg c = fused_tile(n);
+  return (size_t)6 * make_even_tiling(c, n).tiles_per_face() * tile_threads(c.ti) * (3 * sizeof(int4) + 2 * esize);
 }
 #endif
 
@@ -282,6 +295,9 @@ cudaError_t prime_tile() {
   if constexpr (TI == 8 && TJ == 16) {
     e = cudaFuncSetAttribute(k_stage<T, TI, TJ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)std::max(sizeof(T) * FusedShape<TI, TJ>::kWords, spread));
+    if (e != cudaSuccess) return e;
+    e = cudaFuncSetAttribute(k_stage<T, 12, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)std::max(sizeof(T) * FusedShape<12, 16>::kWords, spread));
     if (e != cudaSuccess) return e;
   }
   if ((e = record_wave_slots<T, TI, TJ, false>()) != cudaSuccess) return e;
@@ -407,24 +423,31 @@ cudaError_t launch_phase_uv(const Geo<T>& g, const StageIO<T>& io, TileCfg cfg, 
   return dispatch<T, true>(g, io, cfg, s, full_tiles);
 }
 
-template <typename T>
-cudaError_t launch_stage_tables(const Geo<T>& g, void* out, cudaStream_t s) {
-  const Tiling t = make_even_tiling(kFusedTile, g.n);
+template <typename T, int TI, int TJ>
+static cudaError_t launch_stage_tables_tile(const Geo<T>& g, void* out, cudaStream_t s) {
+  constexpr int kT = TileShape<TI, TJ>::kT;
+  const Tiling t = make_even_tiling({TI, TJ}, g.n);
   const int tiles = 6 * t.tiles_per_face();
   int4* const rec = (int4*)out;
-  k_stage_tables<T, 8, 16><<<tiles, kTileThreads, 0, s>>>(g, t, rec, (T*)(rec + (size_t)tiles * 3 * kTileThreads));
+  k_stage_tables<T, TI, TJ><<<tiles, kT, 0, s>>>(g, t, rec, (T*)(rec + (size_t)tiles * 3 * kT));
   return cudaGetLastError();
 }
 
 template <typename T>
-cudaError_t launch_stage(const Geo<T>& g, const FusedIO<T>& p, const void* tables, cudaStream_t s) {
-  using F = FusedShape<8, 16>;
-  const Tiling t = make_even_tiling(kFusedTile, g.n);
+cudaError_t launch_stage_tables(const Geo<T>& g, void* out, cudaStream_t s) {
+  return fused_tile(g.n).ti == 8 ? launch_stage_tables_tile<T, 8, 16>(g, out, s)
+                                            : launch_stage_tables_tile<T, 12, 16>(g, out, s);
+}
+
+template <typename T, int TI, int TJ>
+static cudaError_t launch_stage_tile(const Geo<T>& g, const FusedIO<T>& p, const void* tables, cudaStream_t s) {
+  using F = FusedShape<TI, TJ>;
+  const Tiling t = make_even_tiling({TI, TJ}, g.n);
   const int4* const rec = (const int4*)tables;
-  const T* const weights = (const T*)(rec + (size_t)6 * t.tiles_per_face() * 3 * kTileThreads);
+  const T* const weights = (const T*)(rec + (size_t)6 * t.tiles_per_face() * 3 * F::kT);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(6 * t.tiles_per_face());
-  cfg.blockDim = dim3(kTileThreads);
+  cfg.blockDim = dim3(F::kT);
   cfg.dynamicSmemBytes = std::max(sizeof(T) * (p.beta_prev != T(0) ? F::kWords : F::kHP),
                                   spread_smem<T>(6 * t.tiles_per_face()));
   cfg.stream = s;
@@ -433,7 +456,13 @@ cudaError_t launch_stage(const Geo<T>& g, const FusedIO<T>& p, const void* table
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k_stage<T, 8, 16>, g, p, t, rec, weights);
+  return cudaLaunchKernelEx(&cfg, k_stage<T, TI, TJ>, g, p, t, rec, weights);
+}
+
+template <typename T>
+cudaError_t launch_stage(const Geo<T>& g, const FusedIO<T>& p, const void* tables, cudaStream_t s) {
+  return fused_tile(g.n).ti == 8 ? launch_stage_tile<T, 8, 16>(g, p, tables, s)
+                                            : launch_stage_tile<T, 12, 16>(g, p, tables, s);
 }
 
 template <typename T, int TI, int TJ>
@@ -452,6 +481,7 @@ cudaError_t launch_const_blocks(const Geo<T>& g, TileCfg c, bool even, T* out, c
   if (c.ti == 15 && c.tj == 32) return launch_const_blocks_tile<T, 15, 32>(g, even, out, s);
   if (c.ti == 16 && c.tj == 32) return launch_const_blocks_tile<T, 16, 32>(g, even, out, s);
   if (c.ti == 8 && c.tj == 16) return launch_const_blocks_tile<T, 8, 16>(g, even, out, s);
+  if (c.ti == 12 && c.tj == 16) return launch_const_blocks_tile<T, 12, 16>(g, even, out, s);
   if (c.ti == 16 && c.tj == 16) return launch_const_blocks_tile<T, 16, 16>(g, even, out, s);
   return cudaErrorInvalidValue;
 }

@@ -47,9 +47,11 @@ template <typename T>
 int phase_full_paths(TileCfg cfg, int n, int full_tiles);
 template <typename T>
 cudaError_t launch_phase_uv(const Geo<T>& g, const StageIO<T>& io, TileCfg cfg, cudaStream_t s, int full_tiles = -1);
-// The fused stage kernel (bt_fused.cuh), its tile shape, and the tables of decoded work it reads (built once
-// per plan, stream ordered).
+// The fused stage kernel (bt_fused.cuh), the tile shape of the phases around it (and of its own tiles, except
+// where fused_tile gives a wider one), and the tables of decoded work it reads (built once per plan, stream
+// ordered).
 constexpr TileCfg kFusedTile{8, 16};
+TileCfg fused_tile(int n);
 template <typename T>
 struct FusedIO;
 size_t stage_table_bytes(int n, size_t esize);

@@ -114,7 +114,7 @@ struct bt_plan {
   }
   size_t even_offset() const { return (stage_offset() + stage_table_bytes(n, esize()) + 255) & ~(size_t)255; }
   size_t scratch_bytes() const {
-    return fused ? even_offset() + const_block_elems(kFusedTile, n) * esize() : stage_offset();
+    return fused ? even_offset() + const_block_elems(fused_tile(n), n) * esize() : stage_offset();
   }
   void* stage_tables() const { return (char*)scratch + stage_offset(); }
   void* even_blocks() const { return (char*)scratch + even_offset(); }
@@ -142,8 +142,9 @@ struct bt_plan {
   Geo<T> geo_fused() const {
     Geo<T> g = geo_arrays<T>();
     g.cblk = (const T*)even_blocks();
-    g.cblk_ti = kFusedTile.ti;
-    g.cblk_tj = kFusedTile.tj;
+    const TileCfg c = fused_tile(n);
+    g.cblk_ti = c.ti;
+    g.cblk_tj = c.tj;
     return g;
   }
   // geometry without constant blocks (the arrays only)

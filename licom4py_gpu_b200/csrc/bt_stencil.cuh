@@ -53,22 +53,32 @@ namespace bt {
 #define BT_M23 (-2.0 / 15.0)
 #define BT_M33 (1.0 / 60.0)
 
+// a x + b y.  float32 names the product that is fused into the sum: left to the
+// compiler the choice differs from kernel to kernel, and with it the last bits of
+// a stage that one kernel or two compute.
+template <typename T>
+__device__ __forceinline__ T lin2(T a, T x, T b, T y) {
+  if constexpr (sizeof(T) == 4)
+    return __fmaf_rn(a, x, __fmul_rn(b, y));
+  else
+    return a * x + b * y;
+}
 // Value at the + face of the centre point of p[0], p[s], .., p[4s] (poly.py:50-56)
 template <typename T>
 __device__ __forceinline__ T rplus(const T* p, int s) {
-  return T(BT_EM23) * p[0] + T(BT_EM13) * p[s] + T(BT_EP03) * p[2 * s] + T(BT_EP13) * p[3 * s] +
+  return lin2(T(BT_EM23), p[0], T(BT_EM13), p[s]) + T(BT_EP03) * p[2 * s] + T(BT_EP13) * p[3 * s] +
          T(BT_EP23) * p[4 * s];
 }
 // Value at the - face of the centre point (poly.py:57-63)
 template <typename T>
 __device__ __forceinline__ T rminus(const T* p, int s) {
-  return T(BT_EP23) * p[0] + T(BT_EP13) * p[s] + T(BT_EP03) * p[2 * s] + T(BT_EM13) * p[3 * s] +
+  return lin2(T(BT_EP23), p[0], T(BT_EP13), p[s]) + T(BT_EP03) * p[2 * s] + T(BT_EM13) * p[3 * s] +
          T(BT_EM23) * p[4 * s];
 }
 // 6-point centred face value between p[2s] and p[3s] (poly.py:120-124)
 template <typename T>
 __device__ __forceinline__ T mid6(const T* p, int s) {
-  return T(BT_M13) * (p[2 * s] + p[3 * s]) + T(BT_M23) * (p[s] + p[4 * s]) +
+  return lin2(T(BT_M13), p[2 * s] + p[3 * s], T(BT_M23), p[s] + p[4 * s]) +
          T(BT_M33) * (p[0] + p[5 * s]);
 }
 // Gravity-wave speed with the 10 m/s floor (barotr_pure.py:21-26); NaN propagates like jnp.maximum.
@@ -91,7 +101,7 @@ __device__ __forceinline__ T fetch_s(const T* F, const Geo<T>& g, int f, int i, 
   const int k = f * g.nh + halo_id(i, j, m);
   const int2 s = g.hsrc[k];
   const T w0 = g.hw[2 * k], w1 = g.hw[2 * k + 1];
-  return w0 * F[s.x] + w1 * F[s.y];
+  return lin2(w0, F[s.x], w1, F[s.y]);
 }
 
 // Vector (covariant u, v) at (f, i, j): the halo value is rotated to lon/lat at
@@ -113,20 +123,20 @@ __device__ __forceinline__ void fetch_v(const T* U, const T* V, const Geo<T>& g,
   const T* C0 = g.c2l + 4 * (long)s.x;
   const T* C1 = g.c2l + 4 * (long)s.y;
   const T u0 = U[s.x], v0 = V[s.x], u1 = U[s.y], v1 = V[s.y];
-  const T ull0 = C0[0] * u0 + C0[1] * v0, vll0 = C0[2] * u0 + C0[3] * v0;
-  const T ull1 = C1[0] * u1 + C1[1] * v1, vll1 = C1[2] * u1 + C1[3] * v1;
-  const T ull = w0 * ull0 + w1 * ull1;
-  const T vll = w0 * vll0 + w1 * vll1;
+  const T ull0 = lin2(C0[0], u0, C0[1], v0), vll0 = lin2(C0[2], u0, C0[3], v0);
+  const T ull1 = lin2(C1[0], u1, C1[1], v1), vll1 = lin2(C1[2], u1, C1[3], v1);
+  const T ull = lin2(w0, ull0, w1, ull1);
+  const T vll = lin2(w0, vll0, w1, vll1);
   const T* L = g.l2c + 4 * o;
-  u = L[0] * ull + L[1] * vll;
-  v = L[2] * ull + L[3] * vll;
+  u = lin2(L[0], ull, L[1], vll);
+  v = lin2(L[2], ull, L[3], vll);
 }
 
 // Contravariant component along axis -2 (x) or axis -1 (y) (remap.py:34-39)
 template <typename T>
 __device__ __forceinline__ T contra(const Geo<T>& g, long o, T u, T v, int y) {
   const T* G = g.gct + 4 * o;
-  return y ? (G[2] * u + G[3] * v) * g.sina[o] : (G[0] * u + G[1] * v) * g.sina[o];
+  return y ? lin2(G[2], u, G[3], v) * g.sina[o] : lin2(G[0], u, G[1], v) * g.sina[o];
 }
 
 // ---------------------------------------------------------------------------
@@ -198,6 +208,10 @@ __device__ __forceinline__ int yface_side(int j, int m) {
 // chain, not two; 8 x 32 and 16 x 16 tiles need two (552 and 544 faces; three
 // with 256 threads), 16 x 32 four (1072).
 constexpr int kTileThreads = 288;
+// Threads of a TI x TJ tile's CTA: 416 for the fused kernel's 12 x 16 tiles (360
+// region points, 412 faces).
+constexpr int tile_threads(int ti) { return ti == 12 ? 416 : kTileThreads; }
+
 
 // Resident CTAs per SM the phase kernels are compiled for (registers 65536 /
 // (288 * blocks), rounded down to a multiple of 8).  A tile spends more than half
@@ -226,6 +240,7 @@ constexpr int up4(int x) { return (x + 3) & ~3; }  // shared-memory offsets in w
 template <int TI, int TJ>
 struct TileShape {
   static_assert(TJ == 16 || TJ == 32, "tile columns must be 16 or 32");
+  static constexpr int kT = tile_threads(TI);
   static constexpr int RI = TI + 6, RJ = TJ + 6;    // stencil region
   static constexpr int VB = RI * TJ;                // vertical-bar points (r * TJ + q)
   static constexpr int NP = VB + 6 * TI;            // region points: vertical bar, then 3 W + 3 E columns per tile row
@@ -234,8 +249,8 @@ struct TileShape {
   static constexpr int C = TI * TJ;                 // cells (a * TJ + q)
   static constexpr int EW = TI > TJ ? TI : TJ;
   static constexpr int NE = 4 * EW;                 // edge slots: 4 kinds x max(TI, TJ) positions
-  static constexpr int KP = (NP + kTileThreads - 1) / kTileThreads;  // region points per thread
-  static constexpr int KC = (C + kTileThreads - 1) / kTileThreads;   // cells per thread
+  static constexpr int KP = (NP + kT - 1) / kT;  // region points per thread
+  static constexpr int KC = (C + kT - 1) / kT;   // cells per thread
   // with one region point per thread its constants (metric, halo weights) are held in registers
   // across the wait for the previous phase; with more they are staged in shared memory
   static constexpr bool kHeld = KP == 1;
@@ -524,7 +539,7 @@ struct HaloRef {
            : side == kN ? (3 + c) * g.m + kHalo + k
                         : 6 * g.m + (side == kE ? 3 * g.n : 0) + 3 * k + c;
   }
-  __device__ __forceinline__ T lerp(const T* band) const { return w0 * band[b0] + w1 * band[b0 + d]; }
+  __device__ __forceinline__ T lerp(const T* band) const { return lin2(w0, band[b0], w1, band[b0 + d]); }
 };
 
 // Halo velocity (ext_vector, cube.py:137-153) from the bands' lon/lat velocity
@@ -532,8 +547,8 @@ struct HaloRef {
 template <typename T>
 __device__ __forceinline__ void halo_uv(const StageIO<T>& io, const HaloRef<T>& r, int plane, const T* l2, T& u, T& v) {
   const T ull = r.lerp(io.band_uv), vll = r.lerp(io.band_uv + plane);
-  u = l2[0] * ull + l2[1] * vll;
-  v = l2[2] * ull + l2[3] * vll;
+  u = lin2(l2[0], ull, l2[1], vll);
+  v = lin2(l2[2], ull, l2[3], vll);
 }
 
 // Words of one band plane.
@@ -719,7 +734,7 @@ __device__ __forceinline__ void line_outside(const StageIO<T>& io, int slot, con
                                              const LayoutH<T, TI, TJ>& L) {
   T u, v;
   halo_uv(io, w.ref, plane, w.l2, u, v);
-  L.s_np[slot] = (w.g0 * u + w.g1 * v) * w.sn;  // remap.py:34-39
+  L.s_np[slot] = lin2(w.g0, u, w.g1, v) * w.sn;  // remap.py:34-39
   if (io.last) L.s_nh[slot] = w.ref.lerp(io.band_h);
 }
 // Both points of a line read directly (first stage of a round: the halo cells are stored).
@@ -791,16 +806,16 @@ __device__ __forceinline__ void face_h(const StageIO<T>& io, const T* ph, int sh
   T cc, coef;
   celerity_coef(mid6(hh, 1), dz, cc, coef);
   const T vis = bc + coef * (he - hw);
-  T fl = dz * vis + (vis > T(0.0) ? he : hw) * vis;
+  T fl = lin2(dz, vis, vis > T(0.0) ? he : hw, vis);
   if (io.last && side >= 0) {  // the neighbour's flux at the same edge face (barotr_pure.py:29-49)
     const T* nh = s_nh + 6 * slot;
     const T ndz = s_ndz[slot];
     const T nvis = bc + nh[2] * (nh[0] - nh[1]);
-    fl = (fl + (ndz * nvis + (nvis > T(0.0) ? nh[0] : nh[1]) * nvis)) / T(2.0);
+    fl = (fl + lin2(ndz, nvis, nvis > T(0.0) ? nh[0] : nh[1], nvis)) / T(2.0);
   }
   const T vt = bc > T(0.0) ? rplus(tt, 1) : rminus(tt + 1, 1);
   fo[0] = fl * len;
-  fo[plane] = T(0.5) * (vis * vis + vt * vt);
+  fo[plane] = T(0.5) * lin2(vis, vis, vt, vt);
   fo[2 * plane] = vt * len;
   fo[3 * plane] = T(0.5) * cc * (ue - uw);
 }
@@ -815,15 +830,15 @@ __device__ __forceinline__ void tile_consts(const Geo<T>& g, const TileBox& b, c
     constexpr int V = 16 / sizeof(T);
     const T* blk = g.cblk + (long)b.idx * S::cW;
 #pragma unroll
-    for (int w = 0; w < S::cW; w += kTileThreads * V) {
+    for (int w = 0; w < S::cW; w += S::kT * V) {
       const int e = w + (int)threadIdx.x * V;
-      if (w + kTileThreads * V <= S::cW || e < S::cW) cp_async<16>(L.s_cell + e, blk + e);
+      if (w + S::kT * V <= S::cW || e < S::cW) cp_async<16>(L.s_cell + e, blk + e);
     }
     return;
   }
   const int m = g.m, o0 = cell32(b.f, b.i0, b.j0, m);
 #pragma unroll 1
-  for (int e = threadIdx.x; e < S::FX; e += kTileThreads) {
+  for (int e = threadIdx.x; e < S::FX; e += S::kT) {
     const int a = e / TJ, q = e % TJ, o = o0 + a * m + q;
     if (a > b.ni || q >= b.nj) continue;
     cp_async_t(L.s_dzx + e, g.dzph_x + o);
@@ -835,7 +850,7 @@ __device__ __forceinline__ void tile_consts(const Geo<T>& g, const TileBox& b, c
     cp_async_t(L.s_cell + 3 * S::C + e, g.a_f + o);
   }
 #pragma unroll 1
-  for (int e = threadIdx.x; e < S::FY; e += kTileThreads) {
+  for (int e = threadIdx.x; e < S::FY; e += S::kT) {
     const int r = e / (TJ + 1), q = e - r * (TJ + 1), o = o0 + r * m + q;
     if (r >= b.ni || q > b.nj) continue;
     cp_async_t(L.s_dzy + e, g.dzph_y + o);
@@ -871,7 +886,7 @@ template <int TI, int TJ>
 __device__ __forceinline__ int line_first() {
   constexpr int line_thread0 = kHalo * TJ;
   const int t = (int)threadIdx.x - line_thread0;
-  return t >= 0 ? t : t + kTileThreads;
+  return t >= 0 ? t : t + TileShape<TI, TJ>::kT;
 }
 
 // Metric, halo sources and line constants of the tile.
@@ -886,7 +901,7 @@ __device__ __forceinline__ void tile_h_points(const Geo<T>& g, const StageIO<T>&
   bool halo = false;
 #pragma unroll
   for (int k = 0; k < S::KP; ++k) {
-    const int p = k * kTileThreads + (int)threadIdx.x;
+    const int p = k * S::kT + (int)threadIdx.x;
     if (p >= S::NP) continue;
     const RegionPoint<TI, TJ, FULL> pt(b, p);
     if (!pt.on) continue;
@@ -913,10 +928,10 @@ __device__ __forceinline__ void tile_h_points(const Geo<T>& g, const StageIO<T>&
   }
   if (!FULL && pre.P > 0) {
 #pragma unroll 1
-    for (int t = line_first<TI, TJ>(); t < 3 * pre.P; t += kTileThreads) {
+    for (int t = line_first<TI, TJ>(); t < 3 * pre.P; t += S::kT) {
       const LinePoint lp(b, pre.cnt, pre.P, t, g.n, S::EW);
       if (io.last) line_depth<T, TI, TJ>(g, lp, L);
-      if (S::kHeld && !io.stored_halo && t < kTileThreads) {
+      if (S::kHeld && !io.stored_halo && t < S::kT) {
         if (!HPre<T, TI, TJ>::kLineHeld) {
           pre.slot = lp.slot_out;
           pre.lref.load(g, lp.nb, lp.ns, lp.d, lp.kk);
@@ -966,7 +981,7 @@ __device__ __forceinline__ void tile_faces(const StageIO<T>& io, const TileBox& 
     face_h<T>(io, hy0 + r * HP + q, 1, L.s_vc + r * RJ + q, L.s_u + r * RJ + q, 1, side,
               (side == kW ? LAY::kSlotW : LAY::kSlotE) + r, L.s_dzy[e], L.s_ddx[e], L.s_np, L.s_nh, L.s_ndz, L.s_fy + e, S::FYP);
   };
-  if constexpr (S::FX + S::FY <= kTileThreads) {
+  if constexpr (S::FX + S::FY <= S::kT) {
     const int t = threadIdx.x;
     if (t < S::FX + S::FY) {
       const bool y = t >= S::FX;
@@ -991,11 +1006,11 @@ __device__ __forceinline__ void tile_faces(const StageIO<T>& io, const TileBox& 
   } else {
     constexpr int XS = (S::FX + 31) & ~31;  // y faces start here
 #pragma unroll
-    for (int z = 0; z < XS + S::FY; z += kTileThreads) {
+    for (int z = 0; z < XS + S::FY; z += S::kT) {
       const int t = z + (int)threadIdx.x;
       if (z < S::FX && t < S::FX)
         x_face(t);
-      else if (z + kTileThreads > XS && t >= XS && t < XS + S::FY)
+      else if (z + S::kT > XS && t >= XS && t < XS + S::FY)
         y_face(t - XS);
     }
   }
@@ -1013,7 +1028,7 @@ __device__ __forceinline__ void tile_cells(const StageIO<T>& io, const TileBox& 
   const int f = b.f, o0 = cell32(f, b.i0, b.j0, m);
 #pragma unroll
   for (int k = 0; k < S::KC; ++k) {
-    const int e = k * kTileThreads + (int)threadIdx.x, a = e / TJ, q = e % TJ;
+    const int e = k * S::kT + (int)threadIdx.x, a = e / TJ, q = e % TJ;
     if (a < ni && q < nj) {
       const T* X = L.s_fx + e;
       const T* Y = L.s_fy + a * (TJ + 1) + q;
@@ -1031,8 +1046,8 @@ __device__ __forceinline__ void tile_cells(const StageIO<T>& io, const TileBox& 
       const T* vx = X + 3 * S::FXP;
       const T* vy = Y + 3 * S::FYP;
       const T vort = rda * (ty[0] + tx[TJ] - ty[1] - tx[0]);
-      const T advx = vort * vct - (kx[TJ] - kx[0]) * rdx;
-      const T advy = -vort * uct - (ky[1] - ky[0]) * rdy;
+      const T advx = lin2(vort, vct, -(kx[TJ] - kx[0]), rdx);
+      const T advy = lin2(-vort, uct, -(ky[1] - ky[0]), rdy);
       const T visx = -(rdx * (vx[TJ] - vx[0]));
       const T visy = -(rdy * (vy[1] - vy[0]));
       if constexpr (kTerms<T> == 6) {
@@ -1067,7 +1082,7 @@ __device__ __forceinline__ void tile_h_main_t(const Geo<T>& g, const StageIO<T>&
   T hv[S::KP], uv[S::KP], vv[S::KP], hpc[S::KC];
 #pragma unroll
   for (int k = 0; k < S::KP; ++k) {
-    const int p = k * kTileThreads + (int)threadIdx.x;
+    const int p = k * S::kT + (int)threadIdx.x;
     if (p >= S::NP) continue;
     const RegionPoint<TI, TJ, FULL> pt(b, p);
     if (!pt.on) continue;
@@ -1090,12 +1105,12 @@ __device__ __forceinline__ void tile_h_main_t(const Geo<T>& g, const StageIO<T>&
   }
 #pragma unroll
   for (int k = 0; k < S::KC; ++k) {
-    const int c = k * kTileThreads + (int)threadIdx.x, a = c / TJ, q = c % TJ;
+    const int c = k * S::kT + (int)threadIdx.x, a = c / TJ, q = c % TJ;
     if (a < ni && q < nj) hpc[k] = io.hp[o0 + a * m + q];
   }
   if (!FULL && pre.P > 0) {
 #pragma unroll 1
-    for (int t = line_first<TI, TJ>(); t < 3 * pre.P; t += kTileThreads) {
+    for (int t = line_first<TI, TJ>(); t < 3 * pre.P; t += S::kT) {
       const LinePoint lp(b, pre.cnt, pre.P, t, n, S::EW);
       if (io.stored_halo) {
         line_stored<T, TI, TJ>(g, io, lp, L);
@@ -1123,7 +1138,7 @@ __device__ __forceinline__ void tile_h_main_t(const Geo<T>& g, const StageIO<T>&
   // h, raw and contravariant velocities (remap.py:34-39)
 #pragma unroll
   for (int k = 0; k < S::KP; ++k) {
-    const int p = k * kTileThreads + (int)threadIdx.x;
+    const int p = k * S::kT + (int)threadIdx.x;
     if (p >= S::NP) continue;
     const RegionPoint<TI, TJ, FULL> pt(b, p);
     if (!pt.on) continue;
@@ -1132,11 +1147,11 @@ __device__ __forceinline__ void tile_h_main_t(const Geo<T>& g, const StageIO<T>&
     const T u = uv[k], v = vv[k];
     L.s_h[pt.r * RJ + pt.c] = hv[k];
     if (pt.vbar) {
-      L.s_uc[pt.r * TJ + pt.c - kHalo] = (G[0] * u + G[1] * v) * sn;
+      L.s_uc[pt.r * TJ + pt.c - kHalo] = lin2(G[0], u, G[1], v) * sn;
       L.s_v[pt.r * TJ + pt.c - kHalo] = v;
     }
     if (pt.hbar) {
-      L.s_vc[(pt.r - kHalo) * RJ + pt.c] = (G[2] * u + G[3] * v) * sn;
+      L.s_vc[(pt.r - kHalo) * RJ + pt.c] = lin2(G[2], u, G[3], v) * sn;
       L.s_u[(pt.r - kHalo) * RJ + pt.c] = u;
     }
   }
@@ -1176,7 +1191,7 @@ __device__ __forceinline__ void tile_uv_pro_t(const Geo<T>& g, const TileBox& b,
   const int ni = FULL ? TI : b.ni, nj = FULL ? TJ : b.nj;
 #pragma unroll
   for (int k = 0; k < S::KC; ++k) {
-    const int c = k * kTileThreads + (int)threadIdx.x, a = c / TJ, q = c % TJ;
+    const int c = k * S::kT + (int)threadIdx.x, a = c / TJ, q = c % TJ;
     if (a < ni && q < nj) {
       pre.rdx[k] = g.rdx[o0 + a * m + q];
       pre.rdy[k] = g.rdy[o0 + a * m + q];
@@ -1191,7 +1206,7 @@ __device__ __forceinline__ void tile_uv_pro_t(const Geo<T>& g, const TileBox& b,
   if (!FULL) {
 #pragma unroll
     for (int k = 0; k < S::KP; ++k) {
-      const int p = k * kTileThreads + (int)threadIdx.x;
+      const int p = k * S::kT + (int)threadIdx.x;
       if (p >= S::NP) continue;
       const RegionPoint<TI, TJ, FULL> pt(b, p);
       if (!pt.on) continue;
@@ -1222,7 +1237,7 @@ __device__ __forceinline__ void tile_uv_main_t(const Geo<T>& g, const StageIO<T>
   T hn[S::KP], hs[S::KP];
 #pragma unroll
   for (int k = 0; k < S::KP; ++k) {
-    const int p = k * kTileThreads + (int)threadIdx.x;
+    const int p = k * S::kT + (int)threadIdx.x;
     if (p >= S::NP) continue;
     const RegionPoint<TI, TJ, FULL> pt(b, p);
     if (!pt.on) continue;
@@ -1248,7 +1263,7 @@ __device__ __forceinline__ void tile_uv_main_t(const Geo<T>& g, const StageIO<T>
   }();
 #pragma unroll
   for (int k = 0; k < S::KC; ++k) {
-    const int c = k * kTileThreads + (int)threadIdx.x, a = c / TJ, q = c % TJ;
+    const int c = k * S::kT + (int)threadIdx.x, a = c / TJ, q = c % TJ;
     if (a < ni && q < nj) {
       upc[k] = io.up[o0 + a * m + q];
       vpc[k] = io.vp[o0 + a * m + q];
@@ -1258,16 +1273,16 @@ __device__ __forceinline__ void tile_uv_main_t(const Geo<T>& g, const StageIO<T>
   }
 #pragma unroll
   for (int k = 0; k < S::KP; ++k) {
-    const int p = k * kTileThreads + (int)threadIdx.x;
+    const int p = k * S::kT + (int)threadIdx.x;
     if (p >= S::NP) continue;
     const RegionPoint<TI, TJ, FULL> pt(b, p);
     if (!pt.on) continue;
-    sm[pt.r * RJ + pt.c] = blend ? (T(1.0) - io.beta) * hn[k] + io.beta * hs[k] : hn[k];
+    sm[pt.r * RJ + pt.c] = blend ? lin2(T(1.0) - io.beta, hn[k], io.beta, hs[k]) : hn[k];
   }
   __syncthreads();
 #pragma unroll
   for (int k = 0; k < S::KC; ++k) {
-    const int c = k * kTileThreads + (int)threadIdx.x, a = c / TJ, q = c % TJ;
+    const int c = k * S::kT + (int)threadIdx.x, a = c / TJ, q = c % TJ;
     if (a < ni && q < nj) {
       T hx[7], hy[7];
 #pragma unroll
@@ -1303,8 +1318,8 @@ __device__ __forceinline__ void tile_uv_main_t(const Geo<T>& g, const StageIO<T>
           ld_quad(g.gct + 4 * (long)o, G);
           sn = g.sina[o];
         }
-        const T ull = c2[0] * u + c2[1] * v, vll = c2[2] * u + c2[3] * v;
-        const T uct = (G[0] * u + G[1] * v) * sn, vct = (G[2] * u + G[3] * v) * sn;
+        const T ull = lin2(c2[0], u, c2[1], v), vll = lin2(c2[2], u, c2[3], v);
+        const T uct = lin2(G[0], u, G[1], v) * sn, vct = lin2(G[2], u, G[3], v) * sn;
         T* const bu = io.band_uv;
         const int plane = band_plane(n);
         for_bands(f, b.i0 + a, b.j0 + q, n, [&](int side, int z) {

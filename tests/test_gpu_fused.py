@@ -5,7 +5,7 @@ rounds must equal the phases' (``set_full_tiles`` forces them) bit for bit;
 float32 is held to 1e-6 relative (max norm), as other forms of the same round,
 whose contraction choices may differ.  Sizes: the smallest it takes, face
 extents that 8 x 16 does and does not divide, uneven splits, more than one tile
-per SM, and a size below its range.
+per SM, sizes where it takes 12 x 16 tiles, and a size below its range.
 """
 import numpy as np
 import pytest
@@ -25,7 +25,7 @@ def inputs(g, seed, dtype):
             for a in (s["h0"], b["h0"], s["ub"], s["vb"], b["ub"], b["vb"])]
 
 
-@pytest.mark.parametrize("n", [17, 18, 25, 33, 41, 48, 58, 72, 80])
+@pytest.mark.parametrize("n", [17, 18, 25, 33, 41, 48, 58, 72, 77, 84, 96])
 @pytest.mark.parametrize("rk", [2, 3])
 def test_fused_round_bitwise_equals_phases_f64(n, rk, grids):
     g = grids(n)
@@ -46,7 +46,7 @@ def test_fused_round_bitwise_equals_phases_f64(n, rk, grids):
     ref.close()
 
 
-@pytest.mark.parametrize("n,rk", [(18, 2), (48, 3), (90, 2), (112, 3)])
+@pytest.mark.parametrize("n,rk", [(18, 2), (48, 3), (90, 2), (96, 3), (112, 3)])
 def test_fused_round_matches_phases_f32(n, rk, grids):
     g = grids(n)
     consts = make_consts(g, 5000.0)
