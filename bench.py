@@ -45,7 +45,10 @@ B_ALG_WORDS = 41  # algorithmic words per cell-update over both RK stages (compu
 #   phase H : h, u, v, [h base], dzph_x, dzph_y, gct(4), sina, rda, c_dy, d_dx -> h     14 / 15
 #   phase UV: u, v, h, new h, [u, v base], gct(4), sina, rda, rdx, rdy, a_f, c_dy,
 #             d_dx, dzph_x, dzph_y -> u, v                                          18 / 20
-KERNEL_WORDS = {"phase_h": 14.5, "phase_uv": 19.0}
+# These count the stage's arithmetic as two independent kernels would have to move it;
+# the phase kernels hand momentum terms over instead of recomputing from the state.
+# stage (fused kernel: phase UV of a stage and phase H of the next): half of B_ALG_WORDS.
+KERNEL_WORDS = {"phase_h": 14.5, "phase_uv": 19.0, "stage": B_ALG_WORDS / 2}
 KERNEL_NAMES = {"phase_h": "k_phase_h", "phase_uv": "k_phase_uv"}
 METRIC = "barotropic cell-updates/s"
 UNIT = "cell-updates/s"
@@ -600,7 +603,7 @@ def form_serving(dev, depth, count):
 # ---------------------------------------------------------------------------
 def run_ours(args, world, rank, local):
     import torch
-    from licom4py_gpu_b200 import barotr
+    from licom4py_gpu_b200 import _native, barotr
     from licom4py_gpu_b200.plan import DIAG_NAMES, BtPlan
     from licom4py_gpu_b200.autotune import choose_config
 
@@ -665,7 +668,11 @@ def run_ours(args, world, rank, local):
     ms = max_over_ranks(ms, world)
     ms_per_step = ms / args.steps
     value = world * cells * nbb * args.steps / (ms * 1e-3)
-    launches_per_step = {"resident": 4, "persistent": 4, "graph": 4 * nbb + 3, "stream": 4 * nbb + 3}[mode]
+    # fused rounds: phase H, 2 nbb - 1 stage kernels and phase UV; halo fill and diagnostics at the end
+    fused_bits = int(_native.lib().bt_plan_get_info(plan._h, _native.BT_INFO_FUSED_ROUND))
+    fused = mode in ("graph", "stream") and bool(fused_bits & 1)
+    per_round = 2 * nbb + 4 if fused else 4 * nbb + 3
+    launches_per_step = {"resident": 4, "persistent": 4, "graph": per_round, "stream": per_round}[mode]
 
     # roofline of the dominant kernel
     peaks = {}
@@ -730,6 +737,25 @@ def run_ours(args, world, rank, local):
                     "peak_source": peak_src, "unit": "GB/s", "frac": achieved / peak, "traffic": traffic,
                     "launch_us": 1e3 * kms / klaunch, "launches_timed": klaunch, "launches_per_step": 1,
                     "alg_bytes_per_launch": alg, "timed_in": "headline run (events around the round kernel)",
+                    "l2_copy_gbs": l2, "frac_of_l2_copy": achieved / l2 if l2 else None}
+    elif fused:
+        # the headline step is a chain of stage kernels: its time over their number
+        launch_us = 1e3 * ms_per_step / (2 * nbb)
+        alg = KERNEL_WORDS["stage"] * 8 * cells
+        achieved = alg / (launch_us * 1e-6) / 1e9
+        l2 = l2_copy_gbs(dev)
+        traffic = None
+        tfile = os.path.join(ROOT, "profiles", f"k_stage_c{n}_f64.json")
+        if os.path.exists(tfile):
+            try:
+                traffic = json.load(open(tfile)).get("dram_bytes_per_launch")
+            except (OSError, ValueError):
+                traffic = None
+        roofline = {"bound": "l2" if 41 * 8 * 6 * (n + 6) ** 2 < 64e6 else "hbm",
+                    "kernel": f"k_stage<double,{12 if fused_bits & 4 else 8},16>", "achieved": achieved, "peak": peak,
+                    "peak_source": peak_src, "unit": "GB/s", "frac": achieved / peak, "traffic": traffic,
+                    "launch_us": launch_us, "launches_per_step": 2 * nbb, "alg_bytes_per_launch": alg,
+                    "timed_in": "headline run: ms_per_step / stages per step",
                     "l2_copy_gbs": l2, "frac_of_l2_copy": achieved / l2 if l2 else None}
     else:
         # graph / stream: the kernels' shares of phase time come from an event-timed stream-mode

@@ -44,7 +44,7 @@ extern "C" {
 #define BT_MODE_GRAPH 1       /* the round is captured once as a CUDA graph and replayed */
 #define BT_MODE_PERSISTENT 2  /* one cooperative launch with grid barriers per round */
 #define BT_MODE_RESIDENT 3    /* one cooperative launch per round, one CTA per tile holding its constants
-                                 and face cache on chip, neighbour tiles synchronised by progress flags;
+                                 and momentum terms on chip, neighbour tiles synchronised by progress flags;
                                  grids whose tiles all fit on the GPU at once (else BT_ENOTSUP) */
 
 /* Plan options (bt_plan_set_option) */
@@ -54,10 +54,11 @@ extern "C" {
 #define BT_OPT_KERNEL_TIMING 3  /* 1 = bracket the round kernel (persistent / resident mode) or each phase
                                    kernel (stream mode) with CUDA events on its stream; setting it resets
                                    the record */
-#define BT_OPT_FULL_TILES 4  /* stream / graph mode, which phase kernels run: -1 (default) by size, the
-                                kernels with a path specialised for full interior tiles when a launch
-                                takes more than one wave of CTAs and the smaller edge-path-only kernels
-                                otherwise; 1 = always the former, 0 = always the latter (same results) */
+#define BT_OPT_FULL_TILES 4  /* stream / graph mode, which kernels run: -1 (default) by size, on small grids
+                                one fused kernel per stage with 8 x 16 tiles (BT_INFO_FUSED_ROUND), else the
+                                phase kernels, with a path specialised for full interior tiles when a launch
+                                takes more than one wave of CTAs and without it otherwise; 1 = always the
+                                phase kernels with that path, 0 = always those without (same results) */
 
 /* Kernel kinds of bt_plan_kernel_time */
 #define BT_KERNEL_ROUND 0     /* the persistent or resident round kernel */
@@ -69,6 +70,9 @@ extern "C" {
 #define BT_INFO_SCRATCH_BYTES 2  /* device scratch owned by the plan */
 #define BT_INFO_FULL_TILES 3     /* stream / graph mode phase kernels at the plan's tile and size: bit 0 set =
                                     phase H runs the kernel with the full-tile path, bit 1 = phase UV */
+#define BT_INFO_FUSED_ROUND 4    /* bit 0 set = RK2 rounds run the fused stage kernel between their first phase H
+                                    and last phase UV, bit 1 = RK3 rounds (stream / graph mode, by size), bit 2 =
+                                    that kernel's tiles are 12 x 16, not 8 x 16 */
 
 typedef struct bt_plan bt_plan;
 
@@ -244,7 +248,7 @@ typedef struct bt_member {
   double dtb;
 } bt_member;
 
-/* Device scratch one member needs for RK order rk (stage fields and face caches). */
+/* Device scratch one member needs for RK order rk (stage fields, momentum terms, bands). */
 int bt_member_scratch_bytes(bt_plan* plan, int rk, unsigned long long* bytes);
 
 /* A batch of dtype BT_F64 / BT_F32 taking up to max_members members per call,

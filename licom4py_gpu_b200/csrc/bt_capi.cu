@@ -274,8 +274,8 @@ cudaError_t run_stage(const bt_plan* p, const Geo<T>& g, const StageIO<T>& io, c
 // Whether stream and graph rounds of plan p run the fused stage kernel: its tile shape is the plan's, nothing
 // asks for the phase kernels by themselves (their timing, one of their builds), and the plan has the buffers.
 bool fused_round(const bt_plan* p, int rk) {
-  return p->fused && (rk == 2 || p->fused_rk3) && p->tile.ti == kFusedTile.ti && p->tile.tj == kFusedTile.tj && !p->timing && p->full_tiles < 0 &&
-         (p->mode == BT_MODE_STREAM || p->mode == BT_MODE_GRAPH);
+  return p->fused && (rk == 2 || p->fused_rk3) && p->tile.ti == kFusedTile.ti && p->tile.tj == kFusedTile.tj &&
+         !p->timing && p->full_tiles < 0 && (p->mode == BT_MODE_STREAM || p->mode == BT_MODE_GRAPH);
 }
 
 // The fused stage kernel's tables and constant blocks, built ahead of the plan's first fused round (like the
@@ -1040,6 +1040,8 @@ long long bt_plan_get_info(bt_plan* p, int key) {
       if (cur >= 0 && cur != p->device) cudaSetDevice(cur);
       return r;
     }
+    case BT_INFO_FUSED_ROUND: return (fused_round(p, 2) ? 1 : 0) | (fused_round(p, 3) ? 2 : 0) |
+                                     (fused_tile(p->n).ti == kFusedTile.ti ? 0 : 4);
     default: return -1;
   }
 }

@@ -74,9 +74,8 @@ struct Geo {
   const int* bsrc;  // (24, 3, n) first source of each band halo cell as a number in band order
                     // (bt_stencil.cuh, band_no); the second is the next one along the edge
   // Tile constant blocks for tiles of cblk_ti x cblk_tj cells (TileShape::cW words
-  // per tile: phase H's cell and face constants of the tile); phase H of full
-  // interior tiles assembles its constants from its own block and its four
-  // neighbours'.  nullptr, or another tile shape: the arrays above are read.
+  // per tile: phase H's cell and face constants of the tile).  nullptr, or
+  // another tile shape: the arrays above are read.
   const T* cblk;
   int cblk_ti, cblk_tj;
   int route[24];    // f*4 + side

@@ -31,7 +31,7 @@
 // alone, so that decoding -- some 300 instructions per thread, which at C96 no
 // earlier kernel's tail would hide, the SMs being full -- is done once per plan
 // (k_stage_tables) and the kernel reads the result: 12 packed ints and two
-// weights per thread.
+// weights per thread, of which tiles away from the face edges need four ints.
 //
 // The arithmetic of each value is the phase kernels' own, so the results are
 // bitwise the same.
@@ -407,10 +407,11 @@ __global__ void __launch_bounds__(TileShape<TI, TJ>::kT) k_stage_tables(Geo<T> g
 
 // One RK stage's phase UV and the next one's phase H (file comment).  Bound by
 // latency while a tile has an SM to itself (the loads' round trip, four barriers,
-// the evaluation and face chains: 5000-8700 cycles from the wait on at C48), by
-// issue slots and the shared-memory pipe with three tiles per SM.  us per
-// substep, two phase kernels per stage / fused: C48 float64 13.1 / 8.9, float32
-// 10.2 / 5.9; C96 float32 10.8 / 8.4; C90 RK3 float32 18.0 / 14.6.
+// the evaluation and face chains: 5000-6600 cycles from the wait on at C48 of
+// float64), by issue slots and the shared-memory pipe with two 12 x 16 tiles per
+// SM, and there by the SMs that hold two edge tiles.  us per substep, two phase
+// kernels per stage / fused: C48 float64 12.1 / 8.2, float32 10.2 / 5.9; C96
+// float64 14.15 / 13.2, float32 10.8 / 8.2; C90 RK3 float32 18.0 / 14.3.
 template <typename T, int TI, int TJ>
 __global__ void __launch_bounds__(TileShape<TI, TJ>::kT, TI == 8 ? 3 : 2)
     k_stage(Geo<T> g, FusedIO<T> p, Tiling t, const int4* rec, const T* weights) {
@@ -468,7 +469,7 @@ __global__ void __launch_bounds__(TileShape<TI, TJ>::kT, TI == 8 ? 3 : 2)
   wait_prior_grid();
   // Only now may the next kernel start: at small sizes it would otherwise start at once, and so would the ones
   // after it as long as SMs have room, and the CTAs of the running kernel would share SMs while others idle
-  // (C48 float64: 14.67 us per substep with the release at the top, 8.79 here).
+  // (C48 float64, before launches were spread evenly: 14.67 us per substep with the release at the top, 8.79 here).
   release_dependents();
 
   // ---- 1. h, and what the evaluations read -------------------------------------

@@ -33,7 +33,7 @@
 
 namespace bt {
 
-// Resident CTAs per SM the kernel is compiled for (register cap 65536 / (256 *
+// Resident CTAs per SM the kernel is compiled for (register cap 65536 / (288 *
 // blocks)).  The float64 layouts of the larger tiles (16 x 16, 8 x 32: over
 // 100 KB) fit only two CTAs per SM anyway, so they get the registers of two.
 template <typename T, int TI, int TJ>

@@ -189,7 +189,8 @@ __device__ __forceinline__ int yface_side(int j, int m) {
 // ---------------------------------------------------------------------------
 // A CTA of kTileThreads threads computes one TI x TJ tile of one face, as lists
 // of independent items spread over the CTA: the points of the tile's stencil
-// region, its faces, its cells.  The lists are row-major, so every global
+// region, its faces, its cells.  (Below, "C96 8 x 16" and the like name a grid and a
+// tile shape; times are us per RK2 substep of a graph round.)  The lists are row-major, so every global
 // access of a warp is a run of consecutive cells and the shared-memory reads
 // are conflict-free or nearly so.
 //
@@ -204,7 +205,7 @@ __device__ __forceinline__ int yface_side(int j, int m) {
 // depend on the state.
 //
 // 288 threads: with 8 x 16 tiles (the one-wave sizes) the 272 region points,
-// the 280 faces and the gather items each fit one pass, so a CTA runs one face
+// the 280 faces and the edge items each fit one pass, so a CTA runs one face
 // chain, not two; 8 x 32 and 16 x 16 tiles need two (552 and 544 faces; three
 // with 256 threads), 16 x 32 four (1072).
 constexpr int kTileThreads = 288;
