@@ -16,7 +16,7 @@
 // calls on any streams are independent and can be captured.  Bound by the 16
 // SMs' share of the memory bandwidth (and by latency below C96); one CTA, as it
 // was, kept a single SM waiting on one load per thread: interior statistics of a
-// C384 float64 field 383 -> 23 us, conservation 848 -> 53 us (launch included).
+// C384 float64 field 383 -> 18.5 us, conservation 848 -> 53 us (launch included).
 
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
@@ -33,7 +33,7 @@ namespace {
 
 namespace cg = cooperative_groups;
 
-constexpr int kRedThreads = 512, kRedWarps = kRedThreads / 32;
+constexpr int kStatThreads = 1024, kConsThreads = 512;
 constexpr int kRedCtas = 16;  // one cluster
 
 struct Kahan {
@@ -53,11 +53,11 @@ struct Kahan {
 
 // Runs item(row offset of column 0, first column) for this warp's strips of W
 // columns: strip u is columns (u % strips) * W .. of interior row u / strips.
-template <int W, typename F>
+template <int WARPS, int W, typename F>
 __device__ __forceinline__ void for_strips(int n, F item) {
   const int m = n + 6;
   const unsigned strips = (n + W - 1) / W, total = 6u * n * strips;
-  for (unsigned u = blockIdx.x * kRedWarps + threadIdx.x / 32; u < total; u += kRedCtas * kRedWarps) {
+  for (unsigned u = blockIdx.x * WARPS + threadIdx.x / 32; u < total; u += kRedCtas * WARPS) {
     const unsigned row = u / strips, f = row / n, i = row - f * n;
     item(cell(f, i + kHalo, kHalo, m), (int)((u - row * strips) * W + (threadIdx.x & 31)));
   }
@@ -73,14 +73,14 @@ __device__ __forceinline__ Kahan warp_sum(Kahan a) {
 }
 
 // Combines the warps' values (lane 0 of each) of all CTAs in a fixed order; thread 0 of CTA 0 gets the result.
-template <typename V, typename F>
+template <int WARPS, typename V, typename F>
 __device__ __forceinline__ V cluster_combine(V v, F join) {
-  __shared__ V part[kRedWarps];
+  __shared__ V part[WARPS];
   cg::cluster_group cl = cg::this_cluster();
   if ((threadIdx.x & 31) == 0) part[threadIdx.x / 32] = v;
   __syncthreads();
   if (threadIdx.x == 0) {
-    for (int w = 1; w < kRedWarps; ++w) join(v, part[w]);
+    for (int w = 1; w < WARPS; ++w) join(v, part[w]);
     part[0] = v;
   }
   cl.sync();
@@ -96,12 +96,14 @@ struct StatsPart {
 };
 
 template <typename T>
-__global__ void __launch_bounds__(kRedThreads) k_stats(int n, const T* F, double* out) {
-  constexpr int K = 8;     // columns per lane and strip
+__global__ void __launch_bounds__(kStatThreads) k_stats(int n, const T* F, double* out) {
+  // columns per lane and strip: 32 warps with 6 loads each in flight (C384 float64 22.9 -> 18.5 us, float32 24.4 ->
+  // 18.6 against 16 warps with 8)
+  constexpr int K = 6;
   constexpr int A = 4;     // sums per lane: independent chains
   StatsPart p{-INFINITY, INFINITY, {}};
   Kahan sum[A];
-  for_strips<32 * K>(n, [&](long o, int j) {
+  for_strips<kStatThreads / 32, 32 * K>(n, [&](long o, int j) {
     T v[K];
 #pragma unroll
     for (int k = 0; k < K; ++k)
@@ -122,7 +124,7 @@ __global__ void __launch_bounds__(kRedThreads) k_stats(int n, const T* F, double
 #pragma unroll
   for (int k = 0; k < A; ++k) p.sum.add(sum[k]);
   p.sum = warp_sum(p.sum);
-  p = cluster_combine(p, [](StatsPart& a, const StatsPart& b) {
+  p = cluster_combine<kStatThreads / 32>(p, [](StatsPart& a, const StatsPart& b) {
     a.mx = fmax(a.mx, b.mx);
     a.mn = fmin(a.mn, b.mn);
     a.sum.add(b.sum);
@@ -139,12 +141,13 @@ struct ConservationPart {
 };
 
 template <typename T>
-__global__ void __launch_bounds__(kRedThreads) k_conservation(int n, const T* H, const T* U, const T* V,
+__global__ void __launch_bounds__(kConsThreads) k_conservation(int n, const T* H, const T* U, const T* V,
                                                             const T* rda, const T* c2l, double depth,
                                                             double* out) {
-  constexpr int K = 3;  // columns per lane and strip, each with its own sums
+  // columns per lane and strip, each with its own sums (1024 threads with 2: C384 float64 52.3 -> 55.0 us)
+  constexpr int K = 3;
   ConservationPart p, q[K];
-  for_strips<32 * K>(n, [&](long o, int j) {
+  for_strips<kConsThreads / 32, 32 * K>(n, [&](long o, int j) {
     T h[K], u[K], v[K], r[K], C[K][4];
 #pragma unroll
     for (int k = 0; k < K; ++k)
@@ -174,7 +177,7 @@ __global__ void __launch_bounds__(kRedThreads) k_conservation(int n, const T* H,
   }
   p.mass = warp_sum(p.mass);
   p.energy = warp_sum(p.energy);
-  p = cluster_combine(p, [](ConservationPart& a, const ConservationPart& b) {
+  p = cluster_combine<kConsThreads / 32>(p, [](ConservationPart& a, const ConservationPart& b) {
     a.mass.add(b.mass);
     a.energy.add(b.energy);
   });
@@ -186,7 +189,7 @@ __global__ void __launch_bounds__(kRedThreads) k_conservation(int n, const T* H,
 
 // One cluster of kRedCtas CTAs (more than the portable 8: the kernel opts in, once per device).
 template <typename... A>
-cudaError_t launch_cluster(void (*kern)(A...), std::atomic<bool>* opted, cudaStream_t s, A... args) {
+cudaError_t launch_cluster(void (*kern)(A...), int threads, std::atomic<bool>* opted, cudaStream_t s, A... args) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
@@ -197,7 +200,7 @@ cudaError_t launch_cluster(void (*kern)(A...), std::atomic<bool>* opted, cudaStr
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(kRedCtas);
-  cfg.blockDim = dim3(kRedThreads);
+  cfg.blockDim = dim3(threads);
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -211,14 +214,14 @@ cudaError_t launch_cluster(void (*kern)(A...), std::atomic<bool>* opted, cudaStr
 template <typename T>
 cudaError_t launch_stats(int n, const void* f, void* out, cudaStream_t s) {
   static std::atomic<bool> opted[64];
-  return launch_cluster<int, const T*, double*>(k_stats<T>, opted, s, n, (const T*)f, (double*)out);
+  return launch_cluster<int, const T*, double*>(k_stats<T>, kStatThreads, opted, s, n, (const T*)f, (double*)out);
 }
 template <typename T>
 cudaError_t launch_conservation(int n, const void* h, const void* u, const void* v, const void* rda, const void* c2l,
                                 double depth, void* out, cudaStream_t s) {
   static std::atomic<bool> opted[64];
   return launch_cluster<int, const T*, const T*, const T*, const T*, const T*, double, double*>(
-      k_conservation<T>, opted, s, n, (const T*)h, (const T*)u, (const T*)v, (const T*)rda, (const T*)c2l, depth,
+      k_conservation<T>, kConsThreads, opted, s, n, (const T*)h, (const T*)u, (const T*)v, (const T*)rda, (const T*)c2l, depth,
       (double*)out);
 }
 

@@ -1,6 +1,6 @@
 """Interior statistics and conservation sums against exactly rounded sums on the host.
 
-Sizes around the kernels' column strips (256 and 96), the smallest, and one
+Sizes around the kernels' column strips (192 and 96), the smallest, and one
 with several strips per warp.  The sums are compensated: what is left is the
 rounding of the compensation and of the final sum and quotient, at most
 4 x 2^-53 of the result (plus 1e-20 of the mean magnitude for the second-order
@@ -18,7 +18,7 @@ pytestmark = pytest.mark.gpu
 EPS = 2.0 ** -53
 
 
-@pytest.mark.parametrize("n", [1, 5, 31, 95, 96, 97, 255, 256, 257])
+@pytest.mark.parametrize("n", [1, 5, 31, 95, 96, 97, 191, 192, 193, 256])
 @pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
 def test_reductions_match_exact_sums(n, dtype):
     rng = np.random.default_rng(n)
