@@ -16,7 +16,7 @@
 // calls on any streams are independent and can be captured.  Bound by the 16
 // SMs' share of the memory bandwidth (and by latency below C96); one CTA, as it
 // was, kept a single SM waiting on one load per thread: interior statistics of a
-// C384 float64 field 383 -> 18.5 us, conservation 848 -> 53 us (launch included).
+// C384 float64 field 383 -> 18.5 us, conservation 848 -> 49 us (launch included).
 
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
@@ -26,6 +26,7 @@
 #include <string>
 
 #include "bt_launch.cuh"
+#include "bt_stencil.cuh"
 #include "licom_bt.h"
 
 namespace bt {
@@ -147,6 +148,7 @@ __global__ void __launch_bounds__(kConsThreads) k_conservation(int n, const T* H
   // columns per lane and strip, each with its own sums (1024 threads with 2: C384 float64 52.3 -> 55.0 us)
   constexpr int K = 3;
   ConservationPart p, q[K];
+  const bool vec = (reinterpret_cast<size_t>(c2l) & 15) == 0;  // 16-byte loads (C384 float64 52.3 -> 49.1 us)
   for_strips<kConsThreads / 32, 32 * K>(n, [&](long o, int j) {
     T h[K], u[K], v[K], r[K], C[K][4];
 #pragma unroll
@@ -157,8 +159,12 @@ __global__ void __launch_bounds__(kConsThreads) k_conservation(int n, const T* H
         u[k] = U[e];
         v[k] = V[e];
         r[k] = rda[e];
+        if (vec) {
+          ld_quad(c2l + 4 * e, C[k]);
+        } else {
 #pragma unroll
-        for (int z = 0; z < 4; ++z) C[k][z] = c2l[4 * e + z];
+          for (int z = 0; z < 4; ++z) C[k][z] = c2l[4 * e + z];
+        }
       }
 #pragma unroll
     for (int k = 0; k < K; ++k)

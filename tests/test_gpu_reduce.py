@@ -45,3 +45,14 @@ def test_reductions_match_exact_sums(n, dtype):
         for g, t in zip(got, (mass, energy)):
             want = math.fsum(t)
             assert abs(g - want) <= 4 * EPS * abs(want) + 1e-20 * np.abs(t).sum()
+
+
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+def test_conservation_of_matrices_off_a_16_byte_boundary(dtype):
+    """Matrices that start off a 16-byte boundary are read one value at a time: the same sums to the bit."""
+    gen = torch.Generator().manual_seed(3)
+    f = [torch.rand((6, 39, 39), generator=gen, dtype=torch.float64).to("cuda", dtype) + 0.5 for _ in range(4)]
+    c = torch.randn((6 * 39 * 39 * 4 + 1,), generator=gen, dtype=torch.float64).to("cuda", dtype)
+    off = c[1:].view(6, 39, 39, 2, 2)
+    assert off.data_ptr() % 16 != 0 and off.clone().data_ptr() % 16 == 0
+    assert torch.equal(conservation(*f, off, 5000.0), conservation(*f, off.clone(), 5000.0))
