@@ -154,7 +154,10 @@ long long bt_plan_get_info(bt_plan* plan, int key);
 /* Advance nbb (>= 1) substeps of RK2 (rk = 2, midpoint, barotr.py:41-61) or
  * RK3 (rk = 3, barotr.py:64-87) with step dtb.  Replaces the call
  * rk_core(barotr_s, barotr_consts, nbb, dtb, px, py) (schedule.py:170) with
- * px = py = 1; STATE_KEYS[16:23] pass through untouched and are not handled here. */
+ * px = py = 1; STATE_KEYS[16:23] pass through untouched and are not handled here.
+ * The first bt_round or bt_stage of a plan with its tile shape prepares tables
+ * and synchronises the stream; from then on a stream-mode round or a stage can be
+ * captured on the caller's stream. */
 int bt_round(bt_plan* plan, const bt_state_in* in, const bt_state_out* out, int nbb, double dtb,
              int rk, void* stream);
 

@@ -96,8 +96,8 @@ int batch_round(bt_batch* b, const bt_member* mem, int count, int rk, cudaStream
     if (gi == (int)plans.size()) {
       if (gi == kMaxGeo) return bfail(BT_EINVAL, "bt_batch_round: more than 16 distinct plans in one call");
       plans.push_back(p);
-      // the member plan's constant blocks for the batch's tile shape, built once per plan
-      const int rc = ensure_const_blocks_any(u.plan, b->tile, s);
+      // what the batch's tile shape needs of the member's plan, built once per plan
+      const int rc = prepare_tile(u.plan, b->tile, s);
       if (rc != BT_OK) return rc;
       hg[gi] = p->geo_tile<T>(b->tile);
     }

@@ -278,22 +278,6 @@ bool fused_round(const bt_plan* p, int rk) {
          !p->timing && p->full_tiles < 0 && (p->mode == BT_MODE_STREAM || p->mode == BT_MODE_GRAPH);
 }
 
-// The fused stage kernel's tables and constant blocks, built ahead of the plan's first fused round (like the
-// tile constant blocks: the stream is synchronised, so rounds on any stream may use them afterwards).
-template <typename T>
-int ensure_stage_tables_t(bt_plan* p, cudaStream_t s) {
-  if (p->stage_ready) return BT_OK;
-  cudaError_t e = launch_stage_tables<T>(p->geo_arrays<T>(), p->stage_tables(), s);
-  if (e == cudaSuccess) e = launch_const_blocks<T>(p->geo_arrays<T>(), fused_tile(p->n), true, (T*)p->even_blocks(), s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  if (e != cudaSuccess) return cuda_fail(e, "fused stage tables");
-  p->stage_ready = true;
-  return BT_OK;
-}
-int ensure_stage_tables(bt_plan* p, cudaStream_t s) {
-  return p->dtype == BT_F64 ? ensure_stage_tables_t<double>(p, s) : ensure_stage_tables_t<float>(p, s);
-}
-
 // The diagnostics of the last stage (input h, u, v) and the halo fill of the result.
 template <typename T>
 cudaError_t enqueue_end(const Geo<T>& g, const bt_state_out& out, T* h, T* u, T* v, cudaStream_t s) {
@@ -466,9 +450,7 @@ namespace bt {
 // Tile constant blocks of plan p for tile shape t (Geo::cblk): built once per
 // shape into a buffer of their own on stream s, which is then synchronised, so
 // rounds on any stream may use them afterwards; without them (allocation
-// failure) the phases read the constant arrays as before.  Runs before any
-// capture of the round (bt_round builds them ahead of its graph), so the
-// first round of a plan per tile shape must not be inside a stream capture.
+// failure) the phases read the constant arrays as before.
 template <typename T>
 int ensure_const_blocks(bt_plan* p, TileCfg t, cudaStream_t s) {
   if (p->cblk_for(t)) return BT_OK;
@@ -493,8 +475,33 @@ int ensure_const_blocks(bt_plan* p, TileCfg t, cudaStream_t s) {
   return BT_OK;
 }
 
-int ensure_const_blocks_any(bt_plan* p, TileCfg t, cudaStream_t s) {
-  return p->dtype == BT_F64 ? ensure_const_blocks<double>(p, t, s) : ensure_const_blocks<float>(p, t, s);
+// The fused stage kernel's tables and the constant blocks of its even split,
+// in the plan's scratch.
+template <typename T>
+int ensure_stage_tables(bt_plan* p, cudaStream_t s) {
+  if (p->stage_ready) return BT_OK;
+  cudaError_t e = launch_stage_tables<T>(p->geo_arrays<T>(), p->stage_tables(), s);
+  if (e == cudaSuccess) e = launch_const_blocks<T>(p->geo_arrays<T>(), fused_tile(p->n), true, (T*)p->even_blocks(), s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  if (e != cudaSuccess) return set_error(BT_ECUDA, std::string("fused stage tables: ") + cudaGetErrorString(e));
+  p->stage_ready = true;
+  return BT_OK;
+}
+
+template <typename T>
+int prepare_tile_t(bt_plan* p, TileCfg t, cudaStream_t s) {
+  const int rc = ensure_const_blocks<T>(p, t, s);
+  if (rc != BT_OK || !p->fused || t.ti != kFusedTile.ti || t.tj != kFusedTile.tj) return rc;
+  return ensure_stage_tables<T>(p, s);
+}
+
+// Everything that rounds and stages of plan p with tiles of shape t read beside
+// the constants and the state.  It does not depend on the entry point, the RK
+// order or the options, so that after the first stage or round of a plan per
+// tile shape -- which must not be inside a stream capture -- every later one
+// only launches kernels.
+int prepare_tile(bt_plan* p, TileCfg t, cudaStream_t s) {
+  return p->dtype == BT_F64 ? prepare_tile_t<double>(p, t, s) : prepare_tile_t<float>(p, t, s);
 }
 }  // namespace bt
 
@@ -868,8 +875,7 @@ int bt_round(bt_plan* p, const bt_state_in* in, const bt_state_out* out, int nbb
       if (!out->diag[k]) return fail(BT_EINVAL, "bt_round: diag outputs must be all set or diag[0] NULL");
   cudaStream_t s = (cudaStream_t)stream;
   {
-    int rc = ensure_const_blocks_any(p, p->tile, s);
-    if (rc == BT_OK && fused_round(p, rk)) rc = ensure_stage_tables(p, s);
+    const int rc = prepare_tile(p, p->tile, s);
     if (rc != BT_OK) return rc;
   }
   if (p->mode == BT_MODE_RESIDENT)
@@ -935,7 +941,7 @@ int bt_stage(bt_plan* p, const bt_state_in* in, const bt_state_out* out, double 
       if (!out->diag[k]) return fail(BT_EINVAL, "bt_stage: diag outputs must be all set or diag[0] NULL");
   cudaStream_t s = (cudaStream_t)stream;
   {
-    const int rc = ensure_const_blocks_any(p, p->tile, s);
+    const int rc = prepare_tile(p, p->tile, s);
     if (rc != BT_OK) return rc;
   }
   cudaError_t e = p->dtype == BT_F64 ? enqueue_stage<double>(p, *in, *out, dt, beta_d, is_laststep ? 1 : 0, s)

@@ -27,8 +27,8 @@ inline bool matrices_aligned(const bt_grid_desc* d) {
 
 struct bt_plan;
 namespace bt {
-// Build the tile constant blocks of plan p for tile shape t if it has none (bt_capi.cu).
-int ensure_const_blocks_any(bt_plan* p, TileCfg t, cudaStream_t s);
+// Build what rounds and stages of plan p with tiles of shape t read, if it is not there yet (bt_capi.cu).
+int prepare_tile(bt_plan* p, TileCfg t, cudaStream_t s);
 }  // namespace bt
 
 struct bt_plan {
@@ -72,7 +72,7 @@ struct bt_plan {
   long long spin_limit = 1ll << 24;
   int full_tiles = -1;  // BT_OPT_FULL_TILES
   bool fused = false;   // the scratch and the halo tables allow the fused stage kernel
-  bool stage_ready = false;  // its tables and constant blocks are built (first use)
+  bool stage_ready = false;  // its tables and constant blocks are built (prepare_tile)
   bool fused_rk3 = false;  // whether RK3 rounds use it too
   int last_grid = 0;
   // optional kernel timing: event pairs on the launch stream around the round
