@@ -53,7 +53,9 @@ extern "C" {
                                 take before it gives up */
 #define BT_OPT_KERNEL_TIMING 3  /* 1 = bracket the round kernel (persistent / resident mode) or each phase
                                    kernel (stream mode) with CUDA events on its stream; setting it resets
-                                   the record */
+                                   the record.  Stream-mode rounds that run the fused stage kernel run the
+                                   phase kernels while it is on (same results); graph mode is not timed and
+                                   not affected */
 #define BT_OPT_FULL_TILES 4  /* stream / graph mode, which kernels run: -1 (default) by size, on small grids
                                 one fused kernel per stage with 8 x 16 tiles (BT_INFO_FUSED_ROUND), else the
                                 phase kernels, with a path specialised for full interior tiles when a launch

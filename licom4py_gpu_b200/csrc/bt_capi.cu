@@ -272,10 +272,11 @@ cudaError_t run_stage(const bt_plan* p, const Geo<T>& g, const StageIO<T>& io, c
 }
 
 // Whether stream and graph rounds of plan p run the fused stage kernel: its tile shape is the plan's, nothing
-// asks for the phase kernels by themselves (their timing, one of their builds), and the plan has the buffers.
+// asks for the phase kernels by themselves (their timing in stream mode, one of their builds), and the plan has
+// the buffers.
 bool fused_round(const bt_plan* p, int rk) {
   return p->fused && (rk == 2 || p->fused_rk3) && p->tile.ti == kFusedTile.ti && p->tile.tj == kFusedTile.tj &&
-         !p->timing && p->full_tiles < 0 && (p->mode == BT_MODE_STREAM || p->mode == BT_MODE_GRAPH);
+         p->full_tiles < 0 && (p->mode == BT_MODE_GRAPH || (p->mode == BT_MODE_STREAM && !p->timing));
 }
 
 // The diagnostics of the last stage (input h, u, v) and the halo fill of the result.

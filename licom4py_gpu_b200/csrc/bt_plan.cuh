@@ -85,7 +85,7 @@ struct bt_plan {
   // Record the start event of a timed kernel of the given kind (nullptr if timing is off).
   cudaError_t time_begin(int kind, cudaStream_t s, cudaEvent_t* stop) const {
     *stop = nullptr;
-    if (!timing) return cudaSuccess;
+    if (!timing || mode == BT_MODE_GRAPH) return cudaSuccess;  // an event in a captured round times nothing
     if (tev_used + 2 > tev.size()) {
       for (int k = 0; k < 2; ++k) {
         cudaEvent_t ev;

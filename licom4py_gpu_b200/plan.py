@@ -119,7 +119,9 @@ class BtPlan:
 
     def enable_kernel_timing(self, on: bool = True) -> None:
         """Bracket the round kernel (persistent / resident mode) or each phase kernel
-        (stream mode) with CUDA events on its stream; resets the record."""
+        (stream mode) with CUDA events on its stream; resets the record.  Stream-mode
+        rounds run the phase kernels while it is on, also where they would run the fused
+        stage kernel (same results); graph mode is not timed and not affected."""
         self.set_option(N.BT_OPT_KERNEL_TIMING, 1 if on else 0)
 
     def set_full_tiles(self, which) -> None:
