@@ -274,13 +274,13 @@ __global__ void __launch_bounds__(kTileThreads, 2) k_batch_round(BatchArgs<T> a)
       const Geo<T>& g = ctx.g;
       const TileBox b = tile_box(make_tiling_dev(TI, TJ, g.n), g.n, tile - __ldg(a.off.tile + k));
       if (!uv) {
-        HPre<T, TI, TJ> pre;
+        HPre<T, TI, TJ> pre{};
         tile_h_pro<T, TI, TJ>(g, ctx.io, b, sm, pre);
-        tile_h_main<T, TI, TJ>(g, ctx.io, b, sm, pre);
+        tile_h_main<T, TI, TJ, true, true>(g, ctx.io, b, sm, pre);
       } else {
-        UvPre<T, TI, TJ> pre;
+        UvPre<T, TI, TJ> pre{};
         tile_uv_pro<T, TI, TJ>(g, b, pre);
-        tile_uv_main<T, TI, TJ>(g, ctx.io, b, sm, pre);
+        tile_uv_main<T, TI, TJ, true, true>(g, ctx.io, b, sm, pre);
       }
     }
     if (!grid_barrier(a.bar, gen, a.err, a.spin_limit)) {

@@ -50,8 +50,11 @@ __global__ void __launch_bounds__(kTileThreads, PhaseBlocksUV<T, TileShape<TI, T
 // its first tile (constants by cp.async, halo descriptors), so those loads
 // overlap the barrier.  The loop runs per RK stage (phase H, barrier, phase
 // UV, barrier) so the two phases' gather states are never live together.
+// float64 runs two CTAs per SM (96 registers: at three the prologue's values, held
+// across the barrier, spill 344-1364 bytes; C96 8 x 16 31.8 -> 28.6 us per substep,
+// C192 16 x 32 75.5 -> 59.3), float32 three (C192 16 x 32 35.2 against 38.2 with two).
 template <typename T, int TI, int TJ>
-__global__ void __launch_bounds__(kTileThreads, 3) k_round(RoundArgs<T> a) {
+__global__ void __launch_bounds__(kTileThreads, sizeof(T) == 8 ? 2 : 3) k_round(RoundArgs<T> a) {
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ StageIO<T> s_io[2];  // stage pointers, alternating between consecutive stages
   T* sm = reinterpret_cast<T*>(smraw);
@@ -60,41 +63,34 @@ __global__ void __launch_bounds__(kTileThreads, 3) k_round(RoundArgs<T> a) {
   const int nstage = a.nbb * nst;
   const int t0 = blockIdx.x;
   unsigned gen = 0;
-  if (threadIdx.x == 0) s_io[0] = round_stage(a, a.step0, 0);
-  __syncthreads();
-  // phase H of stage 0: the first tile's prologue
-  HPre<T, TI, TJ> hpre;
-  if (t0 < ntiles) tile_h_pro<T, TI, TJ>(a.g, s_io[0], tile_box(a.t, a.g.n, t0), sm, hpre);
   for (int sg = 0; sg < nstage; ++sg) {
+    if (threadIdx.x == 0) s_io[sg & 1] = round_stage(a, a.step0 + sg / nst, sg % nst);
+    __syncthreads();
     const StageIO<T>& io = s_io[sg & 1];
+    {
+      HPre<T, TI, TJ> pre{};
+      if (t0 < ntiles) tile_h_pro<T, TI, TJ>(a.g, io, tile_box(a.t, a.g.n, t0), sm, pre);
+      if (sg > 0 && !grid_barrier(a.bar, gen, a.err, a.spin_limit)) {
+        cp_async_wait_all();  // no copy may be left in flight when the CTA leaves
+        return;
+      }
+      int k = 0;
+      for (int tile = t0; tile < ntiles; tile += gridDim.x, ++k) {
+        const TileBox b = tile_box(a.t, a.g.n, tile);
+        if (k > 0) tile_h_pro<T, TI, TJ>(a.g, io, b, sm, pre);
+        tile_h_main<T, TI, TJ, true, true>(a.g, io, b, sm, pre);
+        __syncthreads();
+      }
+    }
+    UvPre<T, TI, TJ> pre{};
+    if (t0 < ntiles) tile_uv_pro<T, TI, TJ>(a.g, tile_box(a.t, a.g.n, t0), pre);
+    if (!grid_barrier(a.bar, gen, a.err, a.spin_limit)) return;
     int k = 0;
     for (int tile = t0; tile < ntiles; tile += gridDim.x, ++k) {
       const TileBox b = tile_box(a.t, a.g.n, tile);
-      if (k > 0) tile_h_pro<T, TI, TJ>(a.g, io, b, sm, hpre);
-      tile_h_main<T, TI, TJ>(a.g, io, b, sm, hpre);
-      __syncthreads();
-    }
-    UvPre<T, TI, TJ> pre;
-    if (t0 < ntiles) tile_uv_pro<T, TI, TJ>(a.g, tile_box(a.t, a.g.n, t0), pre);
-    if (!grid_barrier(a.bar, gen, a.err, a.spin_limit)) {
-      cp_async_wait_all();  // no copy may be left in flight when the CTA leaves
-      return;
-    }
-    k = 0;
-    for (int tile = t0; tile < ntiles; tile += gridDim.x, ++k) {
-      const TileBox b = tile_box(a.t, a.g.n, tile);
       if (k > 0) tile_uv_pro<T, TI, TJ>(a.g, b, pre);
-      tile_uv_main<T, TI, TJ>(a.g, io, b, sm, pre);
+      tile_uv_main<T, TI, TJ, true, true>(a.g, io, b, sm, pre);
       __syncthreads();
-    }
-    if (sg + 1 < nstage) {
-      if (threadIdx.x == 0) s_io[(sg + 1) & 1] = round_stage(a, a.step0 + (sg + 1) / nst, (sg + 1) % nst);
-      __syncthreads();
-      if (t0 < ntiles) tile_h_pro<T, TI, TJ>(a.g, s_io[(sg + 1) & 1], tile_box(a.t, a.g.n, t0), sm, hpre);
-    }
-    if (!grid_barrier(a.bar, gen, a.err, a.spin_limit)) {
-      cp_async_wait_all();
-      return;
     }
   }
 }

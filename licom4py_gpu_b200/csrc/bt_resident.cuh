@@ -107,17 +107,17 @@ template <typename T, int TI, int TJ, bool FULL>
 __device__ __forceinline__ bool res_stage(const RoundArgs<T>& a, const ResSync& rsy, const StageIO<T>& io,
                                           const TileBox& b, T* sm, const ResSm<T>& rs, int tile, int done) {
   {
-    HPre<T, TI, TJ> pre;
+    HPre<T, TI, TJ> pre{};
     tile_h_points<T, TI, TJ, FULL>(a.g, io, b, sm, pre);
     if (done > 0 && !res_wait(rsy, tile, done, a.err, a.spin_limit)) return false;
-    tile_h_main_t<T, TI, TJ, FULL, true>(a.g, io, b, sm, pre, rs);
+    tile_h_main_t<T, TI, TJ, FULL, true, true>(a.g, io, b, sm, pre, rs);
     res_publish(rsy.flags + tile * kResFlagStride, done + 1);
   }
   {
-    UvPre<T, TI, TJ> pre;
+    UvPre<T, TI, TJ> pre{};
     tile_uv_pro_t<T, TI, TJ, FULL>(a.g, b, pre);
     if (!res_wait(rsy, tile, done + 1, a.err, a.spin_limit)) return false;
-    tile_uv_main_t<T, TI, TJ, FULL, true>(a.g, io, b, sm + ResLayout<T, TI, TJ>::kUV, pre, rs);
+    tile_uv_main_t<T, TI, TJ, FULL, true, true>(a.g, io, b, sm + ResLayout<T, TI, TJ>::kUV, pre, rs);
     res_publish(rsy.flags + tile * kResFlagStride, done + 2);
   }
   return true;

@@ -615,6 +615,25 @@ __device__ __forceinline__ void celerity_coef(T hface, T dz, T& c, T& coef) {
   }
 }
 
+// Values of a thread's items that only some threads have, or only some items:
+// assigned under a condition and read under the same one.  In a kernel that loops
+// over tiles or stages (LOOP) such a variable would stay live around the whole
+// loop, because on the other path the register still holds what the iteration
+// before left there; there it is set first.  (k_batch_round float64 16 x 32: 924
+// bytes spilled without, 76 with; a mixed ensemble of 8 C48, 6 C96 and 2 C192
+// members 352 -> 246 us per substep; k_round C192 16 x 32 101 -> 74.5; k_resident
+// C96 8 x 16 27.8 -> 21.3.)  Kernels of one tile have no use for it (float32
+// batch of that ensemble, one launch per phase: 100.8 without, 104.2 with).
+template <bool LOOP, typename V>
+__device__ __forceinline__ void begin_items(V& v) {
+  if constexpr (LOOP) v = V{};
+}
+template <bool LOOP, typename V, int N>
+__device__ __forceinline__ void begin_items(V (&v)[N]) {
+#pragma unroll
+  for (int k = 0; k < N; ++k) begin_items<LOOP>(v[k]);
+}
+
 // ---- phase H ----------------------------------------------------------------
 template <typename T, int TI, int TJ>
 struct LayoutH {
@@ -1069,7 +1088,7 @@ __device__ __forceinline__ void tile_cells(const StageIO<T>& io, const TileBox& 
 // Phase H of one tile: writes the new h and the momentum terms of the tile's
 // interior cells, and the new h of its cells in the face's bands.  RES
 // (tile-resident round): the terms stay on chip.
-template <typename T, int TI, int TJ, bool FULL, bool RES = false>
+template <typename T, int TI, int TJ, bool FULL, bool LOOP, bool RES = false>
 __device__ __forceinline__ void tile_h_main_t(const Geo<T>& g, const StageIO<T>& io, const TileBox& b, T* sm,
                                               const HPre<T, TI, TJ>& pre, const ResSm<T>& rs = ResSm<T>{}) {
   using S = TileShape<TI, TJ>;
@@ -1081,6 +1100,10 @@ __device__ __forceinline__ void tile_h_main_t(const Geo<T>& g, const StageIO<T>&
 
   // region: state of the thread's points (halo points from the bands) and base h of its cells
   T hv[S::KP], uv[S::KP], vv[S::KP], hpc[S::KC];
+  begin_items<LOOP>(hv);
+  begin_items<LOOP>(uv);
+  begin_items<LOOP>(vv);
+  begin_items<LOOP>(hpc);
 #pragma unroll
   for (int k = 0; k < S::KP; ++k) {
     const int p = k * S::kT + (int)threadIdx.x;
@@ -1222,7 +1245,7 @@ __device__ __forceinline__ void tile_uv_pro_t(const Geo<T>& g, const TileBox& b,
 // phase H's terms; the lon/lat and normal contravariant velocity of the tile's
 // cells in the face's bands.  RES (tile-resident round): the terms are in
 // shared memory.
-template <typename T, int TI, int TJ, bool FULL, bool RES = false>
+template <typename T, int TI, int TJ, bool FULL, bool LOOP, bool RES = false>
 __device__ __forceinline__ void tile_uv_main_t(const Geo<T>& g, const StageIO<T>& io, const TileBox& b, T* sm,
                                                const UvPre<T, TI, TJ>& pre, const ResSm<T>& rs = ResSm<T>{}) {
   using S = TileShape<TI, TJ>;
@@ -1236,6 +1259,8 @@ __device__ __forceinline__ void tile_uv_main_t(const Geo<T>& g, const StageIO<T>
 
   // new h of the region, blended with the stage h (fb_scheme, barotr_pure.py:52-54)
   T hn[S::KP], hs[S::KP];
+  begin_items<LOOP>(hn);
+  begin_items<LOOP>(hs);
 #pragma unroll
   for (int k = 0; k < S::KP; ++k) {
     const int p = k * S::kT + (int)threadIdx.x;
@@ -1256,6 +1281,9 @@ __device__ __forceinline__ void tile_uv_main_t(const Geo<T>& g, const StageIO<T>
   }
   // base velocities and terms of the thread's cells
   T upc[S::KC], vpc[S::KC], tm[S::KC][kTerms<T>];
+  begin_items<LOOP>(upc);
+  begin_items<LOOP>(vpc);
+  begin_items<LOOP>(tm);
   const auto ta = [&] {
     if constexpr (RES)
       return TermsAt<T, TI, TJ, false>(rs.terms);
@@ -1349,13 +1377,13 @@ __device__ __forceinline__ void tile_h_pro(const Geo<T>& g, const StageIO<T>& io
   else
     tile_h_pro_t<T, TI, TJ, false>(g, io, b, sm, pre);
 }
-template <typename T, int TI, int TJ, bool FP = true>
+template <typename T, int TI, int TJ, bool FP, bool LOOP>
 __device__ __forceinline__ void tile_h_main(const Geo<T>& g, const StageIO<T>& io, const TileBox& b, T* sm,
                                             const HPre<T, TI, TJ>& pre) {
   if (FP && tile_full(b, g.m, TI, TJ))
-    tile_h_main_t<T, TI, TJ, true>(g, io, b, sm, pre);
+    tile_h_main_t<T, TI, TJ, true, LOOP>(g, io, b, sm, pre);
   else
-    tile_h_main_t<T, TI, TJ, false>(g, io, b, sm, pre);
+    tile_h_main_t<T, TI, TJ, false, LOOP>(g, io, b, sm, pre);
 }
 template <typename T, int TI, int TJ, bool FP = true>
 __device__ __forceinline__ void tile_uv_pro(const Geo<T>& g, const TileBox& b, UvPre<T, TI, TJ>& pre) {
@@ -1364,13 +1392,13 @@ __device__ __forceinline__ void tile_uv_pro(const Geo<T>& g, const TileBox& b, U
   else
     tile_uv_pro_t<T, TI, TJ, false>(g, b, pre);
 }
-template <typename T, int TI, int TJ, bool FP = true>
+template <typename T, int TI, int TJ, bool FP, bool LOOP>
 __device__ __forceinline__ void tile_uv_main(const Geo<T>& g, const StageIO<T>& io, const TileBox& b, T* sm,
                                              const UvPre<T, TI, TJ>& pre) {
   if (FP && tile_full(b, g.m, TI, TJ))
-    tile_uv_main_t<T, TI, TJ, true>(g, io, b, sm, pre);
+    tile_uv_main_t<T, TI, TJ, true, LOOP>(g, io, b, sm, pre);
   else
-    tile_uv_main_t<T, TI, TJ, false>(g, io, b, sm, pre);
+    tile_uv_main_t<T, TI, TJ, false, LOOP>(g, io, b, sm, pre);
 }
 
 // One tile phase with the prologue issued first (the stream/graph kernels).
@@ -1381,7 +1409,7 @@ __device__ __forceinline__ void tile_h(const Geo<T>& g, const StageIO<T>& io, co
   tile_h_pro<T, TI, TJ, FP>(g, io, b, sm, pre);
   wait_prior_grid();
   if (late) release_dependents();
-  tile_h_main<T, TI, TJ, FP>(g, io, b, sm, pre);
+  tile_h_main<T, TI, TJ, FP, false>(g, io, b, sm, pre);
 }
 template <typename T, int TI, int TJ, bool FP = true>
 __device__ __forceinline__ void tile_uv(const Geo<T>& g, const StageIO<T>& io, const TileBox& b, T* sm,
@@ -1390,7 +1418,7 @@ __device__ __forceinline__ void tile_uv(const Geo<T>& g, const StageIO<T>& io, c
   tile_uv_pro<T, TI, TJ, FP>(g, b, pre);
   wait_prior_grid();
   if (late) release_dependents();
-  tile_uv_main<T, TI, TJ, FP>(g, io, b, sm, pre);
+  tile_uv_main<T, TI, TJ, FP, false>(g, io, b, sm, pre);
 }
 
 
