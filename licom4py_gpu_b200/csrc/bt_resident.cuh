@@ -7,7 +7,10 @@
 // everything that does not change during the round on chip:
 //
 //   * the tile's cell and face constants (depths, spacings) are staged into
-//     shared memory once, at launch;
+//     shared memory once, at launch, and for the 8 x 16 tiles, whose threads
+//     have one region point each, the points' metric, halo sources and weights
+//     (ResHeld; the larger shapes read those again in each phase's prologue,
+//     ahead of its wait);
 //   * phase H leaves the momentum terms of the tile's cells in shared memory,
 //     so phase UV reads only the new h of its region and the base velocities.
 //
@@ -34,22 +37,109 @@
 namespace bt {
 
 // Resident CTAs per SM the kernel is compiled for (register cap 65536 / (288 *
-// blocks)).  The float64 layouts of the larger tiles (16 x 16, 8 x 32: over
-// 100 KB) fit only two CTAs per SM anyway, so they get the registers of two.
+// blocks)).  The float64 layouts of the larger tiles (16 x 16: 73 KB, 8 x 32: 83 KB)
+// fit only two CTAs per SM anyway, so they get the registers of two.
 template <typename T, int TI, int TJ>
 struct ResBlocks {
   static constexpr int value = (sizeof(T) == 8 && TI * TJ > 128) ? 2 : 3;
 };
 
-// Shared-memory layout of a resident CTA (words of T): phase H layout,
-// momentum terms, phase UV layout.
+// Shared-memory layout of a resident CTA (words of T): phase H layout, momentum
+// terms, then with one region point per thread what HPre holds of it (ResHeld;
+// phase UV's region h takes the place of phase H's, dead by then, so that three
+// float64 CTAs fit an SM), else phase UV's layout.
 template <typename T, int TI, int TJ>
 struct ResLayout {
   using S = TileShape<TI, TJ>;
-  static constexpr int kTermsAt = up4(S::kWordsH);
-  static constexpr int kUV = up4(kTermsAt + kTerms<T> * S::C);
-  static constexpr int kWords = up4(kUV + S::kWordsUV);
+  static_assert(S::kWordsUV <= S::hUC, "phase UV's region fits phase H's");
+  static constexpr int kTermsAt = up4(S::kWordsH), kHeldAt = up4(kTermsAt + kTerms<T> * S::C);
+  static constexpr int kHeldPlanes = HPre<T, TI, TJ>::kLineHeld ? 14 : 13, kHeldInts = 3 * S::kT * (int)sizeof(int) / (int)sizeof(T);
+  static constexpr int kUV = S::kHeld ? 0 : kHeldAt;
+  static constexpr int kWords = up4(kHeldAt + (S::kHeld ? kHeldPlanes * S::kT + kHeldInts : S::kWordsUV));
   static constexpr size_t kBytes = sizeof(T) * kWords;
+};
+
+// What HPre holds of a thread's region point and line point, kept in shared memory
+// for the whole round where a thread has one of each (TileShape::kHeld): planes
+// of one word per thread -- metric (4), sina, l2c (4), halo weights (2), then the
+// line point's metric (kLineHeld) or weights -- and ints: the numbers of the first
+// halo sources (complemented where the second is the one before) and the line slot.
+// With them read from memory in every phase, as the larger shapes do: C48 float64
+// 19.4 against 17.0 us per substep, C96 float64 21.3 / 19.0, float32 18.1 / 15.6.
+template <typename T, int TI, int TJ>
+struct ResHeld {
+  using S = TileShape<TI, TJ>;
+  using H = HPre<T, TI, TJ>;
+  T* p;
+  int* b;
+  __device__ __forceinline__ explicit ResHeld(T* sm)
+      : p(sm + ResLayout<T, TI, TJ>::kHeldAt + threadIdx.x),
+        b(reinterpret_cast<int*>(sm + ResLayout<T, TI, TJ>::kHeldAt + ResLayout<T, TI, TJ>::kHeldPlanes * S::kT) +
+          threadIdx.x) {}
+  __device__ __forceinline__ void put(const HaloRef<T>& r, int w, int z) const {
+    p[w * S::kT] = r.w0;
+    p[(w + 1) * S::kT] = r.w1;
+    b[z * S::kT] = r.d < 0 ? ~r.b0 : r.b0;
+  }
+  __device__ __forceinline__ void get(HaloRef<T>& r, int w, int z) const {
+    const int e = b[z * S::kT];
+    r.w0 = p[w * S::kT];
+    r.w1 = p[(w + 1) * S::kT];
+    r.b0 = e < 0 ? ~e : e;
+    r.d = e < 0 ? -1 : 1;
+  }
+  __device__ __forceinline__ void store(const H& h) const {
+#pragma unroll
+    for (int z = 0; z < 4; ++z) {
+      p[z * S::kT] = h.g[z];
+      p[(5 + z) * S::kT] = h.halo.l2[z];
+    }
+    p[4 * S::kT] = h.sn;
+    put(h.halo.ref, 9, 0);
+    b[S::kT] = h.slot;
+    if (H::kLineHeld) {
+      p[11 * S::kT] = h.halo.g0;
+      p[12 * S::kT] = h.halo.g1;
+      p[13 * S::kT] = h.halo.sn;
+    } else {
+      put(h.lref, 11, 2);
+    }
+  }
+  __device__ __forceinline__ void load(const Geo<T>& g, const TileBox& box, int stored_halo, H& h) const {
+    h.P = edge_count(box, g.m, g.route, h.cnt);
+#pragma unroll
+    for (int z = 0; z < 4; ++z) {
+      h.g[z] = p[z * S::kT];
+      h.halo.l2[z] = p[(5 + z) * S::kT];
+    }
+    h.sn = p[4 * S::kT];
+    get(h.halo.ref, 9, 0);
+    h.slot = stored_halo ? -1 : b[S::kT];
+    if (H::kLineHeld) {
+      h.halo.g0 = p[11 * S::kT];
+      h.halo.g1 = p[12 * S::kT];
+      h.halo.sn = p[13 * S::kT];
+    } else {
+      get(h.lref, 11, 2);
+    }
+  }
+  // phase UV: the thread's cell and region point (c_block: the tile's cell constants)
+  __device__ __forceinline__ void load(const Geo<T>& g, const TileBox& box, const T* c_block,
+                                       UvPre<T, TI, TJ>& u) const {
+    const int c = threadIdx.x, a = c / TJ, q = c % TJ;
+    get(u.ref[0], 9, 0);
+    if (a < box.ni && q < box.nj) {
+      u.rdx[0] = c_block[S::C + c];
+      u.rdy[0] = c_block[2 * S::C + c];
+      if (in_bands(box.i0 + a, box.j0 + q, g.n)) {
+        ld_quad(g.c2l + 4 * (long)cell32(box.f, box.i0 + a, box.j0 + q, g.m), u.c2);
+        const T* const r = p - c + (a + kHalo) * TJ + q;  // the cell's region point
+#pragma unroll
+        for (int z = 0; z < 4; ++z) u.g[z] = r[z * S::kT];
+        u.sn = r[4 * S::kT];
+      }
+    }
+  }
 };
 
 // Publish that this CTA has completed ``phases`` phases: every thread's global
@@ -106,16 +196,23 @@ __device__ __forceinline__ bool res_wait(const ResSync& s, int tile, int need, i
 template <typename T, int TI, int TJ, bool FULL>
 __device__ __forceinline__ bool res_stage(const RoundArgs<T>& a, const ResSync& rsy, const StageIO<T>& io,
                                           const TileBox& b, T* sm, const ResSm<T>& rs, int tile, int done) {
+  constexpr bool kHeld = TileShape<TI, TJ>::kHeld;
   {
     HPre<T, TI, TJ> pre{};
-    tile_h_points<T, TI, TJ, FULL>(a.g, io, b, sm, pre);
+    if constexpr (kHeld)
+      ResHeld<T, TI, TJ>(sm).load(a.g, b, io.stored_halo, pre);
+    else
+      tile_h_points<T, TI, TJ, FULL>(a.g, io, b, sm, pre);
     if (done > 0 && !res_wait(rsy, tile, done, a.err, a.spin_limit)) return false;
     tile_h_main_t<T, TI, TJ, FULL, true, true>(a.g, io, b, sm, pre, rs);
     res_publish(rsy.flags + tile * kResFlagStride, done + 1);
   }
   {
     UvPre<T, TI, TJ> pre{};
-    tile_uv_pro_t<T, TI, TJ, FULL>(a.g, b, pre);
+    if constexpr (kHeld)
+      ResHeld<T, TI, TJ>(sm).load(a.g, b, sm + LayoutH<T, TI, TJ>::S::hC, pre);
+    else
+      tile_uv_pro_t<T, TI, TJ, FULL>(a.g, b, pre);
     if (!res_wait(rsy, tile, done + 1, a.err, a.spin_limit)) return false;
     tile_uv_main_t<T, TI, TJ, FULL, true, true>(a.g, io, b, sm + ResLayout<T, TI, TJ>::kUV, pre, rs);
     res_publish(rsy.flags + tile * kResFlagStride, done + 2);
@@ -136,6 +233,17 @@ __global__ void __launch_bounds__(kTileThreads, ResBlocks<T, TI, TJ>::value) k_r
   const bool full = tile_full(b, a.g.m, TI, TJ);
   // the constants, once per round (awaited by the first phase's barrier)
   tile_consts<T, TI, TJ>(a.g, b, LayoutH<T, TI, TJ>(sm));
+  if constexpr (TileShape<TI, TJ>::kHeld) {  // with the lines' depths
+    if (threadIdx.x == 0) {
+      s_io.stored_halo = 0;
+      s_io.last = 1;
+    }
+    __syncthreads();
+    HPre<T, TI, TJ> pre{};
+    tile_h_points<T, TI, TJ, false>(a.g, s_io, b, sm, pre);
+    ResHeld<T, TI, TJ>(sm).store(pre);
+    __syncthreads();
+  }
   const int nst = a.rk == 2 ? 2 : 3;
   const int nstage = a.nbb * nst;
   for (int sg = 0; sg < nstage; ++sg) {
