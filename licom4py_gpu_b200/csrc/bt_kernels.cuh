@@ -334,7 +334,7 @@ bool full_path(int n, int full_tiles) {
 }
 
 template <typename T, int TI, int TJ, bool UV>
-cudaError_t launch_tile(const Geo<T>& g, const StageIO<T>& io, cudaStream_t s, int full_tiles) {
+cudaError_t launch_tile(const Geo<T>& g, const StageIO<T>& io, cudaStream_t s, int full_tiles, bool overlap) {
   const size_t smem = tile_smem<T, TI, TJ, UV>();
   Tiling t = make_tiling({TI, TJ}, g.n);
   // up to one tile per SM the next kernel starts only when this one runs: its CTAs, and those of the kernels
@@ -344,7 +344,7 @@ cudaError_t launch_tile(const Geo<T>& g, const StageIO<T>& io, cudaStream_t s, i
   const bool fp = full_path<T, TI, TJ, UV>(g.n, full_tiles);
   auto kern = UV ? (fp ? k_phase_uv<T, TI, TJ, true> : k_phase_uv<T, TI, TJ, false>)
                  : (fp ? k_phase_h<T, TI, TJ, true> : k_phase_h<T, TI, TJ, false>);
-  // programmatic dependent launch: the kernel's constant prologue overlaps the
+  // programmatic dependent launch (overlap): the kernel's constant prologue overlaps the
   // previous kernel's tail; it waits (griddepcontrol.wait) before reading state
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(6 * t.tiles_per_face());
@@ -355,18 +355,18 @@ cudaError_t launch_tile(const Geo<T>& g, const StageIO<T>& io, cudaStream_t s, i
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = overlap ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kern, g, io, t);
 }
 
 template <typename T, bool UV>
-cudaError_t dispatch(const Geo<T>& g, const StageIO<T>& io, TileCfg c, cudaStream_t s, int full_tiles) {
-  if (c.ti == 7 && c.tj == 32) return launch_tile<T, 7, 32, UV>(g, io, s, full_tiles);
-  if (c.ti == 8 && c.tj == 32) return launch_tile<T, 8, 32, UV>(g, io, s, full_tiles);
-  if (c.ti == 15 && c.tj == 32) return launch_tile<T, 15, 32, UV>(g, io, s, full_tiles);
-  if (c.ti == 16 && c.tj == 32) return launch_tile<T, 16, 32, UV>(g, io, s, full_tiles);
-  if (c.ti == 8 && c.tj == 16) return launch_tile<T, 8, 16, UV>(g, io, s, full_tiles);
-  if (c.ti == 16 && c.tj == 16) return launch_tile<T, 16, 16, UV>(g, io, s, full_tiles);
+cudaError_t dispatch(const Geo<T>& g, const StageIO<T>& io, TileCfg c, cudaStream_t s, int full_tiles, bool overlap) {
+  if (c.ti == 7 && c.tj == 32) return launch_tile<T, 7, 32, UV>(g, io, s, full_tiles, overlap);
+  if (c.ti == 8 && c.tj == 32) return launch_tile<T, 8, 32, UV>(g, io, s, full_tiles, overlap);
+  if (c.ti == 15 && c.tj == 32) return launch_tile<T, 15, 32, UV>(g, io, s, full_tiles, overlap);
+  if (c.ti == 16 && c.tj == 32) return launch_tile<T, 16, 32, UV>(g, io, s, full_tiles, overlap);
+  if (c.ti == 8 && c.tj == 16) return launch_tile<T, 8, 16, UV>(g, io, s, full_tiles, overlap);
+  if (c.ti == 16 && c.tj == 16) return launch_tile<T, 16, 16, UV>(g, io, s, full_tiles, overlap);
   return cudaErrorInvalidValue;
 }
 
@@ -410,13 +410,14 @@ int phase_full_paths(TileCfg c, int n, int full_tiles) {
 }
 
 template <typename T>
-cudaError_t launch_phase_h(const Geo<T>& g, const StageIO<T>& io, TileCfg cfg, cudaStream_t s, int full_tiles) {
-  return dispatch<T, false>(g, io, cfg, s, full_tiles);
+cudaError_t launch_phase_h(const Geo<T>& g, const StageIO<T>& io, TileCfg cfg, cudaStream_t s, int full_tiles,
+                           bool overlap) {
+  return dispatch<T, false>(g, io, cfg, s, full_tiles, overlap);
 }
 
 template <typename T>
 cudaError_t launch_phase_uv(const Geo<T>& g, const StageIO<T>& io, TileCfg cfg, cudaStream_t s, int full_tiles) {
-  return dispatch<T, true>(g, io, cfg, s, full_tiles);
+  return dispatch<T, true>(g, io, cfg, s, full_tiles, true);
 }
 
 template <typename T, int TI, int TJ>
@@ -500,7 +501,7 @@ cudaError_t launch_diag(const Geo<T>& g, const T* h, const T* u, const T* v, con
 #define BT_INSTANTIATE(T)                                                                           \
   template cudaError_t prime_kernels<T>();                                                          \
   template int phase_full_paths<T>(TileCfg, int, int);                                              \
-  template cudaError_t launch_phase_h<T>(const Geo<T>&, const StageIO<T>&, TileCfg, cudaStream_t, int);  \
+  template cudaError_t launch_phase_h<T>(const Geo<T>&, const StageIO<T>&, TileCfg, cudaStream_t, int, bool); \
   template cudaError_t launch_phase_uv<T>(const Geo<T>&, const StageIO<T>&, TileCfg, cudaStream_t, int); \
   template cudaError_t launch_fill_halo<T>(const Geo<T>&, T*, T*, T*, cudaStream_t);                \
   template cudaError_t launch_const_blocks<T>(const Geo<T>&, TileCfg, bool, T*, cudaStream_t);         \

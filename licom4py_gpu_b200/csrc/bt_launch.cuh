@@ -40,7 +40,8 @@ cudaError_t prime_kernels();
 // kernel when the launch's CTAs all fit on the device at once).  Results are
 // the same either way.
 template <typename T>
-cudaError_t launch_phase_h(const Geo<T>& g, const StageIO<T>& io, TileCfg cfg, cudaStream_t s, int full_tiles = -1);
+cudaError_t launch_phase_h(const Geo<T>& g, const StageIO<T>& io, TileCfg cfg, cudaStream_t s, int full_tiles = -1,
+                           bool overlap = true);
 // Which kernels those launches take at n: bit 0 set = phase H runs the full-tile
 // kernel, bit 1 = phase UV (-1: unsupported tile shape).
 template <typename T>

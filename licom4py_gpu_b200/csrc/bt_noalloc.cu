@@ -331,8 +331,13 @@ int run_noalloc(unsigned char* base, const bt_grid_desc& d, const bt_state_in& i
   const T* X0[3] = {(const T*)in.h0, (const T*)in.ub, (const T*)in.vb};
   const T* B0[3] = {(const T*)in.h0p, (const T*)in.ubp, (const T*)in.vbp};
   const TileCfg tile{8, 16};
+  // The first phase H waits for k_build_halo to be done: the phases read the halo tables in their prologues, ahead
+  // of the wait from which a kernel's writes are visible to one that overlaps it.  The kernels after it overlap as
+  // they do in a plan's round: they can start only when the first phase H runs.
+  bool overlap = false;
   auto stage = [&](const StageIO<T>& io) {
-    cudaError_t r = launch_phase_h<T>(g, io, tile, s);
+    cudaError_t r = launch_phase_h<T>(g, io, tile, s, -1, overlap);
+    overlap = true;
     return r == cudaSuccess ? launch_phase_uv<T>(g, io, tile, s) : r;
   };
   for (int step = 0; step < nbb && e == cudaSuccess; ++step) {
