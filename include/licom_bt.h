@@ -204,6 +204,14 @@ int bt_interior_stats(int n, int dtype, const void* field, void* out3, void* str
 int bt_conservation(int n, int dtype, const void* h, const void* u, const void* v, const void* rda,
                     const void* a_c2l, double depth, void* out2, void* stream);
 
+/* The same on ``ctas`` CTAs (1, or a cluster of 2, 4, 8 or 16; BT_ECUDA if the
+ * device cannot place it), for inspection and testing.  The calls above (0) take
+ * the largest of these that the device can place.  Sums differ between them by
+ * the order in which they are combined. */
+int bt_interior_stats_on(int ctas, int n, int dtype, const void* field, void* out3, void* stream);
+int bt_conservation_on(int ctas, int n, int dtype, const void* h, const void* u, const void* v, const void* rda,
+                       const void* a_c2l, double depth, void* out2, void* stream);
+
 /* bt_round without any allocation, for callers that cannot allocate device
  * memory (a runtime's custom-call handler given only its operand buffers, a
  * model driver that reserves its GPU memory up front, a service whose memory

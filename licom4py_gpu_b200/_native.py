@@ -51,7 +51,8 @@ _lib = None
 # every symbol declared in include/licom_bt.h
 EXPORTS = ("bt_plan_create", "bt_plan_destroy", "bt_plan_set_tile", "bt_plan_set_mode",
            "bt_plan_set_option", "bt_plan_get_info", "bt_plan_kernel_time", "bt_round",
-           "bt_stage", "bt_fill_halo", "bt_edge_average", "bt_check_device_error", "bt_halo_table_host", "bt_interior_stats", "bt_conservation",
+           "bt_stage", "bt_fill_halo", "bt_edge_average", "bt_check_device_error", "bt_halo_table_host",
+           "bt_interior_stats", "bt_conservation", "bt_interior_stats_on", "bt_conservation_on",
            "bt_round_noalloc",
            "bt_member_scratch_bytes", "bt_batch_create", "bt_batch_destroy", "bt_batch_set_mode",
            "bt_batch_set_tile", "bt_batch_set_option", "bt_batch_get_info", "bt_batch_round",
@@ -86,7 +87,9 @@ def lib():
     L.bt_check_device_error.argtypes = [_vp]
     L.bt_halo_table_host.argtypes = [ctypes.c_int, _vp, _vp, _vp, _vp, _vp, _vp]
     L.bt_interior_stats.argtypes = [ctypes.c_int, ctypes.c_int, _vp, _vp, _vp]
+    L.bt_interior_stats_on.argtypes = [ctypes.c_int] + L.bt_interior_stats.argtypes
     L.bt_conservation.argtypes = [ctypes.c_int, ctypes.c_int, _vp, _vp, _vp, _vp, _vp, ctypes.c_double, _vp, _vp]
+    L.bt_conservation_on.argtypes = [ctypes.c_int] + L.bt_conservation.argtypes
     L.bt_round_noalloc.argtypes = [ctypes.POINTER(GridDesc), ctypes.POINTER(StateIn), ctypes.POINTER(StateOut),
                                    ctypes.c_int, ctypes.c_double, ctypes.c_int, _vp]
     L.bt_member_scratch_bytes.argtypes = [_vp, ctypes.c_int, ctypes.POINTER(ctypes.c_ulonglong)]

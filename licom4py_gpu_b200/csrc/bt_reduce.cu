@@ -13,10 +13,13 @@
 // One cluster of 16 CTAs walks the interior rows in a fixed order, each warp a
 // strip of consecutive columns at a time with all its loads in flight, and
 // combines through distributed shared memory: no scratch memory is used, so
-// calls on any streams are independent and can be captured.  Bound by the 16
-// SMs' share of the memory bandwidth (and by latency below C96); one CTA, as it
+// calls on any streams are independent and can be captured.  Where such a cluster
+// cannot be placed (part of a GPU), a smaller one or a single CTA runs the same
+// code.  Bound by the 16 SMs' share of the memory bandwidth (and by latency below C96); one CTA, as it
 // was, kept a single SM waiting on one load per thread: interior statistics of a
-// C384 float64 field 383 -> 18.5 us, conservation 848 -> 49 us (launch included).
+// C384 float64 field 383 -> 18.5 us, conservation 848 -> 49 us (launch included); on a
+// second stream beside a round they start like a single CTA does (C96 float64 20 us
+// from call to result with 16, 30 with one).
 
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
@@ -35,7 +38,7 @@ namespace {
 namespace cg = cooperative_groups;
 
 constexpr int kStatThreads = 1024, kConsThreads = 512;
-constexpr int kRedCtas = 16;  // one cluster
+constexpr int kRedCtas = 16;  // CTAs of the cluster at most
 
 struct Kahan {
   double s = 0.0, c = 0.0;
@@ -58,7 +61,7 @@ template <int WARPS, int W, typename F>
 __device__ __forceinline__ void for_strips(int n, F item) {
   const int m = n + 6;
   const unsigned strips = (n + W - 1) / W, total = 6u * n * strips;
-  for (unsigned u = blockIdx.x * WARPS + threadIdx.x / 32; u < total; u += kRedCtas * WARPS) {
+  for (unsigned u = blockIdx.x * WARPS + threadIdx.x / 32; u < total; u += gridDim.x * WARPS) {
     const unsigned row = u / strips, f = row / n, i = row - f * n;
     item(cell(f, i + kHalo, kHalo, m), (int)((u - row * strips) * W + (threadIdx.x & 31)));
   }
@@ -86,7 +89,7 @@ __device__ __forceinline__ V cluster_combine(V v, F join) {
   }
   cl.sync();
   if (blockIdx.x == 0 && threadIdx.x == 0)
-    for (int r = 1; r < kRedCtas; ++r) join(v, *cl.map_shared_rank(&part[0], r));
+    for (int r = 1; r < (int)gridDim.x; ++r) join(v, *cl.map_shared_rank(&part[0], r));
   cl.sync();  // no CTA leaves while its shared memory is read
   return v;
 }
@@ -193,45 +196,88 @@ __global__ void __launch_bounds__(kConsThreads) k_conservation(int n, const T* H
   }
 }
 
-// One cluster of kRedCtas CTAs (more than the portable 8: the kernel opts in, once per device).
+// Launch on ``ctas`` CTAs: one cluster, or without one for a single CTA.
 template <typename... A>
-cudaError_t launch_cluster(void (*kern)(A...), int threads, std::atomic<bool>* opted, cudaStream_t s, A... args) {
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  const bool known = dev >= 0 && dev < 64;
-  if (!known || !opted[dev].load(std::memory_order_relaxed)) {
-    if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) != cudaSuccess) return e;
-    if (known) opted[dev].store(true, std::memory_order_relaxed);
-  }
+cudaError_t launch_on(int ctas, void (*kern)(A...), int threads, cudaStream_t s, A... args) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(kRedCtas);
+  cfg.gridDim = dim3(ctas);
   cfg.blockDim = dim3(threads);
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = kRedCtas;
+  attr[0].val.clusterDim.x = ctas;
   attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = ctas > 1 ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
+// The largest cluster of ``kern`` that the current device can hold: kRedCtas (more
+// than the portable 8: the kernel opts in), else half of that and so on, at last 1.
+template <typename K>
+int largest_cluster(K kern, int threads) {
+  for (int ctas = kRedCtas; ctas > 1; ctas /= 2) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(threads);
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = ctas;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int held = 0;
+    if ((ctas <= 8 || cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) &&
+        cudaOccupancyMaxActiveClusters(&held, kern, &cfg) == cudaSuccess && held > 0)
+      return ctas;
+    cudaGetLastError();
+  }
+  return 1;
+}
+
+// Launch on the largest cluster the device holds (asked once per device: ``known``, 0 = not yet), or on ``ctas``
+// CTAs if that is not 0.  A launch that is refused all the same -- the context has fewer SMs than the device, or
+// was reset -- runs on one CTA.
+constexpr int kMaxDevices = 64;
+template <typename... A>
+cudaError_t launch_cluster(int ctas, void (*kern)(A...), int threads, std::atomic<int>* known, cudaStream_t s,
+                           A... args) {
+  if (ctas > 0) {
+    const int most = largest_cluster(kern, threads);
+    return ctas > most ? cudaErrorInvalidClusterSize : launch_on(ctas, kern, threads, s, args...);
+  }
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const bool in_range = dev >= 0 && dev < kMaxDevices;
+  ctas = in_range ? known[dev].load(std::memory_order_relaxed) : 0;
+  if (ctas == 0) {
+    ctas = largest_cluster(kern, threads);
+    if (in_range) known[dev].store(ctas, std::memory_order_relaxed);
+  }
+  e = launch_on(ctas, kern, threads, s, args...);
+  if (e == cudaSuccess || ctas == 1) return e;
+  cudaGetLastError();
+  return launch_on(1, kern, threads, s, args...);
+}
+
 template <typename T>
-cudaError_t launch_stats(int n, const void* f, void* out, cudaStream_t s) {
-  static std::atomic<bool> opted[64];
-  return launch_cluster<int, const T*, double*>(k_stats<T>, kStatThreads, opted, s, n, (const T*)f, (double*)out);
+cudaError_t launch_stats(int ctas, int n, const void* f, void* out, cudaStream_t s) {
+  static std::atomic<int> known[kMaxDevices];
+  return launch_cluster<int, const T*, double*>(ctas, k_stats<T>, kStatThreads, known, s, n, (const T*)f,
+                                                (double*)out);
 }
 template <typename T>
-cudaError_t launch_conservation(int n, const void* h, const void* u, const void* v, const void* rda, const void* c2l,
-                                double depth, void* out, cudaStream_t s) {
-  static std::atomic<bool> opted[64];
+cudaError_t launch_conservation(int ctas, int n, const void* h, const void* u, const void* v, const void* rda,
+                                const void* c2l, double depth, void* out, cudaStream_t s) {
+  static std::atomic<int> known[kMaxDevices];
   return launch_cluster<int, const T*, const T*, const T*, const T*, const T*, double, double*>(
-      k_conservation<T>, kConsThreads, opted, s, n, (const T*)h, (const T*)u, (const T*)v, (const T*)rda, (const T*)c2l, depth,
-      (double*)out);
+      ctas, k_conservation<T>, kConsThreads, known, s, n, (const T*)h, (const T*)u, (const T*)v, (const T*)rda,
+      (const T*)c2l, depth, (double*)out);
 }
 
 int rfail(int code, const std::string& msg) { return set_error(code, msg); }
+bool ctas_ok(int ctas) { return ctas >= 0 && ctas <= kRedCtas && (ctas & (ctas - 1)) == 0; }
 
 }  // namespace
 }  // namespace bt
@@ -240,26 +286,39 @@ using namespace bt;
 
 extern "C" {
 
-int bt_interior_stats(int n, int dtype, const void* field, void* out3, void* stream) {
+int bt_interior_stats_on(int ctas, int n, int dtype, const void* field, void* out3, void* stream) {
   if (n < 1 || !field || !out3) return rfail(BT_EINVAL, "bt_interior_stats: bad argument");
   cudaStream_t s = (cudaStream_t)stream;
   if (dtype != BT_F64 && dtype != BT_F32)
     return rfail(BT_EINVAL, "bt_interior_stats: dtype must be BT_F64 or BT_F32");
-  const cudaError_t e = dtype == BT_F64 ? launch_stats<double>(n, field, out3, s) : launch_stats<float>(n, field, out3, s);
+  if (!ctas_ok(ctas)) return rfail(BT_EINVAL, "bt_interior_stats_on: ctas must be 0, 1, 2, 4, 8 or 16");
+  const cudaError_t e =
+      dtype == BT_F64 ? launch_stats<double>(ctas, n, field, out3, s) : launch_stats<float>(ctas, n, field, out3, s);
   if (e != cudaSuccess) return rfail(BT_ECUDA, std::string("bt_interior_stats: ") + cudaGetErrorString(e));
   return BT_OK;
 }
 
-int bt_conservation(int n, int dtype, const void* h, const void* u, const void* v, const void* rda,
-                    const void* a_c2l, double depth, void* out2, void* stream) {
+int bt_conservation_on(int ctas, int n, int dtype, const void* h, const void* u, const void* v, const void* rda,
+                       const void* a_c2l, double depth, void* out2, void* stream) {
   if (n < 1 || !h || !u || !v || !rda || !a_c2l || !out2) return rfail(BT_EINVAL, "bt_conservation: bad argument");
   cudaStream_t s = (cudaStream_t)stream;
   if (dtype != BT_F64 && dtype != BT_F32)
     return rfail(BT_EINVAL, "bt_conservation: dtype must be BT_F64 or BT_F32");
-  const cudaError_t e = dtype == BT_F64 ? launch_conservation<double>(n, h, u, v, rda, a_c2l, depth, out2, s)
-                                        : launch_conservation<float>(n, h, u, v, rda, a_c2l, depth, out2, s);
+  if (!ctas_ok(ctas)) return rfail(BT_EINVAL, "bt_conservation_on: ctas must be 0, 1, 2, 4, 8 or 16");
+  const cudaError_t e = dtype == BT_F64
+                            ? launch_conservation<double>(ctas, n, h, u, v, rda, a_c2l, depth, out2, s)
+                            : launch_conservation<float>(ctas, n, h, u, v, rda, a_c2l, depth, out2, s);
   if (e != cudaSuccess) return rfail(BT_ECUDA, std::string("bt_conservation: ") + cudaGetErrorString(e));
   return BT_OK;
+}
+
+int bt_interior_stats(int n, int dtype, const void* field, void* out3, void* stream) {
+  return bt_interior_stats_on(0, n, dtype, field, out3, stream);
+}
+
+int bt_conservation(int n, int dtype, const void* h, const void* u, const void* v, const void* rda,
+                    const void* a_c2l, double depth, void* out2, void* stream) {
+  return bt_conservation_on(0, n, dtype, h, u, v, rda, a_c2l, depth, out2, stream);
 }
 
 }  // extern "C"
