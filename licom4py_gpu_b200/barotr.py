@@ -49,8 +49,8 @@ def get_plan(consts: Sequence, dtype=torch.float64, device=None) -> BtPlan:
     if plan is None:
         if len(_PLANS) >= _PLAN_CACHE_MAX:
             _PLANS.pop(next(iter(_PLANS))).close()
-        n = consts[2].shape[-1] - 6  # the drop-in calls pick the tile shape; every shape gives the same result
-        plan = BtPlan(consts, dtype=dtype, device=dev, tile=tuple(heuristic(n, dtype)["tile"]))
+        plan = BtPlan(consts, dtype=dtype, device=dev)
+        plan.set_tile(*heuristic(plan.n, dtype)["tile"])  # the drop-in calls pick the tile shape
         plan._const_refs = tuple(consts[:N_CONSTS])  # keep the key's objects alive
         _PLANS[key] = plan
     return plan
