@@ -373,7 +373,7 @@ cudaError_t enqueue_round_fused(const bt_plan* p, const bt_state_in& in, const b
       f.u_keep = ku[w];
       f.v_keep = kv[w];
     }
-    e = launch_stage<T>(ge, f, p->stage_tables(), s);
+    e = launch_stage<T>(ge, f, p->stage_tables(), p->mode == BT_MODE_STREAM, s);
   }
   if (e != cudaSuccess) return e;
   StageIO<T> last = stage(S - 1);

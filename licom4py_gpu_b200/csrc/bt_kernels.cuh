@@ -223,22 +223,30 @@ size_t tile_smem() {
 }
 
 // Shared memory a one-wave float64 launch of up to two tiles per SM asks for at
-// least, so that no SM takes more tiles than an even spread gives it: the CTAs
-// start as those of the kernel before leave, and without the limit the SMs that
-// are done first take three while others get one.  us per substep without / with
-// it: fused kernel C24 8.05 / 7.71, C48 8.87 / 8.24, C64 12.1 / 9.6, C72 14.2 /
-// 10.0; phase kernels C64 14.2 / 13.6, C72 14.5 / 13.1.  The request stays just
-// above the limit, which leaves the rest to L1 (C72 11.7 with all of it).  With
-// three tiles per SM the registers set the limit already and the larger request
-// only costs (C96 14.2 / 14.6, C128 16 x 16 20.9 / 21.8); phase launches of up to
-// one tile per SM are late (launch_tile) and lose with it (C48 12.1 / 12.9);
-// float32 tiles are short enough for the start of the next kernel's tiles beside
-// them to be worth more (C64 6.99 / 7.11).
+// least, so that no SM takes more than two of its tiles -- or one, if there is one
+// per SM at most and nothing else to run beside it (``alone``): the CTAs start as
+// those of the kernel before leave, and without the limit the SMs that are done
+// first take three while others get one.  us per substep without / with it: fused
+// kernel C24 8.5 / 7.7, C48 9.1 / 8.4, C64 12.2 / 9.8, C72 14.4 / 10.2; phase
+// kernels C64 14.2 / 13.6, C72 14.5 / 13.1.  The request stays just above the
+// limit, which leaves the rest to L1 (C72 11.7 with all of it).  With three tiles
+// per SM the registers set the limit already and the larger request only costs
+// (C96 14.2 / 14.6, C128 16 x 16 20.9 / 21.8); phase launches of up to one tile per
+// SM are late (launch_tile) and lose with it (C48 12.1 / 12.9); float32 tiles are
+// short enough for the start of the next kernel's tiles beside them to be worth
+// more (C64 6.99 / 7.11).
+// One tile per SM leaves the rounds of other plans on other streams no room beside
+// the CTAs that wait for the kernel ahead.  Graph rounds, which several streams can
+// run at once from one thread, allow two: four C48 plans 15.6 us per substep against
+// 23.6, four C36 plans 12.3 / 19.0 (phase kernels 16.3 and 16.0), one C48 plan 8.9 /
+// 8.4.  Stream rounds of one thread are launched too slowly to fill the GPU (four
+// C48 plans 26.2 with one, 24.3 with two; phase kernels 45.7) and keep one: a C48
+// plan 8.3 against 9.6.
 template <typename T>
-size_t spread_smem(int tiles) {
+size_t spread_smem(int tiles, bool alone) {
   constexpr size_t per_sm = 228 * 1024, per_cta = 1024;  // sm_100: shared memory of an SM, reserved by each CTA
   if (sizeof(T) == 4 || tiles > 2 * kSms) return 0;
-  return per_sm / (tiles > kSms ? 3 : 2) - per_cta + 256;
+  return per_sm / (tiles <= kSms && alone ? 2 : 3) - per_cta + 256;
 }
 
 // The persistent kernel runs both phases in one allocation: the larger of the two.
@@ -276,7 +284,7 @@ cudaError_t record_wave_slots() {
 template <typename T, int TI, int TJ>
 cudaError_t prime_tile() {
   cudaError_t e;
-  const size_t spread = spread_smem<T>(1);  // the most it asks for
+  const size_t spread = spread_smem<T>(1, true);  // the most it asks for
   for (auto k : {k_phase_h<T, TI, TJ, true>, k_phase_h<T, TI, TJ, false>})
     if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)std::max(tile_smem<T, TI, TJ, false>(), spread))) != cudaSuccess)
@@ -349,7 +357,7 @@ cudaError_t launch_tile(const Geo<T>& g, const StageIO<T>& io, cudaStream_t s, i
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(6 * t.tiles_per_face());
   cfg.blockDim = dim3(kTileThreads);
-  cfg.dynamicSmemBytes = fp || t.late ? smem : std::max(smem, spread_smem<T>(6 * t.tiles_per_face()));
+  cfg.dynamicSmemBytes = fp || t.late ? smem : std::max(smem, spread_smem<T>(6 * t.tiles_per_face(), false));
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -437,7 +445,8 @@ cudaError_t launch_stage_tables(const Geo<T>& g, void* out, cudaStream_t s) {
 }
 
 template <typename T, int TI, int TJ>
-static cudaError_t launch_stage_tile(const Geo<T>& g, const FusedIO<T>& p, const void* tables, cudaStream_t s) {
+static cudaError_t launch_stage_tile(const Geo<T>& g, const FusedIO<T>& p, const void* tables, bool alone,
+                                     cudaStream_t s) {
   using F = FusedShape<TI, TJ>;
   const Tiling t = make_even_tiling({TI, TJ}, g.n);
   const int4* const rec = (const int4*)tables;
@@ -446,7 +455,7 @@ static cudaError_t launch_stage_tile(const Geo<T>& g, const FusedIO<T>& p, const
   cfg.gridDim = dim3(6 * t.tiles_per_face());
   cfg.blockDim = dim3(F::kT);
   cfg.dynamicSmemBytes = std::max(sizeof(T) * (p.beta_prev != T(0) ? F::kWords : F::kHP),
-                                  spread_smem<T>(6 * t.tiles_per_face()));
+                                  spread_smem<T>(6 * t.tiles_per_face(), alone));
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -457,9 +466,9 @@ static cudaError_t launch_stage_tile(const Geo<T>& g, const FusedIO<T>& p, const
 }
 
 template <typename T>
-cudaError_t launch_stage(const Geo<T>& g, const FusedIO<T>& p, const void* tables, cudaStream_t s) {
-  return fused_tile(g.n).ti == 8 ? launch_stage_tile<T, 8, 16>(g, p, tables, s)
-                                            : launch_stage_tile<T, 12, 16>(g, p, tables, s);
+cudaError_t launch_stage(const Geo<T>& g, const FusedIO<T>& p, const void* tables, bool alone, cudaStream_t s) {
+  return fused_tile(g.n).ti == 8 ? launch_stage_tile<T, 8, 16>(g, p, tables, alone, s)
+                                 : launch_stage_tile<T, 12, 16>(g, p, tables, alone, s);
 }
 
 template <typename T, int TI, int TJ>
@@ -506,7 +515,7 @@ cudaError_t launch_diag(const Geo<T>& g, const T* h, const T* u, const T* v, con
   template cudaError_t launch_fill_halo<T>(const Geo<T>&, T*, T*, T*, cudaStream_t);                \
   template cudaError_t launch_const_blocks<T>(const Geo<T>&, TileCfg, bool, T*, cudaStream_t);         \
   template cudaError_t launch_stage_tables<T>(const Geo<T>&, void*, cudaStream_t);                     \
-  template cudaError_t launch_stage<T>(const Geo<T>&, const FusedIO<T>&, const void*, cudaStream_t);   \
+  template cudaError_t launch_stage<T>(const Geo<T>&, const FusedIO<T>&, const void*, bool, cudaStream_t); \
   template cudaError_t launch_round<T>(const RoundArgs<T>&, TileCfg, int, cudaStream_t, int*);      \
   template cudaError_t launch_diag<T>(const Geo<T>&, const T*, const T*, const T*, const DiagOut<T>&, \
                                       cudaStream_t);

@@ -50,7 +50,7 @@ template <typename T>
 cudaError_t launch_phase_uv(const Geo<T>& g, const StageIO<T>& io, TileCfg cfg, cudaStream_t s, int full_tiles = -1);
 // The fused stage kernel (bt_fused.cuh), the tile shape of the phases around it (and of its own tiles, except
 // where fused_tile gives a wider one), and the tables of decoded work it reads (built once per plan, stream
-// ordered).
+// ordered).  alone: rounds of other plans are not expected beside this one (spread_smem).
 constexpr TileCfg kFusedTile{8, 16};
 TileCfg fused_tile(int n);
 template <typename T>
@@ -59,7 +59,7 @@ size_t stage_table_bytes(int n, size_t esize);
 template <typename T>
 cudaError_t launch_stage_tables(const Geo<T>& g, void* out, cudaStream_t s);
 template <typename T>
-cudaError_t launch_stage(const Geo<T>& g, const FusedIO<T>& p, const void* tables, cudaStream_t s);
+cudaError_t launch_stage(const Geo<T>& g, const FusedIO<T>& p, const void* tables, bool alone, cudaStream_t s);
 // Persistent cooperative launch of a whole round (phases of all substeps);
 // max_ctas > 0 caps the grid.  The grid size used is returned in *grid_out.
 template <typename T>
