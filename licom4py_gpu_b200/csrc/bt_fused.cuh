@@ -522,18 +522,8 @@ __global__ void __launch_bounds__(TileShape<TI, TJ>::kT, TI == 8 ? 3 : 2)
         hy[z] = lin2(T(1.0) - p.beta_prev, hy[z], p.beta_prev, B[(z - 3) * sj]);
       }
     }
-    // agrid.py:55-69, barotr_pure.py:57-60, 149-150
-    const T rdx = s_ec[8 * S::kT + tid], rdy = s_ec[9 * S::kT + tid];
-    const T pgu = T(-9.80) * (rdx * (mid6(hx + 1, 1) - mid6(hx, 1)));
-    const T pgv = T(-9.80) * (rdy * (mid6(hy + 1, 1) - mid6(hy, 1)));
-    T u, v;
-    if constexpr (kTerms<T> == 6) {
-      u = upc + (pgu + tm[0] + tm[1] + tm[2]) * p.dt_prev;
-      v = vpc + (pgv + tm[3] - tm[4] + tm[5]) * p.dt_prev;
-    } else {
-      u = upc + (pgu + tm[0]) * p.dt_prev;
-      v = vpc + (pgv + tm[1]) * p.dt_prev;
-    }
+    const T u = momentum<T, false>(upc, s_ec[8 * S::kT + tid], hx, tm, p.dt_prev);
+    const T v = momentum<T, true>(vpc, s_ec[9 * S::kT + tid], hy, tm, p.dt_prev);
     T G[4];
     ld_pair(s_ec + 2 * tid, G[0], G[1]);
     ld_pair(s_ec + 2 * (tid + S::kT), G[2], G[3]);

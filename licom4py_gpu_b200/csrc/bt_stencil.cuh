@@ -63,23 +63,30 @@ __device__ __forceinline__ T lin2(T a, T x, T b, T y) {
   else
     return a * x + b * y;
 }
+// a x + c, one rounding in float32: named for the same reason.
+template <typename T>
+__device__ __forceinline__ T mad(T a, T x, T c) {
+  if constexpr (sizeof(T) == 4)
+    return __fmaf_rn(a, x, c);
+  else
+    return a * x + c;
+}
 // Value at the + face of the centre point of p[0], p[s], .., p[4s] (poly.py:50-56)
 template <typename T>
 __device__ __forceinline__ T rplus(const T* p, int s) {
-  return lin2(T(BT_EM23), p[0], T(BT_EM13), p[s]) + T(BT_EP03) * p[2 * s] + T(BT_EP13) * p[3 * s] +
-         T(BT_EP23) * p[4 * s];
+  return mad(T(BT_EP23), p[4 * s],
+             mad(T(BT_EP13), p[3 * s], mad(T(BT_EP03), p[2 * s], lin2(T(BT_EM23), p[0], T(BT_EM13), p[s]))));
 }
 // Value at the - face of the centre point (poly.py:57-63)
 template <typename T>
 __device__ __forceinline__ T rminus(const T* p, int s) {
-  return lin2(T(BT_EP23), p[0], T(BT_EP13), p[s]) + T(BT_EP03) * p[2 * s] + T(BT_EM13) * p[3 * s] +
-         T(BT_EM23) * p[4 * s];
+  return mad(T(BT_EM23), p[4 * s],
+             mad(T(BT_EM13), p[3 * s], mad(T(BT_EP03), p[2 * s], lin2(T(BT_EP23), p[0], T(BT_EP13), p[s]))));
 }
 // 6-point centred face value between p[2s] and p[3s] (poly.py:120-124)
 template <typename T>
 __device__ __forceinline__ T mid6(const T* p, int s) {
-  return lin2(T(BT_M13), p[2 * s] + p[3 * s], T(BT_M23), p[s] + p[4 * s]) +
-         T(BT_M33) * (p[0] + p[5 * s]);
+  return mad(T(BT_M33), p[0] + p[5 * s], lin2(T(BT_M13), p[2 * s] + p[3 * s], T(BT_M23), p[s] + p[4 * s]));
 }
 // Gravity-wave speed with the 10 m/s floor (barotr_pure.py:21-26); NaN propagates like jnp.maximum.
 template <typename T>
@@ -282,6 +289,20 @@ struct TileShape {
 // -> 155).
 template <typename T>
 constexpr int kTerms = sizeof(T) == 8 ? 6 : 2;
+
+// New velocity component (Y: along j) of a cell: the base, and dt times the
+// pressure gradient (agrid.py:55-69, barotr_pure.py:57-60) of the 7 h values h
+// along its axis plus the cell's momentum terms (barotr_pure.py:149-150).
+template <typename T, bool Y>
+__device__ __forceinline__ T momentum(T base, T rd, const T* h, const T* tm, T dt) {
+  const T g = rd * (mid6(h + 1, 1) - mid6(h, 1));
+  if constexpr (kTerms<T> == 6) {
+    const T pg = T(-9.80) * g;
+    return base + (Y ? pg + tm[3] - tm[4] + tm[5] : pg + tm[0] + tm[1] + tm[2]) * dt;
+  } else {
+    return mad(mad(T(-9.80), g, tm[Y ? 1 : 0]), dt, base);
+  }
+}
 
 struct TileBox {
   int f, i0, j0, ni, nj;
@@ -825,12 +846,12 @@ __device__ __forceinline__ void face_h(const StageIO<T>& io, const T* ph, int sh
   const T he = rplus(hh, 1), hw = rminus(hh + 1, 1);
   T cc, coef;
   celerity_coef(mid6(hh, 1), dz, cc, coef);
-  const T vis = bc + coef * (he - hw);
+  const T vis = mad(coef, he - hw, bc);
   T fl = lin2(dz, vis, vis > T(0.0) ? he : hw, vis);
   if (io.last && side >= 0) {  // the neighbour's flux at the same edge face (barotr_pure.py:29-49)
     const T* nh = s_nh + 6 * slot;
     const T ndz = s_ndz[slot];
-    const T nvis = bc + nh[2] * (nh[0] - nh[1]);
+    const T nvis = mad(nh[2], nh[0] - nh[1], bc);
     fl = (fl + lin2(ndz, nvis, nvis > T(0.0) ? nh[0] : nh[1], nvis)) / T(2.0);
   }
   const T vt = bc > T(0.0) ? rplus(tt, 1) : rminus(tt + 1, 1);
@@ -1055,7 +1076,7 @@ __device__ __forceinline__ void tile_cells(const StageIO<T>& io, const TileBox& 
       const T* c = L.s_cell + e;
       const T rda = c[0], rdx = c[S::C], rdy = c[2 * S::C], af = c[3 * S::C];
       const T div = rda * (X[TJ] - X[0] + Y[1] - Y[0]);
-      const T hn = hpc[k] - div * io.dt;
+      const T hn = mad(-div, io.dt, hpc[k]);
       io.h_out[o0 + a * m + q] = hn;
       if (!FULL) for_bands(f, b.i0 + a, b.j0 + q, n, [&](int, int z) { io.band_hn[z] = hn; });
       const T uct = L.s_uc[(a + kHalo) * TJ + q], vct = L.s_vc[a * RJ + q + kHalo];
@@ -1068,9 +1089,9 @@ __device__ __forceinline__ void tile_cells(const StageIO<T>& io, const TileBox& 
       const T vort = rda * (ty[0] + tx[TJ] - ty[1] - tx[0]);
       const T advx = lin2(vort, vct, -(kx[TJ] - kx[0]), rdx);
       const T advy = lin2(-vort, uct, -(ky[1] - ky[0]), rdy);
-      const T visx = -(rdx * (vx[TJ] - vx[0]));
-      const T visy = -(rdy * (vy[1] - vy[0]));
       if constexpr (kTerms<T> == 6) {
+        const T visx = -(rdx * (vx[TJ] - vx[0]));
+        const T visy = -(rdy * (vy[1] - vy[0]));
         ta.at(0, a, q) = advx;
         ta.at(1, a, q) = af * vct;
         ta.at(2, a, q) = visx;
@@ -1078,8 +1099,8 @@ __device__ __forceinline__ void tile_cells(const StageIO<T>& io, const TileBox& 
         ta.at(4, a, q) = af * uct;
         ta.at(5, a, q) = visy;
       } else {
-        ta.at(0, a, q) = advx + af * vct + visx;
-        ta.at(1, a, q) = advy - af * uct + visy;
+        ta.at(0, a, q) = mad(-rdx, vx[TJ] - vx[0], mad(af, vct, advx));
+        ta.at(1, a, q) = mad(-rdy, vy[1] - vy[0], mad(-af, uct, advy));
       }
     }
   }
@@ -1319,17 +1340,9 @@ __device__ __forceinline__ void tile_uv_main_t(const Geo<T>& g, const StageIO<T>
         hx[z] = sm[(a + z) * RJ + q + kHalo];
         hy[z] = sm[(a + kHalo) * RJ + q + z];
       }
-      const T pgu = T(-9.80) * (pre.rdx[k] * (mid6(hx + 1, 1) - mid6(hx, 1)));
-      const T pgv = T(-9.80) * (pre.rdy[k] * (mid6(hy + 1, 1) - mid6(hy, 1)));
       const int o = o0 + a * m + q;
-      T u, v;
-      if constexpr (kTerms<T> == 6) {
-        u = upc[k] + (pgu + tm[k][0] + tm[k][1] + tm[k][2]) * io.dt;
-        v = vpc[k] + (pgv + tm[k][3] - tm[k][4] + tm[k][5]) * io.dt;
-      } else {
-        u = upc[k] + (pgu + tm[k][0]) * io.dt;
-        v = vpc[k] + (pgv + tm[k][1]) * io.dt;
-      }
+      const T u = momentum<T, false>(upc[k], pre.rdx[k], hx, tm[k], io.dt);
+      const T v = momentum<T, true>(vpc[k], pre.rdy[k], hy, tm[k], io.dt);
       io.u_out[o] = u;
       io.v_out[o] = v;
       if (!FULL && in_bands(b.i0 + a, b.j0 + q, n)) {
