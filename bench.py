@@ -40,15 +40,15 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 B_ALG_WORDS = 41  # algorithmic words per cell-update over both RK stages (compulsory reads + writes of phase H and UV)
-# Compulsory words per interior cell of each phase kernel, averaged over the two
-# RK2 stages (stage 1 / stage 2): distinct field reads + writes of the kernel's work.
-#   phase H : h, u, v, [h base], dzph_x, dzph_y, gct(4), sina, rda, c_dy, d_dx -> h     14 / 15
-#   phase UV: u, v, h, new h, [u, v base], gct(4), sina, rda, rdx, rdy, a_f, c_dy,
-#             d_dx, dzph_x, dzph_y -> u, v                                          18 / 20
-# These count the stage's arithmetic as two independent kernels would have to move it;
-# the phase kernels hand momentum terms over instead of recomputing from the state.
+# Compulsory words per interior cell of each phase kernel by bytes per word, averaged over
+# the two RK2 stages: distinct field reads + writes of the kernel, the momentum terms that
+# phase H hands to phase UV (6 words in float64, 2 in float32) among them.
+#   phase H : h, u, v, [h base], gct(4), sina, rda, rdx, rdy, a_f, c_dy, d_dx, dzph_x,
+#             dzph_y -> h, terms                                  16.5 + 1 + 6 / 2
+#   phase UV: new h, terms, u, v base, rdx, rdy -> u, v            5 + 6 / 2 + 2
 # stage (fused kernel: phase UV of a stage and phase H of the next): half of B_ALG_WORDS.
-KERNEL_WORDS = {"phase_h": 14.5, "phase_uv": 19.0, "stage": B_ALG_WORDS / 2}
+KERNEL_WORDS = {"phase_h": {8: 23.5, 4: 19.5}, "phase_uv": {8: 13.0, 4: 9.0}}
+STAGE_WORDS = B_ALG_WORDS / 2
 KERNEL_NAMES = {"phase_h": "k_phase_h", "phase_uv": "k_phase_uv"}
 METRIC = "barotropic cell-updates/s"
 UNIT = "cell-updates/s"
@@ -703,7 +703,7 @@ def run_ours(args, world, rank, local):
         dom = max(res, key=lambda k: res[k][0])
         ms, nl = res[dom]
         esz = 8 if dtype == torch.float64 else 4
-        alg = KERNEL_WORDS[dom] * esz * 6 * nn * nn
+        alg = KERNEL_WORDS[dom][esz] * esz * 6 * nn * nn
         achieved = alg / (ms / nl * 1e-3) / 1e9
         traffic = None
         tfile = os.path.join(ROOT, "profiles", f"{KERNEL_NAMES[dom]}_c{nn}_{'f64' if esz == 8 else 'f32'}.json")
@@ -741,7 +741,7 @@ def run_ours(args, world, rank, local):
     elif fused:
         # the headline step is a chain of stage kernels: its time over their number
         launch_us = 1e3 * ms_per_step / (2 * nbb)
-        alg = KERNEL_WORDS["stage"] * 8 * cells
+        alg = STAGE_WORDS * 8 * cells
         achieved = alg / (launch_us * 1e-6) / 1e9
         l2 = l2_copy_gbs(dev)
         traffic = None

@@ -48,15 +48,17 @@ def _store(key: str, cfg: dict) -> None:
 
 
 def heuristic(n: int, dtype: Optional[torch.dtype] = None) -> dict:
-    """Static choice from B200 measurements: CUDA graphs everywhere (at C48-C96
-    the graph with programmatic launch beat the tile-resident and persistent
-    rounds: C96 float64 13.2 us per substep against 28.1 and 29.4), small tiles for small grids.  With ``dtype`` the tile is the fastest
-    one of that type (us per substep): float64 8 x 16 up to C112 (18.8 against 20.7),
-    16 x 16 beyond (C117 20.0 against 23.1; C384 141 against 155 with 8 x 32, 155 with
-    16 x 32) except from C145 to C160, where its 600 tiles are just more than one wave
-    (8 x 32: C145 27.9 against 34.1, C152 26.4 against 28.7; C164 32.8 against 32.2);
-    float32 8 x 16 up to C112 (C112 13.8 against 15.4), 8 x 32 up to C164 (C144 16.9
-    against 20.3), 16 x 32 beyond (C168 22.1 against 22.6; C384 59.5 against 74.5)."""
+    """Static choice from B200 measurements: CUDA graphs everywhere (C96 float64
+    13.2 us per substep against 19.2 in the tile-resident round and 27.8 in the
+    persistent one), small tiles for small grids.  With ``dtype`` the tile is the
+    fastest one of that type (us per substep): float64 8 x 16 up to C112 (18.8
+    against 20.7), 16 x 16 beyond (C117 20.0 against 23.1; C384 141 against 155 with
+    8 x 32, 155 with 16 x 32) except from C145 to C160, where 16 x 16 makes 600 tiles
+    and one wave holds 592, four per SM (8 x 32: C145 27.9 against 34.1, C152 26.4
+    against 28.7; C164 32.8 against 32.2); float32 8 x 16 up to C112 (C112 13.8
+    against 15.4), 8 x 32 up to C164 (C144 16.9 against 20.3), 16 x 32 beyond (C168
+    22.1 against 22.6; C384 59.5 against 74.5).  Without ``dtype``: one shape for
+    both types."""
     if dtype == torch.float64:
         tile = [8, 16] if n <= 112 else [8, 32] if 144 < n <= 160 else [16, 16]
         return {"mode": "graph", "tile": tile, "source": "heuristic"}

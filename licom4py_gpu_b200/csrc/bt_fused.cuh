@@ -410,8 +410,8 @@ __global__ void __launch_bounds__(TileShape<TI, TJ>::kT) k_stage_tables(Geo<T> g
 // the evaluation and face chains: 5000-6600 cycles from the wait on at C48 of
 // float64), by issue slots and the shared-memory pipe with two 12 x 16 tiles per
 // SM, and there by the SMs that hold two edge tiles.  us per substep, two phase
-// kernels per stage / fused: C48 float64 12.1 / 8.2, float32 10.2 / 5.9; C96
-// float64 14.15 / 13.2, float32 10.8 / 8.2; C90 RK3 float32 18.0 / 14.3.
+// kernels per stage / fused: C48 float64 12.3 / 8.8, float32 9.3 / 6.0; C96
+// float64 14.2 / 13.2, float32 11.0 / 8.2; C90 RK3 float32 18.0 / 14.3.
 template <typename T, int TI, int TJ>
 __global__ void __launch_bounds__(TileShape<TI, TJ>::kT, TI == 8 ? 3 : 2)
     k_stage(Geo<T> g, FusedIO<T> p, Tiling t, const int4* rec, const T* weights) {

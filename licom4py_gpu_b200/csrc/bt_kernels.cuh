@@ -23,8 +23,9 @@
 namespace bt {
 
 constexpr int kThreads = 256;  // of the element-wise kernels
+// SMs of a B200, which the tile rules below (fused_tile, spread_smem, late launches) are measured on: they choose
+// between forms of equal results, also where a part of the GPU has fewer.
 constexpr int kSms = 148;
-
 
 // FP: the full-interior-tile path compiled in (multi-wave launches), else
 // every tile runs the edge path (one-wave launches: half the code to fetch).
@@ -200,8 +201,8 @@ Tiling make_even_tiling(TileCfg c, int n) {
 // Tile shape of the fused stage kernel: 8 x 16, and 12 x 16 (416 threads, two CTAs
 // per SM) where that makes three tiles per SM two: it evaluates 1.9 velocities per
 // cell against 2.1, and two tiles of 13 warps spread evenly.  us per substep, 8 x
-// 16 / 12 x 16: float64 C80 13.5 / 12.0, C96 14.25 /
-// 13.2; float32 C80 8.00 / 7.93, C96 8.31 / 8.17, C90 RK3 14.6 / 14.3.
+// 16 / 12 x 16: float64 C80 13.5 / 12.0, C96 14.25 / 13.2; float32 C80 8.00 / 7.93,
+// C96 8.31 / 8.17, C90 RK3 14.6 / 14.3.
 TileCfg fused_tile(int n) {
   const auto tiles = [n](TileCfg c) { return 6 * make_even_tiling(c, n).tiles_per_face(); };
   const TileCfg wide{12, 16};
