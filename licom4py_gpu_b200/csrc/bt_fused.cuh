@@ -522,8 +522,9 @@ __global__ void __launch_bounds__(TileShape<TI, TJ>::kT, TI == 8 ? 3 : 2)
         hy[z] = lin2(T(1.0) - p.beta_prev, hy[z], p.beta_prev, B[(z - 3) * sj]);
       }
     }
-    const T u = momentum<T, false>(upc, s_ec[8 * S::kT + tid], hx, tm, p.dt_prev);
-    const T v = momentum<T, true>(vpc, s_ec[9 * S::kT + tid], hy, tm, p.dt_prev);
+    const T gx = gradient(s_ec[8 * S::kT + tid], hx), gy = gradient(s_ec[9 * S::kT + tid], hy);
+    const T u = momentum<T, false>(upc, gx, tm, p.dt_prev);
+    const T v = momentum<T, true>(vpc, gy, tm, p.dt_prev);
     T G[4];
     ld_pair(s_ec + 2 * tid, G[0], G[1]);
     ld_pair(s_ec + 2 * (tid + S::kT), G[2], G[3]);

@@ -74,19 +74,24 @@ __device__ __forceinline__ T mad(T a, T x, T c) {
 // Value at the + face of the centre point of p[0], p[s], .., p[4s] (poly.py:50-56)
 template <typename T>
 __device__ __forceinline__ T rplus(const T* p, int s) {
-  return mad(T(BT_EP23), p[4 * s],
-             mad(T(BT_EP13), p[3 * s], mad(T(BT_EP03), p[2 * s], lin2(T(BT_EM23), p[0], T(BT_EM13), p[s]))));
+  T r = lin2(T(BT_EM23), p[0], T(BT_EM13), p[s]);
+  r = mad(T(BT_EP03), p[2 * s], r);
+  r = mad(T(BT_EP13), p[3 * s], r);
+  return mad(T(BT_EP23), p[4 * s], r);
 }
 // Value at the - face of the centre point (poly.py:57-63)
 template <typename T>
 __device__ __forceinline__ T rminus(const T* p, int s) {
-  return mad(T(BT_EM23), p[4 * s],
-             mad(T(BT_EM13), p[3 * s], mad(T(BT_EP03), p[2 * s], lin2(T(BT_EP23), p[0], T(BT_EP13), p[s]))));
+  T r = lin2(T(BT_EP23), p[0], T(BT_EP13), p[s]);
+  r = mad(T(BT_EP03), p[2 * s], r);
+  r = mad(T(BT_EM13), p[3 * s], r);
+  return mad(T(BT_EM23), p[4 * s], r);
 }
 // 6-point centred face value between p[2s] and p[3s] (poly.py:120-124)
 template <typename T>
 __device__ __forceinline__ T mid6(const T* p, int s) {
-  return mad(T(BT_M33), p[0] + p[5 * s], lin2(T(BT_M13), p[2 * s] + p[3 * s], T(BT_M23), p[s] + p[4 * s]));
+  const T r = lin2(T(BT_M13), p[2 * s] + p[3 * s], T(BT_M23), p[s] + p[4 * s]);
+  return mad(T(BT_M33), p[0] + p[5 * s], r);
 }
 // Gravity-wave speed with the 10 m/s floor (barotr_pure.py:21-26); NaN propagates like jnp.maximum.
 template <typename T>
@@ -290,17 +295,21 @@ struct TileShape {
 template <typename T>
 constexpr int kTerms = sizeof(T) == 8 ? 6 : 2;
 
+// Gradient of h along one axis at the centre of 7 values (agrid.py:55-69).
+template <typename T>
+__device__ __forceinline__ T gradient(T rd, const T* h) {
+  return rd * (mid6(h + 1, 1) - mid6(h, 1));
+}
 // New velocity component (Y: along j) of a cell: the base, and dt times the
-// pressure gradient (agrid.py:55-69, barotr_pure.py:57-60) of the 7 h values h
-// along its axis plus the cell's momentum terms (barotr_pure.py:149-150).
+// pressure gradient (barotr_pure.py:57-60) of its h gradient ``gr`` plus the
+// cell's momentum terms (barotr_pure.py:149-150).
 template <typename T, bool Y>
-__device__ __forceinline__ T momentum(T base, T rd, const T* h, const T* tm, T dt) {
-  const T g = rd * (mid6(h + 1, 1) - mid6(h, 1));
+__device__ __forceinline__ T momentum(T base, T gr, const T* tm, T dt) {
   if constexpr (kTerms<T> == 6) {
-    const T pg = T(-9.80) * g;
+    const T pg = T(-9.80) * gr;
     return base + (Y ? pg + tm[3] - tm[4] + tm[5] : pg + tm[0] + tm[1] + tm[2]) * dt;
   } else {
-    return mad(mad(T(-9.80), g, tm[Y ? 1 : 0]), dt, base);
+    return mad(mad(T(-9.80), gr, tm[Y ? 1 : 0]), dt, base);
   }
 }
 
@@ -1340,9 +1349,10 @@ __device__ __forceinline__ void tile_uv_main_t(const Geo<T>& g, const StageIO<T>
         hx[z] = sm[(a + z) * RJ + q + kHalo];
         hy[z] = sm[(a + kHalo) * RJ + q + z];
       }
+      const T gx = gradient(pre.rdx[k], hx), gy = gradient(pre.rdy[k], hy);
       const int o = o0 + a * m + q;
-      const T u = momentum<T, false>(upc[k], pre.rdx[k], hx, tm[k], io.dt);
-      const T v = momentum<T, true>(vpc[k], pre.rdy[k], hy, tm[k], io.dt);
+      const T u = momentum<T, false>(upc[k], gx, tm[k], io.dt);
+      const T v = momentum<T, true>(vpc[k], gy, tm[k], io.dt);
       io.u_out[o] = u;
       io.v_out[o] = v;
       if (!FULL && in_bands(b.i0 + a, b.j0 + q, n)) {
