@@ -57,11 +57,12 @@ struct Kahan {
 
 // Runs item(row offset of column 0, first column) for this warp's strips of W
 // columns: strip u is columns (u % strips) * W .. of interior row u / strips.
-template <int WARPS, int W, typename F>
+// CTAS: the cluster's size where it is known when compiled (0: gridDim.x).
+template <int CTAS, int WARPS, int W, typename F>
 __device__ __forceinline__ void for_strips(int n, F item) {
   const int m = n + 6;
   const unsigned strips = (n + W - 1) / W, total = 6u * n * strips;
-  for (unsigned u = blockIdx.x * WARPS + threadIdx.x / 32; u < total; u += gridDim.x * WARPS) {
+  for (unsigned u = blockIdx.x * WARPS + threadIdx.x / 32; u < total; u += (CTAS ? CTAS : gridDim.x) * WARPS) {
     const unsigned row = u / strips, f = row / n, i = row - f * n;
     item(cell(f, i + kHalo, kHalo, m), (int)((u - row * strips) * W + (threadIdx.x & 31)));
   }
@@ -77,7 +78,7 @@ __device__ __forceinline__ Kahan warp_sum(Kahan a) {
 }
 
 // Combines the warps' values (lane 0 of each) of all CTAs in a fixed order; thread 0 of CTA 0 gets the result.
-template <int WARPS, typename V, typename F>
+template <int CTAS, int WARPS, typename V, typename F>
 __device__ __forceinline__ V cluster_combine(V v, F join) {
   __shared__ V part[WARPS];
   cg::cluster_group cl = cg::this_cluster();
@@ -89,7 +90,7 @@ __device__ __forceinline__ V cluster_combine(V v, F join) {
   }
   cl.sync();
   if (blockIdx.x == 0 && threadIdx.x == 0)
-    for (int r = 1; r < (int)gridDim.x; ++r) join(v, *cl.map_shared_rank(&part[0], r));
+    for (int r = 1; r < (CTAS ? CTAS : (int)gridDim.x); ++r) join(v, *cl.map_shared_rank(&part[0], r));
   cl.sync();  // no CTA leaves while its shared memory is read
   return v;
 }
@@ -99,7 +100,7 @@ struct StatsPart {
   Kahan sum;
 };
 
-template <typename T>
+template <typename T, int CTAS>
 __global__ void __launch_bounds__(kStatThreads) k_stats(int n, const T* F, double* out) {
   // columns per lane and strip: 32 warps with 6 loads each in flight (C384 float64 22.9 -> 18.5 us, float32 24.4 ->
   // 18.6 against 16 warps with 8)
@@ -107,7 +108,7 @@ __global__ void __launch_bounds__(kStatThreads) k_stats(int n, const T* F, doubl
   constexpr int A = 4;     // sums per lane: independent chains
   StatsPart p{-INFINITY, INFINITY, {}};
   Kahan sum[A];
-  for_strips<kStatThreads / 32, 32 * K>(n, [&](long o, int j) {
+  for_strips<CTAS, kStatThreads / 32, 32 * K>(n, [&](long o, int j) {
     T v[K];
 #pragma unroll
     for (int k = 0; k < K; ++k)
@@ -128,7 +129,7 @@ __global__ void __launch_bounds__(kStatThreads) k_stats(int n, const T* F, doubl
 #pragma unroll
   for (int k = 0; k < A; ++k) p.sum.add(sum[k]);
   p.sum = warp_sum(p.sum);
-  p = cluster_combine<kStatThreads / 32>(p, [](StatsPart& a, const StatsPart& b) {
+  p = cluster_combine<CTAS, kStatThreads / 32>(p, [](StatsPart& a, const StatsPart& b) {
     a.mx = fmax(a.mx, b.mx);
     a.mn = fmin(a.mn, b.mn);
     a.sum.add(b.sum);
@@ -144,7 +145,7 @@ struct ConservationPart {
   Kahan mass, energy;
 };
 
-template <typename T>
+template <typename T, int CTAS>
 __global__ void __launch_bounds__(kConsThreads) k_conservation(int n, const T* H, const T* U, const T* V,
                                                             const T* rda, const T* c2l, double depth,
                                                             double* out) {
@@ -152,7 +153,7 @@ __global__ void __launch_bounds__(kConsThreads) k_conservation(int n, const T* H
   constexpr int K = 3;
   ConservationPart p, q[K];
   const bool vec = (reinterpret_cast<size_t>(c2l) & 15) == 0;  // 16-byte loads (C384 float64 52.3 -> 49.1 us)
-  for_strips<kConsThreads / 32, 32 * K>(n, [&](long o, int j) {
+  for_strips<CTAS, kConsThreads / 32, 32 * K>(n, [&](long o, int j) {
     T h[K], u[K], v[K], r[K], C[K][4];
 #pragma unroll
     for (int k = 0; k < K; ++k)
@@ -186,7 +187,7 @@ __global__ void __launch_bounds__(kConsThreads) k_conservation(int n, const T* H
   }
   p.mass = warp_sum(p.mass);
   p.energy = warp_sum(p.energy);
-  p = cluster_combine<kConsThreads / 32>(p, [](ConservationPart& a, const ConservationPart& b) {
+  p = cluster_combine<CTAS, kConsThreads / 32>(p, [](ConservationPart& a, const ConservationPart& b) {
     a.mass.add(b.mass);
     a.energy.add(b.energy);
   });
@@ -196,42 +197,48 @@ __global__ void __launch_bounds__(kConsThreads) k_conservation(int n, const T* H
   }
 }
 
-// Launch on ``ctas`` CTAs: one cluster, or without one for a single CTA.
+// The two builds of a reduction: for a cluster of kRedCtas and for any other size.
 template <typename... A>
-cudaError_t launch_on(int ctas, void (*kern)(A...), int threads, cudaStream_t s, A... args) {
+struct Builds {
+  void (*full)(A...);
+  void (*any)(A...);
+  auto of(int ctas) const { return ctas == kRedCtas ? full : any; }
+};
+
+cudaLaunchConfig_t cluster_config(int ctas, int threads, cudaLaunchAttribute* attr) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(ctas);
   cfg.blockDim = dim3(threads);
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = ctas;
-  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr->id = cudaLaunchAttributeClusterDimension;
+  attr->val.clusterDim.x = ctas;
+  attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = ctas > 1 ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kern, args...);
+  cfg.numAttrs = ctas > 1 ? 1 : 0;  // a single CTA needs no cluster
+  return cfg;
 }
 
-// The largest cluster of ``kern`` that the current device can hold: kRedCtas (more
-// than the portable 8: the kernel opts in), else half of that and so on, at last 1.
-template <typename K>
-int largest_cluster(K kern, int threads) {
-  for (int ctas = kRedCtas; ctas > 1; ctas /= 2) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(ctas);
-    cfg.blockDim = dim3(threads);
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = ctas;
-    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
+template <typename... A>
+cudaError_t launch_on(int ctas, const Builds<A...>& k, int threads, cudaStream_t s, A... args) {
+  cudaLaunchAttribute attr;
+  cudaLaunchConfig_t cfg = cluster_config(ctas, threads, &attr);
+  cfg.stream = s;
+  return cudaLaunchKernelEx(&cfg, k.of(ctas), args...);
+}
+
+// The largest cluster that the current device can hold: kRedCtas (more than the
+// portable 8: that build opts in), else half of that and so on, at last 1.
+template <typename... A>
+int largest_cluster(const Builds<A...>& k, int threads) {
+  const bool opted =
+      cudaFuncSetAttribute(k.full, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+  for (int ctas = opted ? kRedCtas : 8; ctas > 1; ctas /= 2) {
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t cfg = cluster_config(ctas, threads, &attr);
     int held = 0;
-    if ((ctas <= 8 || cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) &&
-        cudaOccupancyMaxActiveClusters(&held, kern, &cfg) == cudaSuccess && held > 0)
-      return ctas;
+    if (cudaOccupancyMaxActiveClusters(&held, k.of(ctas), &cfg) == cudaSuccess && held > 0) return ctas;
     cudaGetLastError();
   }
+  cudaGetLastError();
   return 1;
 }
 
@@ -240,40 +247,39 @@ int largest_cluster(K kern, int threads) {
 // was reset -- runs on one CTA.
 constexpr int kMaxDevices = 64;
 template <typename... A>
-cudaError_t launch_cluster(int ctas, void (*kern)(A...), int threads, std::atomic<int>* known, cudaStream_t s,
+cudaError_t launch_cluster(int ctas, const Builds<A...>& k, int threads, std::atomic<int>* known, cudaStream_t s,
                            A... args) {
-  if (ctas > 0) {
-    const int most = largest_cluster(kern, threads);
-    return ctas > most ? cudaErrorInvalidClusterSize : launch_on(ctas, kern, threads, s, args...);
-  }
+  if (ctas > 0)
+    return ctas > largest_cluster(k, threads) ? cudaErrorInvalidClusterSize
+                                              : launch_on<A...>(ctas, k, threads, s, args...);
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   const bool in_range = dev >= 0 && dev < kMaxDevices;
   ctas = in_range ? known[dev].load(std::memory_order_relaxed) : 0;
   if (ctas == 0) {
-    ctas = largest_cluster(kern, threads);
+    ctas = largest_cluster(k, threads);
     if (in_range) known[dev].store(ctas, std::memory_order_relaxed);
   }
-  e = launch_on(ctas, kern, threads, s, args...);
+  e = launch_on<A...>(ctas, k, threads, s, args...);
   if (e == cudaSuccess || ctas == 1) return e;
   cudaGetLastError();
-  return launch_on(1, kern, threads, s, args...);
+  return launch_on<A...>(1, k, threads, s, args...);
 }
 
 template <typename T>
 cudaError_t launch_stats(int ctas, int n, const void* f, void* out, cudaStream_t s) {
   static std::atomic<int> known[kMaxDevices];
-  return launch_cluster<int, const T*, double*>(ctas, k_stats<T>, kStatThreads, known, s, n, (const T*)f,
-                                                (double*)out);
+  return launch_cluster<int, const T*, double*>(ctas, {k_stats<T, kRedCtas>, k_stats<T, 0>}, kStatThreads, known, s, n,
+                                                (const T*)f, (double*)out);
 }
 template <typename T>
 cudaError_t launch_conservation(int ctas, int n, const void* h, const void* u, const void* v, const void* rda,
                                 const void* c2l, double depth, void* out, cudaStream_t s) {
   static std::atomic<int> known[kMaxDevices];
   return launch_cluster<int, const T*, const T*, const T*, const T*, const T*, double, double*>(
-      ctas, k_conservation<T>, kConsThreads, known, s, n, (const T*)h, (const T*)u, (const T*)v, (const T*)rda,
-      (const T*)c2l, depth, (double*)out);
+      ctas, {k_conservation<T, kRedCtas>, k_conservation<T, 0>}, kConsThreads, known, s, n, (const T*)h, (const T*)u,
+      (const T*)v, (const T*)rda, (const T*)c2l, depth, (double*)out);
 }
 
 int rfail(int code, const std::string& msg) { return set_error(code, msg); }
