@@ -179,7 +179,8 @@ int build_halo_host(int n, const T* coef, const int* li, const int* lj, int2* sr
 // tiles per SM (C96; us per substep of a graph round, fused / phases: C48 8.8 / 12.3, C72 10.1 / 13.3, C80 12.0 /
 // 14.6, C96 13.2 / 14.2), in RK3, whose blend doubles the h reads, up to 1.75 of the 12 x 16 tiles (C84; C72 16.8 /
 // 20.4, C80 20.2 / 22.5; C90 22.0 / 21.9, C96 22.0 / 21.7), float32 up to six (C128, 768 tiles; C48 6.0 / 9.3, C96
-// 8.2 / 11.0, C112 13.7 / 15.4, C128 15.0 / 18.2; RK3 C120 25.0 / 24.7, C128 25.1 / 27.2).
+// 8.2 / 11.0, C112 13.7 / 15.4, C128 15.0 / 18.2; RK3 C120 25.0 / 24.7, C128 25.1 / 27.2; above C112 only plans that
+// are given 8 x 16 tiles use it, other shapes being faster there).
 bool fused_size(int n, int dtype, int rk, int sms) {
   const TileCfg c = fused_tile(n);
   const Tiling t = make_even_tiling(c, n);
